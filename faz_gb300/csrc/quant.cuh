@@ -43,8 +43,31 @@ __device__ __forceinline__ int quantize(T &v, T pred, double eb, double recip, i
         return trim - 1;
     }
     T diff = orig - pred;
-    double x = (double)(diff < 0 ? -diff : diff) * recip;
     uval = orig;
+    if constexpr (sizeof(T) == 8) {
+        // The same steps for double data with the comparisons and signs on the
+        // integer pipe: GB300 issues a warp's double-precision instruction
+        // (compares and conversions included) over 16 cycles of one pipe, which
+        // bounds the float64 levels (finest level of 256x384x384 at rel 1e-6:
+        // 1.70 ms with 18 such instructions per point,
+        // 1.43 ms with these and the stencils' scaling off that pipe).
+        const int dh = __double2hiint(diff);
+        const double x = __hiloint2double(dh & 0x7fffffff, __double2loint(diff)) * recip;
+        // x >= 2 * radius (whose low word is zero), infinities and NaN
+        if ((unsigned)__double2hiint(x) >= (unsigned)__double2hiint((double)(2 * radius))) return 0;
+        const int qi = (int)x + 1;
+        if (qi >= 2 * radius) return 0;
+        const int half = qi >> 1;
+        const int code = dh < 0 ? radius - half : radius + half;
+        const double q = (double)(dh < 0 ? -(half << 1) : (half << 1)) * eb;  // +0 for half = 0, as the reference
+        const double dec = pred + q;
+        const double err = dec - orig;
+        const long long eabs = __double_as_longlong(err) & 0x7fffffffffffffffll;
+        if (eabs > __double_as_longlong(eb) || (trim == 2 && code == 1)) return 0;
+        v = dec;
+        return code;
+    }
+    double x = (double)(diff < 0 ? -diff : diff) * recip;
     if (!(x < 2147483647.0)) return 0;
     int qi = (int)x + 1;
     if (qi >= 2 * radius) return 0;
@@ -68,13 +91,8 @@ __device__ __forceinline__ int quantize(T &v, T pred, double eb, double recip, i
 // For float data the reference rounds through double: x = (double)|diff| *
 // (1/eb) truncated to int, and dec = (float)((double)pred + (double)q2 * eb).
 // GB300 runs double arithmetic at a small fraction of its float rate, so the
-// float path below computes both results from float-float products (eb and
-// 1/eb held as float pairs, Dekker products via fmaf) and proves each result
-// equal to the double computation: floor(x) only matters where it changes
-// (floor(x)+1)>>1, i.e. near odd integers, and the final float rounding only
-// where the exact value lies near a midpoint between floats.  Within 2^-20
-// (floor) or 2^-18 ulp (rounding) of such a boundary, on cancellation, at
-// powers of two, zero or non-finite values, the double computation is used.
+// float path computes both results in float and proves each equal to the
+// double computation (fastq.cuh); where it cannot, the double computation runs.
 
 // Double-precision fallbacks of the float path, kept out of line: inlined,
 // the compiler may evaluate them unconditionally (as selects), which on GB300's
@@ -210,29 +228,6 @@ __device__ __forceinline__ void cp_async(void *smem, const void *gmem) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// Straight-line reconstruction pred + q2*eb (dequant_f32 without early
-// exits); returns true when undecided.
-__device__ __forceinline__ bool dequant_f32_straight(float pred, int q2, float eh, float el, float &out) {
-    const float q = int_to_float_small(q2);
-    const float p1 = q * eh;
-    const float e1 = fmaf(q, eh, -p1);
-    const float p2 = q * el;
-    const float s = pred + p1;
-    const float bb = s - pred;
-    const float t = (pred - (s - bb)) + (p1 - bb);
-    const float lo = t + (e1 + p2);
-    const float r = s + lo;
-    const float res = (s - r) + lo;
-    const float ar = fabsf(r);
-    const uint32_t rb = f32_bits(ar);
-    const float bigv = fmaxf(fabsf(pred), fabsf(p1));
-    const float u = f32_from_bits(rb & 0x7f800000u) * 0x1p-23f;
-    const bool und = q2 != 0 && (!(ar >= 0x1p-100f) || ar * 256.0f < bigv || (rb & 0x7fffffu) == 0 ||
-                                 rb >= 0x7f000000u || fabsf(fabsf(res) - 0.5f * u) < u * 0x1p-12f);
-    out = q2 == 0 ? pred + 0.0f : r;
-    return und;
-}
-
 // One quantisation: QM 1 is the straight-line float path (trimToZero 0,
 // eb within the fast range) with the double computation for undecided
 // points; QM 0 is the general path.  v becomes the value the field takes,
@@ -266,7 +261,7 @@ __device__ __forceinline__ T recover_point(T pred, int code, uint64_t pos, const
                                            uint64_t nz, const T *unpred) {
     if constexpr (QM == 1 && sizeof(T) == 4) {
         float out;
-        const bool und = dequant_f32_straight(pred, 2 * (code - a.radius), a.eh, a.el, out);
+        const bool und = dequant_f32_bracket(pred, int_to_float_small(code - a.radius), 2.0f * a.eh, 2.0f * a.el, out);
         if (code == 0 || und) out = recover_dp_f32(pred, code, pos, a.eb, a.radius, 0, zpos, nz, unpred);
         if (a.verify) {
             float ref = recover<float>(pred, code, pos, a.eb, a.radius, 0, zpos, nz, unpred);

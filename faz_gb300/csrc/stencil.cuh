@@ -15,13 +15,13 @@ namespace faz {
 // (shared-memory offsets from the line origin) and the coefficients of the
 // reference's formula, folded so that one expression evaluates all of them
 // in the reference's operation order:
-//   y = ((k1*x1 + k2*x2) + k3*x3) + k4*x4 with 2, 3 or 4 terms, times scale.
+//   y = ((k1*x1 + k2*x2) + k3*x3) - x4 with 2, 3 or 4 terms, times scale.
 // k = +-1 multiplies are exact, so -a + 9b equals (-1)*a + 9*b bit for bit
 // and x - c equals x + (-1)*c.
 template <typename T>
 struct Stencil {
     int i1, i2, i3, i4;  // shared-memory offsets
-    T k1, k2, k3, k4, scale;
+    T k1, k2, k3, scale;
     int nt;              // 1 copy, 2..4 terms, 5 linear1 (double literals)
 };
 
@@ -29,7 +29,7 @@ template <typename T>
 __device__ __forceinline__ Stencil<T> make_stencil(int m, int n, int cubic, int st, int sh) {
     Stencil<T> S;
     int o1 = -1, o2 = 1, o3 = -1, o4 = -1;
-    S.k1 = 1; S.k2 = 1; S.k3 = 0; S.k4 = 0; S.scale = (T)0.5; S.nt = 2;
+    S.k1 = 1; S.k2 = 1; S.k3 = 0; S.scale = (T)0.5; S.nt = 2;
     if (!cubic || n < 5) {
         if (m + 1 >= n) {
             if (n < 4) { S.nt = 1; o1 = -1; o2 = -1; }
@@ -44,7 +44,7 @@ __device__ __forceinline__ Stencil<T> make_stencil(int m, int n, int cubic, int 
         } else if (m == n - 1) { // (3a - 10b + 15c) / 8
             o1 = -5; o2 = -3; o3 = -1; S.k1 = 3; S.k2 = -10; S.k3 = 15; S.nt = 3; S.scale = (T)0.125;
         } else {                 // (-a + 9b + 9c - d) / 16
-            o1 = -3; o2 = -1; o3 = 1; o4 = 3; S.k1 = -1; S.k2 = 9; S.k3 = 9; S.k4 = -1; S.nt = 4;
+            o1 = -3; o2 = -1; o3 = 1; o4 = 3; S.k1 = -1; S.k2 = 9; S.k3 = 9; S.nt = 4;
             S.scale = (T)0.0625;
         }
     }
@@ -56,18 +56,31 @@ __device__ __forceinline__ Stencil<T> make_stencil(int m, int n, int cubic, int 
 }
 
 
+// y * scale, scale a power of two between 1/16 and 1/2: exact for a normal
+// result, where double data takes it off the exponent (an integer add; the
+// double-precision pipe bounds the float64 levels)
+template <typename T>
+__device__ __forceinline__ T scale_pow2(T y, T scale) {
+    if constexpr (sizeof(T) == 8) {
+        const int hi = __double2hiint(y), ex = hi & 0x7ff00000;
+        const int dh = __double2hiint(scale) - 0x3ff00000;
+        if (ex + dh > 0 && ex != 0x7ff00000) return __hiloint2double(hi + dh, __double2loint(y));
+    }
+    return y * scale;
+}
+
 // CUB = 0: a linear level, whose stencils are copy, (a + b) / 2 or linear1
 template <int CUB, typename T>
 __device__ __forceinline__ T eval_stencil(const Stencil<T> &S, const T *p) {
     T x1 = p[S.i1], x2 = p[S.i2];
     if (S.nt == 5) return linear1_any(x1, x2);
-    if (!CUB) return S.nt == 1 ? x1 : (x1 + x2) * S.scale;
+    if (!CUB) return S.nt == 1 ? x1 : scale_pow2(x1 + x2, S.scale);
     T x3 = p[S.i3], x4 = p[S.i4];
     T s2 = S.k1 * x1 + S.k2 * x2;
     T s3 = s2 + S.k3 * x3;
-    T s4 = s3 + S.k4 * x4;
+    T s4 = s3 - x4;  // the only 4-term stencil ends in - d
     T y = S.nt == 4 ? s4 : (S.nt == 3 ? s3 : s2);
-    return S.nt == 1 ? x1 : y * S.scale;
+    return S.nt == 1 ? x1 : scale_pow2(y, S.scale);
 }
 
 // Line counter (outer, inner) of lines enumerated row-major with `inner`

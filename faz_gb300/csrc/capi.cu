@@ -460,7 +460,7 @@ void interp_encode(uint64_t n, int radius, uint16_t *codes, T *scratch, unsigned
     }
     const uint64_t nunpred = e.he.nzero;
     e.unpred = m.alloc<T>(nunpred ? nunpred : 1);
-    if (nunpred) launches(launch_compact_zeros<T>(codes, n, e.he.zc, e.he.zoff, nullptr, scratch, e.unpred, st));
+    if (nunpred) launches(launch_compact_zeros<T>(codes, n, e.he.zc, e.he.zoff, scratch, e.unpred, st));
 }
 
 // The payload of an encoded interpolation compression: the bytes
@@ -1405,84 +1405,119 @@ void parse_payload(const uint8_t *pl, size_t n, int N, Parsed &P) {
 
 }  // namespace
 
-// HuffmanEncoder::load + decode (HuffmanEncoder.hpp:236-296) on the device:
-// reads the tree and bit string at p (advancing it) and writes num codes.
+// HuffmanEncoder::load + decode (HuffmanEncoder.hpp:236-296) on the device.
+// begin() reads the tree and bit string at p (advancing it) and queues the
+// decode of num codes and the count of their zeros; the host waits for nothing,
+// so that the caller can queue what follows.  settle(), once the caller has
+// synchronised the stream, checks the outcome and returns true when the unit
+// starts needed further passes: the codes were decoded again then, and the
+// caller queues its own work again.
 template <typename C>
-void huffman_decode_impl(const uint8_t *&p, const uint8_t *end, uint64_t num, C *codes, DevMem &m, cudaStream_t st,
-                         Counter &launches) {
-    DecodeTablesHost t;
-    std::string err;
-    int rc = parse_tree(p, end, t, err);
-    if (rc) throw Fail{rc, err};
-    if ((size_t)(end - p) < 8) throw Fail{FAZ_ERR_FORMAT, "truncated stream header"};
-    uint64_t nbytes;
-    std::memcpy(&nbytes, p, 8);
-    p += 8;
-    if ((size_t)(end - p) < nbytes) throw Fail{FAZ_ERR_FORMAT, "truncated Huffman bits"};
-    const uint8_t *hbits = p;
-    p += nbytes;
-    if (t.constant || nbytes == 0) {
-        int v = t.constant_state + t.offset;
-        if (v < 0 || (sizeof(C) == 2 && v > 65535)) throw Fail{FAZ_ERR_FORMAT, "Huffman symbol out of range"};
-        launches(launch_fill_u16(codes, num, (C)v, st));
-        return;
-    }
-    const uint64_t nwords = (nbytes + 3) / 4;
-    uint32_t *dbits = m.alloc<uint32_t>(nwords + 16);
-    CK(cudaMemsetAsync(dbits, 0, (nwords + 16) * 4, st));
-    uint32_t *lut = m.alloc<uint32_t>(t.lut.size());
-    uint32_t *dl = m.alloc<uint32_t>(t.nodeCount), *dr = m.alloc<uint32_t>(t.nodeCount);
-    int32_t *ds = m.alloc<int32_t>(t.nodeCount);
-    uint8_t *dleaf = m.alloc<uint8_t>(t.nodeCount);
-    CK(cudaMemcpyAsync(lut, t.lut.data(), t.lut.size() * 4, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(dl, t.left.data(), t.nodeCount * 4, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(dr, t.right.data(), t.nodeCount * 4, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(ds, t.sym.data(), t.nodeCount * 4, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(dleaf, t.leaf.data(), t.nodeCount, cudaMemcpyHostToDevice, st));
-    DecodeTablesDev td{lut, dl, dr, ds, dleaf};
-    const uint64_t nbits = nbytes * 8;
-    const uint64_t nunits = decode_units(nbits);
-    uint64_t *start = m.alloc<uint64_t>(nunits);
-    uint64_t *ea = m.alloc<uint64_t>(nunits), *eb2 = m.alloc<uint64_t>(nunits);
-    unsigned int *cnt = m.alloc<unsigned int>(nunits);
-    uint16_t *bnd = m.alloc<uint16_t>(nunits * decode_boundaries());
-    unsigned long long *cnt64 = m.alloc<unsigned long long>(nunits + 1);
-    unsigned long long *off = m.alloc<unsigned long long>(nunits + 1);
-    unsigned long long *dtmp = m.alloc<unsigned long long>(scan_temp_words(nunits) + 1);
-    int *flags = m.alloc<int>(2);  // [0] changed, [1] damaged tree
-    CK(cudaMemsetAsync(flags, 0, 8, st));
-    launches(launch_init_starts(start, nunits, st));
-    // The bit string comes over in slices on a copy stream while the
-    // speculative decode of the slices already in runs (a unit reads up to 8
-    // words past its CTA's units: each slice's copy carries the next slice's
-    // first 128 bytes).
-    {
-        const uint64_t cta = decode_cta_units();
-        const uint64_t unit_bytes = decode_unit_bits() / 8;
-        // four slices of a bit string of 16 MB or more: each decode launch
-        // still fills the GPU, three quarters of the copy overlap decoding
-        const uint64_t nslices0 = nbytes >= (16u << 20) ? 4 : 1;
-        const uint64_t slice_units = ((nunits + nslices0 - 1) / nslices0 + cta - 1) / cta * cta;
-        const uint64_t nslices = (nunits + slice_units - 1) / slice_units;
+struct HuffDecode {
+    uint64_t num = 0;
+    C *codes = nullptr;
+    uint64_t nranges = 0;              // ranges of the codes with
+    unsigned long long *zc = nullptr;  // their zero counts and
+    unsigned long long *zstart = nullptr;  // first codes
+    struct Status {
+        int changed, damaged;
+        uint64_t total;
+    };
+
+    // zeros: the codes are expected to begin with that many zeros (anchors)
+    void begin(const uint8_t *&p, const uint8_t *end, uint64_t n, C *out, DevMem &m, cudaStream_t st,
+               Counter &launches, uint64_t zeros = 0) {
+        num = n;
+        codes = out;
+        DecodeTablesHost t;
+        std::string err;
+        int rc = parse_tree(p, end, t, err);
+        if (rc) throw Fail{rc, err};
+        if ((size_t)(end - p) < 8) throw Fail{FAZ_ERR_FORMAT, "truncated stream header"};
+        uint64_t nbytes;
+        std::memcpy(&nbytes, p, 8);
+        p += 8;
+        if ((size_t)(end - p) < nbytes) throw Fail{FAZ_ERR_FORMAT, "truncated Huffman bits"};
+        const uint8_t *hbits = p;
+        p += nbytes;
+        if (t.constant || nbytes == 0) {
+            int v = t.constant_state + t.offset;
+            if (v < 0 || (sizeof(C) == 2 && v > 65535)) throw Fail{FAZ_ERR_FORMAT, "Huffman symbol out of range"};
+            launches(launch_fill_u16(codes, num, (C)v, st));
+            nranges = constant_ranges(num);
+            zc = m.alloc<unsigned long long>(2 * nranges);
+            zstart = zc + nranges;
+            launches(launch_constant_ranges(num, v == 0, zstart, zc, st));
+            return;
+        }
+        offset = t.offset;
+        d.run_len = zeros ? leaf_depth(t, -t.offset) : 0;
+        d.run_bits = zeros * d.run_len;
+        d.nwords = (nbytes + 3) / 4;
+        d.nbits = nbytes * 8;
+        d.unit_words = decode_unit_words(d.nbits);
+        const uint64_t unit_bits = 32ull * d.unit_words, cta = decode_cta_units();
+        d.nunits = (d.nbits + unit_bits - 1) / unit_bits;
+        ncta = (d.nunits + cta - 1) / cta;
+        nranges = decode_ranges(d.nunits);
+        // one allocation: bit string, unit records, CTA ends and totals, tables
+        auto up = [](uint64_t b) { return (b + 255) & ~(uint64_t)255; };
+        const size_t lut2n = decode_lut2_entries(t.nodeCount);
+        const uint64_t b_bits = up(4 * d.nwords + 64), b_info = up(4 * d.nunits), b_end = up(4 * ncta),
+                       b_tot = up(8 * (ncta + 1)), b_child = up(4 * t.child.size()), b_lut = up(8ull << kLutBits),
+                       b_lut2 = up(4 * lut2n), b_len2 = up(lut2n), b_rng = up(8 * nranges);
+        uint8_t *w = m.alloc<uint8_t>(b_bits + b_info + 2 * b_end + b_tot + b_child + 3 * b_lut + b_lut2 + b_len2 +
+                                         2 * b_rng + 256);
+        uint32_t *bits = (uint32_t *)w;
+        info = (uint32_t *)(w += b_bits);
+        cend[0] = (uint32_t *)(w += b_info);
+        cend[1] = (uint32_t *)(w += b_end);
+        ctot = (unsigned long long *)(w += b_end);
+        uint32_t *child = (uint32_t *)(w += b_tot);
+        td.child = child;
+        td.lutB = (uint2 *)(w += b_child);
+        td.lutA = (uint16_t *)(w += b_lut);
+        uint32_t *slot_node = (uint32_t *)(w += b_lut);
+        td.lut2 = (uint32_t *)(w += b_lut);
+        td.len2 = w += b_lut2;
+        zc = (unsigned long long *)(w += b_len2);
+        zstart = (unsigned long long *)(w += b_rng);
+        flags = (int *)(w += b_rng);
+        d.w32 = bits;
+        TableStage &ts = t_table_stage;
+        uint8_t *stage = ts.acquire(4 * t.child.size());
+        std::memcpy(stage, t.child.data(), 4 * t.child.size());
+        CK(cudaMemcpyAsync(child, stage, 4 * t.child.size(), cudaMemcpyHostToDevice, st));
+        ts.release(st);
+        CK(cudaMemsetAsync(flags, 0, 8, st));
+        CK(cudaMemsetAsync((uint8_t *)bits + (4 * d.nwords - 4), 0, 68, st));  // past the last byte
+        launches(launch_decode_tables<C>(td, offset, slot_node, (unsigned *)(flags + 2), lut2n, st));
+        // The bit string comes over in slices on a copy stream while the slices
+        // already in are synchronised (a unit reads up to 8 words past its CTA's
+        // units: each slice's copy carries the next slice's first 128 bytes).
+        const uint64_t nslices0 = nbytes >= (16u << 20) ? 8 : 1;
+        const uint64_t slice_ctas = (ncta + nslices0 - 1) / nslices0;
+        const uint64_t nslices = (ncta + slice_ctas - 1) / slice_ctas;
         if (nslices <= 1) {
-            CK(cudaMemcpyAsync(dbits, hbits, nbytes, cudaMemcpyHostToDevice, st));
-            launches(launch_decode_spec(td, dbits, nwords, nbits, nunits, 0, nunits, ea, cnt, bnd, flags + 1, st));
+            CK(cudaMemcpyAsync(bits, hbits, nbytes, cudaMemcpyHostToDevice, st));
+            launches(launch_decode_sync(td, d, 0, ncta, info, cend[0], ctot, flags, st));
         } else {
             StreamGuard cs(nullptr);
             Events ready;
-            CK(cudaEventRecord(ready.a, st));  // dbits cleared
+            CK(cudaEventRecord(ready.a, st));  // the string's tail cleared
             CK(cudaStreamWaitEvent(cs.st, ready.a, 0));
             std::vector<cudaEvent_t> done(nslices, nullptr);
+            const uint64_t slice_bytes = slice_ctas * cta * unit_bits / 8;
             try {
                 for (uint64_t k = 0; k < nslices; k++) {
                     CK(cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming));
-                    const uint64_t b0 = k * slice_units * unit_bytes;
-                    const uint64_t b1 = std::min<uint64_t>(nbytes, (k + 1) * slice_units * unit_bytes + 128);
-                    CK(cudaMemcpyAsync((uint8_t *)dbits + b0, hbits + b0, b1 - b0, cudaMemcpyHostToDevice, cs.st));
+                    const uint64_t b0 = k * slice_bytes;
+                    const uint64_t b1 = std::min<uint64_t>(nbytes, (k + 1) * slice_bytes + 128);
+                    CK(cudaMemcpyAsync((uint8_t *)bits + b0, hbits + b0, b1 - b0, cudaMemcpyHostToDevice, cs.st));
                     CK(cudaEventRecord(done[k], cs.st));
                     CK(cudaStreamWaitEvent(st, done[k], 0));
-                    launches(launch_decode_spec(td, dbits, nwords, nbits, nunits, k * slice_units,
-                                                (k + 1) * slice_units, ea, cnt, bnd, flags + 1, st));
+                    launches(launch_decode_sync(td, d, k * slice_ctas, std::min(ncta, (k + 1) * slice_ctas), info,
+                                                cend[0], ctot, flags, st));
                 }
             } catch (...) {
                 cudaStreamSynchronize(cs.st);
@@ -1490,35 +1525,71 @@ void huffman_decode_impl(const uint8_t *&p, const uint8_t *end, uint64_t num, C 
                     if (e) cudaEventDestroy(e);
                 throw;
             }
-            // the copy stream's work is ordered before st's next launch; the
-            // events go once it has finished
-            CK(cudaStreamSynchronize(cs.st));
+            // the copies are ordered before st's next launch; what destroys the
+            // stream and the events here releases them once they have completed
             for (cudaEvent_t e : done) cudaEventDestroy(e);
         }
+        link(st, launches);
+        write(m, st, launches);
     }
-    int *hflag = (int *)t_pin_small.get(64);
-    bool converged = false;
-    for (int it = 0; it < 1024; it++) {
-        CK(cudaMemsetAsync(flags, 0, 4, st));
-        launches(launch_decode_resync(td, dbits, nwords, nbits, nunits, ea, eb2, cnt, bnd, start, flags, st));
-        CK(cudaMemcpyAsync(hflag, flags, 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        std::swap(ea, eb2);
-        if (hflag[0] < 0 || hflag[1]) throw Fail{FAZ_ERR_FORMAT, "Huffman stream decodes outside the tree"};
-        if (hflag[0] == 0) {
-            converged = true;
-            break;
+
+    bool settle(DevMem &m, cudaStream_t st, Counter &launches) {
+        if (!status) return false;
+        Status s = *status;
+        // a CTA's end moved in the last pass: the next CTA restarts there
+        bool redone = false;
+        for (int it = 0; s.changed && !s.damaged && it < 1024; it++) {
+            CK(cudaMemsetAsync(flags, 0, 4, st));
+            link(st, launches);
+            CK(cudaMemcpyAsync(status, flags, 8, cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+            s = *status;
+            redone = true;
         }
+        if (s.damaged) throw Fail{FAZ_ERR_FORMAT, "Huffman stream decodes outside the tree"};
+        if (s.changed) throw Fail{FAZ_ERR_UNSUPPORTED, "Huffman stream did not synchronise within 1024 passes"};
+        if (redone) {
+            write(m, st, launches);
+            CK(cudaStreamSynchronize(st));
+            s = *status;
+        }
+        if (s.total < num) throw Fail{FAZ_ERR_FORMAT, "Huffman stream holds fewer symbols than the field"};
+        return redone;
     }
-    if (!converged) throw Fail{FAZ_ERR_UNSUPPORTED, "Huffman stream did not synchronise within 1024 passes"};
-    launches(launch_widen_counts(cnt, cnt64, nunits, st));
-    launches(launch_scan_u64(cnt64, off, nunits, dtmp, st));
-    uint64_t total;
-    CK(cudaMemcpyAsync(hflag, off + nunits, 8, cudaMemcpyDeviceToHost, st));
+
+  private:
+    DecodeTablesDev td{};
+    DecodeString d{};
+    uint64_t ncta = 0;
+    int offset = 0;
+    uint32_t *info = nullptr, *cend[2] = {nullptr, nullptr};
+    unsigned long long *ctot = nullptr, *coff = nullptr;
+    int *flags = nullptr;  // changed, damaged, second-table slots
+    Status *status = nullptr;
+
+    void link(cudaStream_t st, Counter &launches) {
+        launches(launch_decode_link(td, d, cend[0], cend[1], info, ctot, flags, st));
+        std::swap(cend[0], cend[1]);
+    }
+    // offsets of the CTAs' codes, the codes, and the outcome to the host
+    void write(DevMem &m, cudaStream_t st, Counter &launches) {
+        if (!coff) coff = m.alloc<unsigned long long>(ncta + 1);
+        CK(cudaMemcpyAsync(coff, ctot, ncta * 8, cudaMemcpyDeviceToDevice, st));
+        launches(launch_scan_small(coff, ncta, st));
+        launches(launch_decode_write(td, d, info, coff, num, offset, codes, zc, zstart, st));
+        if (!status) status = (Status *)t_pin_decode.get(sizeof(Status));
+        CK(cudaMemcpyAsync(status, flags, 8, cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(&status->total, coff + ncta, 8, cudaMemcpyDeviceToHost, st));
+    }
+};
+
+template <typename C>
+void huffman_decode_impl(const uint8_t *&p, const uint8_t *end, uint64_t num, C *codes, DevMem &m, cudaStream_t st,
+                         Counter &launches) {
+    HuffDecode<C> h;
+    h.begin(p, end, num, codes, m, st, launches);
     CK(cudaStreamSynchronize(st));
-    std::memcpy(&total, hflag, 8);
-    if (total < num) throw Fail{FAZ_ERR_FORMAT, "Huffman stream holds fewer symbols than the field"};
-    launches(launch_decode_write(td, dbits, nwords, nbits, nunits, start, off, num, t.offset, codes, st));
+    h.settle(m, st, launches);
 }
 
 void huffman_decode_device(const uint8_t *&p, const uint8_t *end, uint64_t num, uint16_t *codes, DevMem &m,
@@ -1530,32 +1601,44 @@ void huffman_decode_device(const uint8_t *&p, const uint8_t *end, uint64_t num, 
     huffman_decode_impl(p, end, num, codes, m, st, launches);
 }
 
-// Sorted positions of the zero codes (the unpredictable points); returns
-// their count.
+// Sorted positions of the zero codes (the unpredictable points): queues the
+// compaction of the first `expect` of them into zpos and the copy of their
+// count to the returned pinned word, to be read once st is synchronised.
 template <typename C>
-uint64_t zero_positions_impl(const C *codes, uint64_t num, DevMem &m, cudaStream_t st, Counter &launches,
-                             uint64_t *&zpos) {
-    const uint64_t nsub = hist_subchunks(num);
-    unsigned long long *zc = m.alloc<unsigned long long>(nsub + 1);
-    unsigned long long *zoff = m.alloc<unsigned long long>(nsub + 1);
-    unsigned long long *ztmp = m.alloc<unsigned long long>(scan_temp_words(nsub) + 1);
-    launches(launch_count_zeros(codes, num, zc, st));
-    launches(launch_scan_u64(zc, zoff, nsub, ztmp, st));
+const uint64_t *queue_zero_positions(const HuffDecode<C> &h, uint64_t expect, DevMem &m, cudaStream_t st,
+                                     Counter &launches, uint64_t *&zpos) {
+    unsigned long long *zoff = m.alloc<unsigned long long>(h.nranges + 1 + scan_temp_words(h.nranges) + 1);
+    launches(launch_scan_u64(h.zc, zoff, h.nranges, zoff + h.nranges + 1, st));
     uint64_t *hz = (uint64_t *)t_pin_small.get(64);
-    CK(cudaMemcpyAsync(hz, zoff + nsub, 8, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(hz, zoff + h.nranges, 8, cudaMemcpyDeviceToHost, st));
+    zpos = m.alloc<uint64_t>(expect ? expect : 1);
+    if (expect)
+        launches(launch_zero_positions(h.codes, h.num, h.nranges, h.zstart, h.zc, zoff, expect, zpos, st));
+    return hz;
+}
+
+// Decode and compaction with one wait: the codes of an unpredictable-value
+// section of nunpred values.
+template <typename C>
+void decode_with_zeros_impl(const uint8_t *&p, const uint8_t *end, uint64_t num, uint64_t nunpred, C *codes, DevMem &m,
+                            cudaStream_t st, Counter &launches, uint64_t *&zpos) {
+    HuffDecode<C> h;
+    h.begin(p, end, num, codes, m, st, launches);
+    const uint64_t *hz = queue_zero_positions(h, nunpred, m, st, launches, zpos);
     CK(cudaStreamSynchronize(st));
-    const uint64_t nz = *hz;
-    zpos = m.alloc<uint64_t>(nz ? nz : 1);
-    if (nz) launches(launch_compact_zeros<float>(codes, num, zc, zoff, zpos, nullptr, nullptr, st));
-    return nz;
+    if (h.settle(m, st, launches)) {
+        hz = queue_zero_positions(h, nunpred, m, st, launches, zpos);
+        CK(cudaStreamSynchronize(st));
+    }
+    if (*hz != nunpred) throw Fail{FAZ_ERR_FORMAT, "unpredictable count does not match the zero codes"};
 }
-uint64_t zero_positions(const uint16_t *codes, uint64_t num, DevMem &m, cudaStream_t st, Counter &launches,
-                        uint64_t *&zpos) {
-    return zero_positions_impl(codes, num, m, st, launches, zpos);
+void decode_with_zeros(const uint8_t *&p, const uint8_t *end, uint64_t num, uint64_t nunpred, uint16_t *codes,
+                       DevMem &m, cudaStream_t st, Counter &launches, uint64_t *&zpos) {
+    decode_with_zeros_impl(p, end, num, nunpred, codes, m, st, launches, zpos);
 }
-uint64_t zero_positions(const uint32_t *codes, uint64_t num, DevMem &m, cudaStream_t st, Counter &launches,
-                        uint64_t *&zpos) {
-    return zero_positions_impl(codes, num, m, st, launches, zpos);
+void decode_with_zeros(const uint8_t *&p, const uint8_t *end, uint64_t num, uint64_t nunpred, uint32_t *codes,
+                       DevMem &m, cudaStream_t st, Counter &launches, uint64_t *&zpos) {
+    decode_with_zeros_impl(p, end, num, nunpred, codes, m, st, launches, zpos);
 }
 
 namespace {
@@ -1581,10 +1664,9 @@ void decompress_device(const uint8_t *pl, size_t n, Parsed &P, T *dOut, cudaStre
         if (P.nunpred) CK(cudaMemcpyAsync(dunpred, P.unpred, P.nunpred * sizeof(T), cudaMemcpyHostToDevice, st));
         Events ev_dec, ev_pred;
         CK(cudaEventRecord(ev_dec.a, st));
-        huffman_decode_device(p, end, num, codes, m, st, launches);
         uint64_t *zpos = nullptr;
-        const uint64_t nz = zero_positions(codes, num, m, st, launches, zpos);
-        if (nz != P.nunpred) throw Fail{FAZ_ERR_FORMAT, "unpredictable count does not match the zero codes"};
+        const uint64_t nz = P.nunpred;
+        decode_with_zeros(p, end, num, nz, codes, m, st, launches, zpos);
         CK(cudaEventRecord(ev_dec.b, st));
         CK(cudaEventRecord(ev_pred.a, st));
         static const std::vector<uint8_t> none;
@@ -1608,10 +1690,9 @@ void decompress_device(const uint8_t *pl, size_t n, Parsed &P, T *dOut, cudaStre
         if (P.nunpred) CK(cudaMemcpyAsync(dunpred, P.unpred, P.nunpred * sizeof(T), cudaMemcpyHostToDevice, st));
         Events ev_dec, ev_pred;
         CK(cudaEventRecord(ev_dec.a, st));
-        huffman_decode_device(p, end, num, codes, m, st, launches);
         uint64_t *zpos = nullptr;
-        const uint64_t nz = zero_positions(codes, num, m, st, launches, zpos);
-        if (nz != P.nunpred) throw Fail{FAZ_ERR_FORMAT, "unpredictable count does not match the zero codes"};
+        const uint64_t nz = P.nunpred;
+        decode_with_zeros(p, end, num, nz, codes, m, st, launches, zpos);
         CK(cudaEventRecord(ev_dec.b, st));
         unsigned long long *vcount = nullptr;
         if (verify_fast_path()) {
@@ -1635,27 +1716,15 @@ void decompress_device(const uint8_t *pl, size_t n, Parsed &P, T *dOut, cudaStre
     Plan pl_ = make_plan<T>(P.N, P.dims, P.maxStep, (int)P.blocksize, P.fixbs, P.interp, P.dir, P.il, P.dl, P.eb, P.alpha,
                             P.beta, P.radius, P.trim, smem_limit());
     const uint64_t num = pl_.num;
+    // every anchor is an unpredictable value
+    if (pl_.anchor && P.nunpred < pl_.nanchor)
+        throw Fail{FAZ_ERR_FORMAT, "unpredictable count does not match the zero codes"};
     DevMem m(st);
     uint16_t *codes = m.alloc<uint16_t>(num);
     T *dunpred = m.alloc<T>(P.nunpred ? P.nunpred : 1);
     if (P.nunpred) CK(cudaMemcpyAsync(dunpred, P.unpred, P.nunpred * sizeof(T), cudaMemcpyHostToDevice, st));
     Events ev_dec, ev_pred, ev_fin;
     CK(cudaEventRecord(ev_dec.a, st));
-    huffman_decode_device(p, end, num, codes, m, st, launches);
-    CK(cudaEventRecord(ev_dec.b, st));
-    // zero positions for the unpredictable values
-    uint64_t *zpos = nullptr;
-    const uint64_t nz = zero_positions(codes, num, m, st, launches, zpos);
-    if (nz != P.nunpred)
-        throw Fail{FAZ_ERR_FORMAT, "unpredictable count does not match the zero codes"};
-    if (!pl_.anchor) {
-        launches(launch_first_point<T>(true, nullptr, dOut, codes, nullptr, P.eb, P.radius, P.trim, zpos, nz, dunpred, st));
-    } else {
-        int64_t step[3] = {1, 1, 1};
-        int e = 3 - pl_.N;
-        for (int i = 0; i < pl_.N; i++) step[e + i] = (int64_t)pl_.maxStep;
-        launches(launch_anchors<T>(true, nullptr, dOut, codes, nullptr, dunpred, pl_.na, step, pl_.offs3, st));
-    }
     uint64_t *boff = m.alloc<uint64_t>(pl_.block_off.size());
     CK(cudaMemcpyAsync(boff, pl_.block_off.data(), pl_.block_off.size() * 8, cudaMemcpyHostToDevice, st));
     int *kerr = m.alloc<int>(1);
@@ -1665,24 +1734,52 @@ void decompress_device(const uint8_t *pl, size_t n, Parsed &P, T *dOut, cudaStre
         vcount = m.alloc<unsigned long long>(1);
         CK(cudaMemsetAsync(vcount, 0, 8, st));
     }
-    CK(cudaEventRecord(ev_pred.a, st));
-    for (size_t li = 0; li < pl_.lv.size(); li++) {
-        const LevelPlan &L = pl_.lv[li];
-        LevelArgs a = L.args;
-        a.block_off = boff + L.off_index;
-        a.ncodes = num;
-        a.err = kerr;
-        a.verify = vcount;
-        if (li + 1 == pl_.lv.size()) CK(cudaEventRecord(ev_fin.a, st));
-        int nl = 0;
-        CK(launch_level<T>(a, L.nblocks, true, nullptr, dOut, codes, nullptr, zpos, nz, dunpred, st, &nl));
-        launches.n += nl;
+    HuffDecode<uint16_t> h;
+    h.begin(p, end, num, codes, m, st, launches, pl_.anchor ? pl_.nanchor : 0);
+    CK(cudaEventRecord(ev_dec.b, st));
+    // Everything after the decode is queued before its outcome is known: a
+    // damaged stream leaves codes without meaning, which the kernels below take
+    // as any others (positions and unpredictable reads are bounded), and the
+    // call fails below.
+    const uint64_t nz = P.nunpred;
+    const uint64_t *hz = nullptr;
+    int *hk = (int *)t_pin_flag.get(64);
+    auto reconstruct = [&] {
+        uint64_t *zpos = nullptr;
+        hz = queue_zero_positions(h, nz, m, st, launches, zpos);
+        if (!pl_.anchor) {
+            launches(launch_first_point<T>(true, nullptr, dOut, codes, nullptr, P.eb, P.radius, P.trim, zpos, nz,
+                                           dunpred, st));
+        } else {
+            int64_t step[3] = {1, 1, 1};
+            int e = 3 - pl_.N;
+            for (int i = 0; i < pl_.N; i++) step[e + i] = (int64_t)pl_.maxStep;
+            launches(launch_anchors<T>(true, nullptr, dOut, codes, nullptr, dunpred, pl_.na, step, pl_.offs3, st));
+        }
+        CK(cudaEventRecord(ev_pred.a, st));
+        for (size_t li = 0; li < pl_.lv.size(); li++) {
+            const LevelPlan &L = pl_.lv[li];
+            LevelArgs a = L.args;
+            a.block_off = boff + L.off_index;
+            a.ncodes = num;
+            a.err = kerr;
+            a.verify = vcount;
+            if (li + 1 == pl_.lv.size()) CK(cudaEventRecord(ev_fin.a, st));
+            int nl = 0;
+            CK(launch_level<T>(a, L.nblocks, true, nullptr, dOut, codes, nullptr, zpos, nz, dunpred, st, &nl));
+            launches.n += nl;
+        }
+        CK(cudaEventRecord(ev_fin.b, st));
+        CK(cudaEventRecord(ev_pred.b, st));
+        CK(cudaMemcpyAsync(hk, kerr, 4, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+    };
+    reconstruct();
+    if (h.settle(m, st, launches)) {
+        if (vcount) CK(cudaMemsetAsync(vcount, 0, 8, st));
+        reconstruct();
     }
-    CK(cudaEventRecord(ev_fin.b, st));
-    CK(cudaEventRecord(ev_pred.b, st));
-    int *hk = (int *)t_pin_small.get(64);
-    CK(cudaMemcpyAsync(hk, kerr, 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    if (*hz != nz) throw Fail{FAZ_ERR_FORMAT, "unpredictable count does not match the zero codes"};
     if (*hk) throw Fail{FAZ_ERR_DEVICE, "level kernel met an out-of-range stream position"};
     if (vcount) {
         unsigned long long vc = 0;

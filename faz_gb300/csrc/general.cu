@@ -751,7 +751,7 @@ void gen_compress_payload(int N, const uint64_t *dims, int bs, int lo, int lo2, 
     huffman_encode_device(codes, n, radius, m, st, launches, hc, tm);
     const uint64_t nunpred = hc.nzero;
     T *unp = m.alloc<T>(nunpred ? nunpred : 1);
-    if (nunpred) launches(launch_compact_zeros<T>(codes, n, hc.zc, hc.zoff, nullptr, scratch, unp, st));
+    if (nunpred) launches(launch_compact_zeros<T>(codes, n, hc.zc, hc.zoff, scratch, unp, st));
     CK(cudaEventRecord(ev_huff.b, st));
     // SZGeneralFrontend::save: dims, block size, each predictor's save in
     // list order (Lorenzo: its id; regression: id, coefficient count, the two
@@ -927,10 +927,9 @@ void gen_decompress(int N, const uint8_t *pl, size_t psize, const uint64_t *dims
     if (nunpred) CK(cudaMemcpyAsync(dunp, p, nunpred * sizeof(T), cudaMemcpyHostToDevice, st));
     p += nunpred * sizeof(T);
     uint16_t *codes = m.alloc<uint16_t>(n);
-    huffman_decode_device(p, end, n, codes, m, st, launches);
     uint64_t *zpos = nullptr;
-    const uint64_t nz = zero_positions(codes, n, m, st, launches, zpos);
-    if (nz != nunpred) throw Fail{FAZ_ERR_FORMAT, "unpredictable count does not match the zero codes"};
+    const uint64_t nz = nunpred;
+    decode_with_zeros(p, end, n, nz, codes, m, st, launches, zpos);
     CK(cudaEventRecord(ev_dec.b, st));
     {
         const GenArgs ac = a;

@@ -113,6 +113,7 @@ struct Pinned {
 };
 inline thread_local Pinned t_pin_payload;
 inline thread_local Pinned t_pin_small;
+inline thread_local Pinned t_pin_decode;  // outcome of a queued Huffman decode
 inline thread_local Pinned t_pin_flag;  // device status words read after a later synchronisation
 
 // Pinned staging for host-to-device uploads whose copies complete after the
@@ -525,9 +526,11 @@ void huffman_decode_device(const uint8_t *&p, const uint8_t *end, uint64_t num, 
                            cudaStream_t st, Counter &launches);
 void huffman_decode_device(const uint8_t *&p, const uint8_t *end, uint64_t num, uint32_t *codes, DevMem &m,
                            cudaStream_t st, Counter &launches);
-uint64_t zero_positions(const uint16_t *codes, uint64_t num, DevMem &m, cudaStream_t st, Counter &launches,
-                        uint64_t *&zpos);
-uint64_t zero_positions(const uint32_t *codes, uint64_t num, DevMem &m, cudaStream_t st, Counter &launches,
-                        uint64_t *&zpos);
+// Decode num codes that hold nunpred zeros (else FAZ_ERR_FORMAT), with the
+// zeros' sorted positions in zpos.
+void decode_with_zeros(const uint8_t *&p, const uint8_t *end, uint64_t num, uint64_t nunpred, uint16_t *codes,
+                       DevMem &m, cudaStream_t st, Counter &launches, uint64_t *&zpos);
+void decode_with_zeros(const uint8_t *&p, const uint8_t *end, uint64_t num, uint64_t nunpred, uint32_t *codes,
+                       DevMem &m, cudaStream_t st, Counter &launches, uint64_t *&zpos);
 
 }  // namespace faz

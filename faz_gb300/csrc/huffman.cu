@@ -8,6 +8,7 @@
 // (the end of the previous unit's decode) differs, until every unit starts on
 // a codeword boundary (Huffman codes self-synchronise within a few codewords).
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 #include "internal.h"
 
@@ -119,13 +120,12 @@ __global__ void __launch_bounds__(1024) k_count_zeros(const C *__restrict__ code
 }
 
 // Compaction of the zero codes of each warp sub-chunk, in stream order,
-// starting at zoff[sub-chunk]: positions (zpos) and/or the values recorded at
-// those positions (vals from scratch).
+// starting at zoff[sub-chunk]: the values recorded at their positions (vals from
+// scratch).
 template <typename T, typename C>
 __global__ void __launch_bounds__(1024) k_compact_zeros(const C *__restrict__ codes, uint64_t n,
                                                         const unsigned long long *zcount,
-                                                        const unsigned long long *zoff, uint64_t *zpos,
-                                                        const T *scratch, T *vals) {
+                                                        const unsigned long long *zoff, const T *scratch, T *vals) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t sub = (uint64_t)blockIdx.x * HWARPS + w;
     if (zcount[sub] == 0) return;
@@ -159,8 +159,7 @@ __global__ void __launch_bounds__(1024) k_compact_zeros(const C *__restrict__ co
             const int k = __ffs(m) - 1;
             m &= m - 1;
             const uint64_t i = b + 8 * lane + k;
-            if (zpos) zpos[o] = i;
-            if (vals) vals[o] = scratch[i];
+            vals[o] = scratch[i];
             o++;
         }
         run += (unsigned long long)total;
@@ -171,8 +170,7 @@ __global__ void __launch_bounds__(1024) k_compact_zeros(const C *__restrict__ co
         const unsigned int bal = __ballot_sync(0xffffffffu, z);
         if (z) {
             const unsigned long long o = run + __popc(bal & ((1u << lane) - 1));
-            if (zpos) zpos[o] = i;
-            if (vals) vals[o] = scratch[i];
+            vals[o] = scratch[i];
         }
         run += __popc(bal);
     }
@@ -402,211 +400,592 @@ __global__ void __launch_bounds__(ENC_THREADS) k_encode_pack(const C *__restrict
 }
 
 // ------------------------------------------------------------------ decode
-// A CTA decodes DEC_T consecutive units of DEC_UNIT bits from a copy of its
-// segment of the bit string (plus a halo) in shared memory, with the
-// 2^LUT_BITS-entry table beside it.  DEC_UNIT is an odd number of 32-bit
-// words so that the units of a warp start in different banks.
-struct DecTables {
-    const uint32_t *lut;     // 2^LUT_BITS entries: (len << 24) | state, or DEC_NODE | node
-    const uint32_t *left, *right;
-    const int32_t *sym;      // state of a leaf
-    const uint8_t *leaf;
-};
+// The bit string is cut into units of DW 32-bit words, DEC_T units to a CTA.
+//   k_decode_sync   every unit decodes from its nominal start (the codeword
+//                   lengths alone), then the units of a CTA restart at their
+//                   predecessor's end, in shared memory, until none moves;
+//   k_decode_link   the first units of the CTAs restart at the previous CTA's
+//                   end and the change runs on until it meets the recorded
+//                   starts (one thread per CTA: nearly always within a unit);
+//   k_decode_write  decodes the symbols and writes them.
+// A table step takes every whole codeword of the next LUT_BITS bits, and four
+// steps go through one 64-bit window in registers without a test for its end:
+// the decode is bound by issue slots and shared-memory wavefronts, not by memory.
+// For the 134 M codes (82 MB) of a 512^3 field the former per-symbol form (three
+// segment words and a table word per symbol, two resynchronisation passes over
+// every CTA) took 385 + 236 + 337 us, these passes 36 us per
+// eighth of the string (hidden behind its copy but for the last) + 35 + 279 us.
+// DW is odd so that the units of a warp start in different banks.
 static constexpr int LUT_BITS = 12;
-static constexpr uint32_t DEC_NODE = 0x80000000u;
+static constexpr int LUT2_BITS = 8;                  // second table, below each prefix of a longer codeword
+static constexpr uint32_t B_LONG = 1u << 12;         // lutB.y: longer codewords
+static constexpr uint32_t DEC_NODE = 0x80000000u;    // second table: an inner node follows
+static constexpr uint32_t DEC_LEAF = 0x80000000u;    // child: a leaf's state follows
+static constexpr uint32_t DEC_BAD = 0x40000000u;     // child: a leaf with a negative state
 static constexpr int DEC_T = 256;
-static constexpr int DEC_WORDS = 17;                 // words per unit (17: fastest of 9, 13, 17, 33 on GB300)
-static constexpr uint64_t DEC_UNIT = DEC_WORDS * 32; // bits per unit
 static constexpr int DEC_HALO = 8;                   // words past the last unit
-static constexpr int DEC_SEG = DEC_T * DEC_WORDS + DEC_HALO;
 static constexpr int DEC_NB = 16;                    // boundaries recorded per unit
+static constexpr int DEC_STEPS = 4;                  // table steps per 64-bit window
+static_assert(DEC_STEPS * LUT_BITS <= 64, "a window holds its steps");
+static constexpr int DEC_WT = 512;                   // units per CTA of the writing pass
+static constexpr int DEC_ROWS = 3 + 2 * 4 + 1;       // words buffered per thread of it
+// words per unit: long units for long bit strings (fewer restarts), short ones
+// where there would be too few to fill the GPU (a 0.1 MB string has 1,450 units
+// of 17 words, 6 CTAs)
+static constexpr int DEC_LONG = 17, DEC_SHORT = 5;
+static constexpr uint64_t DEC_SHORT_BITS = (uint64_t)1 << 25;
 
-// bits [p, p+64) of the segment (word-grid relative), MSB first
-__device__ __forceinline__ uint64_t seg_peek(const uint32_t *sw, uint32_t p) {
-    uint32_t w = p >> 5, b = p & 31;
-    uint64_t hi = ((uint64_t)sw[w] << 32) | sw[w + 1];
-    if (!b) return hi;
-    return (hi << b) | (sw[w + 2] >> (32 - b));
+// lutA (per LUT_BITS prefix): length of the first codeword, bits and number of
+// the whole codewords in the prefix, 4 bits each; a prefix of longer codewords
+// has length 0 and its second-table slot << 4.
+// lutB: up to three symbols (16 bits each, the third in y's high half; one of 32
+// bits for wide codes), y's low half = their bits | first length << 4 | count << 8
+// | zero symbols << 10; a prefix of longer codewords has y = B_LONG, x = slot.
+// The second tables (per slot and next LUT2_BITS bits): lut2 as below, len2 the
+// codeword's length alone (0: longer still, or damaged).  Longer codewords are
+// a few per cent of the symbols, but with 32 lanes a warp meets one every few
+// steps, so they cost one dependent load and no call.
+__device__ __forceinline__ uint32_t dec_child(const uint32_t *child, uint32_t node, int bit) {
+    return child[2 * (size_t)node + bit];
 }
 
-// one symbol at segment bit p: returns its state (or -1 on a damaged tree)
-// and advances p.  Codes are at most 64 bits long.
-__device__ __forceinline__ int dec_sym(const DecTables &t, const uint32_t *slut, const uint32_t *sw, uint32_t &p) {
-    uint64_t win = seg_peek(sw, p);
-    uint32_t e = slut[win >> (64 - LUT_BITS)];
-    if (!(e & DEC_NODE)) {
-        p += e >> 24;
-        return (int)(e & 0xffffff);
-    }
-    uint32_t node = e & 0xffffff;
-    for (int b = LUT_BITS; b < 64; b++) {
-        int bit = (int)((win >> (63 - b)) & 1);
-        node = bit ? t.right[node] : t.left[node];
-        if (t.leaf[node]) {
-            p += b + 1;
-            return t.sym[node];
+template <typename C>
+__global__ void __launch_bounds__(256) k_decode_lut(const uint32_t *__restrict__ child, int offset, uint16_t *lutA,
+                                                   uint2 *lutB, uint32_t *slot_node, unsigned *nslots) {
+    const uint32_t v = blockIdx.x * 256 + threadIdx.x;
+    uint32_t node = 0;
+    int cnt = 0, bits_all = 0, bits_b = 0, len1 = 0, zeros = 0;
+    uint32_t sx = 0, sy = 0;
+    constexpr int maxsym = sizeof(C) == 2 ? 3 : 1;
+    for (int b = 0; b < LUT_BITS; b++) {
+        const uint32_t ch = dec_child(child, node, (v >> (LUT_BITS - 1 - b)) & 1);
+        if (!(ch & DEC_LEAF)) {
+            node = ch;
+            continue;
         }
+        const C sym = (C)((int)(ch & 0xffffffu) + offset);
+        if (cnt < maxsym) {
+            if (cnt < 2) sx |= (uint32_t)sym << (16 * cnt);
+            else sy = (uint32_t)sym << 16;
+            zeros += sym == 0;
+            bits_b = b + 1;
+        }
+        if (cnt == 0) len1 = b + 1;
+        cnt++;
+        bits_all = b + 1;
+        node = 0;
     }
-    return -1;
+    uint32_t slot = 0;
+    if (cnt == 0) {
+        slot = atomicAdd(nslots, 1u);
+        slot_node[slot] = node;
+    }
+    lutA[v] = (uint16_t)(cnt == 0 ? slot << 4 : len1 | (bits_all << 4) | (cnt << 8));
+    lutB[v] = cnt == 0 ? make_uint2(slot, B_LONG)
+                       : make_uint2(sx, sy | (uint32_t)(bits_b | (len1 << 4) | ((cnt < maxsym ? cnt : maxsym) << 8) |
+                                                        (zeros << 10)));
+}
+
+// Second table: CTA k fills the entries of slot k: (length << 24) | state, or
+// DEC_NODE | node for codewords longer still, or 0 for a leaf without a state.
+__global__ void __launch_bounds__(1 << LUT2_BITS) k_decode_lut2(const uint32_t *__restrict__ child,
+                                                               const uint32_t *__restrict__ slot_node,
+                                                               const unsigned *__restrict__ nslots, uint32_t *lut2,
+                                                               uint8_t *len2) {
+    if (blockIdx.x >= *nslots) return;
+    uint32_t node = slot_node[blockIdx.x], e = 0;
+    int b = 0;
+    for (; b < LUT2_BITS; b++) {
+        const uint32_t ch = dec_child(child, node, (threadIdx.x >> (LUT2_BITS - 1 - b)) & 1);
+        if (ch & DEC_LEAF) {
+            e = ch & DEC_BAD ? 0u : ((uint32_t)(LUT_BITS + b + 1) << 24) | (ch & 0xffffffu);
+            break;
+        }
+        node = ch;
+    }
+    if (b == LUT2_BITS) e = DEC_NODE | node;
+    lut2[((size_t)blockIdx.x << LUT2_BITS) + threadIdx.x] = e;
+    len2[((size_t)blockIdx.x << LUT2_BITS) + threadIdx.x] = (uint8_t)(e & DEC_NODE ? 0u : e >> 24);
+}
+
+// A codeword longer than LUT_BITS + LUT2_BITS at the front of `win`, below
+// second-table entry e: its length (0: damaged tree or longer than 64 bits) and
+// state.
+__device__ __noinline__ uint2 dec_long(const uint32_t *__restrict__ child, uint32_t e, uint64_t win) {
+    if (!(e & DEC_NODE)) return make_uint2(0u, 0u);
+    uint32_t node = e & 0xffffffu;
+    for (int b = LUT_BITS + LUT2_BITS; b < 64; b++) {
+        const uint32_t ch = dec_child(child, node, (int)((win >> (63 - b)) & 1));
+        if (ch & DEC_LEAF) return make_uint2(ch & DEC_BAD ? 0u : (uint32_t)b + 1, ch & 0xffffffu);
+        node = ch;
+    }
+    return make_uint2(0u, 0u);
 }
 
 __device__ __forceinline__ uint32_t bswap_w(uint32_t x) { return __byte_perm(x, 0, 0x0123); }
 
-// Stage the CTA's segment (as big-endian words) and the lookup table.
-__device__ __forceinline__ void dec_stage(const DecTables &t, const uint32_t *__restrict__ w32, uint64_t nwords,
-                                          uint32_t *slut, uint32_t *sw, uint64_t wbase) {
-    for (int i = threadIdx.x; i < (1 << LUT_BITS); i += blockDim.x) slut[i] = t.lut[i];
-    for (int i = threadIdx.x; i < DEC_SEG; i += blockDim.x) {
-        uint64_t gi = wbase + i;
-        sw[i] = gi < nwords ? bswap_w(w32[gi]) : 0u;
+// word i of the bit string, staged in shared memory / read from global memory
+struct WordsShared {
+    const uint32_t *sw;
+    __device__ __forceinline__ uint32_t operator()(uint32_t i) const { return sw[i]; }
+};
+struct WordsGlobal {
+    const uint32_t *w32;
+    uint64_t base, nwords;
+    __device__ __forceinline__ uint32_t operator()(uint32_t i) const {
+        return base + i < nwords ? bswap_w(w32[base + i]) : 0u;
+    }
+};
+
+// 32 and 64 bits of the string from bit p
+template <typename Words>
+__device__ __forceinline__ uint32_t peek32(const Words &words, uint32_t p) {
+    return __funnelshift_l(words((p >> 5) + 1), words(p >> 5), p & 31);
+}
+template <typename Words>
+__device__ __forceinline__ uint64_t peek64(const Words &words, uint32_t p) {
+    const uint32_t w = p >> 5, b = words(w + 1);
+    return ((uint64_t)__funnelshift_l(b, words(w), p & 31) << 32) | __funnelshift_l(words(w + 2), b, p & 31);
+}
+
+// Entry of a slot's second table for the window `win`.
+__device__ __forceinline__ size_t lut2_index(uint32_t slot, uint32_t win) {
+    return ((size_t)slot << LUT2_BITS) + ((win >> (32 - LUT_BITS - LUT2_BITS)) & ((1u << LUT2_BITS) - 1));
+}
+
+// Length of the codeword at bit p (0: damaged).
+template <typename Words>
+__device__ __forceinline__ uint32_t dec_len(const DecodeTablesDev &t, const uint16_t *slut, const Words &words,
+                                            uint32_t p) {
+    const uint32_t win = peek32(words, p), e = slut[win >> (32 - LUT_BITS)];
+    uint32_t n = e & 15;
+    if (n == 0) {
+        const size_t i = lut2_index(e >> 4, win);
+        n = t.len2[i];
+        if (n == 0) n = dec_long(t.child, t.lut2[i], peek64(words, p)).x;
+    }
+    return n;
+}
+
+// Pass codewords from bit p to the first boundary at or past `stop`: returns
+// the boundary and adds the codewords to c.  On damage *err is set and `stop`
+// returned, so that later passes stay within the unit.
+template <typename Words>
+__device__ __forceinline__ uint32_t dec_skip(const DecodeTablesDev &t, const uint16_t *slut, const Words &words,
+                                             uint32_t p, uint32_t stop, unsigned &c, int *err) {
+    // four whole prefixes at a time while they end within the unit
+    while (p + DEC_STEPS * LUT_BITS <= stop) {
+        const uint64_t win = peek64(words, p);
+        uint32_t hi = (uint32_t)(win >> 32), lo = (uint32_t)win;
+#pragma unroll
+        for (int k = 0; k < DEC_STEPS; k++) {
+            const uint32_t e = slut[hi >> (32 - LUT_BITS)];
+            if ((e & 15) == 0) {
+                const uint32_t n = dec_len(t, slut, words, p);
+                if (n == 0) {
+                    atomicExch(err, 1);
+                    return stop;
+                }
+                p += n;
+                c++;
+                break;
+            }
+            const uint32_t b = (e >> 4) & 15;
+            p += b;
+            c += e >> 8;
+            hi = __funnelshift_l(lo, hi, b);
+            lo <<= b;
+        }
+    }
+    while (p + LUT_BITS <= stop) {
+        const uint32_t e = slut[peek32(words, p) >> (32 - LUT_BITS)];
+        if ((e & 15) == 0) break;
+        p += (e >> 4) & 15;
+        c += e >> 8;
+    }
+    while (p < stop) {
+        const uint32_t n = dec_len(t, slut, words, p);
+        if (n == 0) {
+            atomicExch(err, 1);
+            return stop;
+        }
+        p += n;
+        c++;
+    }
+    return p;
+}
+
+// The first run_bits of the string are expected to hold codewords of run_len
+// bits (the anchor grid: the zero code over and over, which a decode that starts
+// between two of them need never fall in step with; the units of such a run
+// then settle one per restart, 0.5 ms for 1152 anchors): units there start at a
+// multiple of run_len.  Like every start it is a guess that the restarts check.
+// info[u]: start of unit u past its nominal start (< 64) | codewords << 8.
+// cend[c]: end of CTA c's last unit past that unit's nominal end.
+template <int DW>
+__global__ void __launch_bounds__(DEC_T) k_decode_sync(DecodeTablesDev t, const uint32_t *__restrict__ w32,
+                                                      uint64_t nwords, uint64_t nbits, uint64_t nunits, uint64_t cta0,
+                                                      uint64_t run_bits, uint32_t run_len,
+                                                      uint32_t *__restrict__ info, uint32_t *__restrict__ cend,
+                                                      unsigned long long *__restrict__ ctot, int *flags) {
+    constexpr uint32_t UNIT = DW * 32;
+    constexpr int SEG = DEC_T * DW + DEC_HALO;
+    __shared__ uint16_t slut[1 << LUT_BITS];
+    __shared__ uint32_t sw[SEG];
+    __shared__ uint16_t bnd[DEC_NB][DEC_T];
+    __shared__ uint32_t send[DEC_T];
+    __shared__ unsigned wsum[DEC_T / 32];
+    const int tid = threadIdx.x;
+    const uint64_t cta = cta0 + blockIdx.x;
+    const uint64_t u0 = cta * DEC_T, g0 = u0 * UNIT;
+    {
+        const uint4 *src = reinterpret_cast<const uint4 *>(t.lutA);
+        for (int i = tid; i < (1 << LUT_BITS) / 8; i += DEC_T) reinterpret_cast<uint4 *>(slut)[i] = src[i];
+        const uint64_t wb = u0 * DW;
+        for (int i = tid; i < SEG; i += DEC_T) sw[i] = wb + i < nwords ? bswap_w(w32[wb + i]) : 0u;
     }
     __syncthreads();
+    const uint64_t u = u0 + tid;
+    const bool act = u < nunits;
+    const uint32_t nominal = (uint32_t)tid * UNIT;
+    uint32_t stop = nominal + UNIT;
+    if (nbits - g0 < stop) stop = (uint32_t)(nbits - g0);
+    const WordsShared words{sw};
+    // speculative decode from the nominal start; its first boundaries are kept
+    unsigned spec_cnt = 0;
+    uint32_t spec_end = nominal, spec_start = nominal;
+    if (act) {
+        if (g0 + nominal < run_bits) {
+            const uint32_t over = (uint32_t)((g0 + nominal) % run_len);
+            if (over) spec_start += run_len - over;
+        }
+        int k = 0;
+        uint32_t p = spec_start;
+        for (; k < DEC_NB && p < stop; k++) {
+            bnd[k][tid] = (uint16_t)(p - nominal);
+            const uint32_t n = dec_len(t, slut, words, p);
+            if (n == 0) break;  // reported by dec_skip
+            p += n;
+        }
+        spec_cnt = k;
+        for (; k < DEC_NB; k++) bnd[k][tid] = 0xffff;
+        spec_end = dec_skip(t, slut, words, p, stop, spec_cnt, flags + 1);
+    }
+    // restart at the predecessor's end until no end moves; a decode that meets
+    // a boundary of the speculative one coincides with it from there
+    uint32_t start = spec_start, end = spec_end;
+    unsigned cnt = spec_cnt;
+    send[tid] = end;
+    for (int it = 0; it < DEC_T; it++) {
+        __syncthreads();
+        const uint32_t s = tid ? send[tid - 1] : spec_start;
+        const uint32_t was = end;
+        if (act && s != start) {
+            start = s;
+            uint32_t p = s;
+            unsigned c = 0;
+            int j = 0;
+            bool met = false;
+            while (p < stop) {
+                const uint32_t off = p - nominal;
+                while (j < DEC_NB && bnd[j][tid] < off) j++;
+                if (j == DEC_NB) break;
+                if (bnd[j][tid] == off) {
+                    met = true;
+                    break;
+                }
+                const uint32_t n = dec_len(t, slut, words, p);
+                if (n == 0) break;
+                c++;
+                p += n;
+            }
+            if (met) {
+                c += spec_cnt - j;
+                end = spec_end;
+            } else {
+                end = dec_skip(t, slut, words, p, stop, c, flags + 1);
+            }
+            cnt = c;
+        }
+        if (!__syncthreads_or(end != was)) break;
+        send[tid] = end;
+    }
+    if (act) info[u] = (start - nominal) | (cnt << 8);
+    if (tid == DEC_T - 1) cend[cta] = end - (nominal + UNIT);
+    unsigned x = act ? cnt : 0;
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if ((tid & 31) == 0) wsum[tid >> 5] = x;
+    __syncthreads();
+    if (tid == 0) {
+        unsigned s = 0;
+        for (int i = 0; i < DEC_T / 32; i++) s += wsum[i];
+        ctot[cta] = s;
+    }
 }
 
-// Speculative pass: unit u decodes from its nominal start u*DEC_UNIT to the
-// first codeword end at or past the unit's end; records the end, the symbol
-// count, and the first DEC_NB codeword boundaries (offsets from the start).
-__global__ void __launch_bounds__(DEC_T) k_decode_spec(DecTables t, const uint32_t *__restrict__ w32, uint64_t nwords,
-                                                      uint64_t nbits, uint64_t nunits, uint64_t ubase,
-                                                      uint64_t *end, unsigned int *cnt, uint16_t *bnd, int *err) {
-    __shared__ uint32_t slut[1 << LUT_BITS];
-    __shared__ uint32_t sw[DEC_SEG];
-    const uint64_t u0 = ubase + (uint64_t)blockIdx.x * DEC_T;
-    dec_stage(t, w32, nwords, slut, sw, u0 * DEC_WORDS);
-    const uint64_t u = u0 + threadIdx.x;
-    if (u >= nunits) return;
-    const uint64_t g0 = u0 * DEC_UNIT;
-    uint64_t lim = (u + 1) * DEC_UNIT;
-    if (lim > nbits) lim = nbits;
-    const uint32_t start = (uint32_t)(u * DEC_UNIT - g0);
-    const uint32_t stop = (uint32_t)(lim - g0);
-    uint32_t p = start;
-    unsigned int c = 0;
-    uint16_t *b = bnd + u * DEC_NB;
-    while (p < stop) {
-        if (c < DEC_NB) b[c] = (uint16_t)(p - start);
-        if (dec_sym(t, slut, sw, p) < 0) {
-            atomicExch(err, 1);
-            break;
-        }
-        c++;
+// Thread c: the units of CTA c from the end of CTA c - 1, until one starts
+// where it was recorded to start.  cend_in / cend_out: ends before and after
+// this pass; *flags = 1 when a CTA's end moved (another pass is needed).
+template <int DW>
+__global__ void __launch_bounds__(64) k_decode_link(DecodeTablesDev t, const uint32_t *__restrict__ w32,
+                                                   uint64_t nwords, uint64_t nbits, uint64_t nunits, uint64_t ncta,
+                                                   const uint32_t *__restrict__ cend_in, uint32_t *__restrict__ cend_out,
+                                                   uint32_t *info, unsigned long long *ctot, int *flags) {
+    constexpr uint32_t UNIT = DW * 32;
+    constexpr int ROW = DW + 4;  // a unit's words and the three past it (odd: distinct banks)
+    __shared__ uint16_t slut[1 << LUT_BITS];
+    __shared__ uint32_t first[64 * ROW];
+    for (int i = threadIdx.x; i < (1 << LUT_BITS) / 8; i += 64)
+        reinterpret_cast<uint4 *>(slut)[i] = reinterpret_cast<const uint4 *>(t.lutA)[i];
+    // the CTAs' first units, where the change nearly always ends: read word by
+    // word from global memory they took 58 us of a 512^3 field's decode
+    for (int i = threadIdx.x; i < 64 * ROW; i += 64) {
+        const uint64_t w = ((uint64_t)blockIdx.x * 64 + i / ROW) * (DEC_T * DW) + i % ROW;
+        first[i] = w < nwords ? bswap_w(w32[w]) : 0u;
     }
-    for (unsigned int k = c; k < DEC_NB; k++) b[k] = 0xffff;
-    end[u] = g0 + p;
-    cnt[u] = c;
+    __syncthreads();
+    const uint64_t c = (uint64_t)blockIdx.x * 64 + threadIdx.x;
+    if (c >= ncta) return;
+    const uint32_t old_end = cend_in[c];
+    uint32_t new_end = old_end;
+    if (c > 0) {
+        const uint64_t u0 = c * DEC_T, g0 = u0 * UNIT;
+        uint32_t s = cend_in[c - 1];
+        long long delta = 0;
+        const WordsShared wf{first + threadIdx.x * ROW};
+        const WordsGlobal wg{w32, u0 * DW, nwords};
+        int k = 0;
+        for (; k < DEC_T && u0 + k < nunits; k++) {
+            const uint32_t rec = info[u0 + k];
+            if ((rec & 255u) == s) break;
+            uint32_t stop = (uint32_t)(k + 1) * UNIT;
+            if (nbits - g0 < stop) stop = (uint32_t)(nbits - g0);
+            unsigned n = 0;
+            const uint32_t e = k == 0 ? dec_skip(t, slut, wf, s, stop, n, flags + 1)
+                                      : dec_skip(t, slut, wg, (uint32_t)k * UNIT + s, stop, n, flags + 1);
+            info[u0 + k] = s | (n << 8);
+            delta += (long long)n - (long long)(rec >> 8);
+            const uint32_t next = (uint32_t)(k + 1) * UNIT;
+            s = e > next ? e - next : 0u;
+        }
+        if (k == DEC_T) new_end = s;
+        if (delta) ctot[c] += (unsigned long long)delta;
+    }
+    cend_out[c] = new_end;
+    if (new_end != old_end) atomicExch(flags, 1);
 }
 
-// Synchronisation pass: unit u restarts at the true end of unit u-1 (given
-// in `start_in`, a copy of the previous pass's ends) and decodes until its
-// position meets a boundary of its speculative decode; from there the two
-// decodes coincide.  Units that do not meet one within the recorded window
-// decode to the end.  Sets *changed when any end moved.
-__global__ void __launch_bounds__(DEC_T) k_decode_resync(DecTables t, const uint32_t *__restrict__ w32,
-                                                        uint64_t nwords, uint64_t nbits, uint64_t nunits,
-                                                        const uint64_t *end_in, uint64_t *end_out,
-                                                        unsigned int *cnt, const uint16_t *bnd, uint64_t *start,
-                                                        int *changed) {
-    __shared__ uint32_t slut[1 << LUT_BITS];
-    __shared__ uint32_t sw[DEC_SEG];
-    const uint64_t u0 = (uint64_t)blockIdx.x * DEC_T;
-    dec_stage(t, w32, nwords, slut, sw, u0 * DEC_WORDS);
-    const uint64_t u = u0 + threadIdx.x;
-    if (u >= nunits) return;
-    const uint64_t g0 = u0 * DEC_UNIT;
-    const uint64_t s_true = u == 0 ? 0 : end_in[u - 1];
-    if (s_true == start[u]) {
-        end_out[u] = end_in[u];
-        return;
+// Decode unit u from its start into out[offset of u...): 16-byte stores of
+// eight 16-bit codes, the ends of a unit's range as single codes.  Warp w's codes
+// begin at zstart[w] and hold zc[w] zeros (for the compaction of the
+// unpredictable ones).  Issue-bound: a step takes up to three symbols; whole
+// words of two codes go to the thread's column of a shared buffer (one bank, no
+// conflicts), from which the threads store together.  Packing in registers with
+// a store whenever a thread's 16 bytes were full took 216 M warp instructions for
+// the 134 M codes of a 512^3 field, this 139 M (0.28 ms).
+template <typename C, int DW>
+__global__ void __launch_bounds__(DEC_WT) k_decode_write(DecodeTablesDev t, const uint32_t *__restrict__ w32,
+                                                        uint64_t nwords, uint64_t nunits,
+                                                        const uint32_t *__restrict__ info,
+                                                        const unsigned long long *__restrict__ coff, uint64_t nout,
+                                                        int offset, C *out, unsigned long long *zc,
+                                                        unsigned long long *zstart) {
+    extern __shared__ __align__(16) unsigned char dsm[];
+    uint2 *slut = reinterpret_cast<uint2 *>(dsm);
+    uint32_t *sw = reinterpret_cast<uint32_t *>(dsm + ((size_t)8 << LUT_BITS));
+    __shared__ unsigned wsum[DEC_WT / 32];
+    constexpr int SEG = DEC_WT * DW + DEC_HALO;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    uint32_t *col = sw + SEG + wid * (DEC_ROWS * 32) + lane;
+    const uint64_t u0 = (uint64_t)blockIdx.x * DEC_WT;
+    {
+        const uint4 *src = reinterpret_cast<const uint4 *>(t.lutB);
+        for (int i = tid; i < (1 << LUT_BITS) / 2; i += DEC_WT) reinterpret_cast<uint4 *>(slut)[i] = src[i];
+        const uint64_t wb = u0 * DW;
+        for (int i = tid; i < SEG; i += DEC_WT) sw[i] = wb + i < nwords ? bswap_w(w32[wb + i]) : 0u;
     }
-    uint64_t lim = (u + 1) * DEC_UNIT;
-    if (lim > nbits) lim = nbits;
-    const uint32_t nominal = (uint32_t)(u * DEC_UNIT - g0);
-    const uint32_t stop = (uint32_t)(lim - g0);
-    if (s_true < g0 || s_true - g0 > stop + 64) {
-        atomicExch(changed, -1);
-        return;
+    const WordsShared words{sw};
+    const uint64_t u = u0 + tid;
+    const uint32_t rec = u < nunits ? info[u] : 0u;
+    unsigned n = rec >> 8, x = n;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
     }
-    uint32_t p = (uint32_t)(s_true - g0);
-    const bool first_pass = start[u] == u * DEC_UNIT;
-    // the speculative boundaries, ascending (unused entries are 0xffff)
-    uint32_t bw[DEC_NB / 2];
-    const uint32_t *b32 = reinterpret_cast<const uint32_t *>(bnd + u * DEC_NB);
-#pragma unroll
-    for (int k = 0; k < DEC_NB / 2; k++) bw[k] = first_pass ? b32[k] : 0xffffffffu;
-    unsigned int c = 0;
-    bool synced = false;
-    int j = 0;  // first speculative boundary not yet passed
-    while (p < stop) {
-        const uint32_t off = p - nominal;
-        while (j < DEC_NB) {
-            uint32_t bj = (bw[j >> 1] >> ((j & 1) * 16)) & 0xffffu;
-            if (bj >= off) break;
-            j++;
+    if (lane == 31) wsum[wid] = x;
+    __syncthreads();
+    if (u0 + (uint64_t)wid * 32 >= nunits) return;  // no unit in this warp
+    uint64_t o = coff[u0 / DEC_T] + (x - n);
+    for (int w = 0; w < wid; w++) o += wsum[w];
+    if (lane == 0) zstart[u >> 5] = o;
+    if (o >= nout) n = 0;
+    else if (nout - o < n) n = (unsigned)(nout - o);
+    uint32_t p = (uint32_t)tid * (DW * 32) + (rec & 255u);
+    unsigned left = n, nz = 0;
+    // a codeword longer than the prefix in `win`, slot e.x, as an entry of one
+    // symbol; returns its bits (0 on damage, reported by the passes before)
+    auto long_entry = [&](uint2 &e, uint32_t win) -> uint32_t {
+        const uint32_t e2 = t.lut2[lut2_index(e.x, win)];
+        uint32_t state = e2 & 0xffffffu, bits = e2 >> 24;
+        if ((int32_t)e2 <= 0) {
+            const uint2 l = dec_long(t.child, e2, peek64(words, p));
+            bits = l.x;
+            state = l.y;
         }
-        if (j < DEC_NB && ((bw[j >> 1] >> ((j & 1) * 16)) & 0xffffu) == off) {
-            c += cnt[u] - j;
-            synced = true;
-            break;
-        }
-        if (dec_sym(t, slut, sw, p) < 0) {
-            atomicExch(changed, -1);
-            return;
-        }
-        c++;
-    }
-    const uint64_t e = synced ? end_in[u] : g0 + p;
-    start[u] = s_true;
-    cnt[u] = c;
-    end_out[u] = e;
-    if (e != end_in[u]) atomicCAS(changed, 0, 1);
-}
-
-// Final pass: decode unit u from its true start into out[off[u]...].
-template <typename C>
-__global__ void __launch_bounds__(DEC_T) k_decode_write(DecTables t, const uint32_t *__restrict__ w32, uint64_t nwords,
-                                                       uint64_t nbits, uint64_t nunits, const uint64_t *start,
-                                                       const unsigned long long *off, uint64_t nout, int offset,
-                                                       C *out) {
-    __shared__ uint32_t slut[1 << LUT_BITS];
-    __shared__ uint32_t sw[DEC_SEG];
-    const uint64_t u0 = (uint64_t)blockIdx.x * DEC_T;
-    dec_stage(t, w32, nwords, slut, sw, u0 * DEC_WORDS);
-    const uint64_t u = u0 + threadIdx.x;
-    if (u >= nunits) return;
-    const uint64_t g0 = u0 * DEC_UNIT;
-    uint64_t lim = (u + 1) * DEC_UNIT;
-    if (lim > nbits) lim = nbits;
-    uint32_t p = (uint32_t)(start[u] - g0);
-    const uint32_t stop = (uint32_t)(lim - g0);
-    uint64_t o = off[u];
+        const C sym = (C)((int)state + offset);
+        e = make_uint2(sym, (1u << 8) | (sym == 0 ? 1u << 10 : 0u));
+        return bits;
+    };
     if constexpr (sizeof(C) != 2) {  // wide codes: one store per symbol
-        while (p < stop && o < nout) {
-            int s = dec_sym(t, slut, sw, p);
-            if (s < 0) return;
-            out[o++] = (C)(s + offset);
+        for (; left; left--) {
+            const uint32_t win = peek32(words, p);
+            uint2 e = slut[win >> (32 - LUT_BITS)];
+            const uint32_t bits = e.y & B_LONG ? long_entry(e, win) : e.y & 15;
+            if (bits == 0) break;
+            p += bits;
+            out[o + (n - left)] = (C)e.x;
+            nz += e.x == 0;
         }
     } else {
-    // 2-byte stores up to a 16-byte boundary, then 8 symbols per store
-    while (p < stop && o < nout && (o & 7)) {
-        int s = dec_sym(t, slut, sw, p);
-        if (s < 0) return;
-        out[o++] = (C)(s + offset);
-    }
-    uint32_t pk[4];
-    int k = 0;
-    while (p < stop && o + k < nout) {
-        int s = dec_sym(t, slut, sw, p);
-        if (s < 0) break;
-        uint32_t v = (uint32_t)(uint16_t)(s + offset);
-        if (k & 1) pk[k >> 1] |= v << 16;
-        else pk[k >> 1] = v;
-        if (++k == 8) {
-            *reinterpret_cast<uint4 *>((uint16_t *)out + o) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            o += 8;
-            k = 0;
+        // the column holds whole words of two codes from ob on (k of them) and
+        // `pend` the low half of the next one when half = 1; the first `lead`
+        // codes at ob belong to the unit before
+        uint16_t *ob = (uint16_t *)out + (o & ~(uint64_t)7);
+        unsigned lead = (unsigned)(o & 7), k = lead >> 1, half = lead & 1;
+        uint32_t pend = 0;
+        // c codes of entry e, (pend,) s0, s1, s2 as two words; rows past the last
+        // whole one are written again
+        auto push = [&](uint2 e, unsigned c) {
+            const uint32_t w0 = __byte_perm(pend, e.x, half ? 0x5410 : 0x7654);
+            const uint32_t w1 = __byte_perm(e.x, e.y, half ? 0x7632 : 0x1076);
+            col[32 * k] = w0;
+            col[32 * k + 32] = w1;
+            const unsigned tot = half + c;
+            pend = tot < 2 ? w0 : w1;
+            k += tot >> 1;
+            half = tot & 1;
+            left -= c;
+        };
+        auto store8 = [&](const uint32_t *cg) {
+            const uint32_t q0 = cg[0], q1 = cg[32], q2 = cg[64], q3 = cg[96];
+            if (lead == 0) {
+                *reinterpret_cast<uint4 *>(ob) = make_uint4(q0, q1, q2, q3);
+            } else {
+                for (unsigned i = lead; i < 8; i++) {
+                    const uint32_t w = i < 4 ? (i < 2 ? q0 : q1) : (i < 6 ? q2 : q3);
+                    ob[i] = (uint16_t)(w >> (16 * (i & 1)));
+                }
+                lead = 0;
+            }
+            ob += 8;
+        };
+        auto flush = [&] {  // whole groups of eight codes; up to three words move down
+            if (k >= 4) {
+                store8(col);
+                if (k >= 8) store8(col + 128);
+                const uint32_t *cl = col + 32 * (k & ~3u);
+                const uint32_t a = cl[0], b = cl[32], c = cl[64];
+                col[0] = a;
+                col[32] = b;
+                col[64] = c;
+                k &= 3;
+            }
+        };
+        while (__any_sync(0xffffffffu, left >= 3 * DEC_STEPS)) {
+            if (left >= 3 * DEC_STEPS) {
+                const uint64_t win = peek64(words, p);
+                uint32_t hi = (uint32_t)(win >> 32), lo = (uint32_t)win;
+#pragma unroll
+                for (int s = 0; s < DEC_STEPS; s++) {
+                    uint2 e = slut[hi >> (32 - LUT_BITS)];
+                    if (e.y & B_LONG) {
+                        // its bits may reach past the window
+                        const uint32_t b = long_entry(e, peek32(words, p));
+                        if (b) {
+                            p += b;
+                            nz += (e.y >> 10) & 3;
+                            push(e, 1);
+                        } else {
+                            left = 0;
+                        }
+                        break;
+                    }
+                    const uint32_t b = e.y & 15;
+                    p += b;
+                    hi = __funnelshift_l(lo, hi, b);
+                    lo <<= b;
+                    nz += (e.y >> 10) & 3;
+                    push(e, (e.y >> 8) & 3);
+                }
+                flush();
+            }
         }
+        while (left) {
+            const uint32_t win = peek32(words, p);
+            uint2 e = slut[win >> (32 - LUT_BITS)];
+            uint32_t b = e.y & 15;
+            if (e.y & B_LONG) b = long_entry(e, win);
+            if (b == 0) break;
+            unsigned c = (e.y >> 8) & 3, z = (e.y >> 10) & 3;
+            if (c > left) {  // the unit's last codes, one or two
+                c = left;
+                z = ((e.x & 0xffffu) == 0) + (c > 1 && (e.x >> 16) == 0);
+            }
+            p += b;
+            nz += z;
+            push(e, c);
+            if (k >= 8) flush();
+        }
+        flush();
+        for (unsigned i = lead; i < 2 * k; i++) ob[i] = (uint16_t)(col[32 * (i >> 1)] >> (16 * (i & 1)));
+        if (half && 2 * k >= lead) ob[2 * k] = (uint16_t)pend;
     }
-    for (int i = 0; i < k; i++) out[o + i] = (C)(uint16_t)(pk[i >> 1] >> ((i & 1) * 16));
+    __syncwarp();
+    for (int d = 16; d > 0; d >>= 1) nz += __shfl_down_sync(0xffffffffu, nz, d);
+    if (lane == 0) zc[u >> 5] = nz;
+}
+
+// The ranges of a stream of one symbol: RANGE codes each, all of them zero or
+// none.
+static constexpr uint64_t RANGE = 4096;
+__global__ void __launch_bounds__(256) k_constant_ranges(uint64_t n, int zero, unsigned long long *zstart,
+                                                        unsigned long long *zcount) {
+    const uint64_t s = ((uint64_t)blockIdx.x * 256 + threadIdx.x) * RANGE;
+    if (s >= n) return;
+    zstart[s / RANGE] = s;
+    zcount[s / RANGE] = zero ? (n - s < RANGE ? n - s : RANGE) : 0;
+}
+
+// Positions of the zero codes of the decoder's warps, in stream order: warp w's
+// codes [zstart[w], zstart[w + 1]) hold zcount[w] zeros, the first of them the
+// zoff[w]-th; the first `cap` positions are written.
+template <typename C>
+__global__ void __launch_bounds__(256) k_zero_positions(const C *__restrict__ codes, uint64_t n, uint64_t nranges,
+                                                       const unsigned long long *__restrict__ zstart,
+                                                       const unsigned long long *__restrict__ zcount,
+                                                       const unsigned long long *__restrict__ zoff, uint64_t cap,
+                                                       uint64_t *zpos) {
+    const uint64_t w = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (w >= nranges || zcount[w] == 0) return;
+    const int lane = threadIdx.x & 31;
+    uint64_t s1 = w + 1 < nranges ? zstart[w + 1] : n;
+    if (s1 > n) s1 = n;
+    unsigned long long run = zoff[w];
+    for (uint64_t b = zstart[w]; b < s1; b += 128) {
+        // four rows of 32 codes in flight
+        bool z[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint64_t i = b + 32 * k + lane;
+            z[k] = i < s1 && codes[i] == 0;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const unsigned bal = __ballot_sync(0xffffffffu, z[k]);
+            const unsigned long long o = run + __popc(bal & ((1u << lane) - 1));
+            if (z[k] && o < cap) zpos[o] = b + 32 * k + lane;
+            run += __popc(bal);
+        }
     }
 }
 
@@ -614,11 +993,6 @@ template <typename C>
 __global__ void k_fill_u16(C *out, uint64_t n, C v) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
         out[i] = v;
-}
-
-__global__ void k_widen_counts(const unsigned int *cnt, unsigned long long *out, uint64_t n) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        out[i] = cnt[i];
 }
 
 // ------------------------------------------------------------ launchers
@@ -655,15 +1029,13 @@ cudaError_t launch_count_zeros(const uint32_t *codes, uint64_t n, unsigned long 
 
 template <typename T, typename C>
 cudaError_t launch_compact_zeros(const C *codes, uint64_t n, const unsigned long long *zcount,
-                                 const unsigned long long *zoff, uint64_t *zpos, const T *scratch, T *vals,
-                                 cudaStream_t st) {
-    k_compact_zeros<T, C><<<grid_for(n, HCHUNK), 1024, 0, st>>>(codes, n, zcount, zoff, zpos, scratch, vals);
+                                 const unsigned long long *zoff, const T *scratch, T *vals, cudaStream_t st) {
+    k_compact_zeros<T, C><<<grid_for(n, HCHUNK), 1024, 0, st>>>(codes, n, zcount, zoff, scratch, vals);
     return cudaGetLastError();
 }
 #define FAZ_INST_COMPACT(T, C)                                                                               \
     template cudaError_t launch_compact_zeros<T, C>(const C *, uint64_t, const unsigned long long *,       \
-                                                    const unsigned long long *, uint64_t *, const T *, T *, \
-                                                    cudaStream_t);
+                                                    const unsigned long long *, const T *, T *, cudaStream_t);
 FAZ_INST_COMPACT(float, uint16_t)
 FAZ_INST_COMPACT(double, uint16_t)
 FAZ_INST_COMPACT(float, uint32_t)
@@ -722,61 +1094,91 @@ cudaError_t launch_encode_pack(const uint32_t *codes, uint64_t n, int offset, co
     return encode_pack_impl(codes, n, offset, code64, packed, len, chunkoff, out, maxlen, st);
 }
 
-uint64_t decode_units(uint64_t nbits) { return (nbits + DEC_UNIT - 1) / DEC_UNIT; }
-uint64_t decode_unit_bits() { return DEC_UNIT; }
-int decode_boundaries() { return DEC_NB; }
-
+int decode_unit_words(uint64_t nbits) { return nbits < DEC_SHORT_BITS ? DEC_SHORT : DEC_LONG; }
 uint64_t decode_cta_units() { return DEC_T; }
+size_t decode_lut2_entries(int nodes) {
+    return std::min<size_t>((size_t)1 << LUT_BITS, (size_t)nodes / 2 + 1) << LUT2_BITS;
+}
 
-cudaError_t launch_decode_spec(const DecodeTablesDev &td, const uint32_t *w32, uint64_t nwords, uint64_t nbits,
-                               uint64_t nunits, uint64_t ubase, uint64_t uend, uint64_t *end, unsigned int *cnt,
-                               uint16_t *bnd, int *err, cudaStream_t st) {
-    DecTables t{td.lut, td.left, td.right, td.sym, td.leaf};
-    if (uend > nunits) uend = nunits;
-    if (uend <= ubase) return cudaSuccess;
-    k_decode_spec<<<grid_for(uend - ubase, DEC_T), DEC_T, 0, st>>>(t, w32, nwords, nbits, uend, ubase, end, cnt, bnd,
-                                                                    err);
+template <typename C>
+cudaError_t launch_decode_tables(const DecodeTablesDev &t, int offset, uint32_t *slot_node, unsigned *nslots,
+                                 size_t lut2_entries, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(nslots, 0, 4, st);
+    if (e != cudaSuccess) return e;
+    k_decode_lut<C><<<(1 << LUT_BITS) / 256, 256, 0, st>>>(t.child, offset, t.lutA, t.lutB, slot_node, nslots);
+    k_decode_lut2<<<(unsigned)(lut2_entries >> LUT2_BITS), 1 << LUT2_BITS, 0, st>>>(t.child, slot_node, nslots, t.lut2,
+                                                                                    t.len2);
+    return cudaGetLastError();
+}
+template cudaError_t launch_decode_tables<uint16_t>(const DecodeTablesDev &, int, uint32_t *, unsigned *, size_t,
+                                                    cudaStream_t);
+template cudaError_t launch_decode_tables<uint32_t>(const DecodeTablesDev &, int, uint32_t *, unsigned *, size_t,
+                                                    cudaStream_t);
+
+cudaError_t launch_decode_sync(const DecodeTablesDev &t, const DecodeString &d, uint64_t cta0, uint64_t cta1,
+                               uint32_t *info, uint32_t *cend, unsigned long long *ctot, int *flags, cudaStream_t st) {
+    if (cta1 <= cta0) return cudaSuccess;
+    auto k = d.unit_words == DEC_LONG ? k_decode_sync<DEC_LONG> : k_decode_sync<DEC_SHORT>;
+    k<<<(unsigned)(cta1 - cta0), DEC_T, 0, st>>>(t, d.w32, d.nwords, d.nbits, d.nunits, cta0, d.run_bits, d.run_len, info,
+                                                 cend, ctot, flags);
     return cudaGetLastError();
 }
 
-cudaError_t launch_decode_resync(const DecodeTablesDev &td, const uint32_t *w32, uint64_t nwords, uint64_t nbits,
-                                 uint64_t nunits, const uint64_t *end_in, uint64_t *end_out, unsigned int *cnt,
-                                 const uint16_t *bnd, uint64_t *start, int *changed, cudaStream_t st) {
-    DecTables t{td.lut, td.left, td.right, td.sym, td.leaf};
-    k_decode_resync<<<grid_for(nunits, DEC_T), DEC_T, 0, st>>>(t, w32, nwords, nbits, nunits, end_in, end_out, cnt,
-                                                                bnd, start, changed);
+cudaError_t launch_decode_link(const DecodeTablesDev &t, const DecodeString &d, const uint32_t *cend_in,
+                               uint32_t *cend_out, uint32_t *info, unsigned long long *ctot, int *flags,
+                               cudaStream_t st) {
+    const uint64_t ncta = (d.nunits + DEC_T - 1) / DEC_T;
+    auto k = d.unit_words == DEC_LONG ? k_decode_link<DEC_LONG> : k_decode_link<DEC_SHORT>;
+    k<<<grid_for(ncta, 64), 64, 0, st>>>(t, d.w32, d.nwords, d.nbits, d.nunits, ncta, cend_in, cend_out, info, ctot,
+                                          flags);
     return cudaGetLastError();
 }
 
 template <typename C>
-cudaError_t decode_write_impl(const DecodeTablesDev &td, const uint32_t *w32, uint64_t nwords, uint64_t nbits,
-                              uint64_t nunits, const uint64_t *start, const unsigned long long *off, uint64_t nout,
-                              int offset, C *out, cudaStream_t st) {
-    DecTables t{td.lut, td.left, td.right, td.sym, td.leaf};
-    k_decode_write<C><<<grid_for(nunits, DEC_T), DEC_T, 0, st>>>(t, w32, nwords, nbits, nunits, start, off, nout,
-                                                                  offset, out);
+cudaError_t launch_decode_write(const DecodeTablesDev &t, const DecodeString &d, const uint32_t *info,
+                                const unsigned long long *coff, uint64_t nout, int offset, C *out,
+                                unsigned long long *zc, unsigned long long *zstart, cudaStream_t st) {
+    auto k = d.unit_words == DEC_LONG ? k_decode_write<C, DEC_LONG> : k_decode_write<C, DEC_SHORT>;
+    const size_t sm = ((size_t)8 << LUT_BITS) + (size_t)(DEC_WT * d.unit_words + DEC_HALO) * 4 +
+                      (size_t)DEC_WT * DEC_ROWS * 4;
+    cudaError_t e = allow_dynamic_smem((const void *)k);
+    if (e != cudaSuccess) return e;
+    k<<<grid_for(d.nunits, DEC_WT), DEC_WT, sm, st>>>(t, d.w32, d.nwords, d.nunits, info, coff, nout, offset, out, zc,
+                                              zstart);
     return cudaGetLastError();
 }
-cudaError_t launch_decode_write(const DecodeTablesDev &td, const uint32_t *w32, uint64_t nwords, uint64_t nbits,
-                                uint64_t nunits, const uint64_t *start, const unsigned long long *off, uint64_t nout,
-                                int offset, uint16_t *out, cudaStream_t st) {
-    return decode_write_impl(td, w32, nwords, nbits, nunits, start, off, nout, offset, out, st);
-}
-cudaError_t launch_decode_write(const DecodeTablesDev &td, const uint32_t *w32, uint64_t nwords, uint64_t nbits,
-                                uint64_t nunits, const uint64_t *start, const unsigned long long *off, uint64_t nout,
-                                int offset, uint32_t *out, cudaStream_t st) {
-    return decode_write_impl(td, w32, nwords, nbits, nunits, start, off, nout, offset, out, st);
+template cudaError_t launch_decode_write<uint16_t>(const DecodeTablesDev &, const DecodeString &, const uint32_t *,
+                                                   const unsigned long long *, uint64_t, int, uint16_t *,
+                                                   unsigned long long *, unsigned long long *, cudaStream_t);
+template cudaError_t launch_decode_write<uint32_t>(const DecodeTablesDev &, const DecodeString &, const uint32_t *,
+                                                   const unsigned long long *, uint64_t, int, uint32_t *,
+                                                   unsigned long long *, unsigned long long *, cudaStream_t);
+
+uint64_t decode_ranges(uint64_t nunits) { return (nunits + 31) / 32; }
+uint64_t constant_ranges(uint64_t n) { return (n + RANGE - 1) / RANGE; }
+cudaError_t launch_constant_ranges(uint64_t n, bool zero, unsigned long long *zstart, unsigned long long *zcount,
+                                   cudaStream_t st) {
+    k_constant_ranges<<<grid_for(constant_ranges(n), 256), 256, 0, st>>>(n, zero, zstart, zcount);
+    return cudaGetLastError();
 }
 
-__global__ void k_init_starts(uint64_t *start, uint64_t n) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        start[i] = i * DEC_UNIT;
+template <typename C>
+cudaError_t launch_zero_positions(const C *codes, uint64_t n, uint64_t nranges, const unsigned long long *zstart,
+                                  const unsigned long long *zcount, const unsigned long long *zoff, uint64_t cap,
+                                  uint64_t *zpos, cudaStream_t st) {
+    k_zero_positions<C><<<grid_for(nranges, 8), 256, 0, st>>>(codes, n, nranges, zstart, zcount, zoff, cap, zpos);
+    return cudaGetLastError();
 }
-cudaError_t launch_init_starts(uint64_t *start, uint64_t n, cudaStream_t st) {
-    unsigned g = grid_for(n, 1024);
-    if (g > 4096) g = 4096;
-    if (g == 0) g = 1;
-    k_init_starts<<<g, 1024, 0, st>>>(start, n);
+template cudaError_t launch_zero_positions<uint16_t>(const uint16_t *, uint64_t, uint64_t, const unsigned long long *,
+                                                     const unsigned long long *, const unsigned long long *, uint64_t,
+                                                     uint64_t *, cudaStream_t);
+template cudaError_t launch_zero_positions<uint32_t>(const uint32_t *, uint64_t, uint64_t, const unsigned long long *,
+                                                     const unsigned long long *, const unsigned long long *, uint64_t,
+                                                     uint64_t *, cudaStream_t);
+
+// one block: exclusive scan of n totals in place, their sum in v[n]
+cudaError_t launch_scan_small(unsigned long long *v, uint64_t n, cudaStream_t st) {
+    k_scan_top<<<1, 1024, 0, st>>>(v, n);
     return cudaGetLastError();
 }
 
@@ -792,14 +1194,6 @@ cudaError_t launch_fill_u16(uint32_t *out, uint64_t n, uint32_t v, cudaStream_t 
     if (g > 4096) g = 4096;
     if (g == 0) g = 1;
     k_fill_u16<uint32_t><<<g, 1024, 0, st>>>(out, n, v);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_widen_counts(const unsigned int *cnt, unsigned long long *out, uint64_t n, cudaStream_t st) {
-    unsigned g = grid_for(n, 1024);
-    if (g > 4096) g = 4096;
-    if (g == 0) g = 1;
-    k_widen_counts<<<g, 1024, 0, st>>>(cnt, out, n);
     return cudaGetLastError();
 }
 

@@ -234,8 +234,8 @@ int build_codebook(const std::vector<int> &syms, const std::vector<uint64_t> &co
     return FAZ_OK;
 }
 
-// HuffmanEncoder::load (include/QoZ/encoder/HuffmanEncoder.hpp:276-296) plus
-// a 2^kLutBits-entry lookup table for the GPU decoder.
+// HuffmanEncoder::load (include/QoZ/encoder/HuffmanEncoder.hpp:276-296): the
+// tree as the child words that the GPU decoder's tables are built from.
 int parse_tree(const uint8_t *&p, const uint8_t *end, DecodeTablesHost &t, std::string &err) {
     auto need = [&](size_t k) { return (size_t)(end - p) >= k; };
     if (!need(12)) {
@@ -259,54 +259,67 @@ int parse_tree(const uint8_t *&p, const uint8_t *end, DecodeTablesHost &t, std::
     const uint8_t *q = p + 1;
     t.offset = offset;
     t.nodeCount = (int)nc;
-    t.left.assign(nc, 0);
-    t.right.assign(nc, 0);
-    t.sym.assign(nc, 0);
-    t.leaf.assign(nc, 0);
-    for (int pass = 0; pass < 2; pass++) {
-        std::vector<uint32_t> &A = pass ? t.right : t.left;
-        for (uint32_t i = 0; i < nc; i++) {
-            uint32_t v;
-            if (w == 1) v = q[0];
-            else if (w == 2) { uint16_t x; std::memcpy(&x, q, 2); v = x; }
-            else std::memcpy(&v, q, 4);
-            q += w;
-            A[i] = v;
+    const uint8_t *ql = q, *qr = q + (size_t)nc * w, *qs = q + 2 * (size_t)nc * w, *qt = qs + (size_t)nc * 4;
+    auto sym = [&](uint32_t i) {
+        int32_t x;
+        std::memcpy(&x, qs + 4 * (size_t)i, 4);
+        return x;
+    };
+    auto index = [&](const uint8_t *a, uint32_t i) -> uint32_t {
+        if (w == 1) return a[i];
+        if (w == 2) {
+            uint16_t x;
+            std::memcpy(&x, a + 2 * (size_t)i, 2);
+            return x;
         }
-    }
-    std::memcpy(t.sym.data(), q, (size_t)nc * 4);
-    q += (size_t)nc * 4;
-    std::memcpy(t.leaf.data(), q, nc);
+        uint32_t x;
+        std::memcpy(&x, a + 4 * (size_t)i, 4);
+        return x;
+    };
     p += bytes;
     // a tree of more than 256 nodes is rebuilt with an internal root
-    bool root_leaf = nc <= 256 && t.leaf[0];
+    const bool root_leaf = nc <= 256 && qt[0];
     t.constant = root_leaf;
-    t.constant_state = t.sym[0];
+    t.constant_state = sym(0);
     if (root_leaf) return FAZ_OK;
-    t.leaf[0] = 0;
     // children are numbered after their parent (preorder): reject anything
     // else so that every walk ends
+    t.child.assign(2 * (size_t)nc, 0);
     for (uint32_t i = 0; i < nc; i++) {
-        if (t.leaf[i]) continue;
-        if (t.left[i] <= i || t.right[i] <= i || t.left[i] >= nc || t.right[i] >= nc) {
-            err = "malformed Huffman tree";
-            return FAZ_ERR_FORMAT;
+        if (i > 0 && qt[i]) continue;
+        for (int k = 0; k < 2; k++) {
+            const uint32_t c = index(k ? qr : ql, i);
+            if (c <= i || c >= nc) {
+                err = "malformed Huffman tree";
+                return FAZ_ERR_FORMAT;
+            }
+            if (qt[c]) {
+                const int32_t s = sym(c);
+                t.child[2 * (size_t)i + k] = kChildLeaf | (s < 0 ? kChildBad : 0u) | ((uint32_t)s & 0xffffffu);
+            } else {
+                t.child[2 * (size_t)i + k] = c;
+            }
         }
-    }
-    const int K = kLutBits;
-    t.lut.assign((size_t)1 << K, 0);
-    for (uint32_t v = 0; v < (1u << K); v++) {
-        uint32_t nd = 0;
-        int b = 0;
-        for (; b < K; b++) {
-            int bit = (v >> (K - 1 - b)) & 1;
-            nd = bit ? t.right[nd] : t.left[nd];
-            if (t.leaf[nd]) break;
-        }
-        if (b < K) t.lut[v] = ((uint32_t)(b + 1) << 24) | ((uint32_t)t.sym[nd] & 0xffffff);
-        else t.lut[v] = 0x80000000u | nd;
     }
     return FAZ_OK;
+}
+
+uint32_t leaf_depth(const DecodeTablesHost &t, int32_t state) {
+    // children are numbered after their parents: one pass carries the depths down
+    const size_t nc = t.child.size() / 2;
+    std::vector<uint8_t> depth(nc, 0);
+    for (size_t i = 0; i < nc; i++) {
+        for (int k = 0; k < 2; k++) {
+            const uint32_t c = t.child[2 * i + k];
+            const uint8_t d = (uint8_t)std::min(255, depth[i] + 1);
+            if (!(c & kChildLeaf)) {
+                if (c < nc) depth[c] = d;
+            } else if (!(c & kChildBad) && (int32_t)(c & 0xffffffu) == state) {
+                return d <= 64 ? d : 0;
+            }
+        }
+    }
+    return 0;
 }
 
 }  // namespace faz

@@ -127,8 +127,7 @@ cudaError_t launch_count_zeros(const uint16_t *codes, uint64_t n, unsigned long 
 cudaError_t launch_count_zeros(const uint32_t *codes, uint64_t n, unsigned long long *zcount, cudaStream_t st);
 template <typename T, typename C>
 cudaError_t launch_compact_zeros(const C *codes, uint64_t n, const unsigned long long *zcount,
-                                 const unsigned long long *zoff, uint64_t *zpos, const T *scratch, T *vals,
-                                 cudaStream_t st);
+                                 const unsigned long long *zoff, const T *scratch, T *vals, cudaStream_t st);
 uint64_t scan_temp_words(uint64_t n);
 cudaError_t launch_scan_u64(const unsigned long long *in, unsigned long long *out, uint64_t n,
                             unsigned long long *temp, cudaStream_t st);
@@ -144,34 +143,54 @@ cudaError_t launch_encode_pack(const uint32_t *codes, uint64_t n, int offset, co
                                const unsigned long long *packed, const uint8_t *len,
                                const unsigned long long *chunkoff, uint32_t *out, int maxlen, cudaStream_t st);
 
+// Huffman decoder (huffman.cu): the tree as child words (leaf flag | state, or
+// node index), and the tables launch_decode_tables builds from it.
 struct DecodeTablesDev {
-    const uint32_t *lut;
-    const uint32_t *left, *right;
-    const int32_t *sym;
-    const uint8_t *leaf;
+    const uint32_t *child;     // 2 per node
+    uint16_t *lutA;            // 2^kLutBits each
+    uint2 *lutB;
+    uint32_t *lut2;            // decode_lut2_entries each
+    uint8_t *len2;
 };
-uint64_t decode_units(uint64_t nbits);
-uint64_t decode_unit_bits();
-int decode_boundaries();
-cudaError_t launch_init_starts(uint64_t *start, uint64_t n, cudaStream_t st);
-// speculative decode of units [ubase, min(uend, nunits)); ubase a multiple of
-// decode_cta_units()
-uint64_t decode_cta_units();
-cudaError_t launch_decode_spec(const DecodeTablesDev &t, const uint32_t *w32, uint64_t nwords, uint64_t nbits,
-                               uint64_t nunits, uint64_t ubase, uint64_t uend, uint64_t *end, unsigned int *cnt,
-                               uint16_t *bnd, int *err, cudaStream_t st);
-cudaError_t launch_decode_resync(const DecodeTablesDev &t, const uint32_t *w32, uint64_t nwords, uint64_t nbits,
-                                 uint64_t nunits, const uint64_t *end_in, uint64_t *end_out, unsigned int *cnt,
-                                 const uint16_t *bnd, uint64_t *start, int *changed, cudaStream_t st);
-cudaError_t launch_decode_write(const DecodeTablesDev &t, const uint32_t *w32, uint64_t nwords, uint64_t nbits,
-                                uint64_t nunits, const uint64_t *start, const unsigned long long *off, uint64_t nout,
-                                int offset, uint16_t *out, cudaStream_t st);
-cudaError_t launch_decode_write(const DecodeTablesDev &t, const uint32_t *w32, uint64_t nwords, uint64_t nbits,
-                                uint64_t nunits, const uint64_t *start, const unsigned long long *off, uint64_t nout,
-                                int offset, uint32_t *out, cudaStream_t st);
+struct DecodeString {
+    const uint32_t *w32;
+    uint64_t nwords, nbits, nunits;
+    int unit_words;
+    uint64_t run_bits;  // leading bits expected to repeat one codeword of run_len bits (0: none)
+    uint32_t run_len;
+};
+int decode_unit_words(uint64_t nbits);  // words per unit of a string of nbits
+uint64_t decode_cta_units();            // units per CTA of the synchronising pass
+size_t decode_lut2_entries(int nodes);
+template <typename C>
+cudaError_t launch_decode_tables(const DecodeTablesDev &t, int offset, uint32_t *slot_node, unsigned *nslots,
+                                 size_t lut2_entries, cudaStream_t st);
+// synchronising pass over CTAs [cta0, cta1); flags[0] = a CTA end moved (set by
+// the link pass), flags[1] = damaged
+cudaError_t launch_decode_sync(const DecodeTablesDev &t, const DecodeString &d, uint64_t cta0, uint64_t cta1,
+                               uint32_t *info, uint32_t *cend, unsigned long long *ctot, int *flags, cudaStream_t st);
+cudaError_t launch_decode_link(const DecodeTablesDev &t, const DecodeString &d, const uint32_t *cend_in,
+                               uint32_t *cend_out, uint32_t *info, unsigned long long *ctot, int *flags,
+                               cudaStream_t st);
+template <typename C>
+cudaError_t launch_decode_write(const DecodeTablesDev &t, const DecodeString &d, const uint32_t *info,
+                                const unsigned long long *coff, uint64_t nout, int offset, C *out,
+                                unsigned long long *zc, unsigned long long *zstart, cudaStream_t st);
+// the zeros of the decoded codes: first code (zstart) and zero count (zcount) of
+// each of decode_ranges(nunits) ranges, zoff the counts' exclusive scan; the
+// first cap positions, sorted
+uint64_t decode_ranges(uint64_t nunits);
+// the ranges of n equal codes
+uint64_t constant_ranges(uint64_t n);
+cudaError_t launch_constant_ranges(uint64_t n, bool zero, unsigned long long *zstart, unsigned long long *zcount,
+                                   cudaStream_t st);
+template <typename C>
+cudaError_t launch_zero_positions(const C *codes, uint64_t n, uint64_t nranges, const unsigned long long *zstart,
+                                  const unsigned long long *zcount, const unsigned long long *zoff, uint64_t cap,
+                                  uint64_t *zpos, cudaStream_t st);
+cudaError_t launch_scan_small(unsigned long long *v, uint64_t n, cudaStream_t st);
 cudaError_t launch_fill_u16(uint16_t *out, uint64_t n, uint16_t v, cudaStream_t st);
 cudaError_t launch_fill_u16(uint32_t *out, uint64_t n, uint32_t v, cudaStream_t st);
-cudaError_t launch_widen_counts(const unsigned int *cnt, unsigned long long *out, uint64_t n, cudaStream_t st);
 
 // ------------------------------------------------------------ Huffman host
 struct Codebook {
@@ -193,12 +212,14 @@ struct DecodeTablesHost {
     int nodeCount = 0;
     bool constant = false;       // single-symbol stream
     int constant_state = 0;
-    std::vector<uint32_t> lut, left, right;
-    std::vector<int32_t> sym;
-    std::vector<uint8_t> leaf;
+    std::vector<uint32_t> child; // 2 per node: node index, or leaf flag | state (kChildLeaf, kChildBad)
 };
-// Parse HuffmanEncoder::save output at p (advances p); builds decode tables.
+constexpr uint32_t kChildLeaf = 0x80000000u;  // a leaf; its state in the low 24 bits
+constexpr uint32_t kChildBad = 0x40000000u;   // with kChildLeaf: a negative state
+// Parse HuffmanEncoder::save output at p (advances p) into the decode tree.
 int parse_tree(const uint8_t *&p, const uint8_t *end, DecodeTablesHost &t, std::string &err);
+// length of the codeword of `state` (0: none, or longer than 64 bits)
+uint32_t leaf_depth(const DecodeTablesHost &t, int32_t state);
 constexpr int kLutBits = 12;
 
 // -------------------------------------------------------------- stream/io

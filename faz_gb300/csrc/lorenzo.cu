@@ -737,8 +737,8 @@ void lorenzo3_compress_payload(const uint64_t *dims, int bs, int pd, int lo, int
     }
     const uint64_t nunpred = hc.nzero;
     T *unp = m.alloc<T>(nunpred ? nunpred : 1);
-    if (nunpred && wide) launches(launch_compact_zeros<T>(codes32, n, hc.zc, hc.zoff, nullptr, scratch, unp, st));
-    if (nunpred && !wide) launches(launch_compact_zeros<T>(codes16, n, hc.zc, hc.zoff, nullptr, scratch, unp, st));
+    if (nunpred && wide) launches(launch_compact_zeros<T>(codes32, n, hc.zc, hc.zoff, scratch, unp, st));
+    if (nunpred && !wide) launches(launch_compact_zeros<T>(codes16, n, hc.zc, hc.zoff, scratch, unp, st));
     CK(cudaEventRecord(ev_huff.b, st));
     trace_step("lorenzo codebooks built");
     // SZFastFrontend::save: params, precision, meanInfo<T>{false, 0}, reg_count,
@@ -879,15 +879,9 @@ void lorenzo3_decompress(const uint8_t *pl, size_t psize, const uint64_t *dims, 
     uint16_t *codes16 = wide ? nullptr : m.alloc<uint16_t>(n);
     uint32_t *codes32 = wide ? m.alloc<uint32_t>(n) : nullptr;
     uint64_t *zpos = nullptr;
-    uint64_t nz;
-    if (wide) {
-        huffman_decode_device(p, end, n, codes32, m, st, launches);
-        nz = zero_positions(codes32, n, m, st, launches, zpos);
-    } else {
-        huffman_decode_device(p, end, n, codes16, m, st, launches);
-        nz = zero_positions(codes16, n, m, st, launches, zpos);
-    }
-    if (nz != nunpred) throw Fail{FAZ_ERR_FORMAT, "unpredictable count does not match the zero codes"};
+    const uint64_t nz = nunpred;
+    if (wide) decode_with_zeros(p, end, n, nz, codes32, m, st, launches, zpos);
+    else decode_with_zeros(p, end, n, nz, codes16, m, st, launches, zpos);
     CK(cudaEventRecord(ev_dec.b, st));
     LorArgs a = make_args<T>(dims, bs, pd, 1, 1, eb, radius);
     a.rp = drec;

@@ -775,7 +775,7 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
         x.launches(launch_scan_u64(zc, zoff, nsub, ztmp, s));
         const uint64_t nunp = h.nzero;
         T *unp = x.m.alloc<T>(nunp ? nunp : 1);
-        if (nunp) x.launches(launch_compact_zeros<T>(x.codes, ns, zc, zoff, nullptr, x.scratch, unp, s));
+        if (nunp) x.launches(launch_compact_zeros<T>(x.codes, ns, zc, zoff, x.scratch, unp, s));
         std::vector<uint8_t> head;
         put<uint8_t>(head, 2);
         put<double>(head, eb);

@@ -331,7 +331,7 @@ void block_interp_tail(int N, const uint64_t *sdims, double eb, int cubic, int d
     trace_step("trial encode queued");
     const uint64_t nunpred = hc.nzero;
     T *unp = m.alloc<T>(nunpred ? nunpred : 1);
-    if (nunpred) launches(launch_compact_zeros<T>(codes, num, hc.zc, hc.zoff, nullptr, scratch, unp, st));
+    if (nunpred) launches(launch_compact_zeros<T>(codes, num, hc.zc, hc.zoff, scratch, unp, st));
     std::vector<uint8_t> h;
     for (int i = 0; i < N; i++) put<uint64_t>(h, sdims[i]);
     put<uint32_t>(h, (uint32_t)bs);

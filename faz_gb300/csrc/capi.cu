@@ -778,29 +778,33 @@ void compress_dispatch(faz_config &c, const T *dX, cudaStream_t st, uint8_t *&pa
         blocked_payload<T>(c, dX, st, payload, psize, tm, launches, sink);
         return;
     }
+    // the Lorenzo compressors assemble the payload where it is to be
     std::vector<uint8_t> pl;
-    if (c.N < 3) {
-        if (c.regression2)
-            throw Fail{FAZ_ERR_UNSUPPORTED, "ALGO_LORENZO_REG on 1-D / 2-D data is implemented without regression2"};
-        gen_compress_payload<T>(c.N, c.dims, c.blockSize, c.lorenzo, c.lorenzo2, c.regression, c.absErrorBound,
-                                c.quantbinCnt / 2, dX, st, launches, tm, pl);
-    } else {
-        if (c.N != 3 || c.regression2)
-            throw Fail{FAZ_ERR_UNSUPPORTED, "ALGO_LORENZO_REG is implemented for 3-D data without regression2"};
-        lorenzo3_compress_payload<T>(c.dims, c.blockSize, c.pred_dim, c.lorenzo, c.lorenzo2, c.regression,
-                                     c.absErrorBound, c.quantbinCnt / 2, dX, st, launches, tm, pl);
+    PayloadView view;
+    if (sink) {
+        view.dst = sink->dst;
+        view.cap = sink->cap;
     }
-    psize = pl.size();
-    if (sink && sink->dst) {
-        if (psize > sink->cap) {
-            sink->too_small = true;
-            throw Fail{FAZ_ERR_ARG, "payload buffer too small: need " + std::to_string(psize) + " bytes"};
+    {
+        ViewScope scope(&view);
+        if (c.N < 3) {
+            if (c.regression2)
+                throw Fail{FAZ_ERR_UNSUPPORTED, "ALGO_LORENZO_REG on 1-D / 2-D data is implemented without regression2"};
+            gen_compress_payload<T>(c.N, c.dims, c.blockSize, c.lorenzo, c.lorenzo2, c.regression, c.absErrorBound,
+                                    c.quantbinCnt / 2, dX, st, launches, tm, pl);
+        } else {
+            if (c.N != 3 || c.regression2)
+                throw Fail{FAZ_ERR_UNSUPPORTED, "ALGO_LORENZO_REG is implemented for 3-D data without regression2"};
+            lorenzo3_compress_payload<T>(c.dims, c.blockSize, c.pred_dim, c.lorenzo, c.lorenzo2, c.regression,
+                                         c.absErrorBound, c.quantbinCnt / 2, dX, st, launches, tm, pl);
         }
-        payload = sink->dst;
-    } else {
-        payload = t_pin_payload.get(psize + 8);
     }
-    std::memcpy(payload, pl.data(), psize);
+    psize = view.size;
+    if (sink && sink->dst && psize > sink->cap) {
+        sink->too_small = true;
+        throw Fail{FAZ_ERR_ARG, "payload buffer too small: need " + std::to_string(psize) + " bytes"};
+    }
+    payload = const_cast<uint8_t *>(view.data);
 }
 
 // Lossless_zstd::compress framing (include/QoZ/lossless/Lossless_zstd.hpp:22-32),

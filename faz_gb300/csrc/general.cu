@@ -818,7 +818,7 @@ void gen_compress_payload(int N, const uint64_t *dims, int bs, int lo, int lo2, 
     size_t total = 0;
     for (const Part &pt : parts) total += pt.dev ? pt.dev_bytes : pt.host.size();
     // device parts come back through the thread's pinned staging buffer
-    uint8_t *pin = t_pin_payload.get(total + 8);
+    uint8_t *pin = payload_buffer(total);
     uint8_t *o = pin;
     for (const Part &pt : parts) {
         if (pt.dev) {

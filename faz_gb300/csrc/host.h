@@ -149,16 +149,23 @@ struct TableStage {
 };
 inline thread_local TableStage t_table_stage;
 
-// Payload producers assemble their bytes in the thread's pinned staging
-// buffer and end with emit_payload: the bytes are copied into `out`, or, while
-// the thread has a view installed (t_payload_view), left where they are, the
-// view pointing at them until the thread assembles its next payload (a
-// tuning trial only measures its payload's zstd size).
+// Payload producers assemble their bytes in payload_buffer(size) and end with
+// emit_payload: the bytes are copied into `out`, or, while the thread has a view
+// installed (t_payload_view), left where they are, the view pointing at them
+// until the thread assembles its next payload (a tuning trial only measures its
+// payload's zstd size).  The buffer is the thread's pinned staging buffer, or the
+// view's own `dst` (a caller's buffer) when the payload fits its `cap` bytes.
 struct PayloadView {
     const uint8_t *data = nullptr;
     size_t size = 0;
+    uint8_t *dst = nullptr;
+    size_t cap = 0;
 };
 inline thread_local PayloadView *t_payload_view = nullptr;
+inline uint8_t *payload_buffer(size_t n) {
+    if (t_payload_view && t_payload_view->dst && n <= t_payload_view->cap) return t_payload_view->dst;
+    return t_pin_payload.get(n + 8);
+}
 inline void emit_payload(std::vector<uint8_t> &out, const uint8_t *pin, size_t n) {
     if (t_payload_view) {
         t_payload_view->data = pin;
@@ -168,6 +175,11 @@ inline void emit_payload(std::vector<uint8_t> &out, const uint8_t *pin, size_t n
     }
     out.assign(pin, pin + n);
 }
+struct ViewScope {
+    PayloadView *before;
+    explicit ViewScope(PayloadView *v) : before(t_payload_view) { t_payload_view = v; }
+    ~ViewScope() { t_payload_view = before; }
+};
 
 // How a call on device buffers reads a NULL stream: the legacy default
 // stream, so that the call is ordered after the caller's default-stream work

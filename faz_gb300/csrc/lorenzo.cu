@@ -7,11 +7,11 @@
 // per block from the original data), keeping the reconstruction in a slab
 // buffer padded with zeros.  That is the same as predicting from a full
 // reconstructed field that reads as zero before the first plane, row and
-// column, so a block depends only on blocks with smaller or equal block
-// coordinates.  Blocks on one diagonal bi + bj + bk = d are therefore
-// independent: one launch per diagonal, one warp per block.  Inside a block
-// the warp walks the point diagonals i + j + k = s in a shared-memory tile
-// that holds the block and its two-deep halo.
+// column, so a block depends only on its seven neighbours with smaller or equal
+// block coordinates, and a block predicted by regression on none.  One launch of
+// persistent warps takes the blocks diagonal by diagonal (bi + bj + bk), one warp
+// per block.  Inside a Lorenzo block the warp walks the point diagonals
+// i + j + k = s in a shared-memory tile that holds the block and its halo.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -202,140 +202,360 @@ __device__ __forceinline__ void lor_st_release(unsigned *p, unsigned v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-__device__ __forceinline__ unsigned lor_ld_relaxed(const unsigned *p) {
+__device__ __forceinline__ unsigned lor_ld_acquire(const unsigned *p) {
     unsigned v;
-    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
 
-// with a relaxed load that saw a release store before it, an acquire pattern
-__device__ __forceinline__ void lor_fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-
-// The original values of block (bi, bj, bk) into the warp's tile (after its
-// (bs + 2)^3 halo part); they depend on no other block, so the persistent
-// kernel loads them before it waits for the block's neighbours.
-template <typename T>
-__device__ __forceinline__ void lor_load_x(const LorArgs &a, int64_t bi, int64_t bj, int64_t bk, T *t,
-                                           const T *__restrict__ X) {
-    const int lane = threadIdx.x & 31;
+// Extents of block (bi, bj, bk) and its place in the field and the stream.
+struct LorBlock {
+    int sx, sy, sz;
+    int64_t g0;     // element of its first point
+    uint64_t pos0;  // stream position of its first code
+    bool full;
+};
+__device__ __forceinline__ LorBlock lor_geom(const LorArgs &a, int64_t bi, int64_t bj, int64_t bk) {
+    LorBlock b;
     const int bs = a.bs;
-    const int sx = (bi + 1) * bs < a.d1 ? bs : (int)(a.d1 - bi * bs);
-    const int sy = (bj + 1) * bs < a.d2 ? bs : (int)(a.d2 - bj * bs);
-    const int sz = (bk + 1) * bs < a.d3 ? bs : (int)(a.d3 - bk * bs);
-    const int64_t x0 = bi * bs, y0 = bj * bs, z0 = bk * bs;
-    const int64_t d0 = a.d2 * a.d3, dd1 = a.d3;
-    T *xs = t + (bs + 2) * (bs + 2) * (bs + 2);
-    const int nv = sx * sy * sz;
+    b.sx = (bi + 1) * bs < a.d1 ? bs : (int)(a.d1 - bi * bs);
+    b.sy = (bj + 1) * bs < a.d2 ? bs : (int)(a.d2 - bj * bs);
+    b.sz = (bk + 1) * bs < a.d3 ? bs : (int)(a.d3 - bk * bs);
+    const int64_t d0 = a.d2 * a.d3;
+    b.g0 = bi * bs * d0 + bj * bs * a.d3 + bk * bs;
+    b.pos0 = (uint64_t)(bi * bs) * (uint64_t)d0 + (uint64_t)(bj * bs) * (uint64_t)(b.sx * a.d3) +
+             (uint64_t)(bk * bs) * (uint64_t)(b.sx * b.sy);
+    b.full = b.sx == bs && b.sy == bs && b.sz == bs;
+    return b;
+}
+
+// Tables of a full block, built once per CTA: lin[e] = i | j << 4 | k << 8 of
+// linear point e; pts the same of the points by diagonal i + j + k (soff: first
+// of each, then their number); halo[h] = i | j << 4 | k << 8 | tile index << 12 of the halo cells of
+// the (bs + 2)^3 tile, the one-deep ones (coordinates >= 1) first.
+struct LorTables {
+    const uint16_t *lin, *pts, *soff;
+    const uint32_t *halo;
+    int n1, nh;  // one-deep halo cells, all of them
+};
+constexpr int kLorSteps = 3 * kLorMaxBs;
+__host__ __device__ constexpr int lor_table_bytes(int bs) {
+    return (4 * ((bs + 2) * (bs + 2) * (bs + 2) - bs * bs * bs) + 2 * (2 * bs * bs * bs + kLorSteps) + 3) / 4 * 4;
+}
+
+__device__ __forceinline__ LorTables lor_tables(int bs, unsigned char *mem) {
+    __shared__ int cur[kLorSteps], hcur[2];
+    const int n = bs * bs * bs, te = bs + 2, tn = te * te * te;
+    LorTables t;
+    t.n1 = (bs + 1) * (bs + 1) * (bs + 1) - n;
+    t.nh = tn - n;
+    uint32_t *halo = reinterpret_cast<uint32_t *>(mem);
+    uint16_t *lin = reinterpret_cast<uint16_t *>(halo + t.nh), *pts = lin + n, *soff = pts + n;
+    for (int i = threadIdx.x; i < kLorSteps; i += blockDim.x) cur[i] = 0;
+    if (threadIdx.x < 2) hcur[threadIdx.x] = threadIdx.x ? t.n1 : 0;
+    __syncthreads();
+    for (int e = threadIdx.x; e < n; e += blockDim.x) {
+        const int i = e / (bs * bs), j = (e / bs) % bs, k = e % bs;
+        lin[e] = (uint16_t)(i | (j << 4) | (k << 8));
+        atomicAdd(&cur[i + j + k], 1);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int sum = 0;
+        for (int d = 0; d < kLorSteps; d++) {
+            const int c = cur[d];
+            soff[d] = (uint16_t)sum;
+            cur[d] = sum;
+            sum += c;
+        }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < n; e += blockDim.x) {
+        const int v = lin[e];
+        pts[atomicAdd(&cur[(v & 15) + ((v >> 4) & 15) + (v >> 8)], 1)] = (uint16_t)v;
+    }
+    for (int e = threadIdx.x; e < tn; e += blockDim.x) {
+        const int i = e / (te * te), j = (e / te) % te, k = e % te;
+        if (i >= 2 && j >= 2 && k >= 2) continue;
+        const int at = atomicAdd(&hcur[i >= 1 && j >= 1 && k >= 1 ? 0 : 1], 1);
+        halo[at] = (uint32_t)i | ((uint32_t)j << 4) | ((uint32_t)k << 8) | ((uint32_t)e << 12);
+    }
+    __syncthreads();
+    t.lin = lin;
+    t.pts = pts;
+    t.soff = soff;
+    t.halo = halo;
+    return t;
+}
+
+// the code kept in the slot of point e's value
+template <typename T>
+__device__ __forceinline__ unsigned *lor_code(T *xs, int e) {
+    return reinterpret_cast<unsigned *>(xs + e);
+}
+
+// What a block needs of its own, before any neighbour is done: its original
+// values (compression), or its codes (decompression; a load per point diagonal
+// would put a memory round trip on each of the block's steps), in linear order or
+// at slot[e].
+template <typename T, bool DECOMP, typename C>
+__device__ __forceinline__ void lor_load_own(const LorArgs &a, const LorBlock &b, const LorTables &tb,
+                                             const uint16_t *slot, T *xs, const T *__restrict__ X,
+                                             const C *__restrict__ codes) {
+    const int lane = threadIdx.x & 31;
+    const int64_t d0 = a.d2 * a.d3;
+    const int nv = b.sx * b.sy * b.sz;
     for (int e0 = lane; e0 < nv; e0 += 32 * kLorBatch) {
         T v[kLorBatch];
+        unsigned c[kLorBatch];
 #pragma unroll
         for (int u = 0; u < kLorBatch; u++) {
             const int e = e0 + 32 * u;
-            const int i = e / (sy * sz), r = e - i * sy * sz, j = r / sz, k = r - j * sz;
-            v[u] = e < nv ? X[(x0 + i) * d0 + (y0 + j) * dd1 + (z0 + k)] : (T)0;
+            v[u] = 0;
+            c[u] = 0;
+            if (e >= nv) continue;
+            if (DECOMP) {
+                c[u] = codes[b.pos0 + e];
+            } else if (b.full) {
+                const int p = tb.lin[e];
+                v[u] = X[b.g0 + (p & 15) * d0 + ((p >> 4) & 15) * a.d3 + (p >> 8)];
+            } else {
+                const int i = e / (b.sy * b.sz), r = e - i * b.sy * b.sz, j = r / b.sz, k = r - j * b.sz;
+                v[u] = X[b.g0 + i * d0 + j * a.d3 + k];
+            }
         }
 #pragma unroll
-        for (int u = 0; u < kLorBatch; u++)
-            if (e0 + 32 * u < nv) xs[e0 + 32 * u] = v[u];
+        for (int u = 0; u < kLorBatch; u++) {
+            if (e0 + 32 * u >= nv) continue;
+            const int e = slot ? slot[e0 + 32 * u] : e0 + 32 * u;
+            if (DECOMP) *lor_code<T>(xs, e) = c[u];
+            else xs[e] = v[u];
+        }
     }
 }
 
-// One block (bi, bj, bk), one warp: the (bs + 2)^3 tile with its two-deep
-// halo of reconstructed values, then the point diagonals i + j + k = s in
-// order, each point predicted from its reconstructed neighbours (in
-// compression the block's original values are already in the tile:
-// lor_load_x).
-template <typename T, bool DECOMP, int QM, typename C>
-__device__ __forceinline__ void lor_block(const LorArgs &a, int64_t bi, int64_t bj, int64_t bk, T *t, int sel,
-                                          const float (&rp)[4], const uint32_t *halo, T *__restrict__ R,
-                                          C *__restrict__ codes, T *__restrict__ scratch,
-                                          const uint64_t *__restrict__ zpos, uint64_t nzp,
-                                          const T *__restrict__ unpred) {
+// The halo of reconstructed values in the tile: one deep, two for the two-layer
+// predictor; zero outside the field.
+template <typename T>
+__device__ __forceinline__ void lor_load_halo(const LorArgs &a, const LorBlock &b, const LorTables &tb, T *t,
+                                              int64_t bi, int64_t bj, int64_t bk, bool two, const T *__restrict__ R) {
     const int lane = threadIdx.x & 31;
-    const int bs = a.bs;
-    const int sx = (bi + 1) * bs < a.d1 ? bs : (int)(a.d1 - bi * bs);
-    const int sy = (bj + 1) * bs < a.d2 ? bs : (int)(a.d2 - bj * bs);
-    const int sz = (bk + 1) * bs < a.d3 ? bs : (int)(a.d3 - bk * bs);
-    const int64_t x0 = bi * bs, y0 = bj * bs, z0 = bk * bs;
-    const int64_t d0 = a.d2 * a.d3, dd1 = a.d3;
-    // tile strides: (tx, ty, 1) over (sx + 2) x (sy + 2) x (sz + 2)
-    const int tz = sz + 2, ty = tz, tx = (sy + 2) * tz;
-    T *xs = t + (bs + 2) * (bs + 2) * (bs + 2);
-    const int tn = (sx + 2) * (sy + 2) * tz;
+    const int64_t x0 = bi * a.bs, y0 = bj * a.bs, z0 = bk * a.bs, d0 = a.d2 * a.d3;
     // loads in batches of kLorBatch per lane, all issued before any is used
-    if (sx == bs && sy == bs && sz == bs) {
-        // a full block: the halo positions come from the CTA's table
-        const int nh = tn - bs * bs * bs;
+    if (b.full) {
+        const int nh = two ? tb.nh : tb.n1;
         for (int h0 = lane; h0 < nh; h0 += 32 * kLorBatch) {
             T v[kLorBatch];
+            uint32_t q[kLorBatch];
 #pragma unroll
             for (int u = 0; u < kLorBatch; u++) {
                 const int h = h0 + 32 * u;
-                const uint32_t p = h < nh ? halo[h] : 0u;
-                const int64_t gx = x0 + (int)(p & 15u) - 2, gy = y0 + (int)((p >> 4) & 15u) - 2,
-                              gz = z0 + (int)((p >> 8) & 15u) - 2;
-                v[u] = (h < nh && gx >= 0 && gy >= 0 && gz >= 0) ? ld_coherent(R + (gx * d0 + gy * dd1 + gz)) : (T)0;
+                q[u] = h < nh ? tb.halo[h] : 0u;
+                const int i = (int)(q[u] & 15u) - 2, j = (int)((q[u] >> 4) & 15u) - 2, k = (int)((q[u] >> 8) & 15u) - 2;
+                v[u] = (h < nh && x0 + i >= 0 && y0 + j >= 0 && z0 + k >= 0)
+                           ? ld_coherent(R + (b.g0 + i * d0 + j * a.d3 + k))
+                           : (T)0;
             }
 #pragma unroll
-            for (int u = 0; u < kLorBatch; u++) {
-                const int h = h0 + 32 * u;
-                if (h < nh) t[halo[h] >> 12] = v[u];
-            }
+            for (int u = 0; u < kLorBatch; u++)
+                if (h0 + 32 * u < nh) t[q[u] >> 12] = v[u];
         }
-    } else
+        return;
+    }
+    const int tz = b.sz + 2, tx = (b.sy + 2) * tz, tn = (b.sx + 2) * tx, lo = two ? 0 : 1;
     for (int e0 = lane; e0 < tn; e0 += 32 * kLorBatch) {
         T v[kLorBatch];
 #pragma unroll
         for (int u = 0; u < kLorBatch; u++) {
             const int e = e0 + 32 * u;
             const int i = e / tx, r = e - i * tx, j = r / tz, k = r - j * tz;
-            const int64_t gx = x0 + i - 2, gy = y0 + j - 2, gz = z0 + k - 2;
-            const bool inside = i >= 2 && j >= 2 && k >= 2;
-            v[u] = (e < tn && !inside && gx >= 0 && gy >= 0 && gz >= 0) ? ld_coherent(R + (gx * d0 + gy * dd1 + gz))
-                                                                       : (T)0;
+            const bool cell = e < tn && (i < 2 || j < 2 || k < 2) && i >= lo && j >= lo && k >= lo;
+            v[u] = (cell && x0 + i >= 2 && y0 + j >= 2 && z0 + k >= 2)
+                       ? ld_coherent(R + (b.g0 + (i - 2) * d0 + (j - 2) * a.d3 + (k - 2)))
+                       : (T)0;
         }
 #pragma unroll
         for (int u = 0; u < kLorBatch; u++)
             if (e0 + 32 * u < tn) t[e0 + 32 * u] = v[u];
     }
-    __syncwarp();
+}
+
+// One block, one warp: a Lorenzo block's points diagonal by diagonal, each
+// predicted from its reconstructed neighbours in the tile; a regression block's
+// points all at once.
+template <typename T, bool DECOMP, int QM, typename C>
+__device__ __forceinline__ void lor_block(const LorArgs &a, const LorBlock &b, const LorTables &tb, T *t, T *xs,
+                                          int sel, const float (&rp)[4], T *__restrict__ R, C *__restrict__ codes,
+                                          T *__restrict__ scratch, const uint64_t *__restrict__ zpos, uint64_t nzp,
+                                          const T *__restrict__ unpred) {
+    const int lane = threadIdx.x & 31;
+    const int64_t d0 = a.d2 * a.d3;
+    // tile strides: (tx, ty, 1) over (sx + 2) x (sy + 2) x (sz + 2)
+    const int ty = b.sz + 2, tx = (b.sy + 2) * ty;
+    auto point = [&](int i, int j, int k, int e, T pred) -> T {
+        const uint64_t pos = b.pos0 + (uint64_t)e;
+        T v;
+        if (!DECOMP) {
+            v = xs[e];
+            T uval;
+            const int code = quant_point<T, QM>(v, pred, a.q, uval);
+            codes[pos] = (C)code;
+            if (code == 0) scratch[pos] = uval;
+        } else {
+            v = recover_point<T, QM>(pred, (int)*lor_code<T>(xs, e), pos, a.q, zpos, nzp, unpred);
+        }
+        R[b.g0 + i * d0 + j * a.d3 + k] = v;
+        return v;
+    };
+    if (sel == 1) {
+        const int nv = b.sx * b.sy * b.sz;
+        for (int e = lane; e < nv; e += 32) {
+            int i, j, k;
+            if (b.full) {
+                const int p = tb.lin[e];
+                i = p & 15;
+                j = (p >> 4) & 15;
+                k = p >> 8;
+            } else {
+                i = e / (b.sy * b.sz);
+                const int r = e - i * b.sy * b.sz;
+                j = r / b.sz;
+                k = r - j * b.sz;
+            }
+            // regression_predict_quantize_3d (MetaRegressionPredictor.hpp:148-189)
+            point(i, j, k, e, (T)(rp[0] * (float)i + rp[1] * (float)j + rp[2] * (float)k + rp[3]));
+        }
+        return;
+    }
     const bool two = sel == 2;
-    const uint64_t boff = (uint64_t)(bi * bs) * (uint64_t)d0 + (uint64_t)(bj * bs) * (uint64_t)(sx * a.d3) +
-                          (uint64_t)(bk * bs) * (uint64_t)(sx * sy);
-    const int nsteps = sx + sy + sz - 2;
-    const int npairs = sx * sy;
-    // a lane's (i, j) pairs: lane, lane + 32, ... (one pair for edges up to 5)
-    const int i0 = lane / sy, j0 = lane - i0 * sy;
+    const int nsteps = b.sx + b.sy + b.sz - 2;
     for (int s = 0; s < nsteps; s++) {
-        int i = i0, j = j0;
-        for (int pr = lane; pr < npairs; pr += 32) {
-            if (pr != lane) {
-                i = pr / sy;
-                j = pr - i * sy;
-            }
-            const int k = s - i - j;
-            if (k < 0 || k >= sz) continue;
+        for (int q = tb.soff[s] + lane; q < tb.soff[s + 1]; q += 32) {
+            const int p = tb.pts[q], i = p & 15, j = (p >> 4) & 15, k = p >> 8;
+            if (i >= b.sx || j >= b.sy || k >= b.sz) continue;
             T *c = t + (i + 2) * tx + (j + 2) * ty + (k + 2);
-            T pred;
-            if (sel == 1) {
-                // regression_predict_quantize_3d (MetaRegressionPredictor.hpp:148-189)
-                pred = (T)(rp[0] * (float)i + rp[1] * (float)j + rp[2] * (float)k + rp[3]);
-            } else {
-                pred = lor_pred(c, tx, ty, a.pd, two);
+            *c = point(i, j, k, (i * b.sy + j) * b.sz + k, lor_pred(c, tx, ty, a.pd, two));
+        }
+        __syncwarp();
+    }
+}
+
+// Tables of the fast path for full one-layer 3-D Lorenzo blocks of edge BS, whose
+// diagonals have a lane per point; step s of lane l is at 32 * s + l: the point's
+// tile index (at) and its element offset from the block's first point (off, < 0:
+// no point); its value or code is at the same place in xs.
+// slot[e]: the step of linear point e.  The halo cells of a lane, in registers:
+// tile index and element offset, and which of the three neighbours behind they
+// need (a cell outside the field reads zero).
+template <int BS>
+struct LorFast {
+    static constexpr int kSteps = 3 * BS - 2;
+    static constexpr int kSlots = 32 * kSteps;
+    static constexpr int kHalo = ((BS + 1) * (BS + 1) * (BS + 1) - BS * BS * BS + 31) / 32;
+    const int *at, *off;
+    const uint16_t *slot;
+    int hat[kHalo], hoff[kHalo];
+    unsigned hneed[kHalo];
+};
+template <>
+struct LorFast<0> {};
+// bytes of the tables above, and of a warp's values in step order (0: no fast path)
+constexpr bool lor_has_fast(int bs) { return bs == 5 || bs == 6; }
+constexpr int lor_fast_bytes(int bs) {
+    return lor_has_fast(bs) ? 8 * 32 * (3 * bs - 1) + 2 * ((bs * bs * bs + 1) / 2 * 2) : 0;
+}
+constexpr int lor_own(int bs) { return lor_has_fast(bs) ? 32 * (3 * bs - 2) : bs * bs * bs; }
+
+template <int BS>
+__device__ __forceinline__ void lor_fast_tables(const LorArgs &a, const LorTables &tb, unsigned char *mem,
+                                                LorFast<BS> &f) {
+    const int d0 = (int)(a.d2 * a.d3), d1 = (int)a.d3;
+    int *at = reinterpret_cast<int *>(mem), *off = at + 32 * (f.kSteps + 1);
+    uint16_t *slot = reinterpret_cast<uint16_t *>(off + 32 * (f.kSteps + 1));
+    for (int i = threadIdx.x; i < 32 * (f.kSteps + 1); i += blockDim.x) {
+        const int s = i >> 5, q = tb.soff[s] + (i & 31);
+        at[i] = ((BS + 2) * (BS + 2) + BS + 2 + 1) * 2;  // any point of the block
+        off[i] = -1;
+        if (s < f.kSteps && q < tb.soff[s + 1]) {
+            const int p = tb.pts[q], x = p & 15, y = (p >> 4) & 15, z = p >> 8;
+            at[i] = ((x + 2) * (BS + 2) + y + 2) * (BS + 2) + z + 2;
+            off[i] = x * d0 + y * d1 + z;
+            slot[(x * BS + y) * BS + z] = (uint16_t)i;
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < f.kHalo; u++) {
+        const int h = (threadIdx.x & 31) + 32 * u;
+        f.hat[u] = -1;
+        f.hoff[u] = 0;
+        f.hneed[u] = 0;
+        if (h < tb.n1) {
+            const uint32_t q = tb.halo[h];
+            const int x = (int)(q & 15u) - 2, y = (int)((q >> 4) & 15u) - 2, z = (int)((q >> 8) & 15u) - 2;
+            f.hat[u] = (int)(q >> 12);
+            f.hoff[u] = x * d0 + y * d1 + z;
+            f.hneed[u] = (x < 0 ? 1u : 0u) | (y < 0 ? 2u : 0u) | (z < 0 ? 4u : 0u);
+        }
+    }
+    f.at = at;
+    f.off = off;
+    f.slot = slot;
+    __syncthreads();
+}
+
+// One such block: a step is the seven neighbours, the prediction, the quantiser
+// and two stores, everything else read a step ahead.  No lane branches away (a
+// lane without a point computes on another's and stores nothing).  The loop is
+// not unrolled: straight-line code for 16 steps misses the instruction cache
+// (2.6 ms for the wavefront of a 100x500x500 field without regression, 1.8 ms this
+// way).
+template <typename T, bool DECOMP, int QM, int BS>
+__device__ __forceinline__ void lor_full(const LorArgs &a, const LorBlock &b, const LorFast<BS> &f, T *t, T *xs,
+                                         T *__restrict__ R, T *__restrict__ scratch,
+                                         const uint64_t *__restrict__ zpos, uint64_t nzp,
+                                         const T *__restrict__ unpred) {
+    constexpr int ty = BS + 2, tx = ty * ty;
+    const int lane = threadIdx.x & 31;
+    const int *at = f.at + lane, *off = f.off + lane;
+    T *x = xs + lane, *r0 = R + b.g0;
+    int an = at[0], on = off[0];
+    T xn = x[0];
+#pragma unroll 1
+    for (int s = 0; s < f.kSteps; s++) {
+        T *c = t + an;
+        const int o = on;
+        T v = xn;
+        T pred = c[-1] + c[-ty] + c[-tx] - c[-ty - 1] - c[-tx - 1] - c[-tx - ty] + c[-tx - ty - 1];
+        an = at[32 * s + 32];
+        on = off[32 * s + 32];
+        if (s + 1 < f.kSteps) xn = x[32 * s + 32];
+        if (!DECOMP) {
+            if (o < 0) v = pred = (T)0;
+            T uval;
+            const int code = quant_point<T, QM>(v, pred, a.q, uval);
+            *lor_code<T>(x, 32 * s) = (unsigned)code;
+            // positions in the unpredictable values: the e-th of the block
+            if (o >= 0 && code == 0) {
+                const int d0 = (int)(a.d2 * a.d3), d1 = (int)a.d3, i = o / d0, j = (o - i * d0) / d1;
+                scratch[b.pos0 + (i * BS + j) * BS + (o - i * d0 - j * d1)] = uval;
             }
-            const uint64_t pos = boff + (uint64_t)((i * sy + j) * sz + k);
-            T v;
-            if (!DECOMP) {
-                v = xs[(i * sy + j) * sz + k];
-                T uval;
-                const int code = quant_point<T, QM>(v, pred, a.q, uval);
-                codes[pos] = (C)code;
-                if (code == 0) scratch[pos] = uval;
-            } else {
-                v = recover_point<T, QM>(pred, (int)codes[pos], pos, a.q, zpos, nzp, unpred);
+        } else {
+            unsigned code;
+            std::memcpy(&code, &v, 4);
+            if (o < 0) {
+                code = (unsigned)a.q.radius;
+                pred = (T)0;
             }
+            uint64_t pos = b.pos0;
+            if (code == 0) {
+                const int d0 = (int)(a.d2 * a.d3), d1 = (int)a.d3, i = o / d0, j = (o - i * d0) / d1;
+                pos += (i * BS + j) * BS + (o - i * d0 - j * d1);
+            }
+            v = recover_point<T, QM>(pred, (int)code, pos, a.q, zpos, nzp, unpred);
+        }
+        if (o >= 0) {
             *c = v;
-            R[(x0 + i) * d0 + (y0 + j) * dd1 + (z0 + k)] = v;
+            r0[o] = v;
         }
         __syncwarp();
     }
@@ -344,40 +564,42 @@ __device__ __forceinline__ void lor_block(const LorArgs &a, int64_t bi, int64_t 
 constexpr unsigned kLorWaitLimit = 1u << 22;  // polls (with back-off) of a block's neighbours before giving up
 
 // The whole wavefront in one launch of persistent CTAs.  A warp takes a
-// ticket, and with it the block order[ticket]: blocks come diagonal by
-// diagonal (bi + bj + bk ascending), so the blocks a block reads - its face
-// neighbours (bi-1, bj, bk), (bi, bj-1, bk), (bi, bj, bk-1), which in turn
-// waited for theirs - hold smaller tickets, taken by warps already running,
-// and every wait ends.  Each wait is bounded all the same (error flag, then
-// the block runs).  A finished block publishes done[b] = 1 with release
-// semantics after its reconstruction is written.
-template <typename T, bool DECOMP, int QM, typename C>
-__global__ void __launch_bounds__(kLorWarps * 32)
+// ticket, and with it the block order[ticket]: blocks come diagonal by diagonal
+// (bi + bj + bk ascending).  A Lorenzo block waits for the seven neighbours it
+// reads; they hold smaller tickets, taken by warps already running, so every
+// wait ends.  A regression block reads none and waits for none.  Each wait is
+// bounded all the same (error flag, then the block runs).  A finished block
+// publishes done[b] = 1 with release semantics after its reconstruction is
+// written.
+//
+// Bound by the latency of the longest chain of Lorenzo blocks (up to the 185
+// diagonals of the 17 x 84 x 84 blocks of a 100x500x500 field), so what is on a
+// block's path counts.  A diagonal of points is one step, a lane per point (27 at
+// most for edge 6; a lane per (i, j) pair took two steps); the halo is one deep
+// unless the two-layer predictor reads it; values and codes are on the SM before
+// the wait; neighbours are polled with acquire loads and the flag is one release
+// store after a warp barrier (a fence per lane on either side took 1,050 cycles
+// each); codes are written after the flag.  The wavefront of that field with
+// regression: 3.18 -> 1.45 ms, 3.49 -> 1.37 ms in decompression; a block on the
+// path takes 8,000 cycles for its 16 steps, 1,750 for the halo, 1,150 to publish.
+// BS: the block edge of lor_full's path, 0 for other edges.
+template <typename T, bool DECOMP, int QM, typename C, int BS>
+__global__ void __launch_bounds__(kLorWarps * 32, 2)
     k_lor_persist(LorArgs a, const uint32_t *__restrict__ order, uint32_t nblocks, unsigned *counter,
                   unsigned *done, int *err, const T *__restrict__ X, T *__restrict__ R,
                   C *__restrict__ codes, T *__restrict__ scratch, const uint16_t *__restrict__ ind,
                   const uint64_t *__restrict__ zpos, uint64_t nzp, const T *__restrict__ unpred) {
     extern __shared__ __align__(16) unsigned char lor_smem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int bs = a.bs;
-    const int tstride = (bs + 2) * (bs + 2) * (bs + 2) + (DECOMP ? 0 : bs * bs * bs);
+    const int bs = BS ? BS : a.bs;
+    const int tile = (bs + 2) * (bs + 2) * (bs + 2), tstride = tile + (BS ? lor_own(BS) : bs * bs * bs);
     T *t = reinterpret_cast<T *>(lor_smem) + (size_t)w * (size_t)tstride;
-    // The halo positions of a full block's tile (i < 2, j < 2 or k < 2 in the
-    // (bs + 2)^3 tile), packed i | j << 4 | k << 8 | tile index << 12, in tile
-    // order: entry = tile index - interior points before it.
-    uint32_t *halo = reinterpret_cast<uint32_t *>(lor_smem + (size_t)kLorWarps * (size_t)tstride * sizeof(T));
-    {
-        const int te = bs + 2, tn = te * te * te;
-        for (int e = threadIdx.x; e < tn; e += blockDim.x) {
-            const int i = e / (te * te), j = (e / te) % te, k = e % te;
-            if (i >= 2 && j >= 2 && k >= 2) continue;
-            int before = (i > 2 ? i - 2 : 0) * bs * bs;
-            if (i >= 2) before += (j > 2 ? j - 2 : 0) * bs;
-            if (i >= 2 && j >= 2) before += k > 2 ? k - 2 : 0;
-            halo[e - before] = (uint32_t)i | ((uint32_t)j << 4) | ((uint32_t)k << 8) | ((uint32_t)e << 12);
-        }
-        __syncthreads();
-    }
+    T *xs = t + tile;
+    const LorTables tb = lor_tables(bs, lor_smem + (size_t)kLorWarps * (size_t)tstride * sizeof(T));
+    LorFast<BS> f;
+    if constexpr (BS != 0)
+        lor_fast_tables<BS>(a, tb,
+                            lor_smem + (size_t)kLorWarps * (size_t)tstride * sizeof(T) + (size_t)lor_table_bytes(bs), f);
     const int64_t plane = a.ny * a.nz;
     // A warp takes its next ticket as it starts a block, so that the atomic's
     // round trip overlaps the block.  The smallest unfinished ticket is then
@@ -391,42 +613,77 @@ __global__ void __launch_bounds__(kLorWarps * 32)
         if (lane == 0) nxt = atomicAdd(counter, 1u);
         const int64_t b = order[tk];
         const int64_t bk = b % a.nz, bj = (b / a.nz) % a.ny, bi = b / plane;
-        const unsigned *deps[3] = {bi > 0 ? done + (b - plane) : nullptr, bj > 0 ? done + (b - a.nz) : nullptr,
-                                   bk > 0 ? done + (b - 1) : nullptr};
-        // the block's own values, its predictor selection and regression
+        const LorBlock g = lor_geom(a, bi, bj, bk);
+        // the block's own values or codes, its predictor selection and regression
         // coefficients need no neighbour: their loads overlap the wait
-        if (!DECOMP) lor_load_x<T>(a, bi, bj, bk, t, X);
         int sel = ind[b];
+        if (sel == 1 && a.rp == nullptr) sel = 0;  // a stream without coefficients
+        const bool fast = BS != 0 && g.full && sel == 0 && a.pd == 3;
+        const uint16_t *slot = nullptr;
+        if constexpr (BS != 0) slot = fast ? f.slot : nullptr;
+        lor_load_own<T, DECOMP, C>(a, g, tb, slot, xs, X, codes);
         float rp[4] = {0, 0, 0, 0};
-        if (sel == 1) {
-            if (a.rp == nullptr) sel = 0;  // a stream without coefficients
-            else
-                for (int c = 0; c < 4; c++) rp[c] = a.rp[4 * b + c];
-        }
-        // every lane polls the (up to three) neighbours' flags together with
-        // relaxed loads; the fence after all are seen set orders the halo
-        // loads after the neighbours' writes
-        {
+        if (sel == 1)
+            for (int c = 0; c < 4; c++) rp[c] = a.rp[4 * b + c];
+        if (sel != 1) {
+            // lanes 0..6 poll one neighbour each.  (Blocks of edge 1 read two
+            // blocks back with two layers: those were done before the neighbour,
+            // which waited for its own.)
+            const int m = lane + 1;
+            const int64_t di = m & 1, dj = (m >> 1) & 1, dk = (m >> 2) & 1;
+            const unsigned *dep =
+                lane < 7 && bi >= di && bj >= dj && bk >= dk ? done + (b - di * plane - dj * a.nz - dk) : nullptr;
             unsigned it = 0;
-            for (;;) {
-                const unsigned f0 = deps[0] ? lor_ld_relaxed(deps[0]) : 1u;
-                const unsigned f1 = deps[1] ? lor_ld_relaxed(deps[1]) : 1u;
-                const unsigned f2 = deps[2] ? lor_ld_relaxed(deps[2]) : 1u;
-                if (__all_sync(0xffffffffu, f0 != 0u && f1 != 0u && f2 != 0u)) break;
+            while (!__all_sync(0xffffffffu, dep ? lor_ld_acquire(dep) != 0u : true)) {
                 if (++it > kLorWaitLimit) {
                     if (lane == 0) atomicExch(err, 1);
                     break;
                 }
-                __nanosleep(32);
+                __nanosleep(20);
             }
-            lor_fence_acq_rel();
+            __syncwarp();
+            if constexpr (BS != 0) {
+                if (fast) {
+                    const unsigned none = (bi > 0 ? 0u : 1u) | (bj > 0 ? 0u : 2u) | (bk > 0 ? 0u : 4u);
+                    const T *r0 = R + g.g0;
+                    T v[LorFast<BS>::kHalo];
+#pragma unroll
+                    for (int u = 0; u < LorFast<BS>::kHalo; u++)
+                        v[u] = f.hat[u] >= 0 && !(f.hneed[u] & none) ? ld_coherent(r0 + f.hoff[u]) : (T)0;
+#pragma unroll
+                    for (int u = 0; u < LorFast<BS>::kHalo; u++)
+                        if (f.hat[u] >= 0) t[f.hat[u]] = v[u];
+                }
+            }
+            if (!fast) lor_load_halo<T>(a, g, tb, t, bi, bj, bk, sel == 2, R);
         }
-        lor_block<T, DECOMP, QM, C>(a, bi, bj, bk, t, sel, rp, halo, R, codes, scratch, zpos, nzp, unpred);
-        // each lane's reconstruction writes are released before the warp's flag
-        lor_fence_acq_rel();
+        __syncwarp();
+        if constexpr (BS != 0) {
+            if (fast) lor_full<T, DECOMP, QM, BS>(a, g, f, t, xs, R, scratch, zpos, nzp, unpred);
+        }
+        if (!fast)
+            lor_block<T, DECOMP, QM, C>(a, g, tb, t, xs, sel, rp, R, codes, scratch, zpos, nzp, unpred);
+        // the barrier orders every lane's reconstruction writes before lane 0's
+        // release store
         __syncwarp();
         if (lane == 0) lor_st_release(done + b, 1u);
+        if constexpr (BS != 0 && !DECOMP) {
+            if (fast)
+                for (int e = lane; e < BS * BS * BS; e += 32)
+                    codes[g.pos0 + e] = (C)*lor_code<T>(xs, f.slot[e]);
+        }
+        __syncwarp();
     }
+}
+
+// Blocks in diagonal order (any order inside a diagonal): base[d] the first place
+// of diagonal d, cnt[d] (zeroed) its places taken.
+__global__ void __launch_bounds__(256) k_lor_order(uint32_t nb, uint32_t ny, uint32_t nz,
+                                                  const uint32_t *__restrict__ base, unsigned *cnt, uint32_t *order) {
+    const uint32_t b = blockIdx.x * 256u + threadIdx.x;
+    if (b >= nb) return;
+    const uint32_t d = b % nz + (b / nz) % ny + b / nz / ny;
+    order[base[d] + atomicAdd(cnt + d, 1u)] = b;
 }
 
 template <typename T>
@@ -461,53 +718,67 @@ const int *launch_wavefront(const LorArgs &a, bool decomp, const T *X, T *R, C *
                             const uint16_t *ind, const uint64_t *zpos, uint64_t nz, const T *unpred, cudaStream_t st,
                             Counter &launches) {
     const bool straight = sizeof(T) == 4 && a.q.fast;
-    // the warps' tiles, then the halo table (4 bytes per halo position)
+    // element offsets of the fast path are 32-bit
+    const bool fast_bs = lor_has_fast(a.bs) && a.d1 * a.d2 * a.d3 < ((int64_t)1 << 31);
+    // the warps' tiles and own values, then the CTA's tables
     const size_t smem = (size_t)kLorWarps *
-                            (size_t)((a.bs + 2) * (a.bs + 2) * (a.bs + 2) + (decomp ? 0 : a.bs * a.bs * a.bs)) *
-                            sizeof(T) +
-                        (size_t)((a.bs + 2) * (a.bs + 2) * (a.bs + 2) - a.bs * a.bs * a.bs) * 4;
+                            (size_t)((a.bs + 2) * (a.bs + 2) * (a.bs + 2) + (fast_bs ? lor_own(a.bs) : a.bs * a.bs * a.bs)) * sizeof(T) +
+                        (size_t)lor_table_bytes(a.bs) + (size_t)lor_fast_bytes(fast_bs ? a.bs : 0);
     void (*k)(LorArgs, const uint32_t *, uint32_t, unsigned *, unsigned *, int *, const T *, T *, C *, T *,
               const uint16_t *, const uint64_t *, uint64_t, const T *);
-    if (!decomp) k = straight ? k_lor_persist<T, false, 1, C> : k_lor_persist<T, false, 0, C>;
-    else k = straight ? k_lor_persist<T, true, 1, C> : k_lor_persist<T, true, 0, C>;
+    // edges 6 (Config's 3-D default) and 5 (the tuner's trial) have lor_full's path
+#define FAZ_LOR_PICK(BS)                                                                                \
+    if (!decomp) k = straight ? k_lor_persist<T, false, 1, C, BS> : k_lor_persist<T, false, 0, C, BS>; \
+    else k = straight ? k_lor_persist<T, true, 1, C, BS> : k_lor_persist<T, true, 0, C, BS>;
+    if (fast_bs && a.bs == 6) {
+        FAZ_LOR_PICK(6)
+    } else if (fast_bs && a.bs == 5) {
+        FAZ_LOR_PICK(5)
+    } else {
+        FAZ_LOR_PICK(0)
+    }
+#undef FAZ_LOR_PICK
     CK(allow_dynamic_smem((const void *)k));
     const uint64_t nb64 = (uint64_t)(a.nx * a.ny * a.nz);
     if (nb64 >= (1ull << 32)) throw Fail{FAZ_ERR_UNSUPPORTED, "too many Lorenzo blocks"};
     const uint32_t nb = (uint32_t)nb64;
-    // blocks in diagonal order (bi + bj + bk ascending, then bi, then bj)
-    std::vector<uint32_t> order;
-    order.reserve(nb);
-    const int64_t last = (a.nx - 1) + (a.ny - 1) + (a.nz - 1);
-    size_t widest = 0;  // blocks on the longest diagonal: the most that are ever ready at once
-    for (int64_t d = 0; d <= last; d++) {
-        const size_t before = order.size();
-        const int64_t bi_lo = std::max<int64_t>(0, d - (a.ny - 1) - (a.nz - 1));
-        const int64_t bi_hi = std::min<int64_t>(a.nx - 1, d);
-        for (int64_t bi = bi_lo; bi <= bi_hi; bi++) {
-            const int64_t r = d - bi;
-            const int64_t bj_lo = std::max<int64_t>(0, r - (a.nz - 1)), bj_hi = std::min<int64_t>(a.ny - 1, r);
-            for (int64_t bj = bj_lo; bj <= bj_hi; bj++)
-                order.push_back((uint32_t)((bi * a.ny + bj) * a.nz + (r - bj)));
-        }
-        widest = std::max(widest, order.size() - before);
-    }
-    if (order.size() != nb) throw Fail{FAZ_ERR_DEVICE, "Lorenzo block order does not cover the blocks"};
+    // blocks per diagonal bi + bj + bk = d: the pairs (bj, bk) of each sum, added
+    // over a window of nx sums
+    const int64_t nd = a.nx + a.ny + a.nz - 2, np = a.ny + a.nz - 1;
+    auto pairs = [&](int64_t s) -> int64_t {
+        return s < 0 || s >= np ? 0 : std::min(std::min(s + 1, np - s), std::min(a.ny, a.nz));
+    };
     DevMem m(st);
-    uint32_t *dorder = m.alloc<uint32_t>(nb);
-    unsigned *sync = m.alloc<unsigned>((size_t)nb + 2);  // counter, done[nb]
-    int *derr = m.alloc<int>(1);
-    CK(cudaMemcpyAsync(dorder, order.data(), (size_t)nb * 4, cudaMemcpyHostToDevice, st));
-    CK(cudaMemsetAsync(sync, 0, ((size_t)nb + 2) * 4, st));
-    CK(cudaMemsetAsync(derr, 0, 4, st));
+    TableStage &ts = t_table_stage;
+    uint32_t *hbase = (uint32_t *)ts.acquire((size_t)nd * 4);
+    int64_t in_diag = 0, total = 0, widest = 0;
+    for (int64_t d = 0; d < nd; d++) {
+        in_diag += pairs(d) - pairs(d - a.nx);
+        hbase[d] = (uint32_t)total;
+        total += in_diag;
+        widest = std::max(widest, in_diag);
+    }
+    if (total != (int64_t)nb) throw Fail{FAZ_ERR_DEVICE, "Lorenzo block order does not cover the blocks"};
+    // zeroed: counter, done[nb], error flag, places taken per diagonal
+    unsigned *sync = m.alloc<unsigned>((size_t)nb + 2 + (size_t)nd);
+    int *derr = (int *)(sync + 1 + nb);
+    unsigned *taken = sync + 2 + nb;
+    uint32_t *dorder = m.alloc<uint32_t>((size_t)nb + (size_t)nd), *dbase = dorder + nb;
+    CK(cudaMemcpyAsync(dbase, hbase, (size_t)nd * 4, cudaMemcpyHostToDevice, st));
+    ts.release(st);
+    CK(cudaMemsetAsync(sync, 0, ((size_t)nb + 2 + (size_t)nd) * 4, st));
+    k_lor_order<<<(unsigned)((nb64 + 255) / 256), 256, 0, st>>>(nb, (uint32_t)a.ny, (uint32_t)a.nz, dbase, taken, dorder);
+    launches(cudaGetLastError());
     int dev = 0, sms = 0, per_sm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kLorWarps * 32, smem));
     if (per_sm < 1) throw Fail{FAZ_ERR_UNSUPPORTED, "Lorenzo block does not fit on an SM"};
-    // never more CTAs than stay resident (waits rely on it), nor more warps than
-    // blocks on the widest diagonal: more would only wait, and hold SMs that
-    // concurrent work (the tuner's other trials) needs
-    const uint64_t want = (widest + kLorWarps - 1) / kLorWarps;
+    // never more CTAs than stay resident (waits rely on it), nor, when every block
+    // waits for its neighbours, more warps than blocks on the widest diagonal: more
+    // would only wait, and hold SMs that concurrent work (the tuner's other trials)
+    // needs.  With regression blocks most tickets run at once.
+    const uint64_t want = ((a.rp ? (uint64_t)nb : (uint64_t)widest) + kLorWarps - 1) / kLorWarps;
     const int grid = (int)std::min<uint64_t>((uint64_t)sms * (uint64_t)per_sm, want);
     k<<<grid, kLorWarps * 32, smem, st>>>(a, dorder, nb, sync, sync + 1, derr, X, R, codes, scratch, ind, zpos, nz,
                                           unpred);
@@ -769,7 +1040,7 @@ void lorenzo3_compress_payload(const uint64_t *dims, int bs, int pd, int lo, int
         h0.size() + hi.nbytes + hreg.size() + rbits + h1.size() + nunpred * sizeof(T) + h2.size() + hc.nbytes;
     // device parts come back through the thread's pinned staging buffer
     // (copies to pageable memory serialise with other threads' copies)
-    uint8_t *pin = t_pin_payload.get(total + 8);
+    uint8_t *pin = payload_buffer(total);
     uint8_t *p = pin;
     std::memcpy(p, h0.data(), h0.size());
     p += h0.size();

@@ -380,10 +380,7 @@ struct Trial {
             pl.clear();
             // the payload stays in the thread's pinned staging buffer
             PayloadView view;
-            struct ViewScope {
-                explicit ViewScope(PayloadView *v) { t_payload_view = v; }
-                ~ViewScope() { t_payload_view = nullptr; }
-            } scope(&view);
+            ViewScope scope(&view);
             bool reported = false;
             size_t early = 0;
             auto report = [&](size_t n) {

@@ -66,53 +66,95 @@ std::vector<int> map_iteration_order(const std::vector<int> &keys) {
 }
 
 // Binary min-heap on freq with the reference's sift rules (qinsert stops on
-// parent <= new, qremove descends to the smaller child while parent > child).
-// Entries carry their node's frequency, so comparisons touch the heap array
-// alone.
+// parent <= new, qremove descends to the smaller child, the left one of equals,
+// while parent > child), which decide between equal counts and so shape the tree.
+// An entry is one word, freq << kNodeBits | node: siblings share a cache line, and
+// a.freq < b.freq is a < (b with its node bits cleared).  The whole codebook of a
+// 65,000-symbol alphabet (float64 at a tight bound) takes 6.9 ms on a Grace core,
+// 5 ms of it here: 13.1 ms with 16-byte entries, an exit test on each level and a
+// comparison sort of the first positions.
 struct Heap {
-    struct E {
-        uint64_t freq;
-        int node;
-    };
-    std::vector<E> q;  // 1-based
-    explicit Heap(size_t cap) {
-        q.reserve(cap + 1);
-        q.push_back({0, -1});
-    }
+    static constexpr int kNodeBits = 19;  // below 2^19 nodes (2^18 + 1 symbols), counts below 2^45
+    static constexpr uint64_t kNode = ((uint64_t)1 << kNodeBits) - 1;
+    std::vector<uint64_t> q;  // 1-based; room for a sibling past the last entry
+    size_t n = 0;
+    explicit Heap(size_t cap) : q(cap + 3) {}
     void insert(int nd, uint64_t fn) {
-        q.push_back({fn, nd});
-        size_t i = q.size() - 1, j;
+        const uint64_t x = fn << kNodeBits | (uint64_t)nd;
+        size_t i = ++n, j;
         while ((j = i >> 1)) {
-            if (q[j].freq <= fn) break;
+            if (!((fn << kNodeBits) < (q[j] & ~kNode))) break;
             q[i] = q[j];
             i = j;
         }
-        q[i] = {fn, nd};
+        q[i] = x;
     }
-    int remove() {
-        const int top = q[1].node;
-        const E last = q.back();
-        q.pop_back();
-        const size_t end = q.size();
-        if (end > 1) {
-            q[1] = last;
-            // the element moved to the top sinks; the choice of the smaller
-            // child is unpredictable, so it is computed without a branch
+    int remove(uint64_t &freq) {
+        const uint64_t top = q[1];
+        freq = top >> kNodeBits;
+        const uint64_t x = q[n--];
+        if (n > 0) {
+            // The last entry x sinks from the top along the path of smaller
+            // children, past those smaller than itself.  Their counts do not
+            // decrease down the path, so the whole path moves up first (a fixed
+            // number of steps, the choice of child without a branch) and x climbs
+            // back to its place, which is near the bottom.
             size_t i = 1, l;
-            const E x = q[1];
-            while ((l = i << 1) < end) {
-                const size_t r = l + 1 < end ? l + 1 : l;
-                l += (size_t)(q[r].freq < q[l].freq);
-                if (!(x.freq > q[l].freq)) break;
+            while ((l = i << 1) < n) {
+                l += (size_t)(q[l + 1] < (q[l] & ~kNode));
+                q[i] = q[l];
+                i = l;
+            }
+            if (l == n) {
+                q[i] = q[l];
+                i = l;
+            }
+            const uint64_t xf = x & ~kNode;
+            while ((l = i >> 1) && !(q[l] < xf)) {
                 q[i] = q[l];
                 i = l;
             }
             q[i] = x;
         }
-        return top;
+        return (int)(top & kNode);
     }
-    size_t size() const { return q.size() - 1; }
 };
+
+// Indices 0 .. v.size() - 1 in ascending order of v (distinct values): a radix
+// sort by 11-bit digits, or std::sort where that is shorter.
+std::vector<int> order_of(const std::vector<uint64_t> &v) {
+    const size_t n = v.size();
+    struct E {
+        uint64_t key;
+        int index;
+    };
+    std::vector<E> a(n);
+    uint64_t all = 0;
+    for (size_t i = 0; i < n; i++) {
+        a[i] = {v[i], (int)i};
+        all |= v[i];
+    }
+    if (n < 512) {
+        std::sort(a.begin(), a.end(), [](const E &x, const E &y) { return x.key < y.key; });
+    } else {
+        std::vector<E> b(n);
+        for (int sh = 0; sh < 64 && (all >> sh) != 0; sh += 11) {
+            uint32_t at[2048] = {0};
+            for (const E &e : a) at[(e.key >> sh) & 2047]++;
+            uint32_t sum = 0;
+            for (uint32_t &c : at) {
+                const uint32_t k = c;
+                c = sum;
+                sum += k;
+            }
+            for (const E &e : a) b[at[(e.key >> sh) & 2047]++] = e;
+            a.swap(b);
+        }
+    }
+    std::vector<int> o(n);
+    for (size_t i = 0; i < n; i++) o[i] = a[i].index;
+    return o;
+}
 
 template <typename W>
 void put_le(std::vector<uint8_t> &o, W v) {
@@ -132,11 +174,13 @@ int build_codebook(const std::vector<int> &syms, const std::vector<uint64_t> &co
     }
     // distinct symbols in order of first occurrence = map insertion order
     // (first positions are distinct stream positions)
-    std::vector<std::pair<uint64_t, int>> byfirst(d);
-    for (size_t i = 0; i < d; i++) byfirst[i] = {first[i], (int)i};
-    std::sort(byfirst.begin(), byfirst.end());
+    if (d >= (size_t)1 << (Heap::kNodeBits - 1)) {
+        err = "too many Huffman symbols";
+        return FAZ_ERR_UNSUPPORTED;
+    }
+    const std::vector<int> byfirst = order_of(first);
     std::vector<int> keys(d);
-    for (size_t i = 0; i < d; i++) keys[i] = syms[byfirst[i].second];
+    for (size_t i = 0; i < d; i++) keys[i] = syms[byfirst[i]];
     std::vector<int> ord = map_iteration_order(keys);
     int mn = *std::min_element(syms.begin(), syms.end());
     int mx = *std::max_element(syms.begin(), syms.end());
@@ -146,27 +190,25 @@ int build_codebook(const std::vector<int> &syms, const std::vector<uint64_t> &co
     // a merged node's children always have smaller indices
     const size_t nn = 2 * d - 1;
     std::vector<int> left(nn, -1), right(nn, -1), state(d);
-    std::vector<uint64_t> freq(nn);
-    Heap h(nn);
+    Heap h(d);
     for (size_t k = 0; k < d; k++) {
-        const int si = byfirst[ord[k]].second;
-        freq[k] = counts[si];
+        const int si = byfirst[ord[k]];
         state[k] = syms[si] - mn;
-        h.insert((int)k, freq[k]);
+        h.insert((int)k, counts[si]);
     }
     size_t next = d;
-    while (h.size() > 1) {
+    while (h.n > 1) {
         // the reference evaluates new_node(0, 0, qremove(), qremove()) right
         // to left: the first node removed is the right child
-        const int b = h.remove();
-        const int a = h.remove();
+        uint64_t fa, fb;
+        const int b = h.remove(fb);
+        const int a = h.remove(fa);
         left[next] = a;
         right[next] = b;
-        freq[next] = freq[a] + freq[b];
-        h.insert((int)next, freq[next]);
+        h.insert((int)next, fa + fb);
         next++;
     }
-    const int root = h.q[1].node;
+    const int root = (int)nn - 1;  // the last node merged
     // code lengths and bits (left 0, right 1), parents before children
     std::vector<uint8_t> len(nn, 0);
     std::vector<uint64_t> bits(nn, 0);

@@ -39,6 +39,7 @@ struct LevelPlan {
     LevelArgs args;
     int64_t nblocks;
     uint64_t off_index;  // first entry of this level in the block-offset table
+    uint64_t pos;        // stream position of its first code
 };
 
 struct Plan {
@@ -51,7 +52,7 @@ struct Plan {
     int64_t na[3] = {1, 1, 1};
     uint64_t nanchor = 0;  // codes before the first level
     std::vector<LevelPlan> lv;
-    std::vector<uint64_t> block_off;
+    uint64_t nblocks = 0;  // of all levels
     uint64_t total_codes = 0;
     size_t max_smem = 0;
 };
@@ -154,21 +155,83 @@ Plan make_plan(int N, const uint64_t *dims, uint64_t maxStep, int blocksize, int
         if (sm > smem_limit)
             throw Fail{FAZ_ERR_UNSUPPORTED, "interpolation block does not fit in shared memory (block size too large)"};
         p.max_smem = std::max(p.max_smem, sm);
-        L.off_index = p.block_off.size();
-        int64_t bc[3];
-        for (int64_t b = 0; b < L.nblocks; b++) {
-            block_coords(a, b, bc);
-            BlockGeom g;
-            block_geom(a, bc, g);
-            p.block_off.push_back(pos);
-            pos += (uint64_t)(g.c1 + g.c2 + g.c3);
-        }
+        L.off_index = p.nblocks;
+        L.pos = pos;
+        p.nblocks += (uint64_t)L.nblocks;
+        pos += codes_before(a, nullptr);
         p.lv.push_back(L);
     }
     p.total_codes = pos;
     if (p.total_codes != p.num && !(p.anchor && (N == 1 || N == 4)))
         throw Fail{FAZ_ERR_UNSUPPORTED, "block decomposition does not cover the field exactly"};
     return p;
+}
+
+// The levels of a plan from number `from` on (at most kMaxPlanLevels) for the
+// kernels that take several; `off`: the plan's block-offset table.
+LevelTable level_table(const Plan &p, size_t from, const uint64_t *off, uint64_t ncodes, int *err,
+                       unsigned long long *verify) {
+    LevelTable t;
+    t.n = (int)std::min<size_t>(p.lv.size() - from, kMaxPlanLevels);
+    for (int i = 0; i < t.n; i++) {
+        const LevelPlan &L = p.lv[from + i];
+        t.a[i] = L.args;
+        t.a[i].block_off = off + L.off_index;
+        t.a[i].ncodes = ncodes;
+        t.a[i].err = err;
+        t.a[i].verify = verify;
+        t.first[i] = L.off_index;
+        t.pos[i] = L.pos;
+    }
+    return t;
+}
+
+// The error bound of a plan made before it was known.
+template <typename T>
+void plan_set_eb(Plan &p, double eb, double alpha, double beta) {
+    const int n = (int)p.lv.size();
+    for (int i = 0; i < n; i++) {
+        LevelArgs &a = p.lv[i].args;
+        a.eb = level_eb(eb, alpha, beta, n - i);
+        a.recip = 1.0 / a.eb;
+        set_fast_path<T>(a);
+    }
+}
+
+// Every block's first stream position into `off` (p.nblocks entries).
+void queue_block_offsets(const Plan &p, uint64_t *off, cudaStream_t st, Counter &launches) {
+    for (size_t from = 0; from < p.lv.size(); from += kMaxPlanLevels) {
+        LevelTable t = level_table(p, from, off, 0, nullptr, nullptr);
+        const uint64_t first = t.first[0], n = t.first[t.n - 1] + (uint64_t)p.lv[from + t.n - 1].nblocks - first;
+        for (int i = 0; i < t.n; i++) t.first[i] -= first;
+        launches(launch_block_offsets(t, n, off + first, st));
+    }
+}
+
+// The first point (without an anchor grid) and every level of a plan.
+template <typename T>
+void queue_levels(const Plan &p, bool decomp, double eb, int radius, int trim, const uint64_t *off, int *err,
+                  unsigned long long *verify, const T *dX, T *W, uint16_t *codes, T *scratch, const uint64_t *zpos,
+                  uint64_t nz, const T *unpred, cudaEvent_t finest, cudaStream_t st, Counter &launches) {
+    size_t li = 0;
+    if (!p.lv.empty()) {
+        const LevelTable t = level_table(p, 0, off, p.num, err, verify);
+        const int n = small_levels(t);
+        if (n > 0) {
+            if (n == (int)p.lv.size()) CK(cudaEventRecord(finest, st));
+            launches(launch_small_levels<T>(t, n, decomp, !p.anchor, eb, dX, W, codes, scratch, zpos, nz, unpred, st));
+            li = (size_t)n;
+        }
+    }
+    if (li == 0 && !p.anchor)
+        launches(launch_first_point<T>(decomp, dX, W, codes, scratch, eb, radius, trim, zpos, nz, unpred, st));
+    for (; li < p.lv.size(); li++) {
+        const LevelTable t = level_table(p, li, off, p.num, err, verify);
+        if (li + 1 == p.lv.size()) CK(cudaEventRecord(finest, st));
+        int nl = 0;
+        CK(launch_level<T>(t.a[0], p.lv[li].nblocks, decomp, dX, W, codes, scratch, zpos, nz, unpred, st, &nl));
+        launches.n += nl;
+    }
 }
 
 // --------------------------------------------------------------- compress
@@ -218,11 +281,10 @@ double device_range(const T *dX, uint64_t n, cudaStream_t st, Counter &launches)
     int nb = (int)std::min<uint64_t>(152 * 4, (n + 4095) / 4096);
     if (nb < 1) nb = 1;
     DevMem m(st);
-    T *pmin = m.alloc<T>(nb), *pmax = m.alloc<T>(nb);
+    T *pmin = m.alloc<T>(2 * nb), *pmax = pmin + nb;
     launches(launch_minmax<T>(dX, n, pmin, pmax, nb, st));
-    std::vector<T> hmin(nb), hmax(nb);
-    CK(cudaMemcpyAsync(hmin.data(), pmin, nb * sizeof(T), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(hmax.data(), pmax, nb * sizeof(T), cudaMemcpyDeviceToHost, st));
+    T *hmin = (T *)t_pin_small.get(2 * nb * sizeof(T)), *hmax = hmin + nb;
+    CK(cudaMemcpyAsync(hmin, pmin, 2 * nb * sizeof(T), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     T mn = hmin[0], mx = hmax[0];
     for (int i = 0; i < nb; i++) {
@@ -295,47 +357,40 @@ struct Sink {
 // `center` is the code the histogram's shared-memory window is centred on.
 template <typename C>
 void huffman_encode_impl(const C *codes, uint64_t n, int center, DevMem &m, cudaStream_t st, Counter &launches,
-                         HuffEncoded &h, faz_timings &tm, const std::function<void(const HuffEncoded &)> &sized) {
+                         HuffEncoded &h, faz_timings &tm, const std::function<void(const HuffEncoded &)> &sized,
+                         bool sliced) {
     const uint64_t nsub = hist_subchunks(n);
     const uint64_t nech = encode_chunks(n);
     // every value a code of this width can take
     const int nsym = sizeof(C) == 2 ? 65536 : std::max(65536, 2 * center + 1);
     // the symbols that occur come back as a compact list (the first
-    // kListHead entries with the count, the rest, if any, in a second copy);
+    // kListHead entries with the counts, the rest, if any, in a second copy);
     // at most min(nsym, n) symbols occur, and the head copy reads kListHead
     constexpr size_t kListHead = 2048;
+    constexpr int kSlices = 8;
     const size_t list_cap = std::max<size_t>(std::min<uint64_t>((uint64_t)nsym, n), kListHead);
     // One allocation holds the work arrays (CUDA calls are few: the tuners
     // run several of these encodes on concurrent host threads, whose calls
-    // serialise in the driver).  In 8-byte words, each part 256-byte aligned:
-    // histogram + list count, first positions, zero counts and offsets, scan
-    // scratch, list, codebook tables (stateNum <= nsym + 1 entries of 17
-    // bytes), chunk bit counts and offsets.
+    // serialise in the driver).  In 8-byte words, each part 256-byte aligned; the
+    // first parts are zeroed together: histogram, first positions, list length and
+    // zero count (before the list); then the list, zero counts and offsets, chunk
+    // bits (in place their offsets), scan scratch, codebook tables (stateNum <=
+    // nsym + 1 entries of 17 bytes).
     auto up = [](uint64_t w) { return (w + 31) & ~(uint64_t)31; };
-    const uint64_t w_hist = up((uint64_t)nsym + 1), w_first = up((uint64_t)nsym), w_z = up(nsub + 1),
-                   w_tmp = up(scan_temp_words(std::max<uint64_t>(nsub, nech)) + 1), w_list = up(3 * list_cap),
-                   w_tab = up(((uint64_t)nsym + 1) * 17 / 8 + 1), w_ch = up(nech + 1);
-    unsigned long long *work =
-        m.alloc<unsigned long long>(w_hist + w_first + 2 * w_z + w_tmp + w_list + w_tab + 2 * w_ch);
-    unsigned long long *hist = work;
-    unsigned int *dnl = reinterpret_cast<unsigned int *>(hist + nsym);
-    unsigned long long *first = hist + w_hist;
-    h.zc = first + w_first;
+    const uint64_t w_hist = up((uint64_t)nsym), w_list = 32 + up(3 * list_cap), w_z = up(nsub + 1),
+                   w_ch = up(nech + 1), w_tmp = up(scan_temp_words(std::max(nsub, nech)) + 1),
+                   w_tab = up(((uint64_t)nsym + 1) * 17 / 8 + 1);
+    unsigned long long *work = m.alloc<unsigned long long>(2 * w_hist + w_list + 2 * w_z + 2 * w_ch + w_tmp + w_tab);
+    unsigned long long *hist = work, *first = hist + w_hist;
+    unsigned long long *dinfo = first + w_hist, *dlist = dinfo + 2;  // [symbols, zeros, list...]
+    h.zc = dinfo + w_list;
     h.zoff = h.zc + w_z;
-    unsigned long long *stmp = h.zoff + w_z;
-    unsigned long long *dlist = stmp + w_tmp;
-    uint8_t *dtab = reinterpret_cast<uint8_t *>(dlist + w_list);
-    unsigned long long *cbits = dlist + w_list + w_tab;
-    unsigned long long *coff = cbits + w_ch;
-    CK(cudaMemsetAsync(hist, 0, ((size_t)nsym + 1) * 8, st));
-    CK(cudaMemsetAsync(first, 0xff, (size_t)nsym * 8, st));
-    launches(launch_histogram(codes, n, center, hist, first, h.zc, st));
-    launches(launch_scan_u64(h.zc, h.zoff, nsub, stmp, st));
-    launches(launch_hist_compact(hist, first, nsym, dlist, dnl, st));
+    unsigned long long *cbits = h.zoff + w_z, *coff = cbits + w_ch, *stmp = coff + w_ch, *dtab = stmp + w_tmp;
+    CK(cudaMemsetAsync(work, 0, (2 * w_hist + 2) * 8, st));
+    launches(launch_histogram(codes, n, center, hist, first, h.zc, dinfo + 1, st));
+    launches(launch_hist_compact(hist, first, nsym, dlist, reinterpret_cast<unsigned *>(dinfo), st));
     uint8_t *hb = t_pin_small.get(16 + kListHead * 24);
-    CK(cudaMemcpyAsync(hb, dnl, 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(hb + 8, h.zoff + nsub, 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(hb + 16, dlist, kListHead * 24, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(hb, dinfo, 16 + kListHead * 24, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (tune_trace()) {
         char msg[96];
@@ -348,6 +403,7 @@ void huffman_encode_impl(const C *codes, uint64_t n, int center, DevMem &m, cuda
     std::memcpy(&h.nzero, hb + 8, 8);
     if (nl > (unsigned int)nsym || nl > list_cap)
         throw Fail{FAZ_ERR_DEVICE, "histogram list longer than the symbol range"};
+    if (h.nzero) launches(launch_scan_u64(h.zc, h.zoff, nsub, stmp, st));
     std::vector<unsigned long long> rest;
     if (nl > kListHead) {
         rest.resize(3 * (size_t)(nl - kListHead));
@@ -370,30 +426,25 @@ void huffman_encode_impl(const C *codes, uint64_t n, int center, DevMem &m, cuda
     trace_step("huffman tree built");
     tm.host_ms += ms_since(th1);
     const Codebook &cb = h.cb;
-    // The three tables (MSB-aligned codes, packed length|code, lengths) go
-    // up in one copy from the thread's pinned staging: pageable copies from
-    // several threads serialise in the driver.  The staging is refilled once
-    // the thread's previous upload from it has completed.
+    // The three tables (MSB-aligned codes, packed length|code, lengths) go up in one
+    // copy from the thread's pinned staging: pageable copies from several threads
+    // serialise in the driver.  The staging is refilled once the thread's previous
+    // upload from it has completed.
     const size_t S = (size_t)cb.stateNum;
     if (S > (size_t)nsym + 1) throw Fail{FAZ_ERR_DEVICE, "Huffman codebook larger than the symbol range"};
     TableStage &ts = t_table_stage;
-    uint8_t *htab = ts.acquire(S * 17);
-    unsigned long long *hcode = reinterpret_cast<unsigned long long *>(htab);
+    unsigned long long *hcode = reinterpret_cast<unsigned long long *>(ts.acquire(S * 17));
     unsigned long long *hpacked = hcode + S;
     std::memcpy(hcode, cb.code.data(), S * 8);
     for (size_t i = 0; i < S; i++) {
         const int l = cb.len[i];
         hpacked[i] = ((unsigned long long)l << 32) | (l >= 1 && l <= 32 ? (cb.code[i] >> (64 - l)) : 0ull);
     }
-    std::memcpy(htab + S * 16, cb.len.data(), S);
-    CK(cudaMemcpyAsync(dtab, htab, S * 17, cudaMemcpyHostToDevice, st));
+    std::memcpy(hcode + 2 * S, cb.len.data(), S);
+    CK(cudaMemcpyAsync(dtab, hcode, S * 17, cudaMemcpyHostToDevice, st));
     ts.release(st);
-    unsigned long long *dcode = reinterpret_cast<unsigned long long *>(dtab);
-    unsigned long long *dpacked = dcode + S;
-    uint8_t *dlen = dtab + S * 16;
     trace_step("huffman tables uploaded");
-    // the encoded size from the counts and code lengths (what the device's
-    // chunk scan adds up)
+    // the encoded size from the counts and code lengths
     uint64_t total_bits = 0;
     for (size_t i = 0; i < syms.size(); i++) total_bits += cnts[i] * (uint64_t)cb.len[syms[i] - cb.offset];
     h.nbytes = (total_bits + 7) / 8;
@@ -403,25 +454,35 @@ void huffman_encode_impl(const C *codes, uint64_t n, int center, DevMem &m, cuda
         trace_step(msg);
     }
     if (sized) sized(h);
-    launches(launch_encode_bits(codes, n, cb.offset, dlen, cbits, st));
-    launches(launch_scan_u64(cbits, coff, nech, stmp, st));
     const uint64_t nwords = (total_bits + 31) / 32 + 1;
     h.bits = m.alloc<uint32_t>(nwords);
     CK(cudaMemsetAsync(h.bits, 0, nwords * 4, st));
-    if (total_bits)
-        launches(launch_encode_pack(codes, n, cb.offset, dcode, dpacked, dlen, coff, h.bits, std::max(cb.maxlen, 1), st));
+    if (!total_bits) return;
+    launches(launch_encode_bits(codes, n, cb.offset, reinterpret_cast<const uint8_t *>(dtab + 2 * S), cbits, st));
+    launches(launch_scan_u64(cbits, coff, nech, stmp, st));
+    const EncodeArgs ea{cb.offset, std::max(cb.maxlen, 1), dtab, dtab + S, coff, h.bits};
+    // strings of 16 MB or more in slices, whose copies overlap the next ones
+    const int slices = sliced && h.nbytes >= (16u << 20) ? kSlices : 1;
+    h.end = (const volatile uint64_t *)t_pin_encode.get(kSlices * 8);
+    for (int k = 0; k < slices; k++) {
+        launches(launch_encode_pack(ea, codes, n, nech * k / slices, nech * (k + 1) / slices,
+                                    slices > 1 ? (unsigned long long *)h.end + k : nullptr, st));
+        if (slices == 1) break;
+        h.done.push_back(std::make_shared<Event>());
+        CK(cudaEventRecord(h.done.back()->e, st));
+    }
 }
 
 void huffman_encode_device(const uint16_t *codes, uint64_t n, int center, DevMem &m, cudaStream_t st,
                            Counter &launches, HuffEncoded &h, faz_timings &tm,
-                           const std::function<void(const HuffEncoded &)> &sized) {
-    huffman_encode_impl(codes, n, center, m, st, launches, h, tm, sized);
+                           const std::function<void(const HuffEncoded &)> &sized, bool sliced) {
+    huffman_encode_impl(codes, n, center, m, st, launches, h, tm, sized, sliced);
 }
 void huffman_encode_device(const uint32_t *codes, uint64_t n, int center, DevMem &m, cudaStream_t st,
                            Counter &launches, HuffEncoded &h, faz_timings &tm,
-                           const std::function<void(const HuffEncoded &)> &sized) {
+                           const std::function<void(const HuffEncoded &)> &sized, bool sliced) {
     if (center < 0 || center > (1 << 20)) throw Fail{FAZ_ERR_UNSUPPORTED, "quantisation radius too large"};
-    huffman_encode_impl(codes, n, center, m, st, launches, h, tm, sized);
+    huffman_encode_impl(codes, n, center, m, st, launches, h, tm, sized, sliced);
 }
 
 // HuffmanEncoder::save header + tree, then the encoded size (HuffmanEncoder.hpp:119-137, 150-227)
@@ -442,22 +503,18 @@ template <typename T>
 struct InterpEncoded {
     HuffEncoded he;
     T *unpred = nullptr;
+    unsigned long long *flags = nullptr;  // pinned: level kernels' error flag, verification disagreements
 };
 
 template <typename T>
 void interp_encode(uint64_t n, int radius, uint16_t *codes, T *scratch, unsigned long long *vcount, const int *lerr,
                    DevMem &m, cudaStream_t st, Counter &launches, faz_timings &tm, InterpEncoded<T> &e) {
-    huffman_encode_device(codes, n, radius, m, st, launches, e.he, tm);
-    if (lerr) {
-        int le = 0;
-        CK(cudaMemcpy(&le, lerr, sizeof(int), cudaMemcpyDeviceToHost));
-        if (le) throw Fail{FAZ_ERR_DEVICE, "an interpolation level kernel gave up waiting for its plane copies"};
-    }
-    if (vcount) {
-        unsigned long long vc = 0;
-        CK(cudaMemcpy(&vc, vcount, 8, cudaMemcpyDeviceToHost));
-        if (vc) throw Fail{FAZ_ERR_DEVICE, "float fast path disagreed with the double path at " + std::to_string(vc) + " points"};
-    }
+    huffman_encode_device(codes, n, radius, m, st, launches, e.he, tm, {}, true);
+    // the levels' flags, read by interp_emit after its wait
+    e.flags = (unsigned long long *)t_pin_flag.get(64);
+    e.flags[0] = e.flags[1] = 0;
+    if (lerr) CK(cudaMemcpyAsync(e.flags, lerr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    if (vcount) CK(cudaMemcpyAsync(e.flags + 1, vcount, 8, cudaMemcpyDeviceToHost, st));
     const uint64_t nunpred = e.he.nzero;
     e.unpred = m.alloc<T>(nunpred ? nunpred : 1);
     if (nunpred) launches(launch_compact_zeros<T>(codes, n, e.he.zc, e.he.zoff, scratch, e.unpred, st));
@@ -513,8 +570,28 @@ void interp_emit(const faz_config &c, const std::vector<uint8_t> &il, const std:
     o += nunpred * sizeof(T);
     std::memcpy(payload + o, tree.data(), tree.size());
     o += tree.size();
-    if (nbytes) CK(cudaMemcpyAsync(payload + o, e.he.bits, nbytes, cudaMemcpyDeviceToHost, st));
+    if (nbytes && e.he.done.empty()) CK(cudaMemcpyAsync(payload + o, e.he.bits, nbytes, cudaMemcpyDeviceToHost, st));
+    if (!e.he.done.empty()) {
+        // each slice's whole words as soon as its launch is done
+        StreamGuard cs(nullptr);
+        uint64_t from = 0;
+        const size_t ns = e.he.done.size();
+        for (size_t k = 0; k < ns; k++) {
+            CK(cudaEventSynchronize(e.he.done[k]->e));
+            const uint64_t to = k + 1 == ns ? nbytes : std::min<uint64_t>(nbytes, e.he.end[k] / 32 * 4);
+            if (to > from)
+                CK(cudaMemcpyAsync(payload + o + from, (const uint8_t *)e.he.bits + from, to - from,
+                                   cudaMemcpyDeviceToHost, cs.st));
+            from = std::max(from, to);
+        }
+        CK(cudaStreamSynchronize(cs.st));
+    }
     CK(cudaStreamSynchronize(st));
+    if (e.flags && (int)e.flags[0])
+        throw Fail{FAZ_ERR_DEVICE, "an interpolation level kernel gave up waiting for its plane copies"};
+    if (e.flags && e.flags[1])
+        throw Fail{FAZ_ERR_DEVICE,
+                   "float fast path disagreed with the double path at " + std::to_string(e.flags[1]) + " points"};
     tm.unpred_count = nunpred;
     tm.payload_bytes = psize;
 }
@@ -557,17 +634,40 @@ struct InterpCodes {
 // 324-461); resolves the error bound of c.
 template <typename T>
 void interp_levels(InterpCodes<T> &r, faz_config &c, const T *dX, cudaStream_t st, Counter &launches) {
-    resolve_eb<T>(c, dX, st, launches);
-    const double eb = c.absErrorBound;
-    if (!(eb > 0) || !std::isfinite(eb)) throw Fail{FAZ_ERR_ARG, "error bound must be positive and finite"};
     const int radius = c.quantbinCnt / 2;
     if (radius > 32768) throw Fail{FAZ_ERR_UNSUPPORTED, "interpolation with more than 65536 bins is not implemented"};
     r.il.assign(c.interpAlgo_list, c.interpAlgo_list + c.interp_list_len);
     r.dl.assign(c.interpDirection_list, c.interpDirection_list + c.interp_list_len);
+    const bool off_lattice = c.fixBlockSize > 0 && !fixbs_aligned(c.N, c.dims, c.maxStep, c.fixBlockSize);
+    DevMem &m = r.m;
+    // What does not depend on the error bound comes before it: the plan, the
+    // memory and the block offsets, so that the wait for the field's range has
+    // only the levels after it.
+    Plan p;
+    T *W = nullptr, *scratch = nullptr;
+    uint16_t *codes = nullptr;
+    uint64_t *boff = nullptr;
+    int *lerr = nullptr;
+    if (c.N != 4 && !off_lattice) {
+        p = make_plan<T>(c.N, c.dims, c.maxStep, c.interpBlockSize, c.fixBlockSize, c.interpAlgo, c.interpDirection,
+                         r.il, r.dl, 1.0, c.alpha, c.beta, radius, c.trimToZero, smem_limit());
+        // one allocation: W, scratch, codes, block offsets, error flag
+        auto up = [](uint64_t b) { return (b + 255) & ~(uint64_t)255; };
+        uint8_t *mem = m.alloc<uint8_t>(2 * up(p.num * sizeof(T)) + up(p.num * 2) + up(p.nblocks * 8) + 256);
+        W = (T *)mem;
+        scratch = (T *)(mem += up(p.num * sizeof(T)));
+        codes = (uint16_t *)(mem += up(p.num * sizeof(T)));
+        boff = (uint64_t *)(mem += up(p.num * 2));
+        lerr = (int *)(mem + up(p.nblocks * 8));
+        CK(cudaMemsetAsync(lerr, 0, sizeof(int), st));
+        queue_block_offsets(p, boff, st, launches);
+    }
+    resolve_eb<T>(c, dX, st, launches);
+    const double eb = c.absErrorBound;
+    if (!(eb > 0) || !std::isfinite(eb)) throw Fail{FAZ_ERR_ARG, "error bound must be positive and finite"};
     if (c.N == 4) {
         // 4-D: one launch per level and sweep (interp4.cu)
-        DevMem &m = r.m;
-        T *W = m.alloc<T>(c.num);
+        W = m.alloc<T>(c.num);
         r.scratch = m.alloc<T>(c.num);
         r.codes = m.alloc<uint16_t>(c.num);
         unsigned long long *vcount = nullptr;
@@ -586,11 +686,10 @@ void interp_levels(InterpCodes<T> &r, faz_config &c, const T *dX, cudaStream_t s
         r.have_levels = false;
         return;
     }
-    if (c.fixBlockSize > 0 && !fixbs_aligned(c.N, c.dims, c.maxStep, c.fixBlockSize)) {
+    if (off_lattice) {
         // blocks of fixBlockSize that leave the coarse lattice: the block
         // wavefront of blocked.cu with the level's interpolator and direction
-        DevMem &m = r.m;
-        T *W = m.alloc<T>(c.num);
+        W = m.alloc<T>(c.num);
         r.scratch = m.alloc<T>(c.num);
         r.codes = m.alloc<uint16_t>(c.num);
         CK(cudaEventRecord(r.ev_pred.a, st));
@@ -604,19 +703,9 @@ void interp_levels(InterpCodes<T> &r, faz_config &c, const T *dX, cudaStream_t s
         r.have_levels = false;
         return;
     }
-    Plan p = make_plan<T>(c.N, c.dims, c.maxStep, c.interpBlockSize, c.fixBlockSize, c.interpAlgo, c.interpDirection,
-                          r.il, r.dl, eb, c.alpha, c.beta, radius, c.trimToZero, smem_limit());
     const uint64_t n = p.num;
-    DevMem &m = r.m;
-    T *W = m.alloc<T>(n);
-    T *scratch = m.alloc<T>(n);
-    uint16_t *codes = m.alloc<uint16_t>(n);
-    uint64_t *boff = m.alloc<uint64_t>(p.block_off.size());
-    CK(cudaMemcpyAsync(boff, p.block_off.data(), p.block_off.size() * 8, cudaMemcpyHostToDevice, st));
-    // first point / anchors
-    if (!p.anchor) {
-        launches(launch_first_point<T>(false, dX, W, codes, scratch, eb, radius, c.trimToZero, nullptr, 0, nullptr, st));
-    } else {
+    plan_set_eb<T>(p, eb, c.alpha, c.beta);
+    if (p.anchor) {
         int64_t step[3] = {1, 1, 1};
         int e = 3 - p.N;
         for (int i = 0; i < p.N; i++) step[e + i] = (int64_t)p.maxStep;
@@ -627,21 +716,9 @@ void interp_levels(InterpCodes<T> &r, faz_config &c, const T *dX, cudaStream_t s
         vcount = m.alloc<unsigned long long>(1);
         CK(cudaMemsetAsync(vcount, 0, 8, st));
     }
-    int *lerr = m.alloc<int>(1);
-    CK(cudaMemsetAsync(lerr, 0, sizeof(int), st));
     CK(cudaEventRecord(r.ev_pred.a, st));
-    for (size_t li = 0; li < p.lv.size(); li++) {
-        const LevelPlan &L = p.lv[li];
-        LevelArgs a = L.args;
-        a.block_off = boff + L.off_index;
-        a.ncodes = n;
-        a.err = lerr;
-        a.verify = vcount;
-        if (li + 1 == p.lv.size()) CK(cudaEventRecord(r.ev_fin.a, st));
-        int nl = 0;
-        CK(launch_level<T>(a, L.nblocks, false, dX, W, codes, scratch, nullptr, 0, nullptr, st, &nl));
-        launches.n += nl;
-    }
+    queue_levels<T>(p, false, eb, radius, c.trimToZero, boff, lerr, vcount, dX, W, codes, scratch, nullptr, 0, nullptr,
+                    r.ev_fin.a, st, launches);
     CK(cudaEventRecord(r.ev_fin.b, st));
     CK(cudaEventRecord(r.ev_pred.b, st));
     r.c = c;
@@ -720,6 +797,10 @@ void blocked_payload(faz_config &c, const T *dX, cudaStream_t st, uint8_t *&payl
 template <typename T>
 void compress_dispatch(faz_config &c, const T *dX, cudaStream_t st, uint8_t *&payload, size_t &psize,
                        faz_timings &tm, Counter &launches, Sink *sink = nullptr) {
+    if (c.cmprAlgo == FAZ_ALGO_INTERP) {  // resolves the error bound itself, beside the range's kernel
+        compress_payload<T>(c, dX, st, payload, psize, tm, launches, sink);
+        return;
+    }
     resolve_eb<T>(c, dX, st, launches);
     if (!(c.absErrorBound > 0) || !std::isfinite(c.absErrorBound))
         throw Fail{FAZ_ERR_ARG, "error bound must be positive and finite"};
@@ -988,20 +1069,20 @@ int compress_batch_impl(int nf, const faz_config *confs, const void *const *d_da
         Events ev_pred;
         CK(cudaEventRecord(ev_pred.a, st));
         if (!fw.empty()) {
-            std::vector<uint64_t> boff;
             std::vector<BatchField> bf(fw.size());
             std::vector<LevelArgs> la;
             std::vector<BatchGroup> groups;
             std::vector<size_t> boff_base(fw.size());
+            size_t nboff = 0;
             bool wide = false;
             size_t smem = 16;
             for (size_t k = 0; k < fw.size(); k++) {
-                boff_base[k] = boff.size();
-                boff.insert(boff.end(), fw[k].p.block_off.begin(), fw[k].p.block_off.end());
+                boff_base[k] = nboff;
+                nboff += fw[k].p.nblocks;
                 wide = wide || (int64_t)fw[k].p.num >= ((int64_t)1 << 31);
             }
-            uint64_t *dboff = m.alloc<uint64_t>(boff.size() + 1);
-            CK(cudaMemcpyAsync(dboff, boff.data(), boff.size() * 8, cudaMemcpyHostToDevice, st));
+            uint64_t *dboff = m.alloc<uint64_t>(nboff + 1);
+            for (size_t k = 0; k < fw.size(); k++) queue_block_offsets(fw[k].p, dboff + boff_base[k], st, launches);
             std::vector<int> first_la(fw.size());
             for (size_t k = 0; k < fw.size(); k++) {
                 const faz_config &c = cs[fw[k].idx];
@@ -1729,8 +1810,8 @@ void decompress_device(const uint8_t *pl, size_t n, Parsed &P, T *dOut, cudaStre
     if (P.nunpred) CK(cudaMemcpyAsync(dunpred, P.unpred, P.nunpred * sizeof(T), cudaMemcpyHostToDevice, st));
     Events ev_dec, ev_pred, ev_fin;
     CK(cudaEventRecord(ev_dec.a, st));
-    uint64_t *boff = m.alloc<uint64_t>(pl_.block_off.size());
-    CK(cudaMemcpyAsync(boff, pl_.block_off.data(), pl_.block_off.size() * 8, cudaMemcpyHostToDevice, st));
+    uint64_t *boff = m.alloc<uint64_t>(pl_.nblocks + 1);
+    queue_block_offsets(pl_, boff, st, launches);
     int *kerr = m.alloc<int>(1);
     CK(cudaMemsetAsync(kerr, 0, 4, st));
     unsigned long long *vcount = nullptr;
@@ -1751,28 +1832,15 @@ void decompress_device(const uint8_t *pl, size_t n, Parsed &P, T *dOut, cudaStre
     auto reconstruct = [&] {
         uint64_t *zpos = nullptr;
         hz = queue_zero_positions(h, nz, m, st, launches, zpos);
-        if (!pl_.anchor) {
-            launches(launch_first_point<T>(true, nullptr, dOut, codes, nullptr, P.eb, P.radius, P.trim, zpos, nz,
-                                           dunpred, st));
-        } else {
+        if (pl_.anchor) {
             int64_t step[3] = {1, 1, 1};
             int e = 3 - pl_.N;
             for (int i = 0; i < pl_.N; i++) step[e + i] = (int64_t)pl_.maxStep;
             launches(launch_anchors<T>(true, nullptr, dOut, codes, nullptr, dunpred, pl_.na, step, pl_.offs3, st));
         }
         CK(cudaEventRecord(ev_pred.a, st));
-        for (size_t li = 0; li < pl_.lv.size(); li++) {
-            const LevelPlan &L = pl_.lv[li];
-            LevelArgs a = L.args;
-            a.block_off = boff + L.off_index;
-            a.ncodes = num;
-            a.err = kerr;
-            a.verify = vcount;
-            if (li + 1 == pl_.lv.size()) CK(cudaEventRecord(ev_fin.a, st));
-            int nl = 0;
-            CK(launch_level<T>(a, L.nblocks, true, nullptr, dOut, codes, nullptr, zpos, nz, dunpred, st, &nl));
-            launches.n += nl;
-        }
+        queue_levels<T>(pl_, true, P.eb, P.radius, P.trim, boff, kerr, vcount, nullptr, dOut, codes, nullptr, zpos, nz,
+                        dunpred, ev_fin.a, st, launches);
         CK(cudaEventRecord(ev_fin.b, st));
         CK(cudaEventRecord(ev_pred.b, st));
         CK(cudaMemcpyAsync(hk, kerr, 4, cudaMemcpyDeviceToHost, st));

@@ -96,6 +96,49 @@ FAZ_HD void block_geom(const LevelArgs &a, const int64_t *bc, BlockGeom &g) {
     g.c3 = (int64_t)(g.n0 - g.k0) * (g.n1 - g.k1) * g.t2;
 }
 
+// Of block b along axis d: the lattice points it emits lines of (0), its emitted
+// even points (1) and its targets per line (2); the codes of a sweep are products
+// of one such number per axis.
+FAZ_HD int64_t axis_count(const LevelArgs &a, int d, int64_t b, int which) {
+    const int64_t beg = b * a.bs;
+    int64_t end = beg + a.bs;
+    if (end > a.dims[d] - 1) end = a.dims[d] - 1;
+    const int64_t n = (end - beg) / a.s + 1, k = b != 0;
+    return which == 0 ? n - k : (which == 1 ? (n + 1) / 2 - k : n / 2);
+}
+// the sum of axis_count over the blocks before b (all but the first and the last
+// are alike)
+FAZ_HD int64_t axis_before(const LevelArgs &a, int d, int64_t b, int which) {
+    return b == 0 ? 0 : axis_count(a, d, 0, which) + (b == 1 ? 0 : (b - 1) * axis_count(a, d, 1, which));
+}
+// Codes of the level in the blocks before block bc (row-major); with bc = null of
+// all of its blocks.
+FAZ_HD uint64_t codes_before(const LevelArgs &a, const int64_t *bc) {
+    uint64_t sum = 0;
+    for (int sw = 0; sw < 3; sw++) {
+        int w[3];  // per axis, in axis order
+        for (int i = 0; i < 3; i++) {
+            // sweep order: the axis swept has targets, those swept before emit
+            // lines at every point, those after at even points
+            const int wi = i == sw ? 2 : (i < sw ? 0 : 1);
+            if (a.perm[i] == 0) w[0] = wi;
+            else if (a.perm[i] == 1) w[1] = wi;
+            else w[2] = wi;
+        }
+        uint64_t t1 = (uint64_t)(axis_before(a, 1, a.nb[1] - 1, w[1]) + axis_count(a, 1, a.nb[1] - 1, w[1]));
+        uint64_t t2 = (uint64_t)(axis_before(a, 2, a.nb[2] - 1, w[2]) + axis_count(a, 2, a.nb[2] - 1, w[2]));
+        if (!bc) {
+            sum += (uint64_t)(axis_before(a, 0, a.nb[0] - 1, w[0]) + axis_count(a, 0, a.nb[0] - 1, w[0])) * t1 * t2;
+            continue;
+        }
+        sum += (uint64_t)axis_before(a, 0, bc[0], w[0]) * t1 * t2 +
+               (uint64_t)axis_count(a, 0, bc[0], w[0]) *
+                   ((uint64_t)axis_before(a, 1, bc[1], w[1]) * t2 +
+                    (uint64_t)axis_count(a, 1, bc[1], w[1]) * (uint64_t)axis_before(a, 2, bc[2], w[2]));
+    }
+    return sum;
+}
+
 // Stream rank of odd lattice index m inside a line of n points
 // (emission order of block_interpolation_1d, SZInterpolationCompressor.hpp:1306-1417):
 // linear / short lines ascend; cubic lines emit interior points 3,5,...,

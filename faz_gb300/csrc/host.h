@@ -16,6 +16,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -113,6 +114,7 @@ struct Pinned {
 };
 inline thread_local Pinned t_pin_payload;
 inline thread_local Pinned t_pin_small;
+inline thread_local Pinned t_pin_encode;  // ends of a sliced bit packing's launches
 inline thread_local Pinned t_pin_decode;  // outcome of a queued Huffman decode
 inline thread_local Pinned t_pin_flag;  // device status words read after a later synchronisation
 
@@ -345,6 +347,14 @@ class TaskThreads {
     bool stop_ = false;
 };
 
+// an event that orders streams (no timing)
+struct Event {
+    cudaEvent_t e = nullptr;
+    Event() { CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)); }
+    ~Event() { cudaEventDestroy(e); }
+    Event(const Event &) = delete;
+};
+
 struct Events {
     cudaEvent_t a = nullptr, b = nullptr;
     Events() {
@@ -522,17 +532,23 @@ struct HuffEncoded {
     uint32_t *bits = nullptr;  // device: the MSB-first bit string
     uint64_t nbytes = 0;
     uint64_t nzero = 0;        // codes equal to 0 (unpredictable points)
-    unsigned long long *zc = nullptr, *zoff = nullptr;  // zero counts per sub-chunk and their exclusive scan
+    unsigned long long *zc = nullptr, *zoff = nullptr;  // zero counts per sub-chunk and their exclusive scan (nzero > 0)
+    // A bit string packed in several launches: after launch k (done[k]) the bits up
+    // to *end[k] are in place, so that their copy can overlap the next launches.
+    // Empty: one launch, in the stream's order.
+    std::vector<std::shared_ptr<Event>> done;
+    const volatile uint64_t *end = nullptr;
 };
 // `sized`, when given, runs as soon as the codebook, the zero count and the
 // encoded size are known on the host (before the encoding kernels finish).
+// `sliced`: long bit strings may be packed in several launches.
 // The uint32_t overloads serve quantisers of more than 65536 bins.
 void huffman_encode_device(const uint16_t *codes, uint64_t n, int center, DevMem &m, cudaStream_t st,
                            Counter &launches, HuffEncoded &h, faz_timings &tm,
-                           const std::function<void(const HuffEncoded &)> &sized = {});
+                           const std::function<void(const HuffEncoded &)> &sized = {}, bool sliced = false);
 void huffman_encode_device(const uint32_t *codes, uint64_t n, int center, DevMem &m, cudaStream_t st,
                            Counter &launches, HuffEncoded &h, faz_timings &tm,
-                           const std::function<void(const HuffEncoded &)> &sized = {});
+                           const std::function<void(const HuffEncoded &)> &sized = {}, bool sliced = false);
 void append_tree(std::vector<uint8_t> &o, const Codebook &cb, uint64_t nbytes);
 void huffman_decode_device(const uint8_t *&p, const uint8_t *end, uint64_t num, uint16_t *codes, DevMem &m,
                            cudaStream_t st, Counter &launches);

@@ -63,6 +63,25 @@ template <typename T>
 cudaError_t launch_minmax(const T *X, uint64_t n, T *pmin, T *pmax, int nblocks, cudaStream_t st);
 template <typename T>
 size_t level_smem_bytes(const LevelArgs &a);
+// The levels of an interpolation plan, coarsest first (a batch of the kernels
+// below takes up to kMaxPlanLevels).
+constexpr int kMaxPlanLevels = 32;
+struct LevelTable {
+    LevelArgs a[kMaxPlanLevels];
+    uint64_t first[kMaxPlanLevels];  // its first entry in the block-offset table
+    uint64_t pos[kMaxPlanLevels];    // stream position of its first code
+    int n;
+};
+// stream position of every block's first code into `off`
+cudaError_t launch_block_offsets(const LevelTable &t, uint64_t nblocks, uint64_t *off, cudaStream_t st);
+// How many of a plan's first levels are small enough for launch_small_levels, and
+// the launch: the first point (unless anchors come instead) and those levels, in
+// one CTA.
+int small_levels(const LevelTable &t);
+template <typename T>
+cudaError_t launch_small_levels(const LevelTable &t, int n, bool decomp, bool first_point, double eb, const T *X, T *W,
+                                uint16_t *codes, T *scratch, const uint64_t *zpos, uint64_t nz, const T *unpred,
+                                cudaStream_t st);
 // One interpolation level; *nlaunch grows by the kernel launches it made.
 template <typename T>
 cudaError_t launch_level(const LevelArgs &a, int64_t nblocks, bool decomp, const T *X, T *W, uint16_t *codes,
@@ -118,11 +137,14 @@ uint64_t hist_subchunks(uint64_t n);
 cudaError_t launch_hist_compact(const unsigned long long *hist, const unsigned long long *first, int nsym,
                                 unsigned long long *list, unsigned int *nlist, cudaStream_t st);
 // Huffman stage kernels; the uint32_t overloads serve quantisers of more than
-// 65536 bins.
+// 65536 bins.  hist[nsym], first[nsym] (complemented positions) and *nzero zeroed
+// by the caller; zcount: hist_subchunks(n) zero counts.
 cudaError_t launch_histogram(const uint16_t *codes, uint64_t n, int center, unsigned long long *hist,
-                             unsigned long long *first, unsigned long long *zcount, cudaStream_t st);
+                             unsigned long long *first, unsigned long long *zcount, unsigned long long *nzero,
+                             cudaStream_t st);
 cudaError_t launch_histogram(const uint32_t *codes, uint64_t n, int center, unsigned long long *hist,
-                             unsigned long long *first, unsigned long long *zcount, cudaStream_t st);
+                             unsigned long long *first, unsigned long long *zcount, unsigned long long *nzero,
+                             cudaStream_t st);
 cudaError_t launch_count_zeros(const uint16_t *codes, uint64_t n, unsigned long long *zcount, cudaStream_t st);
 cudaError_t launch_count_zeros(const uint32_t *codes, uint64_t n, unsigned long long *zcount, cudaStream_t st);
 template <typename T, typename C>
@@ -132,16 +154,23 @@ uint64_t scan_temp_words(uint64_t n);
 cudaError_t launch_scan_u64(const unsigned long long *in, unsigned long long *out, uint64_t n,
                             unsigned long long *temp, cudaStream_t st);
 uint64_t encode_chunks(uint64_t n);
+// bits of every chunk
 cudaError_t launch_encode_bits(const uint16_t *codes, uint64_t n, int offset, const uint8_t *len,
                                unsigned long long *chunkbits, cudaStream_t st);
 cudaError_t launch_encode_bits(const uint32_t *codes, uint64_t n, int offset, const uint8_t *len,
                                unsigned long long *chunkbits, cudaStream_t st);
-cudaError_t launch_encode_pack(const uint16_t *codes, uint64_t n, int offset, const unsigned long long *code64,
-                               const unsigned long long *packed, const uint8_t *len,
-                               const unsigned long long *chunkoff, uint32_t *out, int maxlen, cudaStream_t st);
-cudaError_t launch_encode_pack(const uint32_t *codes, uint64_t n, int offset, const unsigned long long *code64,
-                               const unsigned long long *packed, const uint8_t *len,
-                               const unsigned long long *chunkoff, uint32_t *out, int maxlen, cudaStream_t st);
+// Bit packing of chunks [chunk0, chunk1) of n codes: code tables, the exclusive
+// scan of the chunks' bits, the zeroed output.  host_end (pinned, or null) receives
+// the bits before chunk1.
+struct EncodeArgs {
+    int offset, maxlen;
+    const unsigned long long *code64, *packed, *chunkoff;
+    uint32_t *out;
+};
+cudaError_t launch_encode_pack(const EncodeArgs &a, const uint16_t *codes, uint64_t n, uint64_t chunk0,
+                               uint64_t chunk1, unsigned long long *host_end, cudaStream_t st);
+cudaError_t launch_encode_pack(const EncodeArgs &a, const uint32_t *codes, uint64_t n, uint64_t chunk0,
+                               uint64_t chunk1, unsigned long long *host_end, cudaStream_t st);
 
 // Huffman decoder (huffman.cu): the tree as child words (leaf flag | state, or
 // node index), and the tables launch_decode_tables builds from it.

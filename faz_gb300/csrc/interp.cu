@@ -13,6 +13,7 @@
 // -fmad=false): stencils in T (include/QoZ/utils/Interpolators.hpp:9-36),
 // quantiser in the T/double mix of include/QoZ/quantizer/IntegerQuantizer.hpp:69-179.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
 #include <cfloat>
@@ -305,36 +306,20 @@ __global__ void __launch_bounds__(512, 2) k_interp_level(LevelArgs a, const T *_
     level_block<T, DECOMP, WIDE, QM, false, CUB>(a, blockIdx.x, X, W, codes, scratch, zpos, nz, unpred, smem_raw);
 }
 
-// ------------------------------------------------------ coarse levels
-// Levels with lattice stride s >= 2 hold 1/8 of the field or less, in few
-// blocks (64 at the third level of a 512^3 field, one at the last): one CTA
-// per block leaves most SMs idle while each block's sweeps run one after
-// another.  Instead, each sweep of the level is one launch over every block,
-// one thread per emitted target in stream order (so code stores are
-// contiguous), neighbours read from the reconstruction W (coarse points and
-// the earlier sweeps' targets, written before this launch began), targets
+// ------------------------------------------------------ sweep launches
+// One emitted target of sweep sw (1..3): number x of block g in stream order (so
+// code stores are contiguous), its neighbours read from the reconstruction W
+// (coarse points and the earlier sweeps' targets, written before), the target
 // written back to W.  Every line is computed once, by the block that emits it.
-// CTA c takes chunk c % chunks of block c / chunks.
+// Fields of these kernels hold fewer than 2^31 values: offsets are 32-bit.
 template <typename T, bool DECOMP, int QM, int CUB>
-__global__ void __launch_bounds__(256) k_level_sweep(LevelArgs a, int sw, int64_t chunks, const T *__restrict__ X,
-                                                    T *__restrict__ W, uint16_t *__restrict__ codes,
-                                                    T *__restrict__ scratch, const uint64_t *__restrict__ zpos,
-                                                    uint64_t nz, const T *__restrict__ unpred) {
-    __shared__ BlockGeom sgeo;
-    __shared__ int64_t sbc[3];
-    const int64_t bid = (int64_t)blockIdx.x / chunks;
-    const int64_t x = ((int64_t)blockIdx.x - bid * chunks) * blockDim.x + threadIdx.x;
-    if (threadIdx.x == 0) {
-        block_coords(a, bid, sbc);
-        block_geom(a, sbc, sgeo);
-    }
-    __syncthreads();
-    const BlockGeom &g = sgeo;
-    const int64_t cnt = sw == 1 ? g.c1 : (sw == 2 ? g.c2 : g.c3);
-    if (x >= cnt) return;
-    const int tl = sw == 1 ? g.t0 : (sw == 2 ? g.t1 : g.t2);  // targets per line
-    const int n = sw == 1 ? g.n0 : (sw == 2 ? g.n1 : g.n2);   // lattice points per line
-    const int64_t L = x / tl;
+__device__ __forceinline__ void sweep_target(const LevelArgs &a, const BlockGeom &g, uint64_t base, int sw, uint32_t x,
+                                             const T *__restrict__ X, T *W, uint16_t *__restrict__ codes,
+                                             T *__restrict__ scratch, const uint64_t *__restrict__ zpos, uint64_t nz,
+                                             const T *__restrict__ unpred) {
+    const uint32_t tl = (uint32_t)(sw == 1 ? g.t0 : (sw == 2 ? g.t1 : g.t2));  // targets per line
+    const int n = sw == 1 ? g.n0 : (sw == 2 ? g.n1 : g.n2);                    // lattice points per line
+    const uint32_t L = x / tl;
     const int r = (int)(x - L * tl);
     // target of stream rank r in its line (inverse of line_rank)
     int m;
@@ -346,41 +331,120 @@ __global__ void __launch_bounds__(256) k_level_sweep(LevelArgs a, int sw, int64_
         m = r < cint ? 2 * r + 3 : (r == cint ? 1 : (r == cint + 1 ? ia : n - 1));
     }
     // lattice coordinates along P0, P1, P2 of the line's origin
-    int64_t c0, c1, c2;
-    if (sw == 1) {
-        c0 = 0;
-        c1 = 2 * (L / g.ne2 + g.k1);
-        c2 = 2 * (L % g.ne2 + g.k2);
-    } else if (sw == 2) {
-        c0 = g.k0 + L / g.ne2;
-        c1 = 0;
-        c2 = 2 * (L % g.ne2 + g.k2);
-    } else {
-        const int64_t w1 = g.n1 - g.k1;
-        c0 = g.k0 + L / w1;
-        c1 = g.k1 + L % w1;
-        c2 = 0;
-    }
+    const uint32_t w = (uint32_t)(sw == 3 ? g.n1 - g.k1 : g.ne2);
+    const int hi = (int)(L / w), lo = (int)(L - (uint32_t)hi * w);
+    const int c0 = sw == 1 ? 0 : g.k0 + hi;
+    const int c1 = sw == 1 ? 2 * (hi + g.k1) : (sw == 2 ? 0 : g.k1 + lo);
+    const int c2 = sw == 3 ? 0 : 2 * (lo + g.k2);
     const int P0 = a.perm[0], P1 = a.perm[1], P2 = a.perm[2];
-    const int64_t o0 = pick3(P0, a.offs[0], a.offs[1], a.offs[2]), o1 = pick3(P1, a.offs[0], a.offs[1], a.offs[2]),
-                  o2 = pick3(P2, a.offs[0], a.offs[1], a.offs[2]);
-    const int64_t b0 = pick3(P0, g.beg[0], g.beg[1], g.beg[2]), b1 = pick3(P1, g.beg[0], g.beg[1], g.beg[2]),
-                  b2 = pick3(P2, g.beg[0], g.beg[1], g.beg[2]);
-    const int64_t origin = (b0 + c0 * a.s) * o0 + (b1 + c1 * a.s) * o1 + (b2 + c2 * a.s) * o2;
-    const int64_t st = a.s * (sw == 1 ? o0 : (sw == 2 ? o1 : o2));
-    const Stencil<T> S = make_stencil<T>(m, n, a.cubic, (int)st, 0);
-    const T pred = eval_stencil<CUB>(S, W + origin);
-    const int64_t gi = origin + (int64_t)m * st;
-    const uint64_t pos = a.block_off[bid] + (uint64_t)(sw == 1 ? 0 : (sw == 2 ? g.c1 : g.c1 + g.c2)) + (uint64_t)x;
+    const int s = (int)a.s;
+    const int o0 = s * (int)pick3(P0, a.offs[0], a.offs[1], a.offs[2]),
+              o1 = s * (int)pick3(P1, a.offs[0], a.offs[1], a.offs[2]),
+              o2 = s * (int)pick3(P2, a.offs[0], a.offs[1], a.offs[2]);
+    const int origin = (int)(g.beg[0] * a.offs[0] + g.beg[1] * a.offs[1] + g.beg[2] * a.offs[2]) + c0 * o0 + c1 * o1 +
+                       c2 * o2;
+    const int st = sw == 1 ? o0 : (sw == 2 ? o1 : o2);
+    const Stencil<T> S = make_stencil<T>(m, n, a.cubic, st, 0);
+    const T pred = eval_stencil<CUB>(S, (const T *)W + origin);
+    const int gi = origin + m * st;
+    const uint64_t pos = base + (uint64_t)(sw == 1 ? 0 : (sw == 2 ? g.c1 : g.c1 + g.c2)) + x;
     if (!DECOMP) {
         T v = X[gi], uv;
         const int code = quant_point<T, QM>(v, pred, a, uv);
         codes[pos] = (uint16_t)code;
         if (code == 0) scratch[pos] = uv;
-        W[gi] = v;
+        // a level without finer ones is read by its own later sweeps alone
+        if (a.write_back || sw < 3) W[gi] = v;
     } else {
         W[gi] = recover_point<T, QM>(pred, (int)codes[pos], pos, a, zpos, nz, unpred);
     }
+}
+
+// Levels in few blocks (64 at the third level of a 512^3 field): one CTA per
+// block leaves most SMs idle while each block's sweeps run one after another, so
+// each sweep of the level is one launch over every block, a thread per target.
+// CTA c takes targets of chunk c % chunks of block c / chunks.
+template <typename T, bool DECOMP, int QM, int CUB>
+__global__ void __launch_bounds__(256) k_level_sweep(LevelArgs a, int sw, uint32_t chunks, const T *__restrict__ X,
+                                                    T *W, uint16_t *__restrict__ codes,
+                                                    T *__restrict__ scratch, const uint64_t *__restrict__ zpos,
+                                                    uint64_t nz, const T *__restrict__ unpred) {
+    __shared__ BlockGeom sgeo;
+    __shared__ uint64_t sbase;
+    const uint32_t bid = blockIdx.x / chunks, chunk = blockIdx.x - bid * chunks;
+    if (threadIdx.x == 0) {
+        int64_t bc[3];
+        block_coords(a, bid, bc);
+        block_geom(a, bc, sgeo);
+        sbase = a.block_off[bid];
+    }
+    __syncthreads();
+    const BlockGeom &g = sgeo;
+    const uint32_t cnt = (uint32_t)(sw == 1 ? g.c1 : (sw == 2 ? g.c2 : g.c3));
+    for (uint32_t x = chunk * 256u + threadIdx.x; x < cnt; x += chunks * 256u)
+        sweep_target<T, DECOMP, QM, CUB>(a, g, sbase, sw, x, X, W, codes, scratch, zpos, nz, unpred);
+}
+
+// The coarsest levels hold a few thousand points or fewer: a launch for each of
+// their sweeps is 5 us of latency for almost no work (21 launches on a 512^3 field,
+// 15 on a 33x47x61 one), so one CTA runs the first point and all of them, a
+// barrier between sweeps.
+constexpr int kSmallThreads = 1024;
+constexpr int64_t kSmallTargets = 4 * kSmallThreads;  // of a sweep: beyond some rounds of the CTA launches are faster
+template <typename T, bool DECOMP>
+__global__ void __launch_bounds__(kSmallThreads)
+    k_small_levels(const __grid_constant__ LevelTable t, int n, bool first_point, double eb, const T *__restrict__ X,
+                   T *W, uint16_t *__restrict__ codes, T *__restrict__ scratch, const uint64_t *__restrict__ zpos,
+                   uint64_t nz, const T *__restrict__ unpred) {
+    if (first_point && threadIdx.x == 0) {
+        const LevelArgs &a = t.a[0];
+        if (!DECOMP) {
+            T v = X[0], uv;
+            const int code = quantize(v, (T)0, eb, 1.0 / eb, a.radius, a.trim, uv);
+            codes[0] = (uint16_t)code;
+            if (code == 0) scratch[0] = uv;
+            W[0] = v;
+        } else {
+            W[0] = recover((T)0, (int)codes[0], 0, eb, a.radius, a.trim, zpos, nz, unpred);
+        }
+    }
+    for (int l = 0; l < n; l++) {
+        const LevelArgs &a = t.a[l];
+        const bool straight = sizeof(T) == 4 && a.fast && a.trim == 0;
+        const uint32_t nblocks = (uint32_t)(a.nb[0] * a.nb[1] * a.nb[2]);
+        // the first block has the most targets in every sweep
+        int64_t bc[3] = {0, 0, 0};
+        BlockGeom g;
+        block_geom(a, bc, g);
+        const uint32_t cmax[3] = {(uint32_t)g.c1, (uint32_t)g.c2, (uint32_t)g.c3};
+        for (int sw = 1; sw <= 3; sw++) {
+            __syncthreads();
+            const uint32_t cm = cmax[sw - 1];
+            for (uint32_t i = threadIdx.x; i < nblocks * cm; i += kSmallThreads) {
+                const uint32_t bid = i / cm, x = i - bid * cm;
+                if (nblocks > 1) {
+                    block_coords(a, bid, bc);
+                    block_geom(a, bc, g);
+                }
+                if (x >= (uint32_t)(sw == 1 ? g.c1 : (sw == 2 ? g.c2 : g.c3))) continue;
+                if (straight)
+                    sweep_target<T, DECOMP, 1, 1>(a, g, a.block_off[bid], sw, x, X, W, codes, scratch, zpos, nz, unpred);
+                else
+                    sweep_target<T, DECOMP, 0, 1>(a, g, a.block_off[bid], sw, x, X, W, codes, scratch, zpos, nz, unpred);
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256) k_block_offsets(const __grid_constant__ LevelTable t, uint64_t total,
+                                                      uint64_t *off) {
+    const uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= total) return;
+    int l = 0;
+    while (l + 1 < t.n && t.first[l + 1] <= i) l++;
+    int64_t bc[3];
+    block_coords(t.a[l], (int64_t)(i - t.first[l]), bc);
+    off[i] = t.pos[l] + codes_before(t.a[l], bc);
 }
 
 // ------------------------------------------------------ batched launch
@@ -643,14 +707,13 @@ size_t level_smem_bytes(const LevelArgs &a) {
     return vb + (size_t)a.stage_cap * sizeof(uint16_t);
 }
 
-// Coarse levels (stride >= 2) with few blocks, of fields below 2^31 values:
-// the three sweep launches of k_level_sweep instead of one CTA per block.
+// one launch per sweep (k_level_sweep), of fields below 2^31 values
 template <typename T>
 cudaError_t launch_level_sweeps(const LevelArgs &a, int64_t nblocks, bool decomp, const T *X, T *W, uint16_t *codes,
                                 T *scratch, const uint64_t *zpos, uint64_t nz, const T *unpred, cudaStream_t st,
                                 int *nlaunch) {
     const bool straight = sizeof(T) == 4 && a.fast && a.trim == 0;
-    void (*k)(LevelArgs, int, int64_t, const T *, T *, uint16_t *, T *, const uint64_t *, uint64_t, const T *);
+    void (*k)(LevelArgs, int, uint32_t, const T *, T *, uint16_t *, T *, const uint64_t *, uint64_t, const T *);
     if (a.cubic) {
         if (straight) k = decomp ? k_level_sweep<T, true, 1, 1> : k_level_sweep<T, false, 1, 1>;
         else k = decomp ? k_level_sweep<T, true, 0, 1> : k_level_sweep<T, false, 0, 1>;
@@ -658,21 +721,53 @@ cudaError_t launch_level_sweeps(const LevelArgs &a, int64_t nblocks, bool decomp
         if (straight) k = decomp ? k_level_sweep<T, true, 1, 0> : k_level_sweep<T, false, 1, 0>;
         else k = decomp ? k_level_sweep<T, true, 0, 0> : k_level_sweep<T, false, 0, 0>;
     }
-    // the first block has the most targets in every sweep (no first planes
-    // skipped, full extent)
-    int64_t bc0[3] = {0, 0, 0};
-    BlockGeom g0;
-    block_geom(a, bc0, g0);
-    const int64_t cmax[3] = {g0.c1, g0.c2, g0.c3};
+    // chunks by the targets of a middle block (all but the first along each axis
+    // skip their first planes), or of the only one; a first block's few more
+    // targets go round again
+    int64_t bc[3] = {0, 0, 0}, mid[3];
+    for (int i = 0; i < 3; i++) mid[i] = a.nb[i] > 2 ? 1 : 0;
+    BlockGeom g0, gm;
+    block_geom(a, bc, g0);
+    block_geom(a, mid, gm);
+    const int64_t most[3] = {g0.c1, g0.c2, g0.c3}, usual[3] = {gm.c1, gm.c2, gm.c3};
     for (int sw = 1; sw <= 3; sw++) {
-        if (cmax[sw - 1] <= 0) continue;
-        const int64_t chunks = (cmax[sw - 1] + 255) / 256;
-        k<<<(unsigned)(nblocks * chunks), 256, 0, st>>>(a, sw, chunks, X, W, codes, scratch, zpos, nz, unpred);
+        if (most[sw - 1] <= 0) continue;
+        const int64_t chunks = std::max<int64_t>(1, (usual[sw - 1] + 255) / 256);
+        k<<<(unsigned)(nblocks * chunks), 256, 0, st>>>(a, sw, (uint32_t)chunks, X, W, codes, scratch, zpos, nz, unpred);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         ++*nlaunch;
     }
     return cudaSuccess;
+}
+
+cudaError_t launch_block_offsets(const LevelTable &t, uint64_t nblocks, uint64_t *off, cudaStream_t st) {
+    if (nblocks == 0) return cudaSuccess;
+    k_block_offsets<<<(unsigned)((nblocks + 255) / 256), 256, 0, st>>>(t, nblocks, off);
+    return cudaGetLastError();
+}
+
+int small_levels(const LevelTable &t) {
+    int n = 0;
+    for (; n < t.n; n++) {
+        const LevelArgs &a = t.a[n];
+        if (a.dims[0] * a.dims[1] * a.dims[2] >= ((int64_t)1 << 31)) break;
+        int64_t bc[3] = {0, 0, 0};
+        BlockGeom g;
+        block_geom(a, bc, g);
+        const int64_t nblocks = a.nb[0] * a.nb[1] * a.nb[2];
+        if (nblocks > kSmallTargets || nblocks * std::max({g.c1, g.c2, g.c3}) > kSmallTargets) break;
+    }
+    return n;
+}
+
+template <typename T>
+cudaError_t launch_small_levels(const LevelTable &t, int n, bool decomp, bool first_point, double eb, const T *X, T *W,
+                                uint16_t *codes, T *scratch, const uint64_t *zpos, uint64_t nz, const T *unpred,
+                                cudaStream_t st) {
+    auto k = decomp ? k_small_levels<T, true> : k_small_levels<T, false>;
+    k<<<1, kSmallThreads, 0, st>>>(t, n, first_point, eb, X, W, codes, scratch, zpos, nz, unpred);
+    return cudaGetLastError();
 }
 
 template <typename T>
@@ -685,16 +780,20 @@ cudaError_t launch_level(const LevelArgs &a, int64_t nblocks, bool decomp, const
     int threads = vol >= 8192 ? 512 : (vol >= 1024 ? 256 : (vol >= 256 ? 128 : 64));
     const bool wide = a.dims[0] * a.dims[1] * a.dims[2] >= ((int64_t)1 << 31);
     const bool straight = sizeof(T) == 4 && a.fast && a.trim == 0;
-    // levels with fewer blocks than two per SM (the block kernel would leave
-    // SMs idle) take the sweep launches
+    // The sweep launches instead of a CTA per block: levels with fewer blocks than
+    // two per SM (the block kernel would leave SMs idle; the finest level of a
+    // 33x47x61 field has 8: 67 us there, 3 x 5 us in sweeps), and 2-D fields, whose
+    // 33 x 33 blocks are too small a job for a CTA that stages them (the finest level
+    // of 1800x3600, 6441 blocks: 94 us there, 32 + 53 us in sweeps).
     static const int sms = [] {
         int dev = 0, v = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
         return v > 0 ? v : 1;
     }();
+    const bool flat = a.dims[0] == 1 && a.dims[1] > 1;
     const int64_t per_block = (a.bs / a.s + 1) * (a.bs / a.s + 1) * (a.bs / a.s + 1) / 256 + 1;
-    if (a.s >= 2 && !wide && nblocks < 2 * sms && nblocks * per_block < (1ll << 31))
+    if (!wide && (flat || nblocks < 2 * sms) && nblocks * per_block < (1ll << 31))
         return launch_level_sweeps<T>(a, nblocks, decomp, X, W, codes, scratch, zpos, nz, unpred, st, nlaunch);
     // the finest level of a 3-D float field: plane-parallel kernel (finest.cu).
     // It compresses faster than the block kernel below but decompresses
@@ -762,6 +861,9 @@ cudaError_t launch_anchors(bool decomp, const T *X, T *W, uint16_t *codes, T *sc
     template size_t level_smem_bytes<T>(const LevelArgs &);                                                      \
     template cudaError_t launch_level<T>(const LevelArgs &, int64_t, bool, const T *, T *, uint16_t *, T *,      \
                                          const uint64_t *, uint64_t, const T *, cudaStream_t, int *);            \
+    template cudaError_t launch_small_levels<T>(const LevelTable &, int, bool, bool, double, const T *, T *,      \
+                                                uint16_t *, T *, const uint64_t *, uint64_t, const T *,          \
+                                                cudaStream_t);                                                    \
     template cudaError_t launch_first_point<T>(bool, const T *, T *, uint16_t *, T *, double, int, int,          \
                                                const uint64_t *, uint64_t, const T *, cudaStream_t);             \
     template cudaError_t launch_anchors<T>(bool, const T *, T *, uint16_t *, T *, const T *, const int64_t *,   \

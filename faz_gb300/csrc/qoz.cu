@@ -768,14 +768,17 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
         huffman_encode_device(qb, ns, 32768, x.m, s, x.launches, h, x.tm);
         // unpredictable values in the order the quantiser kept them
         // (block by block, stream order): zeros of the block-major codes
-        const uint64_t nsub = hist_subchunks(ns);
-        unsigned long long *zc = x.m.alloc<unsigned long long>(nsub + 1), *zoff = x.m.alloc<unsigned long long>(nsub + 1);
-        unsigned long long *ztmp = x.m.alloc<unsigned long long>(scan_temp_words(nsub) + 1);
-        x.launches(launch_count_zeros(x.codes, ns, zc, s));
-        x.launches(launch_scan_u64(zc, zoff, nsub, ztmp, s));
         const uint64_t nunp = h.nzero;
-        T *unp = x.m.alloc<T>(nunp ? nunp : 1);
-        if (nunp) x.launches(launch_compact_zeros<T>(x.codes, ns, zc, zoff, x.scratch, unp, s));
+        T *unp = nullptr;
+        if (nunp) {
+            const uint64_t nsub = hist_subchunks(ns);
+            unsigned long long *zc = x.m.alloc<unsigned long long>(2 * (nsub + 1) + scan_temp_words(nsub) + 1),
+                               *zoff = zc + nsub + 1;
+            unp = x.m.alloc<T>(nunp);
+            x.launches(launch_count_zeros(x.codes, ns, zc, s));
+            x.launches(launch_scan_u64(zc, zoff, nsub, zoff + nsub + 1, s));
+            x.launches(launch_compact_zeros<T>(x.codes, ns, zc, zoff, x.scratch, unp, s));
+        }
         std::vector<uint8_t> head;
         put<uint8_t>(head, 2);
         put<double>(head, eb);

@@ -1805,7 +1805,7 @@ void decompress_device(const uint8_t *pl, size_t n, Parsed &P, T *dOut, cudaStre
     if (pl_.anchor && P.nunpred < pl_.nanchor)
         throw Fail{FAZ_ERR_FORMAT, "unpredictable count does not match the zero codes"};
     DevMem m(st);
-    uint16_t *codes = m.alloc<uint16_t>(num);
+    uint16_t *codes = m.alloc<uint16_t>(num + 8);  // the plane kernel reads whole 16 bytes
     T *dunpred = m.alloc<T>(P.nunpred ? P.nunpred : 1);
     if (P.nunpred) CK(cudaMemcpyAsync(dunpred, P.unpred, P.nunpred * sizeof(T), cudaMemcpyHostToDevice, st));
     Events ev_dec, ev_pred, ev_fin;

@@ -795,15 +795,14 @@ cudaError_t launch_level(const LevelArgs &a, int64_t nblocks, bool decomp, const
     const int64_t per_block = (a.bs / a.s + 1) * (a.bs / a.s + 1) * (a.bs / a.s + 1) / 256 + 1;
     if (!wide && (flat || nblocks < 2 * sms) && nblocks * per_block < (1ll << 31))
         return launch_level_sweeps<T>(a, nblocks, decomp, X, W, codes, scratch, zpos, nz, unpred, st, nlaunch);
-    // the finest level of a 3-D float field: plane-parallel kernel (finest.cu).
-    // It compresses faster than the block kernel below but decompresses
-    // slower (0.95 vs 0.86 ms on 512^3), so decompression keeps the block
-    // kernel.  FAZ_FINEST_PLANES (read per call, for comparisons): 0 = block
-    // kernel for both, 2 = plane kernel for both.
+    // the finest level of a 3-D float field: plane-parallel kernel (finest.cu, with
+    // both kernels' times; on 512^3 0.45 ms against 0.83 ms for the block kernel
+    // below, decompression 0.48 against 0.77 ms).  FAZ_FINEST_PLANES=0 (read per
+    // call, for comparisons): the block kernel.
     const char *plane_env = std::getenv("FAZ_FINEST_PLANES");
-    const int plane_mode = plane_env && plane_env[0] == '0' ? 0 : (plane_env && plane_env[0] == '2' ? 2 : 1);
+    const bool planes = !(plane_env && plane_env[0] == '0');
     if constexpr (sizeof(T) == 4) {
-        if ((decomp ? plane_mode == 2 : plane_mode >= 1) && finest_eligible(a, decomp, X, sizeof(T))) {
+        if (planes && finest_eligible(a, decomp, X, W, sizeof(T))) {
             ++*nlaunch;
             return launch_finest(a, nblocks, decomp, reinterpret_cast<const float *>(X), reinterpret_cast<float *>(W),
                                  codes, reinterpret_cast<float *>(scratch), zpos, nz,

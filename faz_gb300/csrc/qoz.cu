@@ -12,9 +12,9 @@
 // mode 1: codes, bit rate after Huffman + zstd, PSNR from summed squared
 // errors).  On the GPU one launch per level and sweep covers every sampled
 // block (one thread per target); each target's error lands at its stream
-// position and k_qz_sum adds the errors in the reference's nesting (per line,
-// then per level block, then a running total), so the sums and therefore
-// the decisions are those of the reference.  The decision logic is the
+// position and k_qz_line_sums / k_qz_sum add the errors in the reference's nesting
+// (per line, then per level block, then a running total), so the sums and
+// therefore the decisions are those of the reference.  The decision logic is the
 // reference's, on the host.
 #include <cuda_runtime.h>
 
@@ -149,6 +149,7 @@ __global__ void k_qz_first(LevelArgs q, T *__restrict__ data, int64_t per, int64
 
 struct SumSeg {
     int64_t off;    // first slot
+    int64_t line0;  // lines of the sweeps before
     int64_t lines;  // lines of this sweep
     int64_t tpl;    // targets per line
     int level_end;  // 1 when this is the level's last sweep
@@ -157,31 +158,73 @@ constexpr int kMaxSegs = 64;
 struct SumPlan {
     int nseg;
     int64_t cpb;
+    int64_t nlines;  // of all sweeps
     SumSeg seg[kMaxSegs];
 };
 
 // Per block: sum of line sums per level block, running total over levels
-// (block_interpolation_1d / block_interpolation / compress accumulation).
-__global__ void k_qz_sum(SumPlan p, const double *__restrict__ err, double *__restrict__ out, uint64_t nblk) {
-    const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nblk) return;
-    const double *e = err + k * (uint64_t)p.cpb;
+// (block_interpolation_1d / block_interpolation / compress accumulation).  The
+// doubles are added in that order exactly, and only the additions of different
+// lines commute with one another: one thread per line for the sums inside the
+// lines, then one chain per block over its line sums, from shared memory.  With
+// both in one thread per block the 35936 errors of a 33^3 block were one chain of
+// dependent loads and additions, 2.46 ms a launch, 95% of the tuner's time on the
+// GPU.
+__global__ void k_qz_line_sums(SumPlan p, const double *__restrict__ err, double *__restrict__ lsum, uint64_t total) {
+    const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= total) return;
+    const uint64_t k = idx / (uint64_t)p.nlines;
+    const int64_t l = (int64_t)(idx - k * (uint64_t)p.nlines);
+    int sgi = 0;
+    while (sgi + 1 < p.nseg && l >= p.seg[sgi + 1].line0) sgi++;
+    const int64_t tpl = p.seg[sgi].tpl;
+    const double *x = err + k * (uint64_t)p.cpb + p.seg[sgi].off + (l - p.seg[sgi].line0) * tpl;
+    double ls = 0;
+#pragma unroll 8
+    for (int64_t t = 0; t < tpl; t++) ls += x[t];
+    lsum[idx] = ls;
+}
+
+constexpr int kSumChunk = 2048;
+__global__ void __launch_bounds__(256) k_qz_sum(SumPlan p, const double *__restrict__ lsum, double *__restrict__ out) {
+    __shared__ double buf[kSumChunk];
+    const double *src = lsum + (uint64_t)blockIdx.x * (uint64_t)p.nlines;
     double total = 0, blk = 0;
-    for (int sgi = 0; sgi < p.nseg; sgi++) {
-        const SumSeg sg = p.seg[sgi];
-        const double *x = e + sg.off;
-        for (int64_t l = 0; l < sg.lines; l++) {
-            double ls = 0;
-            for (int64_t t = 0; t < sg.tpl; t++) ls += x[t];
-            blk += ls;
-            x += sg.tpl;
+    int sgi = 0;
+    for (int64_t c0 = 0; c0 < p.nlines; c0 += kSumChunk) {
+        const int64_t c1 = c0 + kSumChunk < p.nlines ? c0 + kSumChunk : p.nlines;
+        for (int64_t i = c0 + threadIdx.x; i < c1; i += blockDim.x) buf[i - c0] = src[i];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int64_t l = c0; l < c1;) {
+                const int64_t end = p.seg[sgi].line0 + p.seg[sgi].lines;
+                const int n = (int)((end < c1 ? end : c1) - l);
+                const double *b = buf + (l - c0);
+#pragma unroll 8
+                for (int i = 0; i < n; i++) blk += b[i];
+                l += n;
+                if (l < end) break;  // the sweep goes on in the next chunk
+                if (p.seg[sgi].level_end) {
+                    total += blk;
+                    blk = 0;
+                }
+                sgi++;
+            }
         }
-        if (sg.level_end) {
-            total += blk;
-            blk = 0;
-        }
+        __syncthreads();
     }
-    out[k] = total;
+    if (threadIdx.x == 0) out[blockIdx.x] = total;
+}
+
+void launch_qz_sum(const SumPlan &p, const double *err, double *lsum, double *out, uint64_t nblk, cudaStream_t st,
+                   Counter &launches) {
+    const uint64_t total = (uint64_t)p.nlines * nblk;
+    if (total) {
+        k_qz_line_sums<<<(unsigned)((total + 127) / 128), 128, 0, st>>>(p, err, lsum, total);
+        launches(cudaGetLastError());
+    }
+    k_qz_sum<<<(unsigned)nblk, 256, 0, st>>>(p, lsum, out);
+    launches(cudaGetLastError());
 }
 
 // q_bins of CompressTest: for each level range, every block's codes of it.
@@ -230,6 +273,7 @@ struct QzGeom {
     int64_t na[3];         // anchors per axis in tuning mode 1
     int64_t nanchor;
     int64_t cpb;           // stream slots per block (full run, mode 1)
+    int64_t lpb;           // lines per block (full run)
 };
 
 QzGeom make_geom(int N, int64_t bsz, int64_t maxStep) {
@@ -282,6 +326,7 @@ void qz_run(const QzGeom &g, const QzRun &R, T *work, uint16_t *codes, T *scratc
             SumPlan &sp, std::vector<std::pair<int64_t, int64_t>> *level_ranges, cudaStream_t st, Counter &launches) {
     sp.nseg = 0;
     sp.cpb = g.cpb;
+    sp.nlines = 0;
     int64_t pos = 0;
     int start = R.start_level;
     if (!g.anchor) {
@@ -402,7 +447,8 @@ void qz_run(const QzGeom &g, const QzRun &R, T *work, uint16_t *codes, T *scratc
                 launches(cudaGetLastError());
             }
             if (sp.nseg >= kMaxSegs) throw Fail{FAZ_ERR_UNSUPPORTED, "too many tuning levels"};
-            sp.seg[sp.nseg++] = SumSeg{pos, lines, w.tpl, d == g.N - 1 ? 1 : 0};
+            sp.seg[sp.nseg++] = SumSeg{pos, sp.nlines, lines, w.tpl, d == g.N - 1 ? 1 : 0};
+            sp.nlines += lines;
             pos += lines * w.tpl;
         }
         if (level_ranges) {
@@ -412,9 +458,9 @@ void qz_run(const QzGeom &g, const QzRun &R, T *work, uint16_t *codes, T *scratc
     }
 }
 
-// Codes per block of a full tuning-1 run.
-int64_t full_run_slots(const QzGeom &g) {
-    int64_t p = g.anchor ? g.nanchor : 1;
+// Codes and lines per block of a full tuning-1 run.
+void full_run_sizes(QzGeom &g) {
+    int64_t p = g.anchor ? g.nanchor : 1, nl = 0;
     for (int level = g.levels - (g.anchor ? 1 : 0); level > 0; level--) {
         const int64_t s = (int64_t)1 << (level - 1);
         for (int sw = 0; sw < g.N; sw++) {
@@ -422,9 +468,11 @@ int64_t full_run_slots(const QzGeom &g) {
             for (int u = 0; u < g.N; u++)
                 if (u != sw) lines *= (g.bsz - 1) / (u < sw ? s : 2 * s) + 1;
             p += lines * (((g.bsz - 1) / s + 1) / 2);
+            nl += lines;
         }
     }
-    return p;
+    g.cpb = p;
+    g.lpb = nl;
 }
 
 // profiling_block_2d / profiling_block_3d (include/QoZ/utils/Sample.hpp:13-67,
@@ -643,11 +691,11 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
         starts = plain_starts(c.predictorTuningRate);
     }
     QzGeom g = make_geom(N, bsz, (int64_t)c.maxStep);
-    g.cpb = full_run_slots(g);
+    full_run_sizes(g);
     uint64_t nblk = 0, nv = 0, ns = 0;
     T *blocks = nullptr, *work = nullptr, *scratch = nullptr;
     uint16_t *codes = nullptr;
-    double *err = nullptr, *bsum = nullptr;
+    double *err = nullptr, *lsum = nullptr, *bsum = nullptr;
     std::vector<double> hsum;
     // the sampled blocks and the buffers sized by their count
     auto gather = [&](const std::vector<int64_t> &sts) {
@@ -660,6 +708,7 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
         scratch = m.alloc<T>(ns);
         codes = m.alloc<uint16_t>(ns);
         err = m.alloc<double>(ns);
+        lsum = m.alloc<double>(nblk * (uint64_t)g.lpb + 1);
         bsum = m.alloc<double>(nblk);
         hsum.assign(nblk, 0.0);
         int64_t *dstarts = m.alloc<int64_t>(sts.size());
@@ -672,8 +721,7 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
     gather(starts);
     mark("sampled blocks", (double)nblk, (double)nv);
     auto block_sums = [&](const SumPlan &sp) -> double {
-        k_qz_sum<<<(unsigned)((nblk + 63) / 64), 64, 0, st>>>(sp, err, bsum, nblk);
-        launches(cudaGetLastError());
+        launch_qz_sum(sp, err, lsum, bsum, nblk, st, launches);
         CK(cudaMemcpyAsync(hsum.data(), bsum, nblk * 8, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         double s = 0;
@@ -704,17 +752,18 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
         DevMem m;
         T *work, *scratch;
         uint16_t *codes;
-        double *err, *bsum;
+        double *err, *lsum, *bsum;
         std::vector<double> hsum;
         SumPlan sp;
         std::vector<std::pair<int64_t, int64_t>> ranges;
         Counter launches;
         faz_timings tm;
-        CtCtx(cudaStream_t s, uint64_t nv_, uint64_t ns_, uint64_t nblk_) : m(s), hsum(nblk_, 0.0) {
+        CtCtx(cudaStream_t s, uint64_t nv_, uint64_t ns_, uint64_t nblk_, uint64_t lpb_) : m(s), hsum(nblk_, 0.0) {
             work = m.alloc<T>(nv_);
             scratch = m.alloc<T>(ns_);
             codes = m.alloc<uint16_t>(ns_);
             err = m.alloc<double>(ns_);
+            lsum = m.alloc<double>(nblk_ * lpb_ + 1);
             bsum = m.alloc<double>(nblk_);
             std::memset(&tm, 0, sizeof(tm));
         }
@@ -734,8 +783,7 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
         CK(cudaMemcpyAsync(x.work, blocks, nv * sizeof(T), cudaMemcpyDeviceToDevice, s));
         QzRun R{1, g.levels, 0, eb, alpha, beta, c.trimToZero, op, dir, lists ? &il : nullptr, lists ? &dl : nullptr};
         qz_run<T>(g, R, x.work, x.codes, x.scratch, x.err, nblk, x.sp, &x.ranges, s, x.launches);
-        k_qz_sum<<<(unsigned)((nblk + 63) / 64), 64, 0, s>>>(x.sp, x.err, x.bsum, nblk);
-        x.launches(cudaGetLastError());
+        launch_qz_sum(x.sp, x.err, x.lsum, x.bsum, nblk, s, x.launches);
         CK(cudaMemcpyAsync(x.hsum.data(), x.bsum, nblk * 8, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         double se = 0;
@@ -817,7 +865,7 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
     std::unique_ptr<CtCtx> main_ctx;
     auto compress_test = [&](int op, int dir, double alpha, double beta, double eb, double &bitrate, double &psnr,
                              bool lists = true, double pc = 1.0) {
-        if (!main_ctx || main_ctx->hsum.size() != nblk) main_ctx.reset(new CtCtx(st, nv, ns, nblk));
+        if (!main_ctx || main_ctx->hsum.size() != nblk) main_ctx.reset(new CtCtx(st, nv, ns, nblk, (uint64_t)g.lpb));
         compress_test_on(*main_ctx, st, op, dir, alpha, beta, eb, bitrate, psnr, lists, pc);
         launches.n += main_ctx->launches.n;
         main_ctx->launches.n = 0;
@@ -944,7 +992,7 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
             const double alpha = ab.first, beta = ab.second;
             futs.push_back(TaskThreads::get().submit<GridRes>([&, alpha, beta]() {
                 StreamGuard sg(nullptr);
-                CtCtx x(sg.st, nv, ns, nblk);
+                CtCtx x(sg.st, nv, ns, nblk, (uint64_t)g.lpb);
                 GridRes r;
                 compress_test_on(x, sg.st, op0, dir0, alpha, beta, oriabseb, r.br, r.mm, true, pcoeff);
                 CK(cudaStreamSynchronize(sg.st));
@@ -1013,7 +1061,7 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
                 const double alpha = dv.alpha, beta = dv.beta, ebd = dv.eb;
                 dfut.push_back(TaskThreads::get().submit<GridRes>([&, alpha, beta, ebd]() {
                     StreamGuard sg(nullptr);
-                    CtCtx x(sg.st, nv, ns, nblk);
+                    CtCtx x(sg.st, nv, ns, nblk, (uint64_t)g.lpb);
                     GridRes r;
                     compress_test_on(x, sg.st, op0, dir0, alpha, beta, ebd, r.br, r.mm, true, pcoeff);
                     CK(cudaStreamSynchronize(sg.st));

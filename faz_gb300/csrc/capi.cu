@@ -1819,10 +1819,19 @@ const uint64_t *queue_zero_positions(const HuffDecode<C> &h, uint64_t expect, De
 // section of nunpred values.
 template <typename C>
 void decode_with_zeros_impl(const uint8_t *&p, const uint8_t *end, uint64_t num, uint64_t nunpred, C *codes, DevMem &m,
-                            cudaStream_t st, Counter &launches, uint64_t *&zpos) {
+                            cudaStream_t st, Counter &launches, uint64_t *&zpos,
+                            const std::function<void()> &meanwhile) {
     HuffDecode<C> h;
     h.begin(p, end, num, codes, m, st, launches);
     const uint64_t *hz = queue_zero_positions(h, nunpred, m, st, launches, zpos);
+    if (meanwhile) {
+        try {
+            meanwhile();
+        } catch (...) {
+            cudaStreamSynchronize(st);  // the copies from the caller's stream end first
+            throw;
+        }
+    }
     CK(cudaStreamSynchronize(st));
     if (h.settle(m, st, launches)) {
         hz = queue_zero_positions(h, nunpred, m, st, launches, zpos);
@@ -1831,12 +1840,14 @@ void decode_with_zeros_impl(const uint8_t *&p, const uint8_t *end, uint64_t num,
     if (*hz != nunpred) throw Fail{FAZ_ERR_FORMAT, "unpredictable count does not match the zero codes"};
 }
 void decode_with_zeros(const uint8_t *&p, const uint8_t *end, uint64_t num, uint64_t nunpred, uint16_t *codes,
-                       DevMem &m, cudaStream_t st, Counter &launches, uint64_t *&zpos) {
-    decode_with_zeros_impl(p, end, num, nunpred, codes, m, st, launches, zpos);
+                       DevMem &m, cudaStream_t st, Counter &launches, uint64_t *&zpos,
+                       const std::function<void()> &meanwhile) {
+    decode_with_zeros_impl(p, end, num, nunpred, codes, m, st, launches, zpos, meanwhile);
 }
 void decode_with_zeros(const uint8_t *&p, const uint8_t *end, uint64_t num, uint64_t nunpred, uint32_t *codes,
-                       DevMem &m, cudaStream_t st, Counter &launches, uint64_t *&zpos) {
-    decode_with_zeros_impl(p, end, num, nunpred, codes, m, st, launches, zpos);
+                       DevMem &m, cudaStream_t st, Counter &launches, uint64_t *&zpos,
+                       const std::function<void()> &meanwhile) {
+    decode_with_zeros_impl(p, end, num, nunpred, codes, m, st, launches, zpos, meanwhile);
 }
 
 namespace {

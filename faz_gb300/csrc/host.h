@@ -593,10 +593,13 @@ void huffman_decode_device(const uint8_t *&p, const uint8_t *end, uint64_t num, 
 void huffman_decode_device(const uint8_t *&p, const uint8_t *end, uint64_t num, uint32_t *codes, DevMem &m,
                            cudaStream_t st, Counter &launches);
 // Decode num codes that hold nunpred zeros (else FAZ_ERR_FORMAT), with the
-// zeros' sorted positions in zpos.
+// zeros' sorted positions in zpos.  `meanwhile`, when given, runs on the host while
+// the GPU decodes.
 void decode_with_zeros(const uint8_t *&p, const uint8_t *end, uint64_t num, uint64_t nunpred, uint16_t *codes,
-                       DevMem &m, cudaStream_t st, Counter &launches, uint64_t *&zpos);
+                       DevMem &m, cudaStream_t st, Counter &launches, uint64_t *&zpos,
+                       const std::function<void()> &meanwhile = {});
 void decode_with_zeros(const uint8_t *&p, const uint8_t *end, uint64_t num, uint64_t nunpred, uint32_t *codes,
-                       DevMem &m, cudaStream_t st, Counter &launches, uint64_t *&zpos);
+                       DevMem &m, cudaStream_t st, Counter &launches, uint64_t *&zpos,
+                       const std::function<void()> &meanwhile = {});
 
 }  // namespace faz

@@ -18,6 +18,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -1135,6 +1136,10 @@ void lorenzo3_decompress(const uint8_t *pl, size_t psize, const uint64_t *dims, 
     huffman_decode_device(p, end, nb, ind, m, st, launches);
     if (reg_count > nb) throw Fail{FAZ_ERR_FORMAT, "bad regression block count"};
     float *drec = nullptr;
+    // the coefficients' chain, on the host: runs while the GPU decodes the codes
+    // (0.7 of the 1.3 ms before the wavefront of a 100x500x500 field when it came
+    // first)
+    std::function<void()> chain;
     if (reg_count) {
         // decode_regression_coefficients (MetaRegressionPredictor.hpp:42-80)
         need(8);
@@ -1154,9 +1159,11 @@ void lorenzo3_decompress(const uint8_t *pl, size_t psize, const uint64_t *dims, 
         uint64_t nreg = 0;
         for (uint64_t b = 0; b < nb; b++) nreg += hind[b] == 1;
         if (nreg != reg_count) throw Fail{FAZ_ERR_FORMAT, "regression block count does not match the indicators"};
-        reg_chain_decompress<T>(hind, nb, htypes, 4 * reg_count, runp, nrunp, eb_lin, eb_ind, rec);
         drec = m.alloc<float>(4 * nb);
-        CK(cudaMemcpyAsync(drec, rec, nb * 16, cudaMemcpyHostToDevice, st));
+        chain = [=]() {
+            reg_chain_decompress<T>(hind, nb, htypes, 4 * reg_count, runp, nrunp, eb_lin, eb_ind, rec);
+            CK(cudaMemcpyAsync(drec, rec, nb * 16, cudaMemcpyHostToDevice, st));
+        };
     }
     need(1 + 8 + 4 + 8);
     p += 1;
@@ -1181,8 +1188,8 @@ void lorenzo3_decompress(const uint8_t *pl, size_t psize, const uint64_t *dims, 
     uint32_t *codes32 = wide ? m.alloc<uint32_t>(n) : nullptr;
     uint64_t *zpos = nullptr;
     const uint64_t nz = nunpred;
-    if (wide) decode_with_zeros(p, end, n, nz, codes32, m, st, launches, zpos);
-    else decode_with_zeros(p, end, n, nz, codes16, m, st, launches, zpos);
+    if (wide) decode_with_zeros(p, end, n, nz, codes32, m, st, launches, zpos, chain);
+    else decode_with_zeros(p, end, n, nz, codes16, m, st, launches, zpos, chain);
     CK(cudaEventRecord(ev_dec.b, st));
     LorArgs a = make_args<T>(dims, bs, pd, 1, 1, eb, radius);
     a.rp = drec;

@@ -456,17 +456,16 @@ void huffman_encode_impl(const C *codes, uint64_t n, int center, DevMem &m, cuda
     if (sized) sized(h);
     const uint64_t nwords = (total_bits + 31) / 32 + 1;
     h.bits = m.alloc<uint32_t>(nwords);
-    CK(cudaMemsetAsync(h.bits, 0, nwords * 4, st));
     if (!total_bits) return;
-    launches(launch_encode_bits(codes, n, cb.offset, reinterpret_cast<const uint8_t *>(dtab + 2 * S), cbits, st));
-    launches(launch_scan_u64(cbits, coff, nech, stmp, st));
-    const EncodeArgs ea{cb.offset, std::max(cb.maxlen, 1), dtab, dtab + S, coff, h.bits};
+    const EncodeArgs ea{cb.offset, std::max(cb.maxlen, 1), dtab, dtab + S, reinterpret_cast<const uint8_t *>(dtab + 2 * S),
+                        cbits,     coff,                   h.bits};
     // strings of 16 MB or more in slices, whose copies overlap the next ones
     const int slices = sliced && h.nbytes >= (16u << 20) ? kSlices : 1;
     h.end = (const volatile uint64_t *)t_pin_encode.get(kSlices * 8);
     for (int k = 0; k < slices; k++) {
         launches(launch_encode_pack(ea, codes, n, nech * k / slices, nech * (k + 1) / slices,
                                     slices > 1 ? (unsigned long long *)h.end + k : nullptr, st));
+        launches.n += 2;  // three kernels
         if (slices == 1) break;
         h.done.push_back(std::make_shared<Event>());
         CK(cudaEventRecord(h.done.back()->e, st));

@@ -155,11 +155,6 @@ uint64_t scan_temp_words(uint64_t n);
 cudaError_t launch_scan_u64(const unsigned long long *in, unsigned long long *out, uint64_t n,
                             unsigned long long *temp, cudaStream_t st);
 uint64_t encode_chunks(uint64_t n);
-// bits of every chunk
-cudaError_t launch_encode_bits(const uint16_t *codes, uint64_t n, int offset, const uint8_t *len,
-                               unsigned long long *chunkbits, cudaStream_t st);
-cudaError_t launch_encode_bits(const uint32_t *codes, uint64_t n, int offset, const uint8_t *len,
-                               unsigned long long *chunkbits, cudaStream_t st);
 // The stage for a batch of runs of n codes each (the QoZ tuner's tests): run y's
 // codes, and its histogram, positions, counts and list, are a stride from those of
 // the run before (8-byte words); its string's tables and output are tasks[y]; the
@@ -182,12 +177,14 @@ cudaError_t launch_encode_bits_batch(const uint16_t *codes, uint64_t cs, uint64_
 cudaError_t launch_encode_pack_batch(const uint16_t *codes, uint64_t cs, uint64_t n, unsigned runs,
                                      const EncodeTask *tasks, int maxlen, const unsigned long long *chunkoff,
                                      cudaStream_t st);
-// Bit packing of chunks [chunk0, chunk1) of n codes: code tables, the exclusive
-// scan of the chunks' bits, the zeroed output.  host_end (pinned, or null) receives
-// the bits before chunk1.
+// Bit counts, offsets and packing of chunks [chunk0, chunk1) of n codes, after the
+// chunks before them: code tables, bits and offsets per chunk, the output.  Three
+// launches.  host_end (pinned, or null) receives the bits before chunk1.
 struct EncodeArgs {
     int offset, maxlen;
-    const unsigned long long *code64, *packed, *chunkoff;
+    const unsigned long long *code64, *packed;
+    const uint8_t *len;
+    unsigned long long *chunkbits, *chunkoff;
     uint32_t *out;
 };
 cudaError_t launch_encode_pack(const EncodeArgs &a, const uint16_t *codes, uint64_t n, uint64_t chunk0,

@@ -630,8 +630,7 @@ __device__ __forceinline__ void minmax_body(const T *__restrict__ X, uint64_t n,
     const uint64_t nvec = (n - h) / V;
     const uint64_t tid = bid * (uint64_t)blockDim.x + threadIdx.x, nth = (uint64_t)nblocks * blockDim.x;
     const uint4 *xv = reinterpret_cast<const uint4 *>(X + h);
-    for (uint64_t i = tid; i < nvec; i += nth) {
-        uint4 q = __ldg(xv + i);
+    auto take = [&](const uint4 &q) {
         const T *e = reinterpret_cast<const T *>(&q);
 #pragma unroll
         for (int k = 0; k < V; k++) {
@@ -639,7 +638,16 @@ __device__ __forceinline__ void minmax_body(const T *__restrict__ X, uint64_t n,
             mn = v < mn ? v : mn;
             mx = v > mx ? v : mx;
         }
+    };
+    uint64_t iv = tid;
+    for (; iv + 3 * nth < nvec; iv += 4 * nth) {
+        uint4 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) q[u] = __ldg(xv + iv + u * nth);
+#pragma unroll
+        for (int u = 0; u < 4; u++) take(q[u]);
     }
+    for (; iv < nvec; iv += nth) take(__ldg(xv + iv));
     for (uint64_t i = tid; i < h; i += nth) {
         T v = X[i];
         mn = v < mn ? v : mn;

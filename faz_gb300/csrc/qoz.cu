@@ -1100,19 +1100,16 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
         };
         // The tests the search derives (at the bound scaled by a point's bit
         // rate over the best one) follow from the grid's results as long as
-        // no derived test moves the best point, which is rare: when the search
-        // asks for a test that has not run, walk the rest of it under that
-        // assumption and run the derived tests it meets at once.  The search
-        // takes a result only where its bound is the one it asks for.  (One by
-        // one after the best point moved they took 0.63 ms each, 7.6 ms of a 300^3
-        // field's 9.8 ms tuning; 13 at once 0.95.)
+        // no derived test moves the best point, which is rare: walk the
+        // search under that assumption, run the derived tests it meets at
+        // once, and let the search below take a result only where its bound
+        // is the one the search asks for (else that test runs again).
         std::vector<Test> derived;
         std::vector<TestRes> dres;
-        auto derive = [&](size_t a0, size_t b0, double bb, double bm) {
-            derived.clear();
-            for (size_t ai = a0; ai < alist.size(); ai++) {
-                for (size_t bi = ai == a0 ? b0 : 0; bi < blist.size(); bi++) {
-                    const double alpha = alist[ai], beta = blist[bi];
+        {
+            double bb = 9999, bm = 0;
+            for (double alpha : alist) {
+                for (double beta : blist) {
                     if ((alpha >= 1 && alpha > beta) || (alpha < 0 && beta != -1)) continue;
                     double br, mm;
                     grid_result(alpha, beta, br, mm);
@@ -1130,24 +1127,19 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
                 }
             }
             dres = run_tests(derived, pcoeff);
-            mark("derived tests", (double)derived.size());
-        };
-        auto derived_test = [&](size_t ai, size_t bi, double ebd, double &br, double &mm) {
-            const double alpha = alist[ai], beta = blist[bi];
-            for (int pass = 0; pass < 2; pass++) {
-                for (size_t i = 0; i < derived.size(); i++)
-                    if (derived[i].alpha == alpha && derived[i].beta == beta && derived[i].eb == ebd) {
-                        br = dres[i].br;
-                        mm = dres[i].mm;
-                        return;
-                    }
-                if (pass == 0) derive(ai, bi, bestb, bestm);
-            }
+        }
+        mark("derived tests", (double)derived.size());
+        auto derived_test = [&](double alpha, double beta, double ebd, double &br, double &mm) {
+            for (size_t i = 0; i < derived.size(); i++)
+                if (derived[i].alpha == alpha && derived[i].beta == beta && derived[i].eb == ebd) {
+                    br = dres[i].br;
+                    mm = dres[i].mm;
+                    return;
+                }
             compress_test(op0, dir0, alpha, beta, ebd, br, mm, true, pcoeff);
         };
-        for (size_t ai = 0; ai < alist.size(); ai++) {
-            for (size_t bi = 0; bi < blist.size(); bi++) {
-                const double alpha = alist[ai], beta = blist[bi];
+        for (double alpha : alist) {
+            for (double beta : blist) {
                 if ((alpha >= 1 && alpha > beta) || (alpha < 0 && beta != -1)) continue;
                 double br, mm;
                 grid_result(alpha, beta, br, mm);
@@ -1164,7 +1156,7 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
                 } else {
                     const double fix = br / bestb;
                     double br2, m2;
-                    derived_test(ai, bi, oriabseb * fix, br2, m2);
+                    derived_test(alpha, beta, oriabseb * fix, br2, m2);
                     if (cr) m2 = 0;
                     const double a = (mm - m2) / (br - br2);
                     const double b = mm - a * br;

@@ -358,7 +358,7 @@ struct Sink {
 template <typename C>
 void huffman_encode_impl(const C *codes, uint64_t n, int center, DevMem &m, cudaStream_t st, Counter &launches,
                          HuffEncoded &h, faz_timings &tm, const std::function<void(const HuffEncoded &)> &sized,
-                         bool sliced) {
+                         bool sliced, bool zero_scan) {
     const uint64_t nsub = hist_subchunks(n);
     const uint64_t nech = encode_chunks(n);
     // every value a code of this width can take
@@ -403,7 +403,7 @@ void huffman_encode_impl(const C *codes, uint64_t n, int center, DevMem &m, cuda
     std::memcpy(&h.nzero, hb + 8, 8);
     if (nl > (unsigned int)nsym || nl > list_cap)
         throw Fail{FAZ_ERR_DEVICE, "histogram list longer than the symbol range"};
-    if (h.nzero) launches(launch_scan_u64(h.zc, h.zoff, nsub, stmp, st));
+    if (h.nzero && zero_scan) launches(launch_scan_u64(h.zc, h.zoff, nsub, stmp, st));
     std::vector<unsigned long long> rest;
     if (nl > kListHead) {
         rest.resize(3 * (size_t)(nl - kListHead));
@@ -474,130 +474,17 @@ void huffman_encode_impl(const C *codes, uint64_t n, int center, DevMem &m, cuda
 
 void huffman_encode_device(const uint16_t *codes, uint64_t n, int center, DevMem &m, cudaStream_t st,
                            Counter &launches, HuffEncoded &h, faz_timings &tm,
-                           const std::function<void(const HuffEncoded &)> &sized, bool sliced) {
-    huffman_encode_impl(codes, n, center, m, st, launches, h, tm, sized, sliced);
+                           const std::function<void(const HuffEncoded &)> &sized, bool sliced, bool zero_scan) {
+    huffman_encode_impl(codes, n, center, m, st, launches, h, tm, sized, sliced, zero_scan);
 }
 void huffman_encode_device(const uint32_t *codes, uint64_t n, int center, DevMem &m, cudaStream_t st,
                            Counter &launches, HuffEncoded &h, faz_timings &tm,
                            const std::function<void(const HuffEncoded &)> &sized, bool sliced) {
     if (center < 0 || center > (1 << 20)) throw Fail{FAZ_ERR_UNSUPPORTED, "quantisation radius too large"};
-    huffman_encode_impl(codes, n, center, m, st, launches, h, tm, sized, sliced);
+    huffman_encode_impl(codes, n, center, m, st, launches, h, tm, sized, sliced, true);
 }
 
 // HuffmanEncoder::save header + tree, then the encoded size (HuffmanEncoder.hpp:119-137, 150-227)
-// One launch of each kernel for all runs; the codebooks are built on the pool's
-// threads, side by side.  (Run by run, each on a thread and a stream of its own, 18
-// strings of 72 thousand codes took 2.3 ms: 25 calls each, which queue in the
-// driver.)
-void huffman_encode_batch(const uint16_t *codes, uint64_t cs, uint64_t n, unsigned runs, int center, DevMem &m,
-                          cudaStream_t st, Counter &launches, HuffBatch &h, faz_timings &tm) {
-    const uint64_t nsub = hist_subchunks(n), nech = encode_chunks(n);
-    constexpr int nsym = 65536;
-    constexpr size_t kListHead = 2048;
-    const size_t list_cap = std::max<size_t>(std::min<uint64_t>((uint64_t)nsym, n), kListHead);
-    auto up = [](uint64_t w) { return (w + 31) & ~(uint64_t)31; };
-    // per run, in 8-byte words: histogram, first positions, [symbols, zeros, list],
-    // zero counts
-    const uint64_t w_hist = up((uint64_t)nsym), w_list = 32 + up(3 * list_cap), w_run = 2 * w_hist + w_list + up(nsub + 1);
-    unsigned long long *work = m.alloc<unsigned long long>(runs * w_run), *dinfo = work + 2 * w_hist;
-    CK(cudaMemset2DAsync(work, w_run * 8, 0, (2 * w_hist + 2) * 8, runs, st));
-    launches(launch_histogram_batch(codes, n, runs, BatchStride{cs, w_run}, center, nsym, work, work + w_hist,
-                                    dinfo + w_list, dinfo + 1, dinfo + 2, reinterpret_cast<unsigned *>(dinfo), st));
-    launches.n++;  // two kernels
-    constexpr size_t kHead = 16 + kListHead * 24;
-    const uint8_t *hb = t_pin_small.get(runs * kHead);
-    CK(cudaMemcpy2DAsync((void *)hb, kHead, dinfo, w_run * 8, kHead, runs, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    const auto th = clk::now();
-    std::vector<std::vector<unsigned long long>> list(runs);
-    bool more = false;
-    for (unsigned i = 0; i < runs; i++) {
-        unsigned int nl = 0;
-        std::memcpy(&nl, hb + i * kHead, 4);
-        if (nl > list_cap) throw Fail{FAZ_ERR_DEVICE, "histogram list longer than the symbol range"};
-        list[i].resize(3 * (size_t)nl);
-        std::memcpy(list[i].data(), hb + i * kHead + 16, std::min<size_t>(nl, kListHead) * 24);
-        if (nl > kListHead) {
-            more = true;
-            CK(cudaMemcpyAsync(list[i].data() + 3 * kListHead, dinfo + i * w_run + 2 + 3 * kListHead,
-                               (nl - kListHead) * 24, cudaMemcpyDeviceToHost, st));
-        }
-    }
-    if (more) CK(cudaStreamSynchronize(st));
-    // the tables of every run (17 bytes a state, max - min + 2 states) and the tasks
-    // in one upload
-    const size_t tasks_bytes = (runs * sizeof(EncodeTask) + 255) & ~(size_t)255;
-    std::vector<size_t> at(runs + 1, tasks_bytes);
-    for (unsigned i = 0; i < runs; i++) {
-        unsigned long long lo = nsym, hi = 0;
-        for (size_t k = 0; k < list[i].size(); k += 3) {
-            lo = std::min(lo, list[i][k]);
-            hi = std::max(hi, list[i][k]);
-        }
-        const size_t states = list[i].empty() ? 0 : (size_t)(hi - lo) + 2;
-        at[i + 1] = at[i] + ((states * 17 + 255) & ~(size_t)255);
-    }
-    TableStage &ts = t_table_stage;
-    uint8_t *stage = ts.acquire(at[runs]), *dtab = m.alloc<uint8_t>(at[runs]);
-    h.cb.resize(runs);
-    h.nbytes.resize(runs);
-    h.word0.resize(runs);
-    auto build = [&](unsigned i) {
-        const size_t nl = list[i].size() / 3;
-        std::vector<int> syms(nl);
-        std::vector<uint64_t> cnts(nl), firsts(nl);
-        for (size_t k = 0; k < nl; k++) {
-            syms[k] = (int)list[i][3 * k];
-            cnts[k] = list[i][3 * k + 1];
-            firsts[k] = list[i][3 * k + 2];
-        }
-        Codebook &cb = h.cb[i];
-        std::string err;
-        const int rc = build_codebook(syms, cnts, firsts, cb, err);
-        if (rc) throw Fail{rc, err};
-        const size_t S = (size_t)cb.stateNum;
-        if (S * 17 > at[i + 1] - at[i]) throw Fail{FAZ_ERR_DEVICE, "Huffman codebook larger than the symbol range"};
-        unsigned long long *code = reinterpret_cast<unsigned long long *>(stage + at[i]), *packed = code + S;
-        std::memcpy(code, cb.code.data(), S * 8);
-        for (size_t k = 0; k < S; k++) {
-            const int l = cb.len[k];
-            packed[k] = ((unsigned long long)l << 32) | (l >= 1 && l <= 32 ? (cb.code[k] >> (64 - l)) : 0ull);
-        }
-        std::memcpy(packed + S, cb.len.data(), S);
-        uint64_t bits = 0;
-        for (size_t k = 0; k < nl; k++) bits += cnts[k] * (uint64_t)cb.len[syms[k] - cb.offset];
-        h.nbytes[i] = (bits + 7) / 8;
-        return 0;
-    };
-    run_tasks(runs, build);
-    tm.host_ms += ms_since(th);
-    int maxlen = 1;
-    h.words = 0;
-    for (unsigned i = 0; i < runs; i++) {
-        maxlen = std::max(maxlen, h.cb[i].maxlen);
-        h.word0[i] = h.words;
-        h.words += up(h.nbytes[i] / 4 + 2);
-    }
-    h.bits = m.alloc<uint32_t>(h.words);
-    EncodeTask *tasks = reinterpret_cast<EncodeTask *>(stage);
-    for (unsigned i = 0; i < runs; i++) {
-        const size_t S = (size_t)h.cb[i].stateNum;
-        const unsigned long long *code = reinterpret_cast<const unsigned long long *>(dtab + at[i]);
-        tasks[i] = EncodeTask{h.cb[i].offset, code, code + S, reinterpret_cast<const uint8_t *>(code + 2 * S),
-                              h.bits + h.word0[i]};
-    }
-    CK(cudaMemcpyAsync(dtab, stage, at[runs], cudaMemcpyHostToDevice, st));
-    ts.release(st);
-    CK(cudaMemsetAsync(h.bits, 0, h.words * 4, st));
-    const EncodeTask *dtasks = reinterpret_cast<const EncodeTask *>(dtab);
-    const uint64_t nch = runs * nech;
-    unsigned long long *cbits = m.alloc<unsigned long long>(2 * (nch + 1) + scan_temp_words(nch) + 1),
-                       *coff = cbits + nch + 1;
-    launches(launch_encode_bits_batch(codes, cs, n, runs, dtasks, cbits, st));
-    launches(launch_scan_u64(cbits, coff, nch, coff + nch + 1, st));
-    launches(launch_encode_pack_batch(codes, cs, n, runs, dtasks, maxlen, coff, st));
-}
-
 void append_tree(std::vector<uint8_t> &o, const Codebook &cb, uint64_t nbytes) {
     put<int32_t>(o, cb.offset);
     put_be32(o, cb.nodeCount);

@@ -347,34 +347,6 @@ class TaskThreads {
     bool stop_ = false;
 };
 
-// f(0) .. f(n - 1) on the pool's threads (one call: here); the first exception is
-// thrown after all have ended.  Not from a pool thread, which would wait for others.
-template <typename F>
-void run_tasks(uint64_t n, const F &f) {
-    if (n == 1) {
-        f(0);
-        return;
-    }
-    std::vector<std::future<int>> futs;
-    std::exception_ptr first;
-    for (uint64_t i = 0; i < n; i++) {
-        try {
-            futs.push_back(TaskThreads::get().submit<int>([&f, i]() { return f(i); }));
-        } catch (...) {
-            first = std::current_exception();
-            break;
-        }
-    }
-    for (auto &x : futs) {
-        try {
-            (void)x.get();
-        } catch (...) {
-            if (!first) first = std::current_exception();
-        }
-    }
-    if (first) std::rethrow_exception(first);
-}
-
 // an event that orders streams (no timing)
 struct Event {
     cudaEvent_t e = nullptr;
@@ -569,24 +541,16 @@ struct HuffEncoded {
 };
 // `sized`, when given, runs as soon as the codebook, the zero count and the
 // encoded size are known on the host (before the encoding kernels finish).
-// `sliced`: long bit strings may be packed in several launches.
+// `sliced`: long bit strings may be packed in several launches.  `zero_scan`: whether
+// the caller reads zoff.
 // The uint32_t overloads serve quantisers of more than 65536 bins.
 void huffman_encode_device(const uint16_t *codes, uint64_t n, int center, DevMem &m, cudaStream_t st,
                            Counter &launches, HuffEncoded &h, faz_timings &tm,
-                           const std::function<void(const HuffEncoded &)> &sized = {}, bool sliced = false);
+                           const std::function<void(const HuffEncoded &)> &sized = {}, bool sliced = false,
+                           bool zero_scan = true);
 void huffman_encode_device(const uint32_t *codes, uint64_t n, int center, DevMem &m, cudaStream_t st,
                            Counter &launches, HuffEncoded &h, faz_timings &tm,
                            const std::function<void(const HuffEncoded &)> &sized = {}, bool sliced = false);
-// The same for a batch of runs of n codes, run i's at codes + i * cs: the codebooks
-// and, in one area, the bit strings (string i from word word0[i] on).
-struct HuffBatch {
-    std::vector<Codebook> cb;
-    std::vector<uint64_t> nbytes, word0;
-    uint32_t *bits = nullptr;
-    uint64_t words = 0;
-};
-void huffman_encode_batch(const uint16_t *codes, uint64_t cs, uint64_t n, unsigned runs, int center, DevMem &m,
-                          cudaStream_t st, Counter &launches, HuffBatch &h, faz_timings &tm);
 void append_tree(std::vector<uint8_t> &o, const Codebook &cb, uint64_t nbytes);
 void huffman_decode_device(const uint8_t *&p, const uint8_t *end, uint64_t num, uint16_t *codes, DevMem &m,
                            cudaStream_t st, Counter &launches);

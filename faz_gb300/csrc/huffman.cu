@@ -41,12 +41,7 @@ template <typename C>
 __global__ void __launch_bounds__(HTHREADS) k_histogram(const C *__restrict__ codes, uint64_t n, uint64_t nsub,
                                                        uint64_t per_cta, int center, unsigned long long *hist,
                                                        unsigned long long *first, unsigned long long *zcount,
-                                                       unsigned long long *nzero, BatchStride batch) {
-    codes += blockIdx.y * batch.codes;
-    hist += blockIdx.y * batch.words;
-    first += blockIdx.y * batch.words;
-    zcount += blockIdx.y * batch.words;
-    nzero += blockIdx.y * batch.words;
+                                                       unsigned long long *nzero) {
     __shared__ unsigned scnt[HWIN + 1], sfirst[HWIN + 1];
     __shared__ unsigned long long ztotal;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -141,12 +136,7 @@ __global__ void __launch_bounds__(HTHREADS) k_histogram(const C *__restrict__ co
 // *nlist = their number.
 __global__ void __launch_bounds__(256) k_hist_compact(const unsigned long long *__restrict__ hist,
                                                      const unsigned long long *__restrict__ first, int nsym,
-                                                     unsigned long long *list, unsigned int *nlist,
-                                                     BatchStride batch) {
-    hist += blockIdx.y * batch.words;
-    first += blockIdx.y * batch.words;
-    list += blockIdx.y * batch.words;
-    nlist += 2 * blockIdx.y * batch.words;
+                                                     unsigned long long *list, unsigned int *nlist) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     const bool nz = s < nsym && hist[s] != 0;
     const unsigned int m = __ballot_sync(0xffffffffu, nz);
@@ -356,8 +346,9 @@ __device__ __forceinline__ int enc_load(const C *__restrict__ codes, uint64_t n,
 }
 
 template <typename C>
-__device__ __forceinline__ void encode_bits_chunk(const C *__restrict__ codes, uint64_t n, int offset,
-                                                  const uint8_t *__restrict__ len, unsigned long long *chunkbits) {
+__global__ void __launch_bounds__(ENC_THREADS) k_encode_bits(const C *__restrict__ codes, uint64_t n, int offset,
+                                                            const uint8_t *__restrict__ len,
+                                                            unsigned long long *chunkbits) {
     __shared__ unsigned ws[ENC_THREADS / 32];
     C sym[ENC_PER_THREAD];
     const int nvalid =
@@ -380,19 +371,6 @@ __device__ __forceinline__ void encode_bits_chunk(const C *__restrict__ codes, u
         chunkbits[blockIdx.x] = t;
     }
 }
-template <typename C>
-__global__ void __launch_bounds__(ENC_THREADS) k_encode_bits(const C *__restrict__ codes, uint64_t n, int offset,
-                                                            const uint8_t *__restrict__ len,
-                                                            unsigned long long *chunkbits) {
-    encode_bits_chunk(codes, n, offset, len, chunkbits);
-}
-// a batch of strings, nech chunks each (blockIdx.y)
-__global__ void __launch_bounds__(ENC_THREADS) k_encode_bits_batch(const uint16_t *__restrict__ codes, uint64_t cs,
-                                                                  uint64_t n, const EncodeTask *__restrict__ tasks,
-                                                                  uint64_t nech, unsigned long long *chunkbits) {
-    const EncodeTask &t = tasks[blockIdx.y];
-    encode_bits_chunk(codes + blockIdx.y * cs, n, t.offset, t.len, chunkbits + blockIdx.y * nech);
-}
 
 // Each thread packs ENC_PER_THREAD consecutive codes, four at a time while they
 // fit in 32 bits together: about 11 thread instructions a code (pushed one by one
@@ -400,17 +378,18 @@ __global__ void __launch_bounds__(ENC_THREADS) k_encode_bits_batch(const uint16_
 // behind the copy of the eighth before it (227 us in one piece before the copy).  Words in shared memory follow
 // the 32-bit word grid of the output.
 template <typename C>
-__device__ __forceinline__ void encode_pack_chunk(const C *__restrict__ codes, uint64_t n, int offset,
-                                                  const unsigned long long *__restrict__ code64,
-                                                  const unsigned long long *__restrict__ packed,
-                                                  const unsigned long long *__restrict__ chunkoff,
-                                                  unsigned long long bit0, uint64_t chunk, uint32_t *out,
-                                                  unsigned long long *host_end) {
+__global__ void __launch_bounds__(ENC_THREADS) k_encode_pack(const C *__restrict__ codes, uint64_t n, int offset,
+                                                            const unsigned long long *__restrict__ code64,
+                                                            const unsigned long long *__restrict__ packed,
+                                                            const unsigned long long *__restrict__ chunkoff,
+                                                            uint64_t chunk0, uint32_t *out,
+                                                            unsigned long long *host_end) {
     extern __shared__ uint32_t sw[];
     __shared__ unsigned wtot[ENC_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const unsigned long long gbit = chunkoff[chunk] - bit0;
-    const unsigned total = (unsigned)(chunkoff[chunk + 1] - bit0 - gbit);
+    const uint64_t chunk = chunk0 + blockIdx.x;
+    const unsigned long long gbit = chunkoff[chunk];
+    const unsigned total = (unsigned)(chunkoff[chunk + 1] - gbit);
     // the end of a launch's codes, for the host that copies them
     if (host_end && tid == 0 && blockIdx.x == gridDim.x - 1) *(volatile unsigned long long *)host_end = gbit + total;
     if (total == 0) return;
@@ -549,25 +528,6 @@ __global__ void __launch_bounds__(1024) k_scan_chunks(const unsigned long long *
         out[n] = carry;
         clear(carry);
     }
-}
-
-template <typename C>
-__global__ void __launch_bounds__(ENC_THREADS) k_encode_pack(const C *__restrict__ codes, uint64_t n, int offset,
-                                                            const unsigned long long *__restrict__ code64,
-                                                            const unsigned long long *__restrict__ packed,
-                                                            const unsigned long long *__restrict__ chunkoff,
-                                                            uint64_t chunk0, uint32_t *out,
-                                                            unsigned long long *host_end) {
-    encode_pack_chunk(codes, n, offset, code64, packed, chunkoff, 0, chunk0 + blockIdx.x, out, host_end);
-}
-// a batch of strings: their chunks' offsets follow one another in chunkoff
-__global__ void __launch_bounds__(ENC_THREADS) k_encode_pack_batch(const uint16_t *__restrict__ codes, uint64_t cs,
-                                                                  uint64_t n, const EncodeTask *__restrict__ tasks,
-                                                                  uint64_t nech,
-                                                                  const unsigned long long *__restrict__ chunkoff) {
-    const EncodeTask &t = tasks[blockIdx.y];
-    const unsigned long long *off = chunkoff + blockIdx.y * nech;
-    encode_pack_chunk(codes + blockIdx.y * cs, n, t.offset, t.code64, t.packed, off, off[0], blockIdx.x, t.out, nullptr);
 }
 
 // ------------------------------------------------------------------ decode
@@ -1175,7 +1135,7 @@ uint64_t zero_subchunk() { return HSUB; }
 
 cudaError_t launch_hist_compact(const unsigned long long *hist, const unsigned long long *first, int nsym,
                                 unsigned long long *list, unsigned int *nlist, cudaStream_t st) {
-    k_hist_compact<<<(unsigned)((nsym + 255) / 256), 256, 0, st>>>(hist, first, nsym, list, nlist, BatchStride{});
+    k_hist_compact<<<(unsigned)((nsym + 255) / 256), 256, 0, st>>>(hist, first, nsym, list, nlist);
     return cudaGetLastError();
 }
 
@@ -1195,7 +1155,7 @@ cudaError_t histogram_impl(const C *codes, uint64_t n, int center, unsigned long
     if (nsub > used) e = cudaMemsetAsync(zcount + used, 0, (nsub - used) * 8, st);
     if (e != cudaSuccess) return e;
     k_histogram<C><<<grid_for(used, per_cta), HTHREADS, 0, st>>>(codes, n, used, per_cta, center, hist, first, zcount,
-                                                                  nzero, BatchStride{});
+                                                                  nzero);
     return cudaGetLastError();
 }
 cudaError_t launch_histogram(const uint16_t *codes, uint64_t n, int center, unsigned long long *hist,
@@ -1207,22 +1167,6 @@ cudaError_t launch_histogram(const uint32_t *codes, uint64_t n, int center, unsi
                              unsigned long long *first, unsigned long long *zcount, unsigned long long *nzero,
                              cudaStream_t st) {
     return histogram_impl(codes, n, center, hist, first, zcount, nzero, st);
-}
-
-cudaError_t launch_histogram_batch(const uint16_t *codes, uint64_t n, unsigned runs, BatchStride batch, int center,
-                                   int nsym, unsigned long long *hist, unsigned long long *first,
-                                   unsigned long long *zcount, unsigned long long *nzero, unsigned long long *list,
-                                   unsigned int *nlist, cudaStream_t st) {
-    // a sub-chunk or more per warp, about four CTAs per SM over the batch
-    const uint64_t used = (n + HSUB - 1) / HSUB, warps = HTHREADS / 32;
-    uint64_t per_cta = std::max<uint64_t>((used * runs + 607) / 608, std::min<uint64_t>(warps, 4));
-    per_cta = std::min<uint64_t>(per_cta, (1ull << 31) / HSUB);
-    k_histogram<uint16_t><<<dim3(grid_for(used, per_cta), runs), HTHREADS, 0, st>>>(codes, n, used, per_cta, center, hist,
-                                                                                   first, zcount, nzero, batch);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_hist_compact<<<dim3((unsigned)((nsym + 255) / 256), runs), 256, 0, st>>>(hist, first, nsym, list, nlist, batch);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_count_zeros(const uint16_t *codes, uint64_t n, unsigned long long *zcount, cudaStream_t st) {
@@ -1285,23 +1229,6 @@ cudaError_t launch_encode_pack(const EncodeArgs &a, const uint16_t *codes, uint6
 cudaError_t launch_encode_pack(const EncodeArgs &a, const uint32_t *codes, uint64_t n, uint64_t chunk0,
                                uint64_t chunk1, unsigned long long *host_end, cudaStream_t st) {
     return encode_pack_impl(a, codes, n, chunk0, chunk1, host_end, st);
-}
-
-cudaError_t launch_encode_bits_batch(const uint16_t *codes, uint64_t cs, uint64_t n, unsigned runs,
-                                     const EncodeTask *tasks, unsigned long long *chunkbits, cudaStream_t st) {
-    k_encode_bits_batch<<<dim3(grid_for(n, ENC_CHUNK), runs), ENC_THREADS, 0, st>>>(codes, cs, n, tasks,
-                                                                                   encode_chunks(n), chunkbits);
-    return cudaGetLastError();
-}
-cudaError_t launch_encode_pack_batch(const uint16_t *codes, uint64_t cs, uint64_t n, unsigned runs,
-                                     const EncodeTask *tasks, int maxlen, const unsigned long long *chunkoff,
-                                     cudaStream_t st) {
-    const int words = (int)(((uint64_t)ENC_CHUNK * (uint64_t)maxlen + 31) / 32 + 2);
-    cudaError_t e = allow_dynamic_smem((const void *)k_encode_pack_batch);
-    if (e != cudaSuccess) return e;
-    k_encode_pack_batch<<<dim3(grid_for(n, ENC_CHUNK), runs), ENC_THREADS, (size_t)words * 4, st>>>(
-        codes, cs, n, tasks, encode_chunks(n), chunkoff);
-    return cudaGetLastError();
 }
 
 int decode_unit_words(uint64_t nbits) { return nbits < DEC_SHORT_BITS ? DEC_SHORT : DEC_LONG; }

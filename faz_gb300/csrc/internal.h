@@ -155,28 +155,6 @@ uint64_t scan_temp_words(uint64_t n);
 cudaError_t launch_scan_u64(const unsigned long long *in, unsigned long long *out, uint64_t n,
                             unsigned long long *temp, cudaStream_t st);
 uint64_t encode_chunks(uint64_t n);
-// The stage for a batch of runs of n codes each (the QoZ tuner's tests): run y's
-// codes, and its histogram, positions, counts and list, are a stride from those of
-// the run before (8-byte words); its string's tables and output are tasks[y]; the
-// runs' chunks follow one another in chunkbits and their scan.
-struct BatchStride {
-    uint64_t codes = 0, words = 0;
-};
-struct EncodeTask {
-    int offset;
-    const unsigned long long *code64, *packed;
-    const uint8_t *len;
-    uint32_t *out;
-};
-cudaError_t launch_histogram_batch(const uint16_t *codes, uint64_t n, unsigned runs, BatchStride batch, int center,
-                                   int nsym, unsigned long long *hist, unsigned long long *first,
-                                   unsigned long long *zcount, unsigned long long *nzero, unsigned long long *list,
-                                   unsigned int *nlist, cudaStream_t st);
-cudaError_t launch_encode_bits_batch(const uint16_t *codes, uint64_t cs, uint64_t n, unsigned runs,
-                                     const EncodeTask *tasks, unsigned long long *chunkbits, cudaStream_t st);
-cudaError_t launch_encode_pack_batch(const uint16_t *codes, uint64_t cs, uint64_t n, unsigned runs,
-                                     const EncodeTask *tasks, int maxlen, const unsigned long long *chunkoff,
-                                     cudaStream_t st);
 // Bit counts, offsets and packing of chunks [chunk0, chunk1) of n codes, after the
 // chunks before them: code tables, bits and offsets per chunk, the output.  Three
 // launches.  host_end (pinned, or null) receives the bits before chunk1.

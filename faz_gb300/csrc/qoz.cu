@@ -838,8 +838,8 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
     };
     // CompressTests (SZInterp.hpp:1130-1392) of every sampled block: bit rate
     // after Huffman + zstd, PSNR from the summed squared errors.  The tests of one
-    // call run together: their kernels as a batch, codebooks and zstd side by side
-    // on host threads.
+    // call run together: their sweeps, sums and unpredictable values as a batch,
+    // then each one's Huffman and zstd on its own stream and host thread.
     struct Test {
         int op, dir;
         double alpha, beta, eb;
@@ -847,6 +847,8 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
     };
     struct TestRes {
         double br = 0, mm = 0;
+        uint64_t launches = 0;
+        double host_ms = 0;
     };
     auto run_tests = [&](const std::vector<Test> &tests, double pc) {
         std::vector<TestRes> res(tests.size());
@@ -904,49 +906,80 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
             CK(cudaStreamSynchronize(st));
             T *unp = bm.alloc<T>(zat[n]);
             if (zat[n]) launches(launch_compact_zeros<T>(b.codes, n * b.cs, zc, zoff, b.scratch, unp, st));
-            HuffBatch h;
-            huffman_encode_batch(qb, b.cs, ns, (unsigned)n, 32768, bm, st, launches, h, tm);
-            // the strings and the unpredictable values through pinned staging
-            uint8_t *pin = t_pin_payload.get(h.words * 4 + zat[n] * sizeof(T) + 8);
-            const uint8_t *pbits = pin, *punp = pin + h.words * 4;
-            CK(cudaMemcpyAsync(pin, h.bits, h.words * 4, cudaMemcpyDeviceToHost, st));
-            if (zat[n])
-                CK(cudaMemcpyAsync(pin + h.words * 4, unp, zat[n] * sizeof(T), cudaMemcpyDeviceToHost, st));
-            std::vector<T> cur;
-            if (metric_target >= 2) {
-                // the reconstructions are left in the working copies
-                cur.resize(n * nv);
-                CK(cudaMemcpyAsync(cur.data(), b.work, n * nv * sizeof(T), cudaMemcpyDeviceToHost, st));
-            }
             CK(cudaStreamSynchronize(st));
-            mark("  tests encoded", (double)n);
-            run_tasks(n, [&](uint64_t i) {
+            auto finish = [&](uint64_t i, cudaStream_t s) {
                 const Test &t = tests[t0 + i];
+                TestRes r;
+                DevMem xm(s);
+                Counter nl;
+                faz_timings xt;
+                std::memset(&xt, 0, sizeof(xt));
                 double se = 0;
                 for (uint64_t k = 0; k < nblk; k++) se += hsum[i * nblk + k];
+                HuffEncoded h;
+                huffman_encode_device(qb + i * b.cs, ns, 32768, xm, s, nl, h, xt, {}, false, false);
                 const uint64_t nunp = zat[i + 1] - zat[i];
-                std::vector<uint8_t> pl;
-                put<uint8_t>(pl, 2);
-                put<double>(pl, t.eb);
-                put<int32_t>(pl, 32768);
-                put<uint64_t>(pl, nunp);
-                const T *u = reinterpret_cast<const T *>(punp) + zat[i];
-                pl.insert(pl.end(), (const uint8_t *)u, (const uint8_t *)(u + nunp));
-                append_tree(pl, h.cb[i], h.nbytes[i]);
-                const uint8_t *s = pbits + h.word0[i] * 4;
-                pl.insert(pl.end(), s, s + h.nbytes[i]);
+                std::vector<uint8_t> head;
+                put<uint8_t>(head, 2);
+                put<double>(head, t.eb);
+                put<int32_t>(head, 32768);
+                put<uint64_t>(head, nunp);
+                std::vector<uint8_t> tree;
+                append_tree(tree, h.cb, h.nbytes);
+                // the payload through the thread's pinned staging buffer
+                const size_t plen = head.size() + nunp * sizeof(T) + tree.size() + h.nbytes;
+                uint8_t *pl = t_pin_payload.get(plen + 8);
+                std::memcpy(pl, head.data(), head.size());
+                if (nunp)
+                    CK(cudaMemcpyAsync(pl + head.size(), unp + zat[i], nunp * sizeof(T), cudaMemcpyDeviceToHost, s));
+                std::memcpy(pl + head.size() + nunp * sizeof(T), tree.data(), tree.size());
+                if (h.nbytes)
+                    CK(cudaMemcpyAsync(pl + head.size() + nunp * sizeof(T) + tree.size(), h.bits, h.nbytes,
+                                       cudaMemcpyDeviceToHost, s));
+                CK(cudaStreamSynchronize(s));
                 // profiling_coeff scales both (SZInterp.hpp:1364-1370)
                 const double ele = (double)nv;
-                TestRes &r = res[t0 + i];
-                r.br = 8 * (double)zstd_framed_size_host(pl.data(), pl.size()) / ele;
+                mark("  compress test payload", (double)plen, t.alpha);
+                r.br = 8 * (double)zstd_framed_size_host(pl, plen) / ele;
+                mark("  compress test zstd", t.beta, t.eb);
                 r.br *= pc;
                 double mse = se / ele;
                 mse *= pc;
                 r.mm = 20 * std::log10(c.rng) - 10 * std::log10(mse);
-                if (metric_target >= 2)
-                    r.mm = target_metric(std::vector<T>(cur.begin() + i * nv, cur.begin() + (i + 1) * nv));
-                return 0;
-            });
+                if (metric_target >= 2) {
+                    // the reconstructions are left in the working copy
+                    std::vector<T> cur(nv);
+                    CK(cudaMemcpyAsync(cur.data(), b.work + i * nv, nv * sizeof(T), cudaMemcpyDeviceToHost, s));
+                    CK(cudaStreamSynchronize(s));
+                    r.mm = target_metric(cur);
+                }
+                r.launches = nl.n;
+                r.host_ms = xt.host_ms;
+                return r;
+            };
+            if (n == 1) {
+                res[t0] = finish(0, st);
+            } else {
+                std::vector<std::future<TestRes>> futs;
+                for (uint64_t i = 0; i < n; i++)
+                    futs.push_back(TaskThreads::get().submit<TestRes>([&, i]() {
+                        StreamGuard sg(nullptr);
+                        return finish(i, sg.st);
+                    }));
+                std::exception_ptr first;
+                for (uint64_t i = 0; i < n; i++) {
+                    try {
+                        res[t0 + i] = futs[i].get();
+                    } catch (...) {
+                        if (!first) first = std::current_exception();
+                    }
+                }
+                if (first) std::rethrow_exception(first);
+            }
+            for (uint64_t i = 0; i < n; i++) {
+                launches.n += res[t0 + i].launches;
+                tm.host_ms += res[t0 + i].host_ms;
+            }
         }
         return res;
     };

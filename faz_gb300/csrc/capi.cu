@@ -358,7 +358,7 @@ struct Sink {
 template <typename C>
 void huffman_encode_impl(const C *codes, uint64_t n, int center, DevMem &m, cudaStream_t st, Counter &launches,
                          HuffEncoded &h, faz_timings &tm, const std::function<void(const HuffEncoded &)> &sized,
-                         bool sliced, bool zero_scan) {
+                         bool sliced) {
     const uint64_t nsub = hist_subchunks(n);
     const uint64_t nech = encode_chunks(n);
     // every value a code of this width can take
@@ -403,7 +403,7 @@ void huffman_encode_impl(const C *codes, uint64_t n, int center, DevMem &m, cuda
     std::memcpy(&h.nzero, hb + 8, 8);
     if (nl > (unsigned int)nsym || nl > list_cap)
         throw Fail{FAZ_ERR_DEVICE, "histogram list longer than the symbol range"};
-    if (h.nzero && zero_scan) launches(launch_scan_u64(h.zc, h.zoff, nsub, stmp, st));
+    if (h.nzero) launches(launch_scan_u64(h.zc, h.zoff, nsub, stmp, st));
     std::vector<unsigned long long> rest;
     if (nl > kListHead) {
         rest.resize(3 * (size_t)(nl - kListHead));
@@ -474,14 +474,14 @@ void huffman_encode_impl(const C *codes, uint64_t n, int center, DevMem &m, cuda
 
 void huffman_encode_device(const uint16_t *codes, uint64_t n, int center, DevMem &m, cudaStream_t st,
                            Counter &launches, HuffEncoded &h, faz_timings &tm,
-                           const std::function<void(const HuffEncoded &)> &sized, bool sliced, bool zero_scan) {
-    huffman_encode_impl(codes, n, center, m, st, launches, h, tm, sized, sliced, zero_scan);
+                           const std::function<void(const HuffEncoded &)> &sized, bool sliced) {
+    huffman_encode_impl(codes, n, center, m, st, launches, h, tm, sized, sliced);
 }
 void huffman_encode_device(const uint32_t *codes, uint64_t n, int center, DevMem &m, cudaStream_t st,
                            Counter &launches, HuffEncoded &h, faz_timings &tm,
                            const std::function<void(const HuffEncoded &)> &sized, bool sliced) {
     if (center < 0 || center > (1 << 20)) throw Fail{FAZ_ERR_UNSUPPORTED, "quantisation radius too large"};
-    huffman_encode_impl(codes, n, center, m, st, launches, h, tm, sized, sliced, true);
+    huffman_encode_impl(codes, n, center, m, st, launches, h, tm, sized, sliced);
 }
 
 // HuffmanEncoder::save header + tree, then the encoded size (HuffmanEncoder.hpp:119-137, 150-227)

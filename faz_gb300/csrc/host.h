@@ -541,13 +541,11 @@ struct HuffEncoded {
 };
 // `sized`, when given, runs as soon as the codebook, the zero count and the
 // encoded size are known on the host (before the encoding kernels finish).
-// `sliced`: long bit strings may be packed in several launches.  `zero_scan`: whether
-// the caller reads zoff.
+// `sliced`: long bit strings may be packed in several launches.
 // The uint32_t overloads serve quantisers of more than 65536 bins.
 void huffman_encode_device(const uint16_t *codes, uint64_t n, int center, DevMem &m, cudaStream_t st,
                            Counter &launches, HuffEncoded &h, faz_timings &tm,
-                           const std::function<void(const HuffEncoded &)> &sized = {}, bool sliced = false,
-                           bool zero_scan = true);
+                           const std::function<void(const HuffEncoded &)> &sized = {}, bool sliced = false);
 void huffman_encode_device(const uint32_t *codes, uint64_t n, int center, DevMem &m, cudaStream_t st,
                            Counter &launches, HuffEncoded &h, faz_timings &tm,
                            const std::function<void(const HuffEncoded &)> &sized = {}, bool sliced = false);

@@ -1131,7 +1131,6 @@ __global__ void k_fill_u16(C *out, uint64_t n, C v) {
 static inline unsigned grid_for(uint64_t n, uint64_t per) { return (unsigned)((n + per - 1) / per); }
 
 uint64_t hist_subchunks(uint64_t n) { return ((n + HCHUNK - 1) / HCHUNK) * HWARPS; }
-uint64_t zero_subchunk() { return HSUB; }
 
 cudaError_t launch_hist_compact(const unsigned long long *hist, const unsigned long long *first, int nsym,
                                 unsigned long long *list, unsigned int *nlist, cudaStream_t st) {

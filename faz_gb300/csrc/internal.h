@@ -132,7 +132,6 @@ template <typename T, bool WIDE>
 int batch_occupancy(int threads, size_t smem);
 
 uint64_t hist_subchunks(uint64_t n);
-uint64_t zero_subchunk();  // codes per zero count
 // the symbols of non-zero count: list[3k..3k+2] = symbol, count, first
 // position, in no particular order; *nlist (zeroed by the caller) their number
 cudaError_t launch_hist_compact(const unsigned long long *hist, const unsigned long long *first, int nsym,

@@ -10,14 +10,8 @@
 // candidate interpolator and direction per level (tuning mode 2: summed
 // absolute prediction loss), then with every alpha/beta candidate (tuning
 // mode 1: codes, bit rate after Huffman + zstd, PSNR from summed squared
-// errors).  Trials that do not wait for one another's results run as one batch:
-// one launch per level and sweep covers every sampled block of every trial (one
-// thread per target), each trial with its own buffers and its row of the tables.
-// A 256^3 field samples two blocks, 72 thousand points: a trial alone fills a
-// tenth of the GPU and costs its launches, in the driver, which serialises the
-// host threads; 16 selections took 60 sweeps and 16 waits, 1.3 ms, now 0.25; 18
-// alpha/beta tests 270 sweeps on 18 streams, 8 ms with their Huffman and zstd parts,
-// now 2.6.  Each target's error lands at its stream
+// errors).  On the GPU one launch per level and sweep covers every sampled
+// block (one thread per target); each target's error lands at its stream
 // position and k_qz_line_sums / k_qz_sum add the errors in the reference's nesting
 // (per line, then per level block, then a running total), so the sums and
 // therefore the decisions are those of the reference.  The decision logic is the
@@ -62,28 +56,6 @@ struct QzSweep {
     int64_t per;           // values per block
 };
 
-// One trial's part of a launch over a batch of trials (blockIdx.y).
-struct QzTask {
-    QzSweep w;
-    LevelArgs q;
-    uint64_t total;  // targets; 0 when the trial has no such sweep
-    bool straight;   // the exact float path
-};
-// A batch's buffers: each trial's part is a stride from the one before.
-template <typename T>
-struct QzBuffers {
-    T *work, *scratch;
-    uint16_t *codes;
-    double *err, *lsum, *bsum;
-    uint64_t nv, cs, ls;  // strides: values, stream slots, lines
-};
-
-template <typename T>
-__global__ void k_qz_spread(const T *__restrict__ blocks, T *__restrict__ work, uint64_t nv) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nv) work[blockIdx.y * nv + i] = blocks[i];
-}
-
 // target index of rank r in a line of n points (inverse of line_rank)
 __device__ __forceinline__ int64_t target_of_rank(int64_t r, int64_t n, int cubic) {
     if (!cubic || n < 5) return 2 * r + 1;
@@ -98,13 +70,10 @@ __device__ __forceinline__ int64_t target_of_rank(int64_t r, int64_t n, int cubi
 // MODE 1: quantise, store code / unpredictable value / squared error;
 // MODE 2: store |d - pred|, quantise without keeping anything.
 template <typename T, int MODE, int QM>
-__global__ void __launch_bounds__(256) k_qz_sweep(const QzTask *__restrict__ tasks, QzBuffers<T> b) {
+__global__ void k_qz_sweep(QzSweep w, LevelArgs q, T *__restrict__ data, uint16_t *__restrict__ codes,
+                           T *__restrict__ scratch, double *__restrict__ err, uint64_t total) {
     const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const QzTask &task = tasks[blockIdx.y];
-    if (idx >= task.total) return;
-    const QzSweep &w = task.w;
-    const LevelArgs &q = task.q;
-    T *__restrict__ data = b.work + blockIdx.y * b.nv;
+    if (idx >= total) return;
     const uint64_t lines = (uint64_t)(w.cnt[0] * w.cnt[1]);
     const int64_t r = (int64_t)(idx % (uint64_t)w.tpl);
     const uint64_t L = (idx / (uint64_t)w.tpl) % lines;
@@ -128,19 +97,18 @@ __global__ void __launch_bounds__(256) k_qz_sweep(const QzTask *__restrict__ tas
         else if ((n & 1) == 0 && i == n - 1) pred = i_quad3(d[-5 * st], d[-3 * st], d[-st]);
         else pred = i_quad2(d[-3 * st], d[-st], d[st]);
     }
-    const uint64_t pos =
-        blockIdx.y * b.cs + k * (uint64_t)w.cpb + (uint64_t)w.seg_off + L * (uint64_t)w.tpl + (uint64_t)r;
+    const uint64_t pos = k * (uint64_t)w.cpb + (uint64_t)w.seg_off + L * (uint64_t)w.tpl + (uint64_t)r;
     const T orig = *d;
     T v = orig, uval;
     const int code = quant_point<T, QM>(v, pred, q, uval);
     if (MODE == 1) {
-        b.codes[pos] = (uint16_t)code;
-        if (code == 0) b.scratch[pos] = uval;
+        codes[pos] = (uint16_t)code;
+        if (code == 0) scratch[pos] = uval;
         const T df = v - orig;
-        b.err[pos] = (double)(T)(df * df);
+        err[pos] = (double)(T)(df * df);
     } else {
         const T df = orig - pred;
-        b.err[pos] = (double)(df < 0 ? -df : df);
+        err[pos] = (double)(df < 0 ? -df : df);
     }
     *d = v;
 }
@@ -149,8 +117,9 @@ __global__ void __launch_bounds__(256) k_qz_sweep(const QzTask *__restrict__ tas
 // maxStep grid from maxStep on, code 0, the value unpredictable.  Axes below
 // `e` are the 3-D embedding's leading ones.
 template <typename T>
-__global__ void k_qz_anchor(QzBuffers<T> b, int64_t per, int64_t cpb, int64_t nax, int64_t nay, int64_t naz, int64_t ms,
-                            int e, int64_t o0, int64_t o1, uint64_t total) {
+__global__ void k_qz_anchor(const T *__restrict__ data, int64_t per, int64_t cpb, int64_t nax, int64_t nay, int64_t naz,
+                            int64_t ms, int e, int64_t o0, int64_t o1, uint16_t *__restrict__ codes,
+                            T *__restrict__ scratch, uint64_t total) {
     const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const uint64_t na = (uint64_t)(nax * nay * naz);
@@ -158,26 +127,24 @@ __global__ void k_qz_anchor(QzBuffers<T> b, int64_t per, int64_t cpb, int64_t na
     const int64_t z = (int64_t)(a % (uint64_t)naz), y = (int64_t)((a / (uint64_t)naz) % (uint64_t)nay),
                   x = (int64_t)(a / ((uint64_t)naz * (uint64_t)nay));
     const int64_t cx = e > 0 ? 0 : (x + 1) * ms, cy = e > 1 ? 0 : (y + 1) * ms, cz = (z + 1) * ms;
-    const T v = b.work[blockIdx.y * b.nv + k * (uint64_t)per + cx * o0 + cy * o1 + cz];
-    b.codes[blockIdx.y * b.cs + k * (uint64_t)cpb + a] = 0;
-    b.scratch[blockIdx.y * b.cs + k * (uint64_t)cpb + a] = v;
+    const T v = data[k * (uint64_t)per + cx * o0 + cy * o1 + cz];
+    codes[k * (uint64_t)cpb + a] = 0;
+    scratch[k * (uint64_t)cpb + a] = v;
 }
 
 // The first point against prediction 0 (no anchor grid).
 template <typename T, int MODE>
-__global__ void k_qz_first(const QzTask *__restrict__ tasks, QzBuffers<T> b, int64_t per, int64_t cpb, uint64_t nblk) {
+__global__ void k_qz_first(LevelArgs q, T *__restrict__ data, int64_t per, int64_t cpb, uint16_t *__restrict__ codes,
+                           T *__restrict__ scratch, uint64_t nblk) {
     const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nblk) return;
-    const LevelArgs &q = tasks[blockIdx.y].q;
-    T *d = b.work + blockIdx.y * b.nv + k * (uint64_t)per;
-    T v = *d, uval;
+    T v = data[k * (uint64_t)per], uval;
     const int code = quantize<T>(v, (T)0, q.eb, q.recip, q.radius, q.trim, uval);
     if (MODE == 1) {
-        const uint64_t pos = blockIdx.y * b.cs + k * (uint64_t)cpb;
-        b.codes[pos] = (uint16_t)code;
-        if (code == 0) b.scratch[pos] = uval;
+        codes[k * (uint64_t)cpb] = (uint16_t)code;
+        if (code == 0) scratch[k * (uint64_t)cpb] = uval;
     }
-    *d = v;
+    data[k * (uint64_t)per] = v;
 }
 
 struct SumSeg {
@@ -202,14 +169,10 @@ struct SumPlan {
 // lines, then one chain per block over its line sums, from shared memory.  With
 // both in one thread per block the 35936 errors of a 33^3 block were one chain of
 // dependent loads and additions, 2.46 ms a launch, 95% of the tuner's time on the
-// GPU; the whole batch of 16 selections now takes 0.25 ms.
-__global__ void k_qz_line_sums(const SumPlan *__restrict__ plans, const double *__restrict__ errs, uint64_t cs,
-                               double *__restrict__ lsums, uint64_t ls_stride, uint64_t nblk) {
+// GPU.
+__global__ void k_qz_line_sums(SumPlan p, const double *__restrict__ err, double *__restrict__ lsum, uint64_t total) {
     const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const SumPlan &p = plans[blockIdx.y];
-    if (idx >= (uint64_t)p.nlines * nblk) return;
-    const double *err = errs + blockIdx.y * cs;
-    double *lsum = lsums + blockIdx.y * ls_stride;
+    if (idx >= total) return;
     const uint64_t k = idx / (uint64_t)p.nlines;
     const int64_t l = (int64_t)(idx - k * (uint64_t)p.nlines);
     int sgi = 0;
@@ -223,11 +186,9 @@ __global__ void k_qz_line_sums(const SumPlan *__restrict__ plans, const double *
 }
 
 constexpr int kSumChunk = 2048;
-__global__ void __launch_bounds__(256) k_qz_sum(const SumPlan *__restrict__ plans, const double *__restrict__ lsums,
-                                                uint64_t ls_stride, double *__restrict__ out) {
+__global__ void __launch_bounds__(256) k_qz_sum(SumPlan p, const double *__restrict__ lsum, double *__restrict__ out) {
     __shared__ double buf[kSumChunk];
-    const SumPlan &p = plans[blockIdx.y];
-    const double *src = lsums + blockIdx.y * ls_stride + (uint64_t)blockIdx.x * (uint64_t)p.nlines;
+    const double *src = lsum + (uint64_t)blockIdx.x * (uint64_t)p.nlines;
     double total = 0, blk = 0;
     int sgi = 0;
     for (int64_t c0 = 0; c0 < p.nlines; c0 += kSumChunk) {
@@ -252,22 +213,32 @@ __global__ void __launch_bounds__(256) k_qz_sum(const SumPlan *__restrict__ plan
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[(uint64_t)blockIdx.y * gridDim.x + blockIdx.x] = total;
+    if (threadIdx.x == 0) out[blockIdx.x] = total;
+}
+
+void launch_qz_sum(const SumPlan &p, const double *err, double *lsum, double *out, uint64_t nblk, cudaStream_t st,
+                   Counter &launches) {
+    const uint64_t total = (uint64_t)p.nlines * nblk;
+    if (total) {
+        k_qz_line_sums<<<(unsigned)((total + 127) / 128), 128, 0, st>>>(p, err, lsum, total);
+        launches(cudaGetLastError());
+    }
+    k_qz_sum<<<(unsigned)nblk, 256, 0, st>>>(p, lsum, out);
+    launches(cudaGetLastError());
 }
 
 // q_bins of CompressTest: for each level range, every block's codes of it.
-__global__ void k_qz_regroup(const uint16_t *__restrict__ all, uint64_t cs, int64_t cpb,
-                             const int64_t *__restrict__ rlo, const int64_t *__restrict__ rlen,
-                             const int64_t *__restrict__ rout, int nr, uint16_t *__restrict__ out, uint64_t total) {
+__global__ void k_qz_regroup(const uint16_t *__restrict__ codes, int64_t cpb, const int64_t *__restrict__ rlo,
+                             const int64_t *__restrict__ rlen, const int64_t *__restrict__ rout, int nr, uint64_t nblk,
+                             uint16_t *__restrict__ out, uint64_t total) {
     const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
-    const uint16_t *codes = all + blockIdx.y * cs;
     // find the range (few of them)
     int g = 0;
     while (g + 1 < nr && idx >= (uint64_t)rout[g + 1]) g++;
     const uint64_t o = idx - (uint64_t)rout[g];
     const uint64_t k = o / (uint64_t)rlen[g], m = o % (uint64_t)rlen[g];
-    out[blockIdx.y * cs + idx] = codes[k * (uint64_t)cpb + (uint64_t)rlo[g] + m];
+    out[idx] = codes[k * (uint64_t)cpb + (uint64_t)rlo[g] + m];
 }
 
 template <typename T>
@@ -350,23 +321,35 @@ struct QzRun {
     const std::vector<uint8_t> *il, *dl;
 };
 
-// The run's sweeps, first points (first.q) and sums.
 template <typename T>
-void qz_plan(const QzGeom &g, const QzRun &R, uint64_t nblk, std::vector<QzTask> &steps, QzTask &first, SumPlan &sp,
-             std::vector<std::pair<int64_t, int64_t>> *level_ranges) {
+void qz_run(const QzGeom &g, const QzRun &R, T *work, uint16_t *codes, T *scratch, double *err, uint64_t nblk,
+            SumPlan &sp, std::vector<std::pair<int64_t, int64_t>> *level_ranges, cudaStream_t st, Counter &launches) {
     sp.nseg = 0;
     sp.cpb = g.cpb;
     sp.nlines = 0;
     int64_t pos = 0;
     int start = R.start_level;
-    std::memset(&first, 0, sizeof(first));
-    first.q.eb = R.eb;
-    first.q.recip = 1.0 / R.eb;
-    first.q.radius = 32768;
-    first.q.trim = R.trim;
     if (!g.anchor) {
+        LevelArgs q;
+        std::memset(&q, 0, sizeof(q));
+        q.eb = R.eb;
+        q.recip = 1.0 / R.eb;
+        q.radius = 32768;
+        q.trim = R.trim;
+        if (R.mode == 1)
+            k_qz_first<T, 1><<<(unsigned)((nblk + 127) / 128), 128, 0, st>>>(q, work, g.per, g.cpb, codes, scratch, nblk);
+        else
+            k_qz_first<T, 2><<<(unsigned)((nblk + 127) / 128), 128, 0, st>>>(q, work, g.per, g.cpb, codes, scratch, nblk);
+        launches(cudaGetLastError());
         pos = 1;
     } else if (start == g.levels) {
+        if (R.mode == 1 && g.nanchor > 0) {
+            const uint64_t total = (uint64_t)g.nanchor * nblk;
+            // axis strides of the embedded field for the anchor coordinates
+            k_qz_anchor<T><<<(unsigned)((total + 127) / 128), 128, 0, st>>>(
+                work, g.per, g.cpb, g.na[0], g.na[1], g.na[2], g.ms, g.e, g.offs[0], g.offs[1], codes, scratch, total);
+            launches(cudaGetLastError());
+        }
         pos = R.mode == 1 ? g.nanchor : 0;
         start--;
     }
@@ -452,13 +435,17 @@ void qz_plan(const QzGeom &g, const QzRun &R, uint64_t nblk, std::vector<QzTask>
             w.seg_off = pos;
             const int64_t lines = w.cnt[0] * w.cnt[1];
             const uint64_t total = (uint64_t)(lines * w.tpl) * nblk;
-            QzTask task;
-            std::memset(&task, 0, sizeof(task));
-            task.w = w;
-            task.q = q;
-            task.total = total;
-            task.straight = straight;
-            steps.push_back(task);
+            if (total) {
+                const unsigned grid = (unsigned)((total + 255) / 256);
+                if (R.mode == 1) {
+                    if (straight) k_qz_sweep<T, 1, 1><<<grid, 256, 0, st>>>(w, q, work, codes, scratch, err, total);
+                    else k_qz_sweep<T, 1, 0><<<grid, 256, 0, st>>>(w, q, work, codes, scratch, err, total);
+                } else {
+                    if (straight) k_qz_sweep<T, 2, 1><<<grid, 256, 0, st>>>(w, q, work, codes, scratch, err, total);
+                    else k_qz_sweep<T, 2, 0><<<grid, 256, 0, st>>>(w, q, work, codes, scratch, err, total);
+                }
+                launches(cudaGetLastError());
+            }
             if (sp.nseg >= kMaxSegs) throw Fail{FAZ_ERR_UNSUPPORTED, "too many tuning levels"};
             sp.seg[sp.nseg++] = SumSeg{pos, sp.nlines, lines, w.tpl, d == g.N - 1 ? 1 : 0};
             sp.nlines += lines;
@@ -469,75 +456,6 @@ void qz_plan(const QzGeom &g, const QzRun &R, uint64_t nblk, std::vector<QzTask>
             range_lo = pos;
         }
     }
-}
-
-// A batch of runs of one mode over the sampled blocks; the errors' sums (run by
-// run, block by block) land in b.bsum.  ranges: the level ranges, the same for all
-// runs of mode 1.
-template <typename T>
-void qz_run_batch(const QzGeom &g, const std::vector<QzRun> &runs, const T *blocks, const QzBuffers<T> &b, uint64_t nblk,
-                  DevMem &m, std::vector<std::pair<int64_t, int64_t>> *ranges, cudaStream_t st, Counter &launches) {
-    const unsigned n = (unsigned)runs.size();
-    const int mode = runs[0].mode;
-    std::vector<std::vector<QzTask>> steps(n);
-    std::vector<SumPlan> plans(n);
-    std::vector<QzTask> table(n);  // the first points' tasks, then each step's
-    size_t nstep = 0;
-    int64_t max_lines = 0;
-    for (unsigned i = 0; i < n; i++) {
-        qz_plan<T>(g, runs[i], nblk, steps[i], table[i], plans[i], i == 0 ? ranges : nullptr);
-        nstep = std::max(nstep, steps[i].size());
-        max_lines = std::max(max_lines, plans[i].nlines);
-    }
-    QzTask none;
-    std::memset(&none, 0, sizeof(none));
-    none.straight = true;
-    for (size_t k = 0; k < nstep; k++)
-        for (unsigned i = 0; i < n; i++) table.push_back(k < steps[i].size() ? steps[i][k] : none);
-    QzTask *dt = m.alloc<QzTask>(table.size());
-    SumPlan *dp = m.alloc<SumPlan>(n);
-    CK(cudaMemcpyAsync(dt, table.data(), table.size() * sizeof(QzTask), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(dp, plans.data(), n * sizeof(SumPlan), cudaMemcpyHostToDevice, st));
-    k_qz_spread<T><<<dim3((unsigned)((b.nv + 255) / 256), n), 256, 0, st>>>(blocks, b.work, b.nv);
-    launches(cudaGetLastError());
-    if (!g.anchor) {
-        const dim3 grid((unsigned)((nblk + 127) / 128), n);
-        if (mode == 1) k_qz_first<T, 1><<<grid, 128, 0, st>>>(dt, b, g.per, g.cpb, nblk);
-        else k_qz_first<T, 2><<<grid, 128, 0, st>>>(dt, b, g.per, g.cpb, nblk);
-        launches(cudaGetLastError());
-    } else if (mode == 1 && g.nanchor > 0) {
-        const uint64_t total = (uint64_t)g.nanchor * nblk;
-        // axis strides of the embedded field for the anchor coordinates
-        k_qz_anchor<T><<<dim3((unsigned)((total + 127) / 128), n), 128, 0, st>>>(
-            b, g.per, g.cpb, g.na[0], g.na[1], g.na[2], g.ms, g.e, g.offs[0], g.offs[1], total);
-        launches(cudaGetLastError());
-    }
-    for (size_t k = 0; k < nstep; k++) {
-        const QzTask *row = table.data() + (k + 1) * n, *drow = dt + (k + 1) * n;
-        uint64_t total = 0;
-        bool straight = true;
-        for (unsigned i = 0; i < n; i++) {
-            total = std::max(total, row[i].total);
-            straight = straight && row[i].straight;
-        }
-        if (!total) continue;
-        const dim3 grid((unsigned)((total + 255) / 256), n);
-        if (mode == 1) {
-            if (straight) k_qz_sweep<T, 1, 1><<<grid, 256, 0, st>>>(drow, b);
-            else k_qz_sweep<T, 1, 0><<<grid, 256, 0, st>>>(drow, b);
-        } else {
-            if (straight) k_qz_sweep<T, 2, 1><<<grid, 256, 0, st>>>(drow, b);
-            else k_qz_sweep<T, 2, 0><<<grid, 256, 0, st>>>(drow, b);
-        }
-        launches(cudaGetLastError());
-    }
-    if (max_lines) {
-        k_qz_line_sums<<<dim3((unsigned)(((uint64_t)max_lines * nblk + 127) / 128), n), 128, 0, st>>>(dp, b.err, b.cs,
-                                                                                                  b.lsum, b.ls, nblk);
-        launches(cudaGetLastError());
-    }
-    k_qz_sum<<<dim3((unsigned)nblk, n), 256, 0, st>>>(dp, b.lsum, b.ls, b.bsum);
-    launches(cudaGetLastError());
 }
 
 // Codes and lines per block of a full tuning-1 run.
@@ -775,14 +693,24 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
     QzGeom g = make_geom(N, bsz, (int64_t)c.maxStep);
     full_run_sizes(g);
     uint64_t nblk = 0, nv = 0, ns = 0;
-    T *blocks = nullptr;
-    // the sampled blocks
+    T *blocks = nullptr, *work = nullptr, *scratch = nullptr;
+    uint16_t *codes = nullptr;
+    double *err = nullptr, *lsum = nullptr, *bsum = nullptr;
+    std::vector<double> hsum;
+    // the sampled blocks and the buffers sized by their count
     auto gather = [&](const std::vector<int64_t> &sts) {
         nblk = sts.size() / 3;
         if (nblk == 0) throw Fail{FAZ_ERR_UNSUPPORTED, "no block to sample for QoZ tuning"};
         nv = nblk * (uint64_t)g.per;
         ns = nblk * (uint64_t)g.cpb;
         blocks = m.alloc<T>(nv);
+        work = m.alloc<T>(nv);
+        scratch = m.alloc<T>(ns);
+        codes = m.alloc<uint16_t>(ns);
+        err = m.alloc<double>(ns);
+        lsum = m.alloc<double>(nblk * (uint64_t)g.lpb + 1);
+        bsum = m.alloc<double>(nblk);
+        hsum.assign(nblk, 0.0);
         int64_t *dstarts = m.alloc<int64_t>(sts.size());
         CK(cudaMemcpyAsync(dstarts, sts.data(), sts.size() * 8, cudaMemcpyHostToDevice, st));
         k_qz_gather<T><<<(unsigned)((nv + 255) / 256), 256, 0, st>>>(dX, dstarts, (int64_t)c.dims[1],
@@ -792,24 +720,13 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
     };
     gather(starts);
     mark("sampled blocks", (double)nblk, (double)nv);
-    // a batch's buffers, and how many runs make one: runs beyond 1 GB of them wait
-    // for the next batch (that many fill the GPU)
-    auto batch_buffers = [&](DevMem &bm, uint64_t n, int mode) {
-        QzBuffers<T> b;
-        b.nv = nv;
-        b.cs = (ns + zero_subchunk() - 1) / zero_subchunk() * zero_subchunk();
-        b.ls = nblk * (uint64_t)g.lpb;
-        b.work = bm.alloc<T>(n * b.nv);
-        b.scratch = mode == 1 ? bm.alloc<T>(n * b.cs) : nullptr;
-        b.codes = mode == 1 ? bm.alloc<uint16_t>(n * b.cs) : nullptr;
-        b.err = bm.alloc<double>(n * b.cs);
-        b.lsum = bm.alloc<double>(n * b.ls + 1);
-        b.bsum = bm.alloc<double>(n * nblk);
-        return b;
-    };
-    auto batch_limit = [&](size_t n) {
-        const uint64_t run = nv * sizeof(T) + (ns + zero_subchunk()) * (sizeof(T) + 12) + 8 * nblk * (uint64_t)g.lpb;
-        return (size_t)std::min<uint64_t>(n, std::max<uint64_t>(1, (1ull << 30) / run));
+    auto block_sums = [&](const SumPlan &sp) -> double {
+        launch_qz_sum(sp, err, lsum, bsum, nblk, st, launches);
+        CK(cudaMemcpyAsync(hsum.data(), bsum, nblk * 8, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        double s = 0;
+        for (uint64_t k = 0; k < nblk; k++) s += hsum[k];
+        return s;
     };
     const double o_alpha = c.alpha, o_beta = c.beta;
     if (c.autoTuningRate > 0) {
@@ -826,6 +743,31 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
     const int Lsel = c.levelwisePredictionSelection;
     std::vector<uint8_t> il(Lsel > 0 ? Lsel : 0), dl(Lsel > 0 ? Lsel : 0);
     const int dirs[2] = {0, N == 3 ? 5 : 1};
+    SumPlan sp;
+    // One CompressTest (SZInterp.hpp:1130-1392) of every sampled block: bit
+    // rate after Huffman + zstd, PSNR from the summed squared errors.  Its
+    // device buffers and bookkeeping live in a context, so that several tests
+    // can run at once, each on its own stream and host thread.
+    struct CtCtx {
+        DevMem m;
+        T *work, *scratch;
+        uint16_t *codes;
+        double *err, *lsum, *bsum;
+        std::vector<double> hsum;
+        SumPlan sp;
+        std::vector<std::pair<int64_t, int64_t>> ranges;
+        Counter launches;
+        faz_timings tm;
+        CtCtx(cudaStream_t s, uint64_t nv_, uint64_t ns_, uint64_t nblk_, uint64_t lpb_) : m(s), hsum(nblk_, 0.0) {
+            work = m.alloc<T>(nv_);
+            scratch = m.alloc<T>(ns_);
+            codes = m.alloc<uint16_t>(ns_);
+            err = m.alloc<double>(ns_);
+            lsum = m.alloc<double>(nblk_ * lpb_ + 1);
+            bsum = m.alloc<double>(nblk_);
+            std::memset(&tm, 0, sizeof(tm));
+        }
+    };
     // The SSIM and autocorrelation targets score the alpha/beta search's
     // tests by the sampled blocks' reconstructions (tuning_metrics.h): set
     // once the search's sample is in, with the original blocks on the host.
@@ -836,158 +778,99 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
         if (metric_target == 2) return ssim_metric<T>(cubes, horig.data(), cur.data(), nblk);
         return 1.0 - autocorrelation_of<T>(horig.data(), cur.data(), horig.size());
     };
-    // CompressTests (SZInterp.hpp:1130-1392) of every sampled block: bit rate
-    // after Huffman + zstd, PSNR from the summed squared errors.  The tests of one
-    // call run together: their sweeps, sums and unpredictable values as a batch,
-    // then each one's Huffman and zstd on its own stream and host thread.
-    struct Test {
-        int op, dir;
-        double alpha, beta, eb;
-        bool lists;
-    };
-    struct TestRes {
-        double br = 0, mm = 0;
-        uint64_t launches = 0;
-        double host_ms = 0;
-    };
-    auto run_tests = [&](const std::vector<Test> &tests, double pc) {
-        std::vector<TestRes> res(tests.size());
-        const size_t limit = batch_limit(tests.size());
-        for (size_t t0 = 0; t0 < tests.size(); t0 += limit) {
-            const uint64_t n = std::min(limit, tests.size() - t0);
-            DevMem bm(st);
-            const QzBuffers<T> b = batch_buffers(bm, n, 1);
-            std::vector<QzRun> runs;
-            for (uint64_t i = 0; i < n; i++) {
-                const Test &t = tests[t0 + i];
-                runs.push_back({1, g.levels, 0, t.eb, t.alpha, t.beta, c.trimToZero, t.op, t.dir,
-                                t.lists ? &il : nullptr, t.lists ? &dl : nullptr});
-            }
-            std::vector<std::pair<int64_t, int64_t>> ranges;
-            qz_run_batch<T>(g, runs, blocks, b, nblk, bm, &ranges, st, launches);
-            // q_bins: level ranges from the coarsest, each across all blocks
-            // (the anchors travel with the first interpolated level)
-            std::vector<int64_t> rlo, rlen, rout;
-            int64_t o = 0;
-            for (size_t i = 0; i < ranges.size(); i++) {
-                const int64_t lo = i == 0 ? 0 : ranges[i].first, hi = ranges[i].second;
-                if (hi <= lo) continue;
-                rlo.push_back(lo);
-                rlen.push_back(hi - lo);
-                rout.push_back(o);
-                o += (hi - lo) * (int64_t)nblk;
-            }
-            if (o != (int64_t)ns) throw Fail{FAZ_ERR_DEVICE, "tuning codes do not cover the sampled blocks"};
-            std::vector<int64_t> hr;
-            hr.insert(hr.end(), rlo.begin(), rlo.end());
-            hr.insert(hr.end(), rlen.begin(), rlen.end());
-            hr.insert(hr.end(), rout.begin(), rout.end());
-            int64_t *dr = bm.alloc<int64_t>(hr.size());
-            CK(cudaMemcpyAsync(dr, hr.data(), hr.size() * 8, cudaMemcpyHostToDevice, st));
-            uint16_t *qb = bm.alloc<uint16_t>(n * b.cs);
-            const int nr = (int)rlo.size();
-            k_qz_regroup<<<dim3((unsigned)((ns + 255) / 256), (unsigned)n), 256, 0, st>>>(
-                b.codes, b.cs, g.cpb, dr, dr + nr, dr + 2 * nr, nr, qb, ns);
-            launches(cudaGetLastError());
-            // unpredictable values in the order the quantiser kept them (block by
-            // block, stream order): zeros of the block-major codes, of all tests in
-            // one pass (the padding between tests is no zero)
-            if (b.cs > ns)
-                CK(cudaMemset2DAsync(b.codes + ns, b.cs * 2, 1, (b.cs - ns) * 2, n, st));
-            const uint64_t nsub = hist_subchunks(n * b.cs), per_test = b.cs / zero_subchunk();
-            unsigned long long *zc = bm.alloc<unsigned long long>(2 * (nsub + 1) + scan_temp_words(nsub) + 1),
-                               *zoff = zc + nsub + 1;
-            launches(launch_count_zeros(b.codes, n * b.cs, zc, st));
-            launches(launch_scan_u64(zc, zoff, nsub, zoff + nsub + 1, st));
-            std::vector<double> hsum(n * nblk);
-            std::vector<unsigned long long> zat(n + 1);
-            CK(cudaMemcpyAsync(hsum.data(), b.bsum, n * nblk * 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpy2DAsync(zat.data(), 8, zoff, per_test * 8, 8, n + 1, cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-            T *unp = bm.alloc<T>(zat[n]);
-            if (zat[n]) launches(launch_compact_zeros<T>(b.codes, n * b.cs, zc, zoff, b.scratch, unp, st));
-            CK(cudaStreamSynchronize(st));
-            auto finish = [&](uint64_t i, cudaStream_t s) {
-                const Test &t = tests[t0 + i];
-                TestRes r;
-                DevMem xm(s);
-                Counter nl;
-                faz_timings xt;
-                std::memset(&xt, 0, sizeof(xt));
-                double se = 0;
-                for (uint64_t k = 0; k < nblk; k++) se += hsum[i * nblk + k];
-                HuffEncoded h;
-                huffman_encode_device(qb + i * b.cs, ns, 32768, xm, s, nl, h, xt, {}, false, false);
-                const uint64_t nunp = zat[i + 1] - zat[i];
-                std::vector<uint8_t> head;
-                put<uint8_t>(head, 2);
-                put<double>(head, t.eb);
-                put<int32_t>(head, 32768);
-                put<uint64_t>(head, nunp);
-                std::vector<uint8_t> tree;
-                append_tree(tree, h.cb, h.nbytes);
-                // the payload through the thread's pinned staging buffer
-                const size_t plen = head.size() + nunp * sizeof(T) + tree.size() + h.nbytes;
-                uint8_t *pl = t_pin_payload.get(plen + 8);
-                std::memcpy(pl, head.data(), head.size());
-                if (nunp)
-                    CK(cudaMemcpyAsync(pl + head.size(), unp + zat[i], nunp * sizeof(T), cudaMemcpyDeviceToHost, s));
-                std::memcpy(pl + head.size() + nunp * sizeof(T), tree.data(), tree.size());
-                if (h.nbytes)
-                    CK(cudaMemcpyAsync(pl + head.size() + nunp * sizeof(T) + tree.size(), h.bits, h.nbytes,
-                                       cudaMemcpyDeviceToHost, s));
-                CK(cudaStreamSynchronize(s));
-                // profiling_coeff scales both (SZInterp.hpp:1364-1370)
-                const double ele = (double)nv;
-                mark("  compress test payload", (double)plen, t.alpha);
-                r.br = 8 * (double)zstd_framed_size_host(pl, plen) / ele;
-                mark("  compress test zstd", t.beta, t.eb);
-                r.br *= pc;
-                double mse = se / ele;
-                mse *= pc;
-                r.mm = 20 * std::log10(c.rng) - 10 * std::log10(mse);
-                if (metric_target >= 2) {
-                    // the reconstructions are left in the working copy
-                    std::vector<T> cur(nv);
-                    CK(cudaMemcpyAsync(cur.data(), b.work + i * nv, nv * sizeof(T), cudaMemcpyDeviceToHost, s));
-                    CK(cudaStreamSynchronize(s));
-                    r.mm = target_metric(cur);
-                }
-                r.launches = nl.n;
-                r.host_ms = xt.host_ms;
-                return r;
-            };
-            if (n == 1) {
-                res[t0] = finish(0, st);
-            } else {
-                std::vector<std::future<TestRes>> futs;
-                for (uint64_t i = 0; i < n; i++)
-                    futs.push_back(TaskThreads::get().submit<TestRes>([&, i]() {
-                        StreamGuard sg(nullptr);
-                        return finish(i, sg.st);
-                    }));
-                std::exception_ptr first;
-                for (uint64_t i = 0; i < n; i++) {
-                    try {
-                        res[t0 + i] = futs[i].get();
-                    } catch (...) {
-                        if (!first) first = std::current_exception();
-                    }
-                }
-                if (first) std::rethrow_exception(first);
-            }
-            for (uint64_t i = 0; i < n; i++) {
-                launches.n += res[t0 + i].launches;
-                tm.host_ms += res[t0 + i].host_ms;
-            }
+    auto compress_test_on = [&](CtCtx &x, cudaStream_t s, int op, int dir, double alpha, double beta, double eb,
+                                double &bitrate, double &psnr, bool lists, double pc) {
+        CK(cudaMemcpyAsync(x.work, blocks, nv * sizeof(T), cudaMemcpyDeviceToDevice, s));
+        QzRun R{1, g.levels, 0, eb, alpha, beta, c.trimToZero, op, dir, lists ? &il : nullptr, lists ? &dl : nullptr};
+        qz_run<T>(g, R, x.work, x.codes, x.scratch, x.err, nblk, x.sp, &x.ranges, s, x.launches);
+        launch_qz_sum(x.sp, x.err, x.lsum, x.bsum, nblk, s, x.launches);
+        CK(cudaMemcpyAsync(x.hsum.data(), x.bsum, nblk * 8, cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        double se = 0;
+        for (uint64_t k = 0; k < nblk; k++) se += x.hsum[k];
+        // q_bins: level ranges from the coarsest, each across all blocks
+        // (the anchors travel with the first interpolated level)
+        std::vector<int64_t> rlo, rlen, rout;
+        int64_t o = 0;
+        for (size_t i = 0; i < x.ranges.size(); i++) {
+            const int64_t lo = i == 0 ? 0 : x.ranges[i].first, hi = x.ranges[i].second;
+            if (hi <= lo) continue;
+            rlo.push_back(lo);
+            rlen.push_back(hi - lo);
+            rout.push_back(o);
+            o += (hi - lo) * (int64_t)nblk;
         }
-        return res;
+        if (o != (int64_t)ns) throw Fail{FAZ_ERR_DEVICE, "tuning codes do not cover the sampled blocks"};
+        int64_t *dr = x.m.alloc<int64_t>(3 * rlo.size() + 3);
+        std::vector<int64_t> hr;
+        hr.insert(hr.end(), rlo.begin(), rlo.end());
+        hr.insert(hr.end(), rlen.begin(), rlen.end());
+        hr.insert(hr.end(), rout.begin(), rout.end());
+        CK(cudaMemcpyAsync(dr, hr.data(), hr.size() * 8, cudaMemcpyHostToDevice, s));
+        uint16_t *qb = x.m.alloc<uint16_t>(ns);
+        const int nr = (int)rlo.size();
+        k_qz_regroup<<<(unsigned)((ns + 255) / 256), 256, 0, s>>>(x.codes, g.cpb, dr, dr + nr, dr + 2 * nr, nr, nblk,
+                                                                  qb, ns);
+        x.launches(cudaGetLastError());
+        HuffEncoded h;
+        huffman_encode_device(qb, ns, 32768, x.m, s, x.launches, h, x.tm);
+        // unpredictable values in the order the quantiser kept them
+        // (block by block, stream order): zeros of the block-major codes
+        const uint64_t nunp = h.nzero;
+        T *unp = nullptr;
+        if (nunp) {
+            const uint64_t nsub = hist_subchunks(ns);
+            unsigned long long *zc = x.m.alloc<unsigned long long>(2 * (nsub + 1) + scan_temp_words(nsub) + 1),
+                               *zoff = zc + nsub + 1;
+            unp = x.m.alloc<T>(nunp);
+            x.launches(launch_count_zeros(x.codes, ns, zc, s));
+            x.launches(launch_scan_u64(zc, zoff, nsub, zoff + nsub + 1, s));
+            x.launches(launch_compact_zeros<T>(x.codes, ns, zc, zoff, x.scratch, unp, s));
+        }
+        std::vector<uint8_t> head;
+        put<uint8_t>(head, 2);
+        put<double>(head, eb);
+        put<int32_t>(head, 32768);
+        put<uint64_t>(head, nunp);
+        std::vector<uint8_t> tree;
+        append_tree(tree, h.cb, h.nbytes);
+        // the payload through the thread's pinned staging buffer
+        const size_t plen = head.size() + nunp * sizeof(T) + tree.size() + h.nbytes;
+        uint8_t *pl = t_pin_payload.get(plen + 8);
+        std::memcpy(pl, head.data(), head.size());
+        if (nunp) CK(cudaMemcpyAsync(pl + head.size(), unp, nunp * sizeof(T), cudaMemcpyDeviceToHost, s));
+        std::memcpy(pl + head.size() + nunp * sizeof(T), tree.data(), tree.size());
+        if (h.nbytes)
+            CK(cudaMemcpyAsync(pl + head.size() + nunp * sizeof(T) + tree.size(), h.bits, h.nbytes,
+                               cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        // profiling_coeff scales both (SZInterp.hpp:1364-1370)
+        const double ele = (double)nv;
+        mark("  compress test payload", (double)plen, alpha);
+        bitrate = 8 * (double)zstd_framed_size_host(pl, plen) / ele;
+        mark("  compress test zstd", beta, eb);
+        bitrate *= pc;
+        double mse = se / ele;
+        mse *= pc;
+        psnr = 20 * std::log10(c.rng) - 10 * std::log10(mse);
+        if (metric_target >= 2) {
+            // the reconstructions are left in the working copy
+            std::vector<T> cur(nv);
+            CK(cudaMemcpyAsync(cur.data(), x.work, nv * sizeof(T), cudaMemcpyDeviceToHost, s));
+            CK(cudaStreamSynchronize(s));
+            psnr = target_metric(cur);
+        }
     };
+    // tests on the tuner's own stream
+    std::unique_ptr<CtCtx> main_ctx;
     auto compress_test = [&](int op, int dir, double alpha, double beta, double eb, double &bitrate, double &psnr,
                              bool lists = true, double pc = 1.0) {
-        const TestRes r = run_tests({{op, dir, alpha, beta, eb, lists}}, pc)[0];
-        bitrate = r.br;
-        psnr = r.mm;
+        if (!main_ctx || main_ctx->hsum.size() != nblk) main_ctx.reset(new CtCtx(st, nv, ns, nblk, (uint64_t)g.lpb));
+        compress_test_on(*main_ctx, st, op, dir, alpha, beta, eb, bitrate, psnr, lists, pc);
+        launches.n += main_ctx->launches.n;
+        main_ctx->launches.n = 0;
+        tm.host_ms += main_ctx->tm.host_ms;
+        main_ctx->tm.host_ms = 0;
     };
     // without the alpha/beta search (autoTuningRate = 0) the decisions
     // compare compression ratios of CompressTests (TUNING_TARGET_CR)
@@ -1000,40 +883,20 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
         best_lorenzo_ratio = sizeof(T) * 8.0 / br;
     }
     if (Lsel > 0) {
-        // per-level selection by summed prediction loss (tuning mode 2); every
-        // run starts from the original blocks, so all of them make one batch
-        std::vector<QzRun> runs;
+        // per-level selection by summed prediction loss (tuning mode 2)
         for (int level = Lsel; level > 0; level--) {
             int start_level = level == Lsel ? 9999 : level, end_level = level - 1;
             if (start_level <= 0 || start_level > g.levels) start_level = g.levels;
             if (end_level >= start_level || end_level < 0) end_level = 0;
-            for (int op = 0; op < 2; op++)
-                for (int di = 0; di < 2; di++)
-                    runs.push_back({2, start_level, end_level, c.absErrorBound, c.alpha, c.beta, c.trimToZero, op,
-                                    dirs[di], nullptr, nullptr});
-        }
-        std::vector<double> loss(runs.size()), hsum;
-        const size_t limit = batch_limit(runs.size());
-        for (size_t r0 = 0; r0 < runs.size(); r0 += limit) {
-            const std::vector<QzRun> part(runs.begin() + r0, runs.begin() + std::min(r0 + limit, runs.size()));
-            DevMem bm(st);
-            const QzBuffers<T> b = batch_buffers(bm, part.size(), 2);
-            qz_run_batch<T>(g, part, blocks, b, nblk, bm, nullptr, st, launches);
-            hsum.resize(part.size() * nblk);
-            CK(cudaMemcpyAsync(hsum.data(), b.bsum, hsum.size() * 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-            for (size_t i = 0; i < part.size(); i++) {
-                double s = 0;
-                for (uint64_t k = 0; k < nblk; k++) s += hsum[i * nblk + k];
-                loss[r0 + i] = s;
-            }
-        }
-        for (int level = Lsel; level > 0; level--) {
             int best_op = 1, best_dir = 0;
             double best = DBL_MAX;
             for (int op = 0; op < 2; op++)
                 for (int di = 0; di < 2; di++) {
-                    const double cur = loss[(size_t)(Lsel - level) * 4 + 2 * op + di];
+                    CK(cudaMemcpyAsync(work, blocks, nv * sizeof(T), cudaMemcpyDeviceToDevice, st));
+                    QzRun R{2, start_level, end_level, c.absErrorBound, c.alpha, c.beta, c.trimToZero, op, dirs[di],
+                            nullptr, nullptr};
+                    qz_run<T>(g, R, work, codes, scratch, err, nblk, sp, nullptr, st, launches);
+                    const double cur = block_sums(sp);
                     if (cur < best) {
                         best = cur;
                         best_op = op;
@@ -1060,18 +923,17 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
         // ratio of a CompressTest per candidate (SZInterp.hpp:2036-2076)
         int best_op = FAZ_INTERP_ALGO_CUBIC, best_dir = 0;
         double best_cr = 0;
-        std::vector<Test> tests;
         for (int op = 0; op < 2; op++)
-            for (int di = 0; di < 2; di++) tests.push_back({op, dirs[di], c.alpha, c.beta, c.absErrorBound, true});
-        const std::vector<TestRes> res = run_tests(tests, 1.0);
-        for (size_t i = 0; i < tests.size(); i++) {
-            const double cr = sizeof(T) * 8.0 / res[i].br;
-            if (cr > best_cr) {
-                best_cr = cr;
-                best_op = tests[i].op;
-                best_dir = tests[i].dir;
+            for (int di = 0; di < 2; di++) {
+                double br, mm;
+                compress_test(op, dirs[di], c.alpha, c.beta, c.absErrorBound, br, mm);
+                const double cr = sizeof(T) * 8.0 / br;
+                if (cr > best_cr) {
+                    best_cr = cr;
+                    best_op = op;
+                    best_dir = dirs[di];
+                }
             }
-        }
         c.interpAlgo = best_op;
         c.interpDirection = (uint8_t)best_dir;
         if (cr_tests) best_interp_cr = best_cr;
@@ -1101,14 +963,21 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
                    (alpha < 1 && alpha * (max_interp_level - 1) <= beta);
         };
         // The grid's CompressTests at the bound itself are independent of
-        // one another: all of them run at once.  The search below reads their
-        // results in the reference's order (a test it never reaches is simply
-        // unused) and runs the tests it derives on the way - a bound scaled by a
-        // ratio found so far - one by one.
+        // one another: all of them run at once, each with its own stream,
+        // buffers and host thread.  The search below reads their results in
+        // the reference's order (a test it never reaches is simply unused)
+        // and runs the tests it derives on the way - a bound scaled by a ratio
+        // found so far - one by one.
+        struct GridRes {
+            double br = 0, mm = 0;
+            uint64_t launches = 0;
+            double host_ms = 0;
+        };
         std::vector<std::pair<double, double>> grid;
         for (double alpha : alist)
             for (double beta : blist)
                 if (!((alpha >= 1 && alpha > beta) || (alpha < 0 && beta != -1))) grid.emplace_back(alpha, beta);
+        CK(cudaStreamSynchronize(st));  // the sampled blocks are gathered
         if (c.tuningTarget >= 2) {
             horig.resize(nv);
             CK(cudaMemcpyAsync(horig.data(), blocks, nv * sizeof(T), cudaMemcpyDeviceToHost, st));
@@ -1118,9 +987,34 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
             metric_target = c.tuningTarget;
         }
         const int op0 = c.interpAlgo, dir0 = c.interpDirection;
-        std::vector<Test> gtests;
-        for (const auto &ab : grid) gtests.push_back({op0, dir0, ab.first, ab.second, oriabseb, true});
-        const std::vector<TestRes> gres = run_tests(gtests, pcoeff);
+        std::vector<std::future<GridRes>> futs;
+        for (const auto &ab : grid) {
+            const double alpha = ab.first, beta = ab.second;
+            futs.push_back(TaskThreads::get().submit<GridRes>([&, alpha, beta]() {
+                StreamGuard sg(nullptr);
+                CtCtx x(sg.st, nv, ns, nblk, (uint64_t)g.lpb);
+                GridRes r;
+                compress_test_on(x, sg.st, op0, dir0, alpha, beta, oriabseb, r.br, r.mm, true, pcoeff);
+                CK(cudaStreamSynchronize(sg.st));
+                r.launches = x.launches.n;
+                r.host_ms = x.tm.host_ms;
+                return r;
+            }));
+        }
+        std::vector<GridRes> gres(grid.size());
+        {
+            std::exception_ptr first;
+            for (size_t i = 0; i < futs.size(); i++) {
+                try {
+                    gres[i] = futs[i].get();
+                    launches.n += gres[i].launches;
+                    tm.host_ms += gres[i].host_ms;
+                } catch (...) {
+                    if (!first) first = std::current_exception();
+                }
+            }
+            if (first) std::rethrow_exception(first);
+        }
         mark("grid tests", (double)grid.size());
         auto grid_result = [&](double alpha, double beta, double &br, double &mm) {
             for (size_t i = 0; i < grid.size(); i++)
@@ -1137,8 +1031,11 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
         // search under that assumption, run the derived tests it meets at
         // once, and let the search below take a result only where its bound
         // is the one the search asks for (else that test runs again).
-        std::vector<Test> derived;
-        std::vector<TestRes> dres;
+        struct Derived {
+            double alpha, beta, eb;
+            GridRes r;
+        };
+        std::vector<Derived> derived;
         {
             double bb = 9999, bm = 0;
             for (double alpha : alist) {
@@ -1154,19 +1051,43 @@ void qoz_tune_device(faz_config &c, const T *dX, cudaStream_t st, Counter &launc
                         if (stop_here(alpha, beta)) break;
                         continue;
                     } else {
-                        derived.push_back({op0, dir0, alpha, beta, oriabseb * (br / bb), true});
+                        derived.push_back({alpha, beta, oriabseb * (br / bb), GridRes{}});
                     }
                     if (stop_here(alpha, beta)) break;
                 }
             }
-            dres = run_tests(derived, pcoeff);
+            std::vector<std::future<GridRes>> dfut;
+            for (const Derived &dv : derived) {
+                const double alpha = dv.alpha, beta = dv.beta, ebd = dv.eb;
+                dfut.push_back(TaskThreads::get().submit<GridRes>([&, alpha, beta, ebd]() {
+                    StreamGuard sg(nullptr);
+                    CtCtx x(sg.st, nv, ns, nblk, (uint64_t)g.lpb);
+                    GridRes r;
+                    compress_test_on(x, sg.st, op0, dir0, alpha, beta, ebd, r.br, r.mm, true, pcoeff);
+                    CK(cudaStreamSynchronize(sg.st));
+                    r.launches = x.launches.n;
+                    r.host_ms = x.tm.host_ms;
+                    return r;
+                }));
+            }
+            std::exception_ptr first;
+            for (size_t i = 0; i < dfut.size(); i++) {
+                try {
+                    derived[i].r = dfut[i].get();
+                    launches.n += derived[i].r.launches;
+                    tm.host_ms += derived[i].r.host_ms;
+                } catch (...) {
+                    if (!first) first = std::current_exception();
+                }
+            }
+            if (first) std::rethrow_exception(first);
         }
         mark("derived tests", (double)derived.size());
         auto derived_test = [&](double alpha, double beta, double ebd, double &br, double &mm) {
-            for (size_t i = 0; i < derived.size(); i++)
-                if (derived[i].alpha == alpha && derived[i].beta == beta && derived[i].eb == ebd) {
-                    br = dres[i].br;
-                    mm = dres[i].mm;
+            for (const Derived &dv : derived)
+                if (dv.alpha == alpha && dv.beta == beta && dv.eb == ebd) {
+                    br = dv.r.br;
+                    mm = dv.r.mm;
                     return;
                 }
             compress_test(op0, dir0, alpha, beta, ebd, br, mm, true, pcoeff);

@@ -1,9 +1,8 @@
-"""The QoZ tuner's batches of trials and their error sums (k_qz_sweep,
-k_qz_line_sums, k_qz_sum in qoz.cu) on sampled blocks of few and many lines: below
-one chunk of the chain kernel and across one chunk's end, one block and several,
-and trials that do not fit in one batch.  The sums decide the interpolators,
-directions, alpha and beta, which the stream records: streams equal the oracle's
-byte for byte."""
+"""The QoZ tuner's error sums (k_qz_line_sums, k_qz_sum in qoz.cu) on sampled
+blocks of few and many lines: below one chunk of the chain kernel and across one
+chunk's end, one block and several.  The sums decide the
+interpolators, directions, alpha and beta, which the stream records: streams
+equal the oracle's byte for byte."""
 import numpy as np
 import pytest
 
@@ -27,7 +26,6 @@ CASES = [
     ((100, 101, 99), 32, 0.1, np.float32),    # 33^3: 2.6 thousand
     ((100, 101, 99), 32, 0.1, np.float64),
     ((210, 333), 32, 0.2, np.float32),        # 33^2: a hundred
-    ((200, 200, 200), 32, 0.5, np.float32),   # 108 blocks: the trials in several batches
 ]
 
 

@@ -147,10 +147,10 @@ def make_conf(F, dims, eb, interp, algo="auto"):
 
 # DRAM traffic of one finest-level compress launch (the plane kernel
 # k_finest), measured with ncu (dram__bytes_read.sum + dram__bytes_write.sum =
-# 335.69 MB + 95.54 MB) on a 256x512x512 float32 field, cubic, rel eb 1e-3;
+# 336.04 MB + 97.93 MB) on a 256x512x512 float32 field, cubic, rel eb 1e-3;
 # traffic grows with the number of values, so it is scaled to the benchmarked
 # field by its value count.
-FINEST_TRAFFIC_BYTES = 431225856
+FINEST_TRAFFIC_BYTES = 433970432
 FINEST_TRAFFIC_VALUES = 256 * 512 * 512
 
 

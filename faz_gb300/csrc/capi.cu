@@ -374,7 +374,7 @@ void huffman_encode_impl(const C *codes, uint64_t n, int center, DevMem &m, cuda
     // serialise in the driver).  In 8-byte words, each part 256-byte aligned; the
     // first parts are zeroed together: histogram, first positions, list length and
     // zero count (before the list); then the list, zero counts and offsets, chunk
-    // bits (in place their offsets), scan scratch, codebook tables (stateNum <=
+    // bits and their offsets, scan scratch, codebook tables (stateNum <=
     // nsym + 1 entries of 17 bytes).
     auto up = [](uint64_t w) { return (w + 31) & ~(uint64_t)31; };
     const uint64_t w_hist = up((uint64_t)nsym), w_list = 32 + up(3 * list_cap), w_z = up(nsub + 1),

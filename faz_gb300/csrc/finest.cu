@@ -20,12 +20,13 @@
 // neighbours, and the 16 targets of the line are independent of one another; its
 // 16 codes are one run of 32 bytes in the stream, put together in registers and
 // moved with 16-byte accesses.  Sweep 2 takes both planes' columns at once, a plane
-// to a half-warp, sweep 3 a plane's rows.  The kernel is issue-bound: with a
-// target to a lane (five shared loads, stencil coefficients selected per lane and a
-// 2-byte store each) it took 169 thread instructions a target, 0.60 ms for the 117
-// M targets of a 512^3 field; now 95 and 0.45 ms (decompression 0.48 ms, 0.77 ms in
-// the block kernel), with 16 warps an SM: registers (a line a lane) and shared
-// memory (two planes a warp) both end there.
+// to a half-warp, sweep 3 a plane's rows.  Bound by instructions: with a target to a
+// lane (five shared loads, stencil coefficients selected per lane and a 2-byte store
+// each) it took 169 thread instructions a target, 0.60 ms for the 117 M targets of a
+// 512^3 field; now 95 and 0.45 ms (decompression 0.48 ms, 0.77 ms in the block
+// kernel).  58% of the issue slots are used: 16 warps an SM (registers, a line a
+// lane, and shared memory, two planes a warp, both end there) wait for their own
+// arithmetic first, then for instruction fetch; DRAM is at 21%.
 //
 // Stream positions are the ones of interp.cu (closed form from level, block,
 // sweep, line and index; common.cuh): sweep-1 codes of a block interleave all

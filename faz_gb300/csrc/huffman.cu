@@ -373,8 +373,8 @@ __global__ void __launch_bounds__(ENC_THREADS) k_encode_bits(const C *__restrict
 }
 
 // Each thread packs ENC_PER_THREAD consecutive codes, four at a time while they
-// fit in 32 bits together: about 11 thread instructions a code (pushed one by one
-// and looked up twice 40).  The 134 M codes of a 512^3 field: 26 us per eighth,
+// fit in 32 bits together: about 30 thread instructions a code (pushed one by one
+// 40, and 80% of the issue slots used; now 52%).  The 134 M codes of a 512^3 field: 26 us per eighth,
 // behind the copy of the eighth before it (227 us in one piece before the copy).  Words in shared memory follow
 // the 32-bit word grid of the output.
 template <typename C>
@@ -491,8 +491,8 @@ __global__ void __launch_bounds__(ENC_THREADS) k_encode_pack(const C *__restrict
     }
 }
 // Where the chunks' bits begin: out[i] = out[0] + in[0] + .. + in[i - 1] for i <= n
-// (`first`: out[0] = 0), by one CTA (33,000 chunks 10 us, the three launches of
-// the general scan 13).  Also clears the words of the string in which a chunk
+// (`first`: out[0] = 0), by one CTA (a slice's 4096 chunks 8 us, a small string's
+// 4; the general scan's three launches 13 and 9).  Also clears the words of the string in which a chunk
 // begins or ends, which the packing ORs into (the words inside the chunks it
 // stores); not the one a slice before this has begun.
 __global__ void __launch_bounds__(1024) k_scan_chunks(const unsigned long long *__restrict__ in, uint64_t n,

@@ -1546,7 +1546,7 @@ struct HuffDecode {
         nranges = decode_ranges(d.nunits);
         // one allocation: bit string, unit records, CTA ends and totals, tables
         auto up = [](uint64_t b) { return (b + 255) & ~(uint64_t)255; };
-        const size_t lut2n = decode_lut2_entries(t.nodeCount);
+        const size_t lut2n = decode_lut2_entries(decode_slots(t));
         const uint64_t b_bits = up(4 * d.nwords + 64), b_info = up(4 * d.nunits), b_end = up(4 * ncta),
                        b_tot = up(8 * (ncta + 1)), b_child = up(4 * t.child.size()), b_lut = up(8ull << kLutBits),
                        b_lut2 = up(4 * lut2n), b_len2 = up(lut2n), b_rng = up(8 * nranges);

@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(1024) k_scan_chunks(const unsigned long long *
 // every CTA) took 385 + 236 + 337 us, these passes 36 us per
 // eighth of the string (hidden behind its copy but for the last) + 35 + 279 us.
 // DW is odd so that the units of a warp start in different banks.
-static constexpr int LUT_BITS = 12;
+static constexpr int LUT_BITS = kLutBits;
 static constexpr int LUT2_BITS = 8;                  // second table, below each prefix of a longer codeword
 static constexpr uint32_t B_LONG = 1u << 12;         // lutB.y: longer codewords
 static constexpr uint32_t DEC_NODE = 0x80000000u;    // second table: an inner node follows
@@ -1232,9 +1232,7 @@ cudaError_t launch_encode_pack(const EncodeArgs &a, const uint32_t *codes, uint6
 
 int decode_unit_words(uint64_t nbits) { return nbits < DEC_SHORT_BITS ? DEC_SHORT : DEC_LONG; }
 uint64_t decode_cta_units() { return DEC_T; }
-size_t decode_lut2_entries(int nodes) {
-    return std::min<size_t>((size_t)1 << LUT_BITS, (size_t)nodes / 2 + 1) << LUT2_BITS;
-}
+size_t decode_lut2_entries(size_t slots) { return slots << LUT2_BITS; }
 
 template <typename C>
 cudaError_t launch_decode_tables(const DecodeTablesDev &t, int offset, uint32_t *slot_node, unsigned *nslots,

@@ -325,8 +325,11 @@ int parse_tree(const uint8_t *&p, const uint8_t *end, DecodeTablesHost &t, std::
     t.constant_state = sym(0);
     if (root_leaf) return FAZ_OK;
     // children are numbered after their parent (preorder): reject anything
-    // else so that every walk ends
+    // else so that every walk ends.  Two parents of one node are taken as they
+    // always were (every walk still ends), but such a tree has more prefixes than
+    // its nodes bound: see decode_slots.
     t.child.assign(2 * (size_t)nc, 0);
+    std::vector<uint8_t> named(nc, 0);
     for (uint32_t i = 0; i < nc; i++) {
         if (i > 0 && qt[i]) continue;
         for (int k = 0; k < 2; k++) {
@@ -340,10 +343,20 @@ int parse_tree(const uint8_t *&p, const uint8_t *end, DecodeTablesHost &t, std::
                 t.child[2 * (size_t)i + k] = kChildLeaf | (s < 0 ? kChildBad : 0u) | ((uint32_t)s & 0xffffffu);
             } else {
                 t.child[2 * (size_t)i + k] = c;
+                t.shared |= named[c] != 0;
+                named[c] = 1;
             }
         }
     }
     return FAZ_OK;
+}
+
+// A prefix without a leaf ends at an inner node.  Where every inner node has one parent,
+// m such nodes of one depth are distinct and have at least m - 1 inner nodes above them;
+// where one has two, every prefix may end at the same node.
+size_t decode_slots(const DecodeTablesHost &t) {
+    const size_t all = (size_t)1 << kLutBits;
+    return t.shared ? all : std::min(all, (size_t)t.nodeCount / 2 + 1);
 }
 
 uint32_t leaf_depth(const DecodeTablesHost &t, int32_t state) {

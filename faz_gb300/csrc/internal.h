@@ -175,7 +175,7 @@ struct DecodeTablesDev {
     const uint32_t *child;     // 2 per node
     uint16_t *lutA;            // 2^kLutBits each
     uint2 *lutB;
-    uint32_t *lut2;            // decode_lut2_entries each
+    uint32_t *lut2;            // decode_lut2_entries(decode_slots) each
     uint8_t *len2;
 };
 struct DecodeString {
@@ -187,7 +187,7 @@ struct DecodeString {
 };
 int decode_unit_words(uint64_t nbits);  // words per unit of a string of nbits
 uint64_t decode_cta_units();            // units per CTA of the synchronising pass
-size_t decode_lut2_entries(int nodes);
+size_t decode_lut2_entries(size_t slots);
 template <typename C>
 cudaError_t launch_decode_tables(const DecodeTablesDev &t, int offset, uint32_t *slot_node, unsigned *nslots,
                                  size_t lut2_entries, cudaStream_t st);
@@ -238,6 +238,7 @@ struct DecodeTablesHost {
     int nodeCount = 0;
     bool constant = false;       // single-symbol stream
     int constant_state = 0;
+    bool shared = false;         // two parents name one inner node (a damaged stream)
     std::vector<uint32_t> child; // 2 per node: node index, or leaf flag | state (kChildLeaf, kChildBad)
 };
 constexpr uint32_t kChildLeaf = 0x80000000u;  // a leaf; its state in the low 24 bits
@@ -247,6 +248,9 @@ int parse_tree(const uint8_t *&p, const uint8_t *end, DecodeTablesHost &t, std::
 // length of the codeword of `state` (0: none, or longer than 64 bits)
 uint32_t leaf_depth(const DecodeTablesHost &t, int32_t state);
 constexpr int kLutBits = 12;
+// Bound on the kLutBits-bit prefixes that hold no whole codeword: each takes a
+// slot of the decoder's second tables.
+size_t decode_slots(const DecodeTablesHost &t);
 
 // -------------------------------------------------------------- stream/io
 void config_save(const faz_config &c, std::vector<uint8_t> &out);

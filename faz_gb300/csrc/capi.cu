@@ -170,7 +170,7 @@ Plan make_plan(int N, const uint64_t *dims, uint64_t maxStep, int blocksize, int
 // The levels of a plan from number `from` on (at most kMaxPlanLevels) for the
 // kernels that take several; `off`: the plan's block-offset table.
 LevelTable level_table(const Plan &p, size_t from, const uint64_t *off, uint64_t ncodes, int *err,
-                       unsigned long long *verify) {
+                       unsigned long long *verify, const int *hold = nullptr) {
     LevelTable t;
     t.n = (int)std::min<size_t>(p.lv.size() - from, kMaxPlanLevels);
     for (int i = 0; i < t.n; i++) {
@@ -180,6 +180,7 @@ LevelTable level_table(const Plan &p, size_t from, const uint64_t *off, uint64_t
         t.a[i].ncodes = ncodes;
         t.a[i].err = err;
         t.a[i].verify = verify;
+        t.a[i].hold = hold;
         t.first[i] = L.off_index;
         t.pos[i] = L.pos;
     }
@@ -212,10 +213,11 @@ void queue_block_offsets(const Plan &p, uint64_t *off, cudaStream_t st, Counter 
 template <typename T>
 void queue_levels(const Plan &p, bool decomp, double eb, int radius, int trim, const uint64_t *off, int *err,
                   unsigned long long *verify, const T *dX, T *W, uint16_t *codes, T *scratch, const uint64_t *zpos,
-                  uint64_t nz, const T *unpred, cudaEvent_t finest, cudaStream_t st, Counter &launches) {
+                  uint64_t nz, const T *unpred, cudaEvent_t finest, cudaStream_t st, Counter &launches,
+                  const int *hold = nullptr) {
     size_t li = 0;
     if (!p.lv.empty()) {
-        const LevelTable t = level_table(p, 0, off, p.num, err, verify);
+        const LevelTable t = level_table(p, 0, off, p.num, err, verify, hold);
         const int n = small_levels(t);
         if (n > 0) {
             if (n == (int)p.lv.size()) CK(cudaEventRecord(finest, st));
@@ -224,9 +226,9 @@ void queue_levels(const Plan &p, bool decomp, double eb, int radius, int trim, c
         }
     }
     if (li == 0 && !p.anchor)
-        launches(launch_first_point<T>(decomp, dX, W, codes, scratch, eb, radius, trim, zpos, nz, unpred, st));
+        launches(launch_first_point<T>(decomp, dX, W, codes, scratch, eb, radius, trim, zpos, nz, unpred, st, hold));
     for (; li < p.lv.size(); li++) {
-        const LevelTable t = level_table(p, li, off, p.num, err, verify);
+        const LevelTable t = level_table(p, li, off, p.num, err, verify, hold);
         if (li + 1 == p.lv.size()) CK(cudaEventRecord(finest, st));
         int nl = 0;
         CK(launch_level<T>(t.a[0], p.lv[li].nblocks, decomp, dX, W, codes, scratch, zpos, nz, unpred, st, &nl));
@@ -1503,10 +1505,6 @@ struct HuffDecode {
     uint64_t nranges = 0;              // ranges of the codes with
     unsigned long long *zc = nullptr;  // their zero counts and
     unsigned long long *zstart = nullptr;  // first codes
-    struct Status {
-        int changed, damaged;
-        uint64_t total;
-    };
 
     // zeros: the codes are expected to begin with that many zeros (anchors)
     void begin(const uint8_t *&p, const uint8_t *end, uint64_t n, C *out, DevMem &m, cudaStream_t st,
@@ -1618,14 +1616,13 @@ struct HuffDecode {
     }
 
     bool settle(DevMem &m, cudaStream_t st, Counter &launches) {
-        if (!status) return false;
-        Status s = *status;
+        DecodeStatus s = *status;
         // a CTA's end moved in the last pass: the next CTA restarts there
         bool redone = false;
         for (int it = 0; s.changed && !s.damaged && it < 1024; it++) {
             CK(cudaMemsetAsync(flags, 0, 4, st));
             link(st, launches);
-            CK(cudaMemcpyAsync(status, flags, 8, cudaMemcpyDeviceToHost, st));
+            outcome(nullptr, 0, nullptr, st, launches);
             CK(cudaStreamSynchronize(st));
             s = *status;
             redone = true;
@@ -1634,12 +1631,21 @@ struct HuffDecode {
         if (s.changed) throw Fail{FAZ_ERR_UNSUPPORTED, "Huffman stream did not synchronise within 1024 passes"};
         if (redone) {
             write(m, st, launches);
+            outcome(nullptr, 0, nullptr, st, launches);
             CK(cudaStreamSynchronize(st));
             s = *status;
         }
         if (s.total < num) throw Fail{FAZ_ERR_FORMAT, "Huffman stream holds fewer symbols than the field"};
         return redone;
     }
+
+    // What settle() reads, queued behind the decode (and the count of its zeros, if
+    // given); *hold = 0 when the codes are a field's with `expect` zeros.
+    void outcome(const unsigned long long *zeros, uint64_t expect, int *hold, cudaStream_t st, Counter &launches) {
+        status = (DecodeStatus *)t_pin_decode.get(sizeof(DecodeStatus));
+        launches(launch_decode_outcome(flags, coff ? coff + ncta : nullptr, num, zeros, expect, hold, status, st));
+    }
+    uint64_t zeros() const { return status->zeros; }
 
   private:
     DecodeTablesDev td{};
@@ -1649,21 +1655,18 @@ struct HuffDecode {
     uint32_t *info = nullptr, *cend[2] = {nullptr, nullptr};
     unsigned long long *ctot = nullptr, *coff = nullptr;
     int *flags = nullptr;  // changed, damaged, second-table slots
-    Status *status = nullptr;
+    DecodeStatus *status = nullptr;  // pinned
 
     void link(cudaStream_t st, Counter &launches) {
         launches(launch_decode_link(td, d, cend[0], cend[1], info, ctot, flags, st));
         std::swap(cend[0], cend[1]);
     }
-    // offsets of the CTAs' codes, the codes, and the outcome to the host
+    // offsets of the CTAs' codes, and the codes
     void write(DevMem &m, cudaStream_t st, Counter &launches) {
         if (!coff) coff = m.alloc<unsigned long long>(ncta + 1);
         CK(cudaMemcpyAsync(coff, ctot, ncta * 8, cudaMemcpyDeviceToDevice, st));
         launches(launch_scan_small(coff, ncta, st));
         launches(launch_decode_write(td, d, info, coff, num, offset, codes, zc, zstart, st));
-        if (!status) status = (Status *)t_pin_decode.get(sizeof(Status));
-        CK(cudaMemcpyAsync(status, flags, 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(&status->total, coff + ncta, 8, cudaMemcpyDeviceToHost, st));
     }
 };
 
@@ -1672,6 +1675,7 @@ void huffman_decode_impl(const uint8_t *&p, const uint8_t *end, uint64_t num, C 
                          Counter &launches) {
     HuffDecode<C> h;
     h.begin(p, end, num, codes, m, st, launches);
+    h.outcome(nullptr, 0, nullptr, st, launches);
     CK(cudaStreamSynchronize(st));
     h.settle(m, st, launches);
 }
@@ -1686,19 +1690,17 @@ void huffman_decode_device(const uint8_t *&p, const uint8_t *end, uint64_t num, 
 }
 
 // Sorted positions of the zero codes (the unpredictable points): queues the
-// compaction of the first `expect` of them into zpos and the copy of their
-// count to the returned pinned word, to be read once st is synchronised.
+// compaction of the first `expect` of them into zpos and the decode's outcome with
+// their count.
 template <typename C>
-const uint64_t *queue_zero_positions(const HuffDecode<C> &h, uint64_t expect, DevMem &m, cudaStream_t st,
-                                     Counter &launches, uint64_t *&zpos) {
+void queue_zero_positions(HuffDecode<C> &h, uint64_t expect, DevMem &m, cudaStream_t st, Counter &launches,
+                          uint64_t *&zpos, int *hold = nullptr) {
     unsigned long long *zoff = m.alloc<unsigned long long>(h.nranges + 1 + scan_temp_words(h.nranges) + 1);
     launches(launch_scan_u64(h.zc, zoff, h.nranges, zoff + h.nranges + 1, st));
-    uint64_t *hz = (uint64_t *)t_pin_small.get(64);
-    CK(cudaMemcpyAsync(hz, zoff + h.nranges, 8, cudaMemcpyDeviceToHost, st));
+    h.outcome(zoff + h.nranges, expect, hold, st, launches);
     zpos = m.alloc<uint64_t>(expect ? expect : 1);
     if (expect)
         launches(launch_zero_positions(h.codes, h.num, h.nranges, h.zstart, h.zc, zoff, expect, zpos, st));
-    return hz;
 }
 
 // Decode and compaction with one wait: the codes of an unpredictable-value
@@ -1709,7 +1711,7 @@ void decode_with_zeros_impl(const uint8_t *&p, const uint8_t *end, uint64_t num,
                             const std::function<void()> &meanwhile) {
     HuffDecode<C> h;
     h.begin(p, end, num, codes, m, st, launches);
-    const uint64_t *hz = queue_zero_positions(h, nunpred, m, st, launches, zpos);
+    queue_zero_positions(h, nunpred, m, st, launches, zpos);
     if (meanwhile) {
         try {
             meanwhile();
@@ -1720,10 +1722,10 @@ void decode_with_zeros_impl(const uint8_t *&p, const uint8_t *end, uint64_t num,
     }
     CK(cudaStreamSynchronize(st));
     if (h.settle(m, st, launches)) {
-        hz = queue_zero_positions(h, nunpred, m, st, launches, zpos);
+        queue_zero_positions(h, nunpred, m, st, launches, zpos);
         CK(cudaStreamSynchronize(st));
     }
-    if (*hz != nunpred) throw Fail{FAZ_ERR_FORMAT, "unpredictable count does not match the zero codes"};
+    if (h.zeros() != nunpred) throw Fail{FAZ_ERR_FORMAT, "unpredictable count does not match the zero codes"};
 }
 void decode_with_zeros(const uint8_t *&p, const uint8_t *end, uint64_t num, uint64_t nunpred, uint16_t *codes,
                        DevMem &m, cudaStream_t st, Counter &launches, uint64_t *&zpos,
@@ -1822,7 +1824,7 @@ void decompress_device(const uint8_t *pl, size_t n, Parsed &P, T *dOut, cudaStre
     CK(cudaEventRecord(ev_dec.a, st));
     uint64_t *boff = m.alloc<uint64_t>(pl_.nblocks + 1);
     queue_block_offsets(pl_, boff, st, launches);
-    int *kerr = m.alloc<int>(1);
+    int *kerr = m.alloc<int>(2), *hold = kerr + 1;
     CK(cudaMemsetAsync(kerr, 0, 4, st));
     unsigned long long *vcount = nullptr;
     if (verify_fast_path()) {
@@ -1832,25 +1834,25 @@ void decompress_device(const uint8_t *pl, size_t n, Parsed &P, T *dOut, cudaStre
     HuffDecode<uint16_t> h;
     h.begin(p, end, num, codes, m, st, launches, pl_.anchor ? pl_.nanchor : 0);
     CK(cudaEventRecord(ev_dec.b, st));
-    // Everything after the decode is queued before its outcome is known: a
-    // damaged stream leaves codes without meaning, which the kernels below take
-    // as any others (positions and unpredictable reads are bounded), and the
-    // call fails below.
+    // Everything after the decode is queued before the host knows its outcome.  The
+    // device does: where the codes are no field's (a damaged stream, or unit starts
+    // that settle() moves again) the kernels below return at once, and dOut stays as
+    // the caller left it.
     const uint64_t nz = P.nunpred;
-    const uint64_t *hz = nullptr;
     int *hk = (int *)t_pin_flag.get(64);
     auto reconstruct = [&] {
         uint64_t *zpos = nullptr;
-        hz = queue_zero_positions(h, nz, m, st, launches, zpos);
+        queue_zero_positions(h, nz, m, st, launches, zpos, hold);
         if (pl_.anchor) {
             int64_t step[3] = {1, 1, 1};
             int e = 3 - pl_.N;
             for (int i = 0; i < pl_.N; i++) step[e + i] = (int64_t)pl_.maxStep;
-            launches(launch_anchors<T>(true, nullptr, dOut, codes, nullptr, dunpred, pl_.na, step, pl_.offs3, st));
+            launches(
+                launch_anchors<T>(true, nullptr, dOut, codes, nullptr, dunpred, pl_.na, step, pl_.offs3, st, hold));
         }
         CK(cudaEventRecord(ev_pred.a, st));
         queue_levels<T>(pl_, true, P.eb, P.radius, P.trim, boff, kerr, vcount, nullptr, dOut, codes, nullptr, zpos, nz,
-                        dunpred, ev_fin.a, st, launches);
+                        dunpred, ev_fin.a, st, launches, hold);
         CK(cudaEventRecord(ev_fin.b, st));
         CK(cudaEventRecord(ev_pred.b, st));
         CK(cudaMemcpyAsync(hk, kerr, 4, cudaMemcpyDeviceToHost, st));
@@ -1861,7 +1863,7 @@ void decompress_device(const uint8_t *pl, size_t n, Parsed &P, T *dOut, cudaStre
         if (vcount) CK(cudaMemsetAsync(vcount, 0, 8, st));
         reconstruct();
     }
-    if (*hz != nz) throw Fail{FAZ_ERR_FORMAT, "unpredictable count does not match the zero codes"};
+    if (h.zeros() != nz) throw Fail{FAZ_ERR_FORMAT, "unpredictable count does not match the zero codes"};
     if (*hk) throw Fail{FAZ_ERR_DEVICE, "level kernel met an out-of-range stream position"};
     if (vcount) {
         unsigned long long vc = 0;

@@ -39,6 +39,7 @@ struct LevelArgs {
     const uint64_t *block_off;  // stream position of each block's first code
     uint64_t ncodes;     // codes in the whole stream (bounds every code read)
     int *err;            // set to 1 by a kernel that met an out-of-range position
+    const int *hold;     // decompression: where not 0, the codes are no field's and W is left as it is
     // float fast path: eb and 1/eb split into float pairs, largest float <= eb
     float eh, el, rh, rl, eblo, twor_f;
     float eb_half0;      // |diff| below this float gives half index 0 for sure

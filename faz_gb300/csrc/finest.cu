@@ -392,7 +392,9 @@ __global__ void __launch_bounds__(FW * 32, 2)
         }
         cp_async_wait_all();
     }
+    int hold = 0;  // read here, with the loads above on their way
     if (DECOMP) {
+        if (a.hold) hold = *a.hold;
         // the block's sweep-1 codes (they interleave all planes)
         const int cnt = (int)g.c1;
         const int a0 = (8 - sh1) & 7;
@@ -406,6 +408,7 @@ __global__ void __launch_bounds__(FW * 32, 2)
         }
     }
     __syncthreads();
+    if (DECOMP && hold) return;
 
     const int t = lane & 15, half = lane >> 4;
     const int np = n0 - k0;   // planes with emitted codes

@@ -1316,6 +1316,24 @@ cudaError_t launch_scan_small(unsigned long long *v, uint64_t n, cudaStream_t st
     return cudaGetLastError();
 }
 
+// one launch in the place of four copies of a word each
+__global__ void k_decode_outcome(const int *flags, const unsigned long long *total, uint64_t need,
+                                 const unsigned long long *zeros, uint64_t expect, int *hold, DecodeStatus *host) {
+    DecodeStatus s;
+    s.changed = flags ? flags[0] : 0;
+    s.damaged = flags ? flags[1] : 0;
+    s.total = total ? *total : need;
+    s.zeros = zeros ? *zeros : 0;
+    if (hold) *hold = s.changed || s.damaged || s.total < need || s.zeros != expect;
+    *host = s;
+}
+cudaError_t launch_decode_outcome(const int *flags, const unsigned long long *total, uint64_t need,
+                                  const unsigned long long *zeros, uint64_t expect, int *hold, DecodeStatus *host,
+                                  cudaStream_t st) {
+    k_decode_outcome<<<1, 1, 0, st>>>(flags, total, need, zeros, expect, hold, host);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_fill_u16(uint16_t *out, uint64_t n, uint16_t v, cudaStream_t st) {
     unsigned g = grid_for(n, 1024);
     if (g > 4096) g = 4096;

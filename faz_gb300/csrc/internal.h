@@ -95,10 +95,12 @@ cudaError_t launch_finest(const LevelArgs &a, int64_t nblocks, bool decomp, cons
                           cudaStream_t st);
 template <typename T>
 cudaError_t launch_first_point(bool decomp, const T *X, T *W, uint16_t *codes, T *scratch, double eb, int radius,
-                               int trim, const uint64_t *zpos, uint64_t nz, const T *unpred, cudaStream_t st);
+                               int trim, const uint64_t *zpos, uint64_t nz, const T *unpred, cudaStream_t st,
+                               const int *hold = nullptr);
 template <typename T>
 cudaError_t launch_anchors(bool decomp, const T *X, T *W, uint16_t *codes, T *scratch, const T *unpred,
-                           const int64_t *na, const int64_t *step, const int64_t *offs, cudaStream_t st);
+                           const int64_t *na, const int64_t *step, const int64_t *offs, cudaStream_t st,
+                           const int *hold = nullptr);
 
 // Batched compression: every field's first point / anchors and levels in one
 // persistent launch from a device work queue (interp.cu).
@@ -215,6 +217,17 @@ cudaError_t launch_zero_positions(const C *codes, uint64_t n, uint64_t nranges, 
                                   const unsigned long long *zcount, const unsigned long long *zoff, uint64_t cap,
                                   uint64_t *zpos, cudaStream_t st);
 cudaError_t launch_scan_small(unsigned long long *v, uint64_t n, cudaStream_t st);
+// The outcome of a queued decode (flags and total null: a constant string; zeros null:
+// not counted) into pinned memory, to be read once the stream is synchronised.
+// *hold, when given: 0 where the codes are a field's, flags clear, at least `need` of
+// them and `expect` zeros.
+struct DecodeStatus {
+    int changed, damaged;
+    unsigned long long total, zeros;
+};
+cudaError_t launch_decode_outcome(const int *flags, const unsigned long long *total, uint64_t need,
+                                  const unsigned long long *zeros, uint64_t expect, int *hold, DecodeStatus *host,
+                                  cudaStream_t st);
 cudaError_t launch_fill_u16(uint16_t *out, uint64_t n, uint16_t v, cudaStream_t st);
 cudaError_t launch_fill_u16(uint32_t *out, uint64_t n, uint32_t v, cudaStream_t st);
 

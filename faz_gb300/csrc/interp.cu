@@ -303,6 +303,7 @@ __global__ void __launch_bounds__(512, 2) k_interp_level(LevelArgs a, const T *_
                                                       const uint64_t *__restrict__ zpos, uint64_t nz,
                                                       const T *__restrict__ unpred) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    if (DECOMP && a.hold && *a.hold) return;
     level_block<T, DECOMP, WIDE, QM, false, CUB>(a, blockIdx.x, X, W, codes, scratch, zpos, nz, unpred, smem_raw);
 }
 
@@ -371,14 +372,17 @@ __global__ void __launch_bounds__(256) k_level_sweep(LevelArgs a, int sw, uint32
                                                     uint64_t nz, const T *__restrict__ unpred) {
     __shared__ BlockGeom sgeo;
     __shared__ uint64_t sbase;
+    __shared__ int shold;
     const uint32_t bid = blockIdx.x / chunks, chunk = blockIdx.x - bid * chunks;
     if (threadIdx.x == 0) {
         int64_t bc[3];
         block_coords(a, bid, bc);
         block_geom(a, bc, sgeo);
         sbase = a.block_off[bid];
+        shold = DECOMP && a.hold ? *a.hold : 0;
     }
     __syncthreads();
+    if (DECOMP && shold) return;
     const BlockGeom &g = sgeo;
     const uint32_t cnt = (uint32_t)(sw == 1 ? g.c1 : (sw == 2 ? g.c2 : g.c3));
     for (uint32_t x = chunk * 256u + threadIdx.x; x < cnt; x += chunks * 256u)
@@ -396,6 +400,7 @@ __global__ void __launch_bounds__(kSmallThreads)
     k_small_levels(const __grid_constant__ LevelTable t, int n, bool first_point, double eb, const T *__restrict__ X,
                    T *W, uint16_t *__restrict__ codes, T *__restrict__ scratch, const uint64_t *__restrict__ zpos,
                    uint64_t nz, const T *__restrict__ unpred) {
+    if (DECOMP && t.a[0].hold && *t.a[0].hold) return;
     if (first_point && threadIdx.x == 0) {
         const LevelArgs &a = t.a[0];
         if (!DECOMP) {
@@ -593,7 +598,8 @@ __global__ void k_first_point(const T *X, T *W, uint16_t *codes, T *scratch, dou
 
 template <typename T>
 __global__ void k_first_point_dec(const uint16_t *codes, T *W, double eb, int radius, int trim,
-                                  const uint64_t *zpos, uint64_t nz, const T *unpred) {
+                                  const uint64_t *zpos, uint64_t nz, const T *unpred, const int *hold) {
+    if (hold && *hold) return;
     if (threadIdx.x == 0 && blockIdx.x == 0) W[0] = recover((T)0, (int)codes[0], 0, eb, radius, trim, zpos, nz, unpred);
 }
 
@@ -601,7 +607,8 @@ __global__ void k_first_point_dec(const uint16_t *codes, T *W, double eb, int ra
 template <typename T, bool DECOMP>
 __global__ void k_anchors(const T *X, T *W, uint16_t *codes, T *scratch, const T *unpred, int64_t na0, int64_t na1,
                           int64_t na2, int64_t step0, int64_t step1, int64_t step2, int64_t o0, int64_t o1,
-                          int64_t o2) {
+                          int64_t o2, const int *hold) {
+    if (DECOMP && hold && *hold) return;
     int64_t total = na0 * na1 * na2;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         int64_t z = i % na2, r = i / na2;
@@ -841,25 +848,27 @@ cudaError_t launch_level(const LevelArgs &a, int64_t nblocks, bool decomp, const
 
 template <typename T>
 cudaError_t launch_first_point(bool decomp, const T *X, T *W, uint16_t *codes, T *scratch, double eb, int radius,
-                               int trim, const uint64_t *zpos, uint64_t nz, const T *unpred, cudaStream_t st) {
+                               int trim, const uint64_t *zpos, uint64_t nz, const T *unpred, cudaStream_t st,
+                               const int *hold) {
     if (!decomp) k_first_point<T><<<1, 32, 0, st>>>(X, W, codes, scratch, eb, 1.0 / eb, radius, trim);
-    else k_first_point_dec<T><<<1, 32, 0, st>>>(codes, W, eb, radius, trim, zpos, nz, unpred);
+    else k_first_point_dec<T><<<1, 32, 0, st>>>(codes, W, eb, radius, trim, zpos, nz, unpred, hold);
     return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_anchors(bool decomp, const T *X, T *W, uint16_t *codes, T *scratch, const T *unpred,
-                           const int64_t *na, const int64_t *step, const int64_t *offs, cudaStream_t st) {
+                           const int64_t *na, const int64_t *step, const int64_t *offs, cudaStream_t st,
+                           const int *hold) {
     int64_t total = na[0] * na[1] * na[2];
     int blocks = (int)((total + 255) / 256);
     if (blocks > 4096) blocks = 4096;
     if (blocks < 1) blocks = 1;
     if (!decomp)
         k_anchors<T, false><<<blocks, 256, 0, st>>>(X, W, codes, scratch, unpred, na[0], na[1], na[2], step[0], step[1],
-                                                     step[2], offs[0], offs[1], offs[2]);
+                                                     step[2], offs[0], offs[1], offs[2], hold);
     else
         k_anchors<T, true><<<blocks, 256, 0, st>>>(X, W, codes, scratch, unpred, na[0], na[1], na[2], step[0], step[1],
-                                                    step[2], offs[0], offs[1], offs[2]);
+                                                    step[2], offs[0], offs[1], offs[2], hold);
     return cudaGetLastError();
 }
 
@@ -872,9 +881,9 @@ cudaError_t launch_anchors(bool decomp, const T *X, T *W, uint16_t *codes, T *sc
                                                 uint16_t *, T *, const uint64_t *, uint64_t, const T *,          \
                                                 cudaStream_t);                                                    \
     template cudaError_t launch_first_point<T>(bool, const T *, T *, uint16_t *, T *, double, int, int,          \
-                                               const uint64_t *, uint64_t, const T *, cudaStream_t);             \
+                                               const uint64_t *, uint64_t, const T *, cudaStream_t, const int *); \
     template cudaError_t launch_anchors<T>(bool, const T *, T *, uint16_t *, T *, const T *, const int64_t *,   \
-                                           const int64_t *, const int64_t *, cudaStream_t);                      \
+                                           const int64_t *, const int64_t *, cudaStream_t, const int *);         \
     template cudaError_t launch_interp_batch<T>(const BatchGroup *, int, const BatchField *, const LevelArgs *,   \
                                                 uint64_t, unsigned long long *, unsigned *, int *, bool, int, int,\
                                                 size_t, cudaStream_t);                                           \

@@ -1,5 +1,6 @@
 """Payloads that no compressor writes.  A tree in which nodes have two parents
-decodes as a walk over it says."""
+decodes as a walk over it says.  Damage that the Huffman stage finds is refused, and
+the caller's output stays as it was."""
 import struct
 
 import numpy as np
@@ -66,3 +67,55 @@ def test_nodes_with_two_parents(depth):
     got = _decode(payload, torch.full((N,), 7.0, device="cuda"))
     assert np.abs(got - x).max() <= 1.0
     assert np.array_equal(got, np.where(x > 0, 2.0, 0.0).astype(np.float32))
+
+
+# one CTA's levels alone, sweep launches with an anchor grid, the block kernel
+# (float64), the plane kernel
+FIELDS = [((20001,), {}, np.float32), ((90, 80, 70), dict(maxStep=16, alpha=1.5, beta=2.0), np.float32),
+          ((231, 230, 229), {}, np.float64), ((231, 262, 264), {}, np.float32)]
+
+
+@pytest.mark.parametrize("damage", ["string cut", "one value less", "one value more", "negative state"])
+@pytest.mark.parametrize("dims,kw,dtype", FIELDS)
+def test_damage_leaves_the_output(dims, kw, dtype, damage):
+    rng = np.random.default_rng(sum(dims))
+    x = rng.normal(0, 3, dims).astype(dtype)
+    x.reshape(-1)[rng.integers(0, x.size, 50)] = 1e9  # unpredictable values
+    conf = F.Config(*dims)
+    conf.cmprAlgo, conf.errorBoundMode, conf.absErrorBound = F.ALGO_INTERP, F.EB_ABS, 0.5
+    for k, v in kw.items():
+        setattr(conf, k, v)
+    good = bytes(F.compress_payload_device(conf, torch.from_numpy(x).cuda())[0])
+    head = 8 * len(dims) + 4 * 3 + 8 * 3 + 4 + 1 + 4 + 8 + 4 + 4 + 1 + 8 + 4
+    nunpred, = struct.unpack_from("<Q", good, head)
+    assert nunpred > 0
+    tree = head + 8 + nunpred * x.itemsize
+    nodes, = struct.unpack_from(">I", good, tree + 4)
+    assert 3 < nodes <= 256  # one-byte indices
+    at = tree + 13 + 2 * nodes + 4 * nodes + nodes
+    nbytes, = struct.unpack_from("<Q", good, at)
+    assert at + 8 + nbytes == len(good)
+    if damage == "string cut":
+        bad = good[:at] + struct.pack("<Q", nbytes // 2) + good[at + 8:at + 8 + nbytes // 2]
+    elif damage == "one value less":
+        bad = good[:head] + struct.pack("<Q", nunpred - 1) + good[head + 8:tree - x.itemsize] + good[tree:]
+    elif damage == "one value more":
+        bad = good[:head] + struct.pack("<Q", nunpred + 1) + good[head + 8:tree] + good[tree - x.itemsize:]
+    else:  # of a rare symbol, one with a long codeword
+        types = good[tree + 13 + 6 * nodes:at]
+        left, right = good[tree + 13:tree + 13 + nodes], good[tree + 13 + nodes:tree + 13 + 2 * nodes]
+        depth = [0] * nodes
+        for i in range(nodes):
+            if not types[i]:
+                depth[left[i]] = depth[right[i]] = depth[i] + 1
+        leaf = max((d, i) for i, d in enumerate(depth) if types[i])[1]
+        assert depth[leaf] > 12
+        state = tree + 13 + 2 * nodes + 4 * leaf
+        bad = good[:state] + struct.pack("<i", -1) + good[state + 4:]
+    out = torch.full(dims, 7.0, dtype=torch.from_numpy(x).dtype, device="cuda")
+    with pytest.raises(F.FazError) as e:
+        F.decompress_payload_device(len(dims), bad, out)
+    assert e.value.code == -4
+    assert bool((out == 7.0).all())
+    F.decompress_payload_device(len(dims), good, out)
+    assert np.abs(out.cpu().numpy() - x).max() <= 0.5

@@ -1712,14 +1712,7 @@ void decode_with_zeros_impl(const uint8_t *&p, const uint8_t *end, uint64_t num,
     HuffDecode<C> h;
     h.begin(p, end, num, codes, m, st, launches);
     queue_zero_positions(h, nunpred, m, st, launches, zpos);
-    if (meanwhile) {
-        try {
-            meanwhile();
-        } catch (...) {
-            cudaStreamSynchronize(st);  // the copies from the caller's stream end first
-            throw;
-        }
-    }
+    if (meanwhile) meanwhile();
     CK(cudaStreamSynchronize(st));
     if (h.settle(m, st, launches)) {
         queue_zero_positions(h, nunpred, m, st, launches, zpos);
@@ -1743,6 +1736,7 @@ namespace {
 template <typename T>
 void decompress_device(const uint8_t *pl, size_t n, Parsed &P, T *dOut, cudaStream_t st, faz_timings &tm,
                        Counter &launches) {
+    WaitOnThrow wait(st);
     const uint8_t *end = pl + n;
     const uint8_t *p = P.unpred;
     if ((size_t)(end - p) / sizeof(T) < P.nunpred) throw Fail{FAZ_ERR_FORMAT, "truncated unpredictable values"};

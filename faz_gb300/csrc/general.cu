@@ -846,6 +846,7 @@ void gen_compress_payload(int N, const uint64_t *dims, int bs, int lo, int lo2, 
 template <typename T>
 void gen_decompress(int N, const uint8_t *pl, size_t psize, const uint64_t *dims, int lo, int lo2, int reg, T *dOut,
                     cudaStream_t st, Counter &launches, faz_timings &tm) {
+    WaitOnThrow wait(st);
     const uint8_t *p = pl, *end = pl + psize;
     auto need = [&](size_t k) {
         if ((size_t)(end - p) < k) throw Fail{FAZ_ERR_FORMAT, "truncated Lorenzo stream"};

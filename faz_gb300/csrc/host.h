@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <functional>
 #include <memory>
 #include <mutex>
@@ -181,6 +182,19 @@ struct ViewScope {
     PayloadView *before;
     explicit ViewScope(PayloadView *v) : before(t_payload_view) { t_payload_view = v; }
     ~ViewScope() { t_payload_view = before; }
+};
+
+// Waits for the stream when its scope is left by an exception: copies from the
+// caller's payload or into the caller's or the thread's pinned buffers end before the
+// call returns its error and those buffers are free to be used again.
+struct WaitOnThrow {
+    cudaStream_t st;
+    int before = std::uncaught_exceptions();
+    explicit WaitOnThrow(cudaStream_t s) : st(s) {}
+    ~WaitOnThrow() {
+        if (std::uncaught_exceptions() > before) cudaStreamSynchronize(st);
+    }
+    WaitOnThrow(const WaitOnThrow &) = delete;
 };
 
 // How a call on device buffers reads a NULL stream: the legacy default

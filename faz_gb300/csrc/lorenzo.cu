@@ -1102,6 +1102,7 @@ void lorenzo3_compress_payload(const uint64_t *dims, int bs, int pd, int lo, int
 template <typename T>
 void lorenzo3_decompress(const uint8_t *pl, size_t psize, const uint64_t *dims, T *dOut, cudaStream_t st,
                          Counter &launches, faz_timings &tm) {
+    WaitOnThrow wait(st);
     const uint8_t *p = pl, *end = pl + psize;
     auto need = [&](size_t k) {
         if ((size_t)(end - p) < k) throw Fail{FAZ_ERR_FORMAT, "truncated Lorenzo stream"};

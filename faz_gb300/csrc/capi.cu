@@ -575,6 +575,7 @@ void interp_emit(const faz_config &c, const std::vector<uint8_t> &il, const std:
     if (!e.he.done.empty()) {
         // each slice's whole words as soon as its launch is done
         StreamGuard cs(nullptr);
+        WaitOnThrow wait(cs.st);
         uint64_t from = 0;
         const size_t ns = e.he.done.size();
         for (size_t k = 0; k < ns; k++) {
@@ -603,6 +604,7 @@ void interp_payload_tail(const faz_config &c, const std::vector<uint8_t> &il, co
                          double eb, int radius, uint64_t n, uint16_t *codes, T *scratch, unsigned long long *vcount,
                          DevMem &m, cudaStream_t st, Counter &launches, faz_timings &tm, Sink *sink,
                          uint8_t *&payload, size_t &psize, cudaEvent_t huff_end = nullptr, const int *lerr = nullptr) {
+    WaitOnThrow wait(st);  // a batch runs this on a stream of each field
     InterpEncoded<T> e;
     interp_encode<T>(n, radius, codes, scratch, vcount, lerr, m, st, launches, tm, e);
     if (huff_end) CK(cudaEventRecord(huff_end, st));
@@ -798,6 +800,7 @@ void blocked_payload(faz_config &c, const T *dX, cudaStream_t st, uint8_t *&payl
 template <typename T>
 void compress_dispatch(faz_config &c, const T *dX, cudaStream_t st, uint8_t *&payload, size_t &psize,
                        faz_timings &tm, Counter &launches, Sink *sink = nullptr) {
+    WaitOnThrow wait(st);
     if (c.cmprAlgo == FAZ_ALGO_INTERP) {  // resolves the error bound itself, beside the range's kernel
         compress_payload<T>(c, dX, st, payload, psize, tm, launches, sink);
         return;

@@ -33,10 +33,11 @@
 // planes, so they are staged in shared memory and moved once per block; sweep-2
 // and sweep-3 codes of a plane are contiguous.
 //
-// Requirements (finest_eligible): float data on the exact float quantiser
+// Requirements (finest_possible): float data on the exact float quantiser
 // path, P2 the contiguous axis, a 3-D field below 2^31 values, rows of 16-byte
 // multiples in 16-byte aligned buffers (the tensor map's strides and x coordinates,
-// decompression's 16-byte stores) and blocks of edge 32, so that most lines have 32
+// decompression's 16-byte stores) and blocks of an edge up to 32 that is a multiple
+// of 4.  It is used (finest_faster) for edge 32, where most lines have 32
 // or 33 points.  Decompression moreover wants three quarters of the blocks to have
 // both in-plane extents full: its single targets wait for their codes.  Measured
 // against the block kernel of interp.cu, the line between them (finest level, ms,
@@ -686,14 +687,21 @@ EncodeTiledFn encode_tiled() {
 
 }  // namespace
 
-bool finest_eligible(const LevelArgs &a, bool decomp, const void *X, const void *W, size_t elem) {
-    if (elem != 4 || a.s != 1 || a.bs != 32 || a.write_back || !a.fast || a.trim != 0) return false;
+bool finest_possible(const LevelArgs &a, bool decomp, const void *X, const void *W) {
+    // block begins along the contiguous axis are TMA x coordinates: the edge is a
+    // multiple of 4 values
+    if (a.s != 1 || a.bs > 32 || (a.bs & 3) || a.write_back || !a.fast || a.trim != 0) return false;
     if (a.perm[2] != 2 || a.perm[0] > 1 || a.perm[1] > 1) return false;
     if (a.dims[0] < FROWS || a.dims[1] < FROWS || a.dims[2] < FX || (a.dims[2] & 3)) return false;
     if (a.dims[0] * a.dims[1] * a.dims[2] >= ((int64_t)1 << 31)) return false;
-    if (!decomp) return ((uintptr_t)X & 15) == 0 && encode_tiled() != nullptr;
+    if (decomp) return ((uintptr_t)W & 15) == 0;
+    return ((uintptr_t)X & 15) == 0 && encode_tiled() != nullptr;
+}
+
+bool finest_faster(const LevelArgs &a, bool decomp) {
+    if (a.bs != 32) return false;
     const int64_t d1 = a.dims[a.perm[1]], d2 = a.dims[2];
-    return ((uintptr_t)W & 15) == 0 && 4 * (d1 / 32) * (d2 / 32) >= 3 * ((d1 + 31) / 32) * ((d2 + 31) / 32);
+    return !decomp || 4 * (d1 / 32) * (d2 / 32) >= 3 * ((d1 + 31) / 32) * ((d2 + 31) / 32);
 }
 
 cudaError_t launch_finest(const LevelArgs &a, int64_t nblocks, bool decomp, const float *X, float *W,

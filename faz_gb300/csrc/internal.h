@@ -88,8 +88,10 @@ cudaError_t launch_level(const LevelArgs &a, int64_t nblocks, bool decomp, const
                          T *scratch, const uint64_t *zpos, uint64_t nz, const T *unpred, cudaStream_t st,
                          int *nlaunch);
 // The finest level of a 3-D float field, plane by plane with TMA-staged
-// planes (finest.cu): whether a level qualifies, and its launch.
-bool finest_eligible(const LevelArgs &a, bool decomp, const void *X, const void *W, size_t elem);
+// planes (finest.cu): whether it can take a level, whether it is faster there than
+// the block kernel, and its launch.
+bool finest_possible(const LevelArgs &a, bool decomp, const void *X, const void *W);
+bool finest_faster(const LevelArgs &a, bool decomp);
 cudaError_t launch_finest(const LevelArgs &a, int64_t nblocks, bool decomp, const float *X, float *W,
                           uint16_t *codes, float *scratch, const uint64_t *zpos, uint64_t nz, const float *unpred,
                           cudaStream_t st);

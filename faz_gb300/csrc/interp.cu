@@ -806,18 +806,20 @@ cudaError_t launch_level(const LevelArgs &a, int64_t nblocks, bool decomp, const
         cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
         return v > 0 ? v : 1;
     }();
+    // FAZ_FINEST_PLANES (read per call, for comparisons): the finest level of any field
+    // in the block kernel (0), or in the plane kernel wherever that can run (2).
+    const char *plane_env = std::getenv("FAZ_FINEST_PLANES");
+    const bool only_blocks = plane_env && plane_env[0] == '0', only_planes = plane_env && plane_env[0] == '2';
+    const bool forced = a.s == 1 && (only_blocks || only_planes);
     const bool flat = a.dims[0] == 1 && a.dims[1] > 1;
     const int64_t per_block = (a.bs / a.s + 1) * (a.bs / a.s + 1) * (a.bs / a.s + 1) / 256 + 1;
-    if (!wide && (flat || nblocks < 2 * sms) && nblocks * per_block < (1ll << 31))
+    if (!forced && !wide && (flat || nblocks < 2 * sms) && nblocks * per_block < (1ll << 31))
         return launch_level_sweeps<T>(a, nblocks, decomp, X, W, codes, scratch, zpos, nz, unpred, st, nlaunch);
     // the finest level of a 3-D float field: plane-parallel kernel (finest.cu, with
     // both kernels' times; on 512^3 0.45 ms against 0.83 ms for the block kernel
-    // below, decompression 0.48 against 0.77 ms).  FAZ_FINEST_PLANES=0 (read per
-    // call, for comparisons): the block kernel.
-    const char *plane_env = std::getenv("FAZ_FINEST_PLANES");
-    const bool planes = !(plane_env && plane_env[0] == '0');
+    // below, decompression 0.48 against 0.77 ms)
     if constexpr (sizeof(T) == 4) {
-        if (planes && finest_eligible(a, decomp, X, W, sizeof(T))) {
+        if (!only_blocks && finest_possible(a, decomp, X, W) && (only_planes || finest_faster(a, decomp))) {
             ++*nlaunch;
             return launch_finest(a, nblocks, decomp, reinterpret_cast<const float *>(X), reinterpret_cast<float *>(W),
                                  codes, reinterpret_cast<float *>(scratch), zpos, nz,

@@ -49,7 +49,9 @@ __device__ __forceinline__ void move_codes(uint16_t *g, uint16_t *stg, int64_t c
 
 // --------------------------------------------------------- level kernel
 // One CTA per block.  Each half-warp takes one line at a time; lane t of the
-// half-warp owns target 2t+1 of the line.  Shared-memory strides along every
+// half-warp owns target 2t+1 of the line (blocks of more than 33 points an axis have
+// more than 16 targets a line, taken 16 at a time, the lines once for each sixteen:
+// no target of a sweep depends on another of it).  Shared-memory strides along every
 // sweep axis are odd multiples of the lane step, so the half-warps read
 // distinct banks.  Lanes past the line's targets run the same code on a valid
 // target and store nothing.
@@ -125,47 +127,50 @@ __device__ __forceinline__ void level_block(const LevelArgs &a, const int64_t bi
         }
         const int st = n1 * h2;
         const int lines = ((n1 + 1) / 2) * h2;
-        const bool act = t < g.t0;
-        const int m0 = act ? 2 * t + 1 : 1;
-        const Stencil<T> S = make_stencil<T>(m0, n0, cubic, st, 0);
-        const int rk = line_rank(m0, n0, cubic);
-        const Off gl = (Off)m0 * G0;
-        LineCursor lc;
-        lc.init(hw, nhw, h2);  // outer = e1, inner = e2
-        for (int l = hw; l < lines; l += nhw, lc.next()) {
-            const int e1 = lc.outer, e2 = lc.inner;
-            const int col = 2 * e1 * h2 + e2;
-            const bool emit = act && e1 >= k1 && e2 >= k2;
-            const int rank = ((e1 - k1) * g.ne2 + (e2 - k2)) * g.t0 + rk;
-            const T pred = eval_stencil<CUB>(S, V + col);
-            const int idx = m0 * st + col;
-            const Off gi = gl + (Off)(2 * e1) * G1 + (Off)(2 * e2) * G2;
-            if (!DECOMP) {
-                T v = V[idx], uv;
-                const int code = quant_point<T, QM>(v, pred, a, uv);
-                if (act) V[idx] = v;
-                if (emit) {
-                    sg[rank] = (uint16_t)code;
-                    if (code == 0) scratch[base + rank] = uv;
-                    if (wb) W[gi] = v;
-                }
-            } else if (act) {
-                uint64_t pos;
-                int code;
-                if (emit) {
-                    pos = base + rank;
-                    code = sg[rank];
-                } else {
-                    pos = owner_pos_sweep1(a, g, bc, P1, P2, e1, e2, n2) + rk;
-                    if (pos >= a.ncodes) {
-                        atomicExch(a.err, 1);
-                        pos = 0;
+        for (int tb = 0; tb < g.t0; tb += 16) {
+            const int tt = tb + t;
+            const bool act = tt < g.t0;
+            const int m0 = act ? 2 * tt + 1 : 1;
+            const Stencil<T> S = make_stencil<T>(m0, n0, cubic, st, 0);
+            const int rk = line_rank(m0, n0, cubic);
+            const Off gl = (Off)m0 * G0;
+            LineCursor lc;
+            lc.init(hw, nhw, h2);  // outer = e1, inner = e2
+            for (int l = hw; l < lines; l += nhw, lc.next()) {
+                const int e1 = lc.outer, e2 = lc.inner;
+                const int col = 2 * e1 * h2 + e2;
+                const bool emit = act && e1 >= k1 && e2 >= k2;
+                const int rank = ((e1 - k1) * g.ne2 + (e2 - k2)) * g.t0 + rk;
+                const T pred = eval_stencil<CUB>(S, V + col);
+                const int idx = m0 * st + col;
+                const Off gi = gl + (Off)(2 * e1) * G1 + (Off)(2 * e2) * G2;
+                if (!DECOMP) {
+                    T v = V[idx], uv;
+                    const int code = quant_point<T, QM>(v, pred, a, uv);
+                    if (act) V[idx] = v;
+                    if (emit) {
+                        sg[rank] = (uint16_t)code;
+                        if (code == 0) scratch[base + rank] = uv;
+                        if (wb) W[gi] = v;
                     }
-                    code = codes[pos];
+                } else if (act) {
+                    uint64_t pos;
+                    int code;
+                    if (emit) {
+                        pos = base + rank;
+                        code = sg[rank];
+                    } else {
+                        pos = owner_pos_sweep1(a, g, bc, P1, P2, e1, e2, n2) + rk;
+                        if (pos >= a.ncodes) {
+                            atomicExch(a.err, 1);
+                            pos = 0;
+                        }
+                        code = codes[pos];
+                    }
+                    const T v = recover_point<T, QM>(pred, code, pos, a, zpos, nz, unpred);
+                    V[idx] = v;
+                    if (emit) W[gi] = v;
                 }
-                const T v = recover_point<T, QM>(pred, code, pos, a, zpos, nz, unpred);
-                V[idx] = v;
-                if (emit) W[gi] = v;
             }
         }
         __syncthreads();
@@ -187,48 +192,51 @@ __device__ __forceinline__ void level_block(const LevelArgs &a, const int64_t bi
             __syncthreads();
         }
         const int lines = (n0 - k0) * h2;
-        const bool act = t < g.t1;
-        const int m1 = act ? 2 * t + 1 : 1;
-        const Stencil<T> S = make_stencil<T>(m1, n1, cubic, h2, 0);
-        const int rk = line_rank(m1, n1, cubic);
-        const Off gl = (Off)m1 * G1;
-        LineCursor lc;
-        lc.init(hw, nhw, h2);  // outer = m0 - k0, inner = e2
-        for (int l = hw; l < lines; l += nhw, lc.next()) {
-            const int q = lc.outer, e2 = lc.inner;
-            const int m0 = k0 + q;
-            const int col = m0 * n1 * h2 + e2;
-            const bool emit = act && e2 >= k2;
-            const int rank = (q * g.ne2 + (e2 - k2)) * g.t1 + rk;
-            const T pred = eval_stencil<CUB>(S, V + col);
-            const int idx = col + m1 * h2;
-            const Off gi = (Off)m0 * G0 + gl + (Off)(2 * e2) * G2;
-            if (!DECOMP) {
-                T v = V[idx], uv;
-                const int code = quant_point<T, QM>(v, pred, a, uv);
-                if (act) V[idx] = v;
-                if (emit) {
-                    sg[rank] = (uint16_t)code;
-                    if (code == 0) scratch[sbase + rank] = uv;
-                    if (wb) W[gi] = v;
-                }
-            } else if (act) {
-                uint64_t pos;
-                int code;
-                if (emit) {
-                    pos = sbase + rank;
-                    code = sg[rank];
-                } else {
-                    pos = owner_pos_sweep2(a, g, bc, P2, q) + rk;
-                    if (pos >= a.ncodes) {
-                        atomicExch(a.err, 1);
-                        pos = 0;
+        for (int tb = 0; tb < g.t1; tb += 16) {
+            const int tt = tb + t;
+            const bool act = tt < g.t1;
+            const int m1 = act ? 2 * tt + 1 : 1;
+            const Stencil<T> S = make_stencil<T>(m1, n1, cubic, h2, 0);
+            const int rk = line_rank(m1, n1, cubic);
+            const Off gl = (Off)m1 * G1;
+            LineCursor lc;
+            lc.init(hw, nhw, h2);  // outer = m0 - k0, inner = e2
+            for (int l = hw; l < lines; l += nhw, lc.next()) {
+                const int q = lc.outer, e2 = lc.inner;
+                const int m0 = k0 + q;
+                const int col = m0 * n1 * h2 + e2;
+                const bool emit = act && e2 >= k2;
+                const int rank = (q * g.ne2 + (e2 - k2)) * g.t1 + rk;
+                const T pred = eval_stencil<CUB>(S, V + col);
+                const int idx = col + m1 * h2;
+                const Off gi = (Off)m0 * G0 + gl + (Off)(2 * e2) * G2;
+                if (!DECOMP) {
+                    T v = V[idx], uv;
+                    const int code = quant_point<T, QM>(v, pred, a, uv);
+                    if (act) V[idx] = v;
+                    if (emit) {
+                        sg[rank] = (uint16_t)code;
+                        if (code == 0) scratch[sbase + rank] = uv;
+                        if (wb) W[gi] = v;
                     }
-                    code = codes[pos];
+                } else if (act) {
+                    uint64_t pos;
+                    int code;
+                    if (emit) {
+                        pos = sbase + rank;
+                        code = sg[rank];
+                    } else {
+                        pos = owner_pos_sweep2(a, g, bc, P2, q) + rk;
+                        if (pos >= a.ncodes) {
+                            atomicExch(a.err, 1);
+                            pos = 0;
+                        }
+                        code = codes[pos];
+                    }
+                    const T v = recover_point<T, QM>(pred, code, pos, a, zpos, nz, unpred);
+                    V[idx] = v;
+                    if (emit) W[gi] = v;
                 }
-                const T v = recover_point<T, QM>(pred, code, pos, a, zpos, nz, unpred);
-                V[idx] = v;
-                if (emit) W[gi] = v;
             }
         }
         __syncthreads();
@@ -253,43 +261,46 @@ __device__ __forceinline__ void level_block(const LevelArgs &a, const int64_t bi
         }
         const int w1 = n1 - k1;
         const int lines = (n0 - k0) * w1;
-        const bool act = t < g.t2;
-        const int m2 = act ? 2 * t + 1 : 1;
-        const Stencil<T> S = make_stencil<T>(m2, n2, cubic, 1, 1);
-        const int rk = line_rank(m2, n2, cubic);
-        const Off gl = (Off)m2 * G2 + (Off)k0 * G0 + (Off)k1 * G1;
-        LineCursor lc, lp;  // line being computed / being loaded
-        lc.init(hw, nhw, w1);
-        lp = lc;
-        T xa = 0, xb = 0;
-        int lpi = hw;
-        if (!DECOMP) {
-            if (lpi < lines) xa = X[gl + (Off)lp.outer * G0 + (Off)lp.inner * G1];
-            lpi += nhw;
-            lp.next();
-        }
-        for (int l = hw; l < lines; l += nhw, lc.next()) {
+        for (int tb = 0; tb < g.t2; tb += 16) {
+            const int tt = tb + t;
+            const bool act = tt < g.t2;
+            const int m2 = act ? 2 * tt + 1 : 1;
+            const Stencil<T> S = make_stencil<T>(m2, n2, cubic, 1, 1);
+            const int rk = line_rank(m2, n2, cubic);
+            const Off gl = (Off)m2 * G2 + (Off)k0 * G0 + (Off)k1 * G1;
+            LineCursor lc, lp;  // line being computed / being loaded
+            lc.init(hw, nhw, w1);
+            lp = lc;
+            T xa = 0, xb = 0;
+            int lpi = hw;
             if (!DECOMP) {
-                xb = lpi < lines ? X[gl + (Off)lp.outer * G0 + (Off)lp.inner * G1] : (T)0;
+                if (lpi < lines) xa = X[gl + (Off)lp.outer * G0 + (Off)lp.inner * G1];
                 lpi += nhw;
                 lp.next();
             }
-            const int q0 = lc.outer, q1 = lc.inner;
-            const T *row = V + ((k0 + q0) * n1 + (k1 + q1)) * h2;
-            const T pred = eval_stencil<CUB>(S, row);
-            const int rank = l * g.t2 + rk;
-            const Off gi = gl + (Off)q0 * G0 + (Off)q1 * G1;
-            if (!DECOMP) {
-                T v = xa, uv;
-                const int code = quant_point<T, QM>(v, pred, a, uv);
-                if (act) {
-                    sg[rank] = (uint16_t)code;
-                    if (code == 0) scratch[sbase + rank] = uv;
-                    if (wb) W[gi] = v;
+            for (int l = hw; l < lines; l += nhw, lc.next()) {
+                if (!DECOMP) {
+                    xb = lpi < lines ? X[gl + (Off)lp.outer * G0 + (Off)lp.inner * G1] : (T)0;
+                    lpi += nhw;
+                    lp.next();
                 }
-                xa = xb;
-            } else if (act) {
-                W[gi] = recover_point<T, QM>(pred, (int)sg[rank], sbase + rank, a, zpos, nz, unpred);
+                const int q0 = lc.outer, q1 = lc.inner;
+                const T *row = V + ((k0 + q0) * n1 + (k1 + q1)) * h2;
+                const T pred = eval_stencil<CUB>(S, row);
+                const int rank = l * g.t2 + rk;
+                const Off gi = gl + (Off)q0 * G0 + (Off)q1 * G1;
+                if (!DECOMP) {
+                    T v = xa, uv;
+                    const int code = quant_point<T, QM>(v, pred, a, uv);
+                    if (act) {
+                        sg[rank] = (uint16_t)code;
+                        if (code == 0) scratch[sbase + rank] = uv;
+                        if (wb) W[gi] = v;
+                    }
+                    xa = xb;
+                } else if (act) {
+                    W[gi] = recover_point<T, QM>(pred, (int)sg[rank], sbase + rank, a, zpos, nz, unpred);
+                }
             }
         }
         __syncthreads();

@@ -806,11 +806,6 @@ cudaError_t launch_level(const LevelArgs &a, int64_t nblocks, bool decomp, const
     int threads = vol >= 8192 ? 512 : (vol >= 1024 ? 256 : (vol >= 256 ? 128 : 64));
     const bool wide = a.dims[0] * a.dims[1] * a.dims[2] >= ((int64_t)1 << 31);
     const bool straight = sizeof(T) == 4 && a.fast && a.trim == 0;
-    // The sweep launches instead of a CTA per block: levels with fewer blocks than
-    // two per SM (the block kernel would leave SMs idle; the finest level of a
-    // 33x47x61 field has 8: 67 us there, 3 x 5 us in sweeps), and 2-D fields, whose
-    // 33 x 33 blocks are too small a job for a CTA that stages them (the finest level
-    // of 1800x3600, 6441 blocks: 94 us there, 32 + 53 us in sweeps).
     static const int sms = [] {
         int dev = 0, v = 0;
         cudaGetDevice(&dev);
@@ -822,9 +817,42 @@ cudaError_t launch_level(const LevelArgs &a, int64_t nblocks, bool decomp, const
     const char *plane_env = std::getenv("FAZ_FINEST_PLANES");
     const bool only_blocks = plane_env && plane_env[0] == '0', only_planes = plane_env && plane_env[0] == '2';
     const bool forced = a.s == 1 && (only_blocks || only_planes);
-    const bool flat = a.dims[0] == 1 && a.dims[1] > 1;
+    // The sweep launches, a thread per target, or a CTA per block, by what the finest
+    // level takes (us, compression / decompression, sweeps | a CTA per block; blocks of
+    // 32 points an edge where none is named):
+    //   - 3-D levels of fewer blocks than two per SM leave SMs idle: sweeps.  float64:
+    //     168^3 185 / 137 | 266 / 195.  float32 only while the one wave of blocks
+    //     (about 55 us) takes longer: 120^3 41 / 37 | 56 / 45, but 140^3 57 / 51 |
+    //     47 / 45, 193x193x192 117 / 102 | 51 / 45 (plane kernel); edge 40, one wave of
+    //     longer blocks, 161^3 78 / 70 | 96 / 94, 200^3 123 / 105 | 96 / 96.
+    //   - 2-D levels of many points, whose blocks are too small a job for a CTA that
+    //     stages them: 1200^2 27 / 25 | 27 / 29, 1800x3600 82 / 72 | 94 / 95, edge 16
+    //     134 / 113 | 178 / 175; but 1000^2 25 / 20 | 20 / 23, 300^2 14 / 14 | 10 / 12,
+    //     30x100000 43 / 39 | 35 / 35.  Coarser ones of as few blocks as above, or from
+    //     2^21 points on (all levels of 1800x3600 205 / 187 | 197 / 186, of 3600^2
+    //     325 / 279 | 330 / 287; float64, edge 16, of 1800x3600 497 / 404 | 526 / 407).
+    //   - 2-D at other edges.  8: 1800x3600 452 / 346 | 422 / 418, float64 627 / 552 |
+    //     842 / 588; 16: float64 1000^2 57 / 49 | 72 / 55, 300^2 16 / 14 | 16 / 16; 4:
+    //     1800x3600 1793 / 1434 | 1141 / 1157 (the sweeps' CTAs are mostly empty); 128:
+    //     float64 300^2 18 / 18 | 84 / 55, 1800x3600 199 / 138 | 229 / 142, float32 300^2
+    //     14 / 14 | 23 / 25.
+    constexpr bool f32 = sizeof(T) == 4;
+    const int64_t edge = a.bs / a.s;
+    int64_t points = 1;
+    for (int i = 0; i < 3; i++) points *= (a.dims[i] - 1) / a.s + 1;
+    const bool flat = a.dims[0] == 1 && a.dims[1] > 1, few = nblocks < 2 * sms;
+    bool sweeps = few;
+    if (flat && (a.s == 1 || !few)) {
+        const bool strip = a.dims[1] < 2 * a.bs || a.dims[2] < 2 * a.bs;
+        if (edge < 8) sweeps = false;
+        else if (edge > 32 || (!f32 && edge < 32)) sweeps = true;
+        else if (edge < 16) sweeps = decomp && a.s == 1 && points >= 1 << 20;
+        else sweeps = !strip && points >= (f32 && a.s > 1 ? 1 << 21 : 1 << 20);
+    } else if (f32 && a.s == 1) {
+        sweeps = few && points < (edge <= 32 ? 1 << 21 : 1 << 22);
+    }
     const int64_t per_block = (a.bs / a.s + 1) * (a.bs / a.s + 1) * (a.bs / a.s + 1) / 256 + 1;
-    if (!forced && !wide && (flat || nblocks < 2 * sms) && nblocks * per_block < (1ll << 31))
+    if (sweeps && !forced && !wide && nblocks * per_block < (1ll << 31))
         return launch_level_sweeps<T>(a, nblocks, decomp, X, W, codes, scratch, zpos, nz, unpred, st, nlaunch);
     // the finest level of a 3-D float field: plane-parallel kernel (finest.cu, with
     // both kernels' times; on 512^3 0.45 ms against 0.83 ms for the block kernel

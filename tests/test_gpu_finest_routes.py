@@ -1,9 +1,9 @@
-"""Each kernel of the finest level on fields of every size.  By default few-block
-fields take the sweep launches; FAZ_FINEST_PLANES sends the finest level of any field
-to the block kernel (0), or to the plane kernel wherever that can run (2).  Payloads
-equal the oracle's byte for byte, decoded fields bit for bit (the arithmetic is the
-reference's, so no tolerance), and the launch counts say that another kernel ran:
-three sweeps, or one launch."""
+"""Each kernel of the finest level on fields of every size.  By default small 3-D and
+large 2-D fields take the sweep launches; FAZ_FINEST_PLANES sends the finest level of
+any field to the block kernel (0), or to the plane kernel wherever that can run (2).
+Payloads equal the oracle's byte for byte, decoded fields bit for bit (the arithmetic is
+the reference's, so no tolerance), and the launch counts say which kernel ran: three
+sweeps (two of a 2-D field), or one launch."""
 import numpy as np
 import pytest
 
@@ -40,7 +40,7 @@ def _run(conf, t, ref_payload, ref, monkeypatch, mode):
     return n
 
 
-def _check(dims, interp, direction, dtype, modes, monkeypatch, **kw):
+def _check(dims, interp, direction, dtype, modes, monkeypatch, fewer=(2, 2), **kw):
     x = spectral_field(dims, slope=-3.0, noise=0.02, seed=sum(dims) + direction).astype(dtype)
     conf = F.Config(*dims)
     conf.cmprAlgo, conf.errorBoundMode, conf.relErrorBound = F.ALGO_INTERP, F.EB_REL, 1e-3
@@ -53,8 +53,7 @@ def _check(dims, interp, direction, dtype, modes, monkeypatch, **kw):
     sweeps = _run(conf, t, payload, ref, monkeypatch, None)
     for mode in modes:
         one = _run(conf, t, payload, ref, monkeypatch, mode)
-        # three sweeps (two of a 2-D field, one of a 1-D one) or one launch
-        assert [a - b for a, b in zip(sweeps, one)] == [len(dims) - 1] * 2
+        assert [a - b for a, b in zip(sweeps, one)] == list(fewer)
 
 
 @pytest.mark.parametrize("direction", range(6))
@@ -65,11 +64,22 @@ def test_block_kernel(dims, dtype, interp, direction, monkeypatch):
     _check(dims, interp, direction, dtype, ["0"], monkeypatch)
 
 
-@pytest.mark.parametrize("dims", [(700, 300), (65, 1000), (129, 97)])
-@pytest.mark.parametrize("direction", [0, 1])
-@pytest.mark.parametrize("dtype", [np.float32, np.float64])
-def test_block_kernel_flat(dims, dtype, direction, monkeypatch):
-    _check(dims, CUB, direction, dtype, ["0"], monkeypatch)
+# fields on either side of the rule between the sweeps and a CTA per block: launches that
+# one launch saves in compression and in decompression
+@pytest.mark.parametrize("dims,dtype,edge,fewer", [
+    # 2-D: 2^20 points, two blocks across, each range of edges
+    ((1024, 1024), np.float32, 32, (1, 1)), ((1024, 1023), np.float32, 32, (0, 0)),
+    ((1024, 1024), np.float64, 16, (1, 1)), ((300, 700), np.float64, 16, (1, 1)), ((300, 700), np.float64, 32, (0, 0)),
+    ((64, 17000), np.float32, 32, (1, 1)), ((63, 17000), np.float32, 32, (0, 0)),
+    ((17000, 63), np.float32, 32, (0, 0)), ((1025, 1030), np.float32, 4, (0, 0)),
+    ((1025, 1030), np.float32, 14, (0, 1)), ((300, 400), np.float64, 8, (1, 1)),
+    ((300, 400), np.float64, 6, (0, 0)), ((192, 320), np.float64, 64, (1, 1)), ((640, 641), np.float32, 64, (1, 1)),
+    # 3-D: 2^21 points, two blocks an SM
+    ((128, 128, 127), np.float32, 32, (2, 2)), ((128, 128, 128), np.float32, 32, (0, 0)),
+    ((130, 129, 128), np.float32, 38, (2, 2)), ((128, 128, 128), np.float64, 32, (2, 2)),
+    ((160, 192, 320), np.float64, 32, (2, 2)), ((170, 192, 320), np.float64, 32, (0, 0))])
+def test_rule(dims, dtype, edge, fewer, monkeypatch):
+    _check(dims, CUB, 1, dtype, ["0"], monkeypatch, fewer, interpBlockSize=edge)
 
 
 @pytest.mark.parametrize("interp", [LIN, CUB])

@@ -265,8 +265,10 @@ __device__ __forceinline__ void run_load(const uint16_t *src, uint32_t (&R)[8]) 
 
 // One line per lane (`act`), `line` in shared memory with stride st, its codes at
 // cb[off..off + 16) (stream position base + off).  `width` lanes make a run.
-// Values: already in v; the odd ones become the reconstruction.
-template <bool DECOMP, int CUB>
+// Values: already in v; the odd ones become the reconstruction.  VERIFY: every target
+// that the float proofs decided is computed again by the double computation, and the
+// differences counted.
+template <bool DECOMP, int CUB, bool VERIFY>
 __device__ __forceinline__ void line_run(const LevelArgs &a, float (&v)[33], const float *line, int st, int n, bool act,
                                          int width, int in_run, int lanes, uint16_t *cb, float *ub, uint64_t base,
                                          int off, const uint64_t *__restrict__ zpos, uint64_t nz,
@@ -284,6 +286,22 @@ __device__ __forceinline__ void line_run(const LevelArgs &a, float (&v)[33], con
         from_stream<CUB>(R, n, N);
     }
     unsigned bad = line_targets<DECOMP, CUB>(v, n, a, N);
+    if constexpr (VERIFY) {
+#pragma unroll 1
+        for (unsigned todo = act ? ~bad & 0xffffu : 0u; todo; todo &= todo - 1) {
+            const unsigned bit = todo & (0u - todo);
+            uint32_t Nm[8], c;
+            float val;
+#pragma unroll
+            for (int i = 0; i < 8; i++) Nm[i] = N[i];
+            line_redo<DECOMP, CUB>(a, bit, line, st, n, base + (uint64_t)off, zpos, nz, unpred, Nm, &c, &val);
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+                if (bit == 1u << k && (c != ((N[k >> 1] >> (16 * (k & 1))) & 0xffffu) ||
+                                       __float_as_uint(val) != __float_as_uint(v[2 * k + 1])))
+                    atomicAdd(a.verify, 1ull);
+        }
+    }
     if (!act) bad = 0;
     while (bad) {
         uint32_t Nm[8], c;
@@ -348,7 +366,7 @@ __device__ __forceinline__ void one_target(const LevelArgs &a, float *line, int 
 // at even P2 indices (each value written where its original was read, once the
 // original is no longer needed) and, in decompression, at odd ones too, to be
 // written to W.  W holds the coarse points (earlier levels) in both directions.
-template <bool DECOMP, int CUB>
+template <bool DECOMP, int CUB, bool VERIFY>
 __global__ void __launch_bounds__(FW * 32, 2)
     k_finest(LevelArgs a, const __grid_constant__ CUtensorMap tm, float *W, uint16_t *__restrict__ codes,
              float *__restrict__ scratch, const uint64_t *__restrict__ zpos, uint64_t nz,
@@ -415,9 +433,8 @@ __global__ void __launch_bounds__(FW * 32, 2)
     const int np = n0 - k0;   // planes with emitted codes
     const int w1 = n1 - k1;   // emitted rows (sweep 3)
     const int w2 = n2 - k2;   // emitted columns
-    // lines of 32 or 33 points in both sweeps: a line to a lane (verification wants
-    // every target's double computation: target by target)
-    const bool lines = n1 >= 32 && n2 >= 32 && a.verify == nullptr;
+    // lines of 32 or 33 points in both sweeps: a line to a lane
+    const bool lines = n1 >= 32 && n2 >= 32;
     uint32_t phase = 0;
     // planes in pairs (an odd and an even P0 index) per warp, so that warps
     // get the same work
@@ -537,7 +554,7 @@ __global__ void __launch_bounds__(FW * 32, 2)
 #pragma unroll
             for (int r = 0; r < 32; r++) v[r] = DECOMP && (r & 1) ? 0.0f : col[r * FX];
             v[32] = n1 == 33 ? col[32 * FX] : 0.0f;
-            line_run<DECOMP, CUB>(a, v, col, FX, n1, act, 16, t, h2 - 1, cb, ub, base, act ? pb + (e2 - k2) * 16 : 0,
+            line_run<DECOMP, CUB, VERIFY>(a, v, col, FX, n1, act, 16, t, h2 - 1, cb, ub, base, act ? pb + (e2 - k2) * 16 : 0,
                                   zpos, nz, unpred);
             if (act) {
 #pragma unroll
@@ -595,7 +612,7 @@ __global__ void __launch_bounds__(FW * 32, 2)
                     v[4 * c + 3] = q.w;
                 }
                 v[32] = n2 == 33 ? row[32] : 0.0f;
-                line_run<DECOMP, CUB>(a, v, row, 1, n2, act, 32, lane, n1 - 1, cb, ub, base,
+                line_run<DECOMP, CUB, VERIFY>(a, v, row, 1, n2, act, 32, lane, n1 - 1, cb, ub, base,
                                       act ? pb0 + (s * w1 + m1 - k1) * 16 : 0, zpos, nz, unpred);
                 if (DECOMP && act) {
 #pragma unroll
@@ -722,8 +739,13 @@ cudaError_t launch_finest(const LevelArgs &a, int64_t nblocks, bool decomp, cons
         if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
     }
     void (*k)(LevelArgs, const CUtensorMap, float *, uint16_t *, float *, const uint64_t *, uint64_t, const float *);
-    if (decomp) k = a.cubic ? k_finest<true, 1> : k_finest<true, 0>;
-    else k = a.cubic ? k_finest<false, 1> : k_finest<false, 0>;
+    if (a.verify) {
+        if (decomp) k = a.cubic ? k_finest<true, 1, true> : k_finest<true, 0, true>;
+        else k = a.cubic ? k_finest<false, 1, true> : k_finest<false, 0, true>;
+    } else {
+        if (decomp) k = a.cubic ? k_finest<true, 1, false> : k_finest<true, 0, false>;
+        else k = a.cubic ? k_finest<false, 1, false> : k_finest<false, 0, false>;
+    }
     cudaError_t e = allow_dynamic_smem((const void *)k);
     if (e != cudaSuccess) return e;
     k<<<(unsigned)nblocks, FW * 32, FSMEM, st>>>(a, tm, W, codes, scratch, zpos, nz, unpred);

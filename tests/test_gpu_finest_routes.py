@@ -89,3 +89,33 @@ def test_rule(dims, dtype, edge, fewer, monkeypatch):
                                      ((96, 64, 64), dict(maxStep=16, alpha=1.5, beta=3.0))])
 def test_plane_kernel(dims, kw, direction, interp, monkeypatch):
     _check(dims, interp, direction, np.float32, ["0", "2"], monkeypatch, **kw)
+
+
+@pytest.mark.parametrize("mode", [None, "0", "2"])
+@pytest.mark.parametrize("interp", [LIN, CUB])
+@pytest.mark.parametrize("whole", [True, False])
+def test_verified(whole, interp, mode, monkeypatch):
+    """FAZ_VERIFY_FASTPATH in each kernel of the finest level: the call fails where the
+    float proofs and the double computation differ.  Whole numbers at a bound of one
+    half lie on the bins' edges.  Blocks of 32 and 33 points, whose lines the plane
+    kernel keeps in registers, and shorter ones."""
+    dims = (97, 100, 132)
+    x = spectral_field(dims, slope=-3.0, noise=0.02, seed=11)
+    conf = F.Config(*dims)
+    conf.cmprAlgo, conf.interpAlgo, conf.errorBoundMode = F.ALGO_INTERP, interp, F.EB_ABS
+    conf.absErrorBound = 0.5 if whole else 0.013
+    if whole:
+        x = np.rint(x).astype(np.float32)
+    monkeypatch.setenv("FAZ_VERIFY_FASTPATH", "1")
+    if mode is None:
+        monkeypatch.delenv("FAZ_FINEST_PLANES", raising=False)
+    else:
+        monkeypatch.setenv("FAZ_FINEST_PLANES", mode)
+    stream, want = O.compress(conf, x)
+    ref, _ = O.decompress(stream)
+    t = torch.from_numpy(x).cuda()
+    payload, _ = F.compress_payload_device(conf, t)
+    assert bytes(payload) == want
+    out = torch.empty_like(t)
+    F.decompress_payload_device(3, payload, out)
+    assert out.cpu().numpy().tobytes() == ref.tobytes()

@@ -280,7 +280,7 @@ void check_config(const faz_config &c) {
 // in the element type.
 template <typename T>
 double device_range(const T *dX, uint64_t n, cudaStream_t st, Counter &launches) {
-    int nb = (int)std::min<uint64_t>(152 * 4, (n + 4095) / 4096);
+    int nb = (int)std::min<uint64_t>(4 * (uint64_t)sm_count(), (n + 4095) / 4096);
     if (nb < 1) nb = 1;
     DevMem m(st);
     T *pmin = m.alloc<T>(2 * nb), *pmax = pmin + nb;

@@ -146,10 +146,11 @@ FAZ_HD bool dequant_f32_bracket(float pred, float half, float eh2, float el2, fl
 // diff's sign to within |y| 2^-23 (rh and the product round once each), so
 // rint(y) is the signed half unless y lies within |y| 2^-22 of a half-integer;
 // half >= radius (also NaN and infinities) is unpredictable.  The kernels that
-// call this are issue-bound, so instructions count: with the former form
-// (floor and midpoint cases spelled out, about twice the instructions) the
-// finest level of a 512^3 field took 0.80 ms, now 0.60 ms, and its inverse 0.87
-// against 0.77 ms.
+// call this are issue-bound, so instructions count: in the kernel that had a target to
+// a lane, the finest level of a 512^3 field took 0.80 ms with the former form (floor and
+// midpoint cases spelled out, about twice the instructions) and 0.60 ms with this one
+// (finest.cu has the present kernel's times).  rl, the low part of 1/eb, is not needed
+// to decide; half_index_f32 takes the same arguments.
 FAZ_HD int quantize_f32_straight(float orig, float pred, float rh, float rl, float eh, float el, float eblo,
                                  float twor_f, int radius, float &out, bool &undecided) {
     (void)rl;

@@ -153,9 +153,8 @@ __global__ void __launch_bounds__(256) k_hist_compact(const unsigned long long *
     }
 }
 
-// Zero-code count per warp sub-chunk (decompress side).
-template <typename C>
-__global__ void __launch_bounds__(1024) k_count_zeros(const C *__restrict__ codes, uint64_t n,
+// Zero-code count per warp sub-chunk, where no histogram of the same codes gives it.
+__global__ void __launch_bounds__(1024) k_count_zeros(const uint16_t *__restrict__ codes, uint64_t n,
                                                       unsigned long long *zcount) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t s0 = (uint64_t)blockIdx.x * HCHUNK + (uint64_t)w * HSUB;
@@ -182,7 +181,7 @@ __global__ void __launch_bounds__(1024) k_compact_zeros(const C *__restrict__ co
     if (s1 > n) s1 = n;
     unsigned long long run = zoff[sub];
     // 256 codes per warp step, four steps' loads in flight: lane L reads codes
-    // [b + 8L, b + 8L + 8) with one 16-byte load (s0 is a multiple of 8192 and codes
+    // [b + 8L, b + 8L + 8) with one 16-byte load (s0 is a multiple of HSUB and codes
     // is 256-byte aligned), so the zeros of a step come in stream order lane by lane
     uint64_t b = s0;
     for (; sizeof(C) == 2 && b + 1024 <= s1; b += 1024) {
@@ -1146,8 +1145,8 @@ cudaError_t histogram_impl(const C *codes, uint64_t n, int center, unsigned long
     const uint64_t used = (n + HSUB - 1) / HSUB, nsub = hist_subchunks(n);
     // four CTAs per SM in one wave, at least a sub-chunk per warp each; a CTA's run
     // stays below 2^32 codes
-    const uint64_t warps = HTHREADS / 32;
-    uint64_t per_cta = std::max<uint64_t>((used + 607) / 608, std::min<uint64_t>(warps, 4));
+    const uint64_t warps = HTHREADS / 32, wave = 4 * (uint64_t)sm_count();
+    uint64_t per_cta = std::max<uint64_t>((used + wave - 1) / wave, std::min<uint64_t>(warps, 4));
     per_cta = std::min<uint64_t>(per_cta, (1ull << 31) / HSUB);
     // the sub-chunks past the last code
     cudaError_t e = cudaSuccess;
@@ -1169,11 +1168,7 @@ cudaError_t launch_histogram(const uint32_t *codes, uint64_t n, int center, unsi
 }
 
 cudaError_t launch_count_zeros(const uint16_t *codes, uint64_t n, unsigned long long *zcount, cudaStream_t st) {
-    k_count_zeros<uint16_t><<<grid_for(n, HCHUNK), 1024, 0, st>>>(codes, n, zcount);
-    return cudaGetLastError();
-}
-cudaError_t launch_count_zeros(const uint32_t *codes, uint64_t n, unsigned long long *zcount, cudaStream_t st) {
-    k_count_zeros<uint32_t><<<grid_for(n, HCHUNK), 1024, 0, st>>>(codes, n, zcount);
+    k_count_zeros<<<grid_for(n, HCHUNK), 1024, 0, st>>>(codes, n, zcount);
     return cudaGetLastError();
 }
 

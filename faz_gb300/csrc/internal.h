@@ -61,6 +61,7 @@ inline cudaError_t allow_dynamic_smem(const void *func) {
 // ---------------------------------------------------------------- kernels
 template <typename T>
 cudaError_t launch_minmax(const T *X, uint64_t n, T *pmin, T *pmax, int nblocks, cudaStream_t st);
+int sm_count();  // SMs of the device current at the first call
 template <typename T>
 size_t level_smem_bytes(const LevelArgs &a);
 // The levels of an interpolation plan, coarsest first (a batch of the kernels
@@ -150,7 +151,6 @@ cudaError_t launch_histogram(const uint32_t *codes, uint64_t n, int center, unsi
                              unsigned long long *first, unsigned long long *zcount, unsigned long long *nzero,
                              cudaStream_t st);
 cudaError_t launch_count_zeros(const uint16_t *codes, uint64_t n, unsigned long long *zcount, cudaStream_t st);
-cudaError_t launch_count_zeros(const uint32_t *codes, uint64_t n, unsigned long long *zcount, cudaStream_t st);
 template <typename T, typename C>
 cudaError_t launch_compact_zeros(const C *codes, uint64_t n, const unsigned long long *zcount,
                                  const unsigned long long *zoff, const T *scratch, T *vals, cudaStream_t st);

@@ -1,13 +1,17 @@
 // interp.cu - multilevel interpolation predictor + linear quantiser kernels.
 //
-// One CTA per interpolation block and level (SZInterpolationCompressor.hpp
-// 384-461 compress, 106-196 decompress).  The block's lattice points with an
-// even index along the last sweep axis live in shared memory; sweep 1 and 2
-// targets are computed there, sweep 3 targets stream from global memory.
-// Lines on the block's first planes, which the reference assigns to the
-// previous block, are recomputed (never emitted) so that every block of a
-// level runs independently.  Codes of a sweep are staged in shared memory and
-// written to their stream positions in one coalesced pass.
+// A level (SZInterpolationCompressor.hpp 384-461 compress, 106-196 decompress) runs in
+// one of four ways; launch_level says which, by size:
+//   - k_small_levels: the coarsest levels together, in one CTA;
+//   - k_level_sweep: a launch per sweep, a thread per target (few or flat blocks);
+//   - k_finest (finest.cu): the finest level of 3-D float fields, by planes;
+//   - k_interp_level: a CTA per interpolation block.
+// The last one keeps the block's lattice points with an even index along the last sweep
+// axis in shared memory; sweep 1 and 2 targets are computed there, sweep 3 targets
+// stream from global memory.  Lines on the block's first planes, which the reference
+// assigns to the previous block, are recomputed (never emitted) so that every block of a
+// level runs independently.  Codes of a sweep are staged in shared memory and written
+// to their stream positions in one coalesced pass.
 //
 // Arithmetic follows the reference's types and operation order (compiled with
 // -fmad=false): stencils in T (include/QoZ/utils/Interpolators.hpp:9-36),
@@ -796,6 +800,16 @@ cudaError_t launch_small_levels(const LevelTable &t, int n, bool decomp, bool fi
     return cudaGetLastError();
 }
 
+int sm_count() {
+    static const int sms = [] {
+        int dev = 0, v = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        return v > 0 ? v : 1;
+    }();
+    return sms;
+}
+
 template <typename T>
 cudaError_t launch_level(const LevelArgs &a, int64_t nblocks, bool decomp, const T *X, T *W, uint16_t *codes,
                          T *scratch, const uint64_t *zpos, uint64_t nz, const T *unpred, cudaStream_t st,
@@ -806,12 +820,7 @@ cudaError_t launch_level(const LevelArgs &a, int64_t nblocks, bool decomp, const
     int threads = vol >= 8192 ? 512 : (vol >= 1024 ? 256 : (vol >= 256 ? 128 : 64));
     const bool wide = a.dims[0] * a.dims[1] * a.dims[2] >= ((int64_t)1 << 31);
     const bool straight = sizeof(T) == 4 && a.fast && a.trim == 0;
-    static const int sms = [] {
-        int dev = 0, v = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-        return v > 0 ? v : 1;
-    }();
+    const int sms = sm_count();
     // FAZ_FINEST_PLANES (read per call, for comparisons): the finest level of any field
     // in the block kernel (0), or in the plane kernel wherever that can run (2).
     const char *plane_env = std::getenv("FAZ_FINEST_PLANES");

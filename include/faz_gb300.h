@@ -193,7 +193,11 @@ int faz_compress_device(const faz_config *conf, int dtype, const void *d_data,
                         faz_timings *timings);
 
 /* Same as faz_decompress writing into device memory d_out, which holds
- * conf->num values on entry (a stream with a larger field is rejected). */
+ * conf->num values on entry (a stream with a larger field is rejected).
+ * A stream refused for its headers or its Huffman section leaves d_out as it
+ * was; after an error found later, in the predictors' own data or in another
+ * slab of an OpenMP stream, its contents are undefined.  The call has finished
+ * with its buffers when it returns, also with an error. */
 int faz_decompress_device(faz_config *conf, int dtype, const char *cmp,
                           size_t cmp_size, void *d_out, void *stream,
                           faz_timings *timings);
@@ -212,7 +216,7 @@ int faz_compress_device_payload(const faz_config *conf, int dtype, const void *d
                                 faz_config *conf_out, faz_timings *timings);
 
 /* Decode a pre-zstd payload of an N-dimensional field into device memory
- * d_out holding `capacity` values. */
+ * d_out holding `capacity` values (after an error as faz_decompress_device). */
 int faz_decompress_payload_device(int N, int dtype, const char *payload, size_t size,
                                   void *d_out, uint64_t capacity, void *stream,
                                   faz_timings *timings);

@@ -242,6 +242,7 @@ void check_config(const faz_config &c) {
     uint64_t num = 1;
     for (int i = 0; i < c.N; i++) {
         if (c.dims[i] == 0) throw Fail{FAZ_ERR_ARG, "zero dimension"};
+        if (num > UINT64_MAX / c.dims[i]) throw Fail{FAZ_ERR_ARG, "num does not match dims"};
         num *= c.dims[i];
     }
     if (num != c.num) throw Fail{FAZ_ERR_ARG, "num does not match dims"};
@@ -1454,7 +1455,12 @@ V rd(const uint8_t *&p, const uint8_t *end) {
 void parse_payload(const uint8_t *pl, size_t n, int N, Parsed &P) {
     const uint8_t *p = pl, *end = pl + n;
     P.N = N;
-    for (int i = 0; i < N; i++) P.dims[i] = rd<uint64_t>(p, end);
+    uint64_t num = 1;  // the caller compares it with its buffer: no wrap past 2^64
+    for (int i = 0; i < N; i++) {
+        P.dims[i] = rd<uint64_t>(p, end);
+        if (P.dims[i] && num > UINT64_MAX / P.dims[i]) throw Fail{FAZ_ERR_FORMAT, "field too large"};
+        num *= P.dims[i];
+    }
     P.blocksize = rd<uint32_t>(p, end);
     P.interp = rd<int32_t>(p, end);
     P.dir = rd<int32_t>(p, end);

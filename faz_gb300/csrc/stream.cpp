@@ -348,7 +348,10 @@ int config_load(faz_config &c, const uint8_t *p, size_t n, size_t *used) {
     }
     if (r.bad) return FAZ_ERR_FORMAT;
     uint64_t num = 1;
-    for (int i = 0; i < t.N; i++) num *= t.dims[i];
+    for (int i = 0; i < t.N; i++) {
+        if (t.dims[i] && num > UINT64_MAX / t.dims[i]) return FAZ_ERR_FORMAT;
+        num *= t.dims[i];
+    }
     if (num != t.num) return FAZ_ERR_FORMAT;
     // fields the trailer does not carry keep their defaults
     t.rng = -1;

@@ -277,9 +277,7 @@ BlkPlan make_blk_plan(const uint64_t *dims, uint64_t maxStep, int B) {
         if (maxStep & (maxStep - 1)) throw Fail{FAZ_ERR_UNSUPPORTED, "maxStep must be a power of two on the GPU path"};
         p.anchor = true;
         p.levels += 1;
-        int lm = 0;
-        while (((uint64_t)1 << (lm + 1)) <= maxStep) lm++;
-        lm += 1;
+        const int lm = floor_log2(maxStep) + 1;
         if (lm <= p.levels) p.levels = lm;
         p.nanchor = 1;
         for (int i = 0; i < 3; i++) {
@@ -471,9 +469,7 @@ bool fixbs_aligned(int N, const uint64_t *dims, uint64_t maxStep, int fixbs) {
     for (int i = 0; i < 3; i++) levels = std::max(levels, ceil_log2(dims3[i]));
     if (maxStep > 0) {
         levels += 1;
-        int lm = 0;
-        while (((uint64_t)1 << (lm + 1)) <= maxStep) lm++;
-        lm += 1;
+        const int lm = floor_log2(maxStep) + 1;
         if (lm <= levels) levels = lm;
         levels -= 1;
     }

@@ -90,9 +90,7 @@ Plan make_plan(int N, const uint64_t *dims, uint64_t maxStep, int blocksize, int
     if (maxStep > 0) {
         p.anchor = true;
         p.levels += 1;
-        int lm = 0;
-        while (((uint64_t)1 << (lm + 1)) <= maxStep) lm++;
-        lm += 1;
+        const int lm = floor_log2(maxStep) + 1;
         if (lm <= p.levels) p.levels = lm;
         if (maxStep & (maxStep - 1)) throw Fail{FAZ_ERR_UNSUPPORTED, "maxStep must be a power of two on the GPU path"};
         if (N != 2 && N != 3) throw Fail{FAZ_ERR_UNSUPPORTED, "an anchor grid needs 2-D or 3-D data"};

@@ -19,6 +19,8 @@ namespace faz {
 // per (device, kernel).  Setting the limit to each launch's own need instead
 // races: host threads launching the same kernel concurrently (the tuner's
 // trials) can lower it between another thread's set and launch.
+// largest l with 2^l <= d (d >= 1)
+inline int floor_log2(uint64_t d) { return 63 - __builtin_clzll(d); }
 // smallest l with 2^l >= d (ceil(log2(d)) for d >= 1)
 inline int ceil_log2(uint64_t d) {
     int l = 0;

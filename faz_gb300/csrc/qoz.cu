@@ -295,9 +295,7 @@ QzGeom make_geom(int N, int64_t bsz, int64_t maxStep) {
     if (maxStep > 0) {
         g.anchor = true;
         g.levels += 1;
-        int lm = 0;
-        while (((uint64_t)1 << (lm + 1)) <= (uint64_t)maxStep) lm++;
-        lm += 1;
+        const int lm = floor_log2((uint64_t)maxStep) + 1;
         if (lm <= g.levels) g.levels = lm;
         for (int i = 0; i < 3; i++) g.na[i] = 1;
         g.nanchor = 1;
